@@ -79,6 +79,7 @@ SIGNATURES = {
     "pie_status_string": (C.c_char_p, [_i]),
     "pie_last_cuda_error": (C.c_char_p, []),
     "pie_launch_count": (C.c_ulonglong, []),
+    "pie_pipeline_error": (C.c_uint, []),
     "pie_quantize": (_i, [_vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _vp]),
     "pie_dequantize": (_i, [_vp, _vp, _vp, _vp, _vp, _ll, _ll, _i, _i, _i, _vp]),
     "pie_qmv_workspace_bytes": (_sz, [_i, _ll, _i, _i, _i, _i]),

@@ -1,0 +1,538 @@
+// Persistent tcgen05 GEMM core, sm_100a:  acc[m, n] = sum_k x[m, k] w[n, k]  (bf16 operands, fp32 in tensor memory), shared
+// by the prefill quantized GEMM (pie_qmm.cu: w is dequantised into shared memory on the way) and the dense linear of the
+// hybrid families (hyb_umma.cu: w arrives by TMA).  What bounds it is the tensor pipe; the shape of the kernel follows from
+// keeping that pipe fed:
+//   * CG = 2: a CTA pair (two SMs) owns a 256 x 256 tile, cta_group::2.  Each CTA stages 128 rows of x and HALF of the w rows
+//     (128), so a 64-element K step moves 32 KB into each SM for 512 tensor-pipe cycles (64 B / cycle of shared-memory reads
+//     and 64 of writes, the 128 the SM has); a 128 x 256 tile of one CTA would need 192.
+//   * CG = 1: one CTA owns a 128 x BN tile: few rows or few tiles, where the pair would leave SMs idle.  SPLIT cuts K over the
+//     ranks of a cluster; partial tiles meet in the owners' shared memory and are added in rank order (no workspace, no
+//     atomics, the same sum every time).
+//   * operands by TMA into an S-deep ring of 128-byte-swizzled stages; one thread issues the MMAs; two accumulator buffers, so
+//     the epilogue of a tile runs under the main loop of the next; a CTA (pair) walks tiles blockIdx, + grid, ... with the row
+//     tiles of a group of `group_m` innermost, so that what is in flight at once shares rows of x and of w in L2.
+//   * QB = 4 / 8: a further TMA warp brings the packed rows of w, 128 bytes each, and groups of four warps turn them into
+//     the stage's bf16 rows, w_hat = bf16(scale q + bias) rounded once (fused bf16x2 / fp32 multiply-add): a thread takes one
+//     row of a K step, the groups take the K steps in turn (one step's chain of wait, load, store and proxy fence is longer
+//     than its MMAs).
+// No wait is unbounded: one that expires raises g_gemm_error and a CTA-wide flag, every role leaves its loop, copies in flight
+// are given time to land, tensor memory is freed and the kernel returns.
+#pragma once
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "pie_ptx.cuh"
+#include "pie_umma.cuh"
+
+namespace pie {
+
+static __device__ unsigned int g_gemm_error = 0;   // 1: a pipeline wait of this library's GEMM expired
+
+// ---------------------------------------------------------------------------------------------------- cluster / mbarrier
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {   // every thread of every CTA of the cluster, warps converged
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+  uint32_t d;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(addr), "r"(rank));
+  return d;
+}
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
+}
+constexpr uint32_t kGemmWaitLimit = 1u << 22;
+// false: the wait expired here or the CTA is already leaving
+__device__ __forceinline__ bool gemm_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  uint32_t ok, spins = 0;
+  while (true) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    if (ok) return true;
+    if (++spins > kGemmWaitLimit || *abort_flag) {
+      *abort_flag = 1;
+      atomicExch(&g_gemm_error, 1u);
+      return false;
+    }
+  }
+}
+
+// the same for a whole warp whose lanes go on together: one lane's expiry takes the warp out
+__device__ __forceinline__ bool gemm_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, gemm_wait(bar, parity, abort_flag));
+}
+
+// ---------------------------------------------------------------------------------------------------- TMA / MMA, 1 or 2 CTAs
+template <int CG>
+__device__ __forceinline__ void gemm_tma_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+  if (CG == 2)   // the barrier may be the leader CTA's
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void gemm_mma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accum) {
+  if (CG == 2)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accum)
+        : "memory");
+  else
+    umma_bf16(tmem_d, da, db, idesc, accum);
+}
+// arrives on `bar` (in both CTAs of a pair) once every MMA issued so far has finished
+template <int CG>
+__device__ __forceinline__ void gemm_commit(uint32_t bar) {
+  if (CG == 2)
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+        "h"((uint16_t)3) : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// ---------------------------------------------------------------------------------------------------- arguments
+struct GemmArgs {
+  int M, N, K;            // one product; K a multiple of 64
+  int mt, nt, nb;         // tiles along m and n, independent products
+  int zx, zw;             // 0: one x / one w for all products
+  int group_m;            // row tiles walked together
+  int k_per;              // SPLIT: K steps (of 64) per cluster rank
+  const uint16_t* scales; // QB: [N, K / 64] bf16
+  const uint16_t* biases;
+  int scale_vec;          // QB: rows of scales / biases can be read 16 bytes (8 K steps) at a time
+};
+
+template <int CG, int BN, int QB, bool SPLIT>
+struct GemmTile {
+  static constexpr int BM = 128 * CG, NB = BN / CG;              // tile rows; w rows staged by one CTA
+  static constexpr int A_STAGE = 128 * 128, B_STAGE = NB * 128;  // bytes of one 64-element K step
+  static constexpr int CHUNK = NB * 128, RING = QB ? 3 : 0;      // packed rows: 128 bytes each, 256 (4-bit) / 128 (8-bit) of K
+  static constexpr int S = QB ? 5 : (CG == 2 ? 6 : 6);
+  static constexpr int EPI_WARPS = QB ? 4 : 8;
+  static constexpr int W_TMA = EPI_WARPS, W_MMA = EPI_WARPS + 1, W_PACK = EPI_WARPS + 2, W_DEQ = EPI_WARPS + 4;
+  static constexpr int GROUPS = 3;                                // dequantising groups of four warps, a K step each in turn
+  static constexpr int THREADS = 32 * (QB ? W_DEQ + 4 * GROUPS : EPI_WARPS + 4);
+  static constexpr int SMEM = 1024 + S * (A_STAGE + B_STAGE) + RING * CHUNK;
+  static constexpr int TMEM_COLS = 2 * BN;
+  static_assert(SMEM <= 227 * 1024 && TMEM_COLS <= 512 && BN % 32 == 0, "tile");
+  static_assert(!QB || NB == 128, "the dequantising threads are laid out for 128 rows");
+  static_assert(!(SPLIT && CG == 2), "K is split over single CTAs");
+};
+
+// eight 4-bit codes of one word -> eight bf16 scale * q + bias in order.  128 + q is a bf16 number (one mask-or for two codes);
+// subtracting 128 is exact, and the fused multiply-add rounds once.
+__device__ __forceinline__ uint4 gemm_dequant4(uint32_t w, uint32_t s2, uint32_t b2) {
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t p = ((w >> (4 * j)) & 0x000f000fu) | 0x43004300u;
+    o[j] = fma_bf16x2(fma_bf16x2(p, 0x3f803f80u, 0xc300c300u), s2, b2);
+  }
+  return make_uint4(__byte_perm(o[0], o[1], 0x5410), __byte_perm(o[2], o[3], 0x5410), __byte_perm(o[0], o[1], 0x7632),
+                    __byte_perm(o[2], o[3], 0x7632));
+}
+// four 8-bit codes of one word -> four bf16: 2^23 + q is one byte permutation, the rest is fp32 and one rounding
+__device__ __forceinline__ uint2 gemm_dequant8(uint32_t w, float s, float b) {
+  float q[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) q[j] = fmaf(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + j)) - 8388608.f, s, b);
+  return make_uint2(pack_bf16(q[0], q[1]), pack_bf16(q[2], q[3]));
+}
+
+struct GemmTileAt { int z, m, n; };
+__device__ __forceinline__ GemmTileAt gemm_tile_at(const GemmArgs& a, int t) {
+  const int per = a.mt * a.nt, z = t / per, r = t - z * per;
+  const int span = a.group_m * a.nt, g = r / span, rr = r - g * span, first = g * a.group_m;
+  const int gm = min(a.group_m, a.mt - first);
+  return {z, first + rr % gm, rr / gm};
+}
+
+// Epi: void operator()(int z, int row, int col0, const uint32_t (&v)[32]) for 32 columns of one row (any row / column, the
+// callee checks the bounds).
+template <int CG, int BN, int QB, bool SPLIT, class Epi>
+__global__ void __launch_bounds__(GemmTile<CG, BN, QB, SPLIT>::THREADS, 1)
+gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ GemmArgs a,
+            const __grid_constant__ Epi epi) {
+  using T = GemmTile<CG, BN, QB, SPLIT>;
+  constexpr int S = T::S, RING = T::RING > 0 ? T::RING : 1, KPC = QB == 4 ? 4 : 2;   // K steps per packed chunk
+  constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(T::BM >> 4) << 24);
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[S], empty_bar[S], tfull_bar[2], tempty_bar[2], pfull_bar[RING], pempty_bar[RING];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  // programmatic dependents of this launch may start; what this one reads was written by launches before it
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const uint32_t rank = (CG == 2 || SPLIT) ? cluster_rank() : 0;
+  const uint32_t lead = CG == 2 ? 0 : rank;      // the CTA that issues this CTA's MMAs
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t smA = base, smB = base + S * T::A_STAGE, smP = smB + S * T::B_STAGE;
+  const int nk_all = a.K / 64;
+  const int k_lo = SPLIT ? (int)rank * a.k_per : 0, k_hi = SPLIT ? min(nk_all, k_lo + a.k_per) : nk_all;
+  constexpr int CL = CG;                         // CTAs per tile step of the grid; SPLIT: the whole cluster shares blockIdx.y
+  const int first_tile = SPLIT ? (int)blockIdx.y : (int)blockIdx.x / CL, tile_step = SPLIT ? (int)gridDim.y : (int)gridDim.x / CL;
+  const int ntiles = a.mt * a.nt * a.nb;
+
+  if (tid == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(&full_bar[s], 1 + (QB ? 4 * CG : 0));
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tfull_bar[b], 1);
+      mbar_init(&tempty_bar[b], T::EPI_WARPS * CG);
+    }
+    for (int p = 0; p < RING; ++p) {
+      mbar_init(&pfull_bar[p], 1);
+      mbar_init(&pempty_bar[p], 4 * KPC);
+    }
+    abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == T::W_MMA) {
+    if (CG == 2) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                   "n"(T::TMEM_COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                   "n"(T::TMEM_COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+  }
+  if (warp == T::W_TMA && lane == 0) { tma_prefetch_desc(&map_x); tma_prefetch_desc(&map_w); }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (CG == 2 || SPLIT) cluster_sync_all();      // the peers' barriers are set up
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  volatile int* const abortp = &abort_flag;
+
+  if (warp < T::EPI_WARPS) {
+    // ---------------------------------------------------------------- epilogue: TMEM lane quadrant warp % 4
+    const int quad = warp & 3, row_in = quad * 32 + lane;
+    constexpr int PARTS = T::EPI_WARPS / 4, RUNS = BN / 32 / PARTS;   // 32-column runs of this warp
+    const int c_lo = (warp >> 2) * RUNS;
+    if (!SPLIT) {
+      int i = 0;
+      for (int t = first_tile; t < ntiles; t += tile_step, ++i) {
+        const GemmTileAt at = gemm_tile_at(a, t);
+        const int b = i & 1;
+        if (!gemm_wait_warp(smem_u32(&tfull_bar[b]), (i >> 1) & 1, abortp)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int row = at.m * T::BM + (int)(CG == 2 ? rank : 0) * 128 + row_in;
+#pragma unroll 1
+        for (int c = 0; c < RUNS; ++c) {
+          uint32_t v[32];
+          tmem_ld32(tmem + (uint32_t)(b * BN + (c_lo + c) * 32) + ((uint32_t)(quad * 32) << 16), v);
+          if (c == RUNS - 1) {   // the accumulator may be overwritten
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+              if (CG == 2) mbar_arrive_remote(map_to_rank(smem_u32(&tempty_bar[b]), lead));
+              else mbar_arrive(&tempty_bar[b]);
+            }
+          }
+          epi(at.z, row, at.n * BN + (c_lo + c) * 32, v);
+        }
+      }
+    } else {
+      gemm_wait_warp(smem_u32(&tfull_bar[0]), 0, abortp);
+    }
+  } else if (warp == T::W_TMA) {
+    // ---------------------------------------------------------------- operands that arrive as they are
+    if (lane == 0) {
+      int it = 0;
+      bool alive = true;
+      for (int t = first_tile; t < ntiles && alive; t += tile_step) {
+        const GemmTileAt at = gemm_tile_at(a, t);
+        const int row = at.m * T::BM + (int)(CG == 2 ? rank : 0) * 128, col = at.n * BN + (int)(CG == 2 ? rank : 0) * T::NB;
+        for (int kb = k_lo; kb < k_hi; ++kb, ++it) {
+          const int s = it % S;
+          if (!(alive = gemm_wait(smem_u32(&empty_bar[s]), ((it / S) & 1) ^ 1, abortp))) break;
+          const uint32_t bar = CG == 2 ? map_to_rank(smem_u32(&full_bar[s]), lead) : smem_u32(&full_bar[s]);
+          if (rank == lead) mbar_arrive_expect_tx(&full_bar[s], CG * (T::A_STAGE + (QB ? 0 : T::B_STAGE)));
+          gemm_tma_3d<CG>(smA + s * T::A_STAGE, &map_x, bar, kb * 64, row, at.z * a.zx);
+          if (!QB) gemm_tma_3d<CG>(smB + s * T::B_STAGE, &map_w, bar, kb * 64, col, at.z * a.zw);
+        }
+        if (SPLIT) break;
+      }
+      if (!alive)   // copies that were requested land within microseconds; nothing of them may outlive the CTA
+        for (int w = 0; w < 1000; ++w) __nanosleep(1000);
+    }
+  } else if (warp == T::W_MMA) {
+    // ---------------------------------------------------------------- MMA issue
+    if (rank == lead) {
+      int it = 0, i = 0;
+      bool alive = true;
+      for (int t = first_tile; t < ntiles && alive; t += tile_step, ++i) {
+        const int b = i & 1;
+        alive = gemm_wait_warp(smem_u32(&tempty_bar[b]), ((i >> 1) & 1) ^ 1, abortp);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int kb = k_lo; kb < k_hi && alive; ++kb, ++it) {
+          const int s = it % S;
+          if (!(alive = gemm_wait_warp(smem_u32(&full_bar[s]), (it / S) & 1, abortp))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (lane == 0) {
+            const uint64_t da = umma_desc_sw128(smA + s * T::A_STAGE), db = umma_desc_sw128(smB + s * T::B_STAGE);
+#pragma unroll
+            for (int k4 = 0; k4 < 4; ++k4)   // 16 elements of K: 32 bytes inside the swizzle atom
+              gemm_mma<CG>(tmem + b * BN, da + 2 * k4, db + 2 * k4, IDESC, (kb > k_lo || k4 > 0) ? 1u : 0u);
+            gemm_commit<CG>(smem_u32(&empty_bar[s]));
+            if (kb == k_hi - 1) gemm_commit<CG>(smem_u32(&tfull_bar[b]));
+          }
+          __syncwarp();
+        }
+        if (SPLIT) break;
+      }
+    }
+  } else if (QB && warp == T::W_PACK) {
+    // ---------------------------------------------------------------- packed rows of w
+    if (lane == 0) {
+      int pc = 0;
+      bool alive = true;
+      for (int t = first_tile; t < ntiles && alive; t += tile_step) {
+        const GemmTileAt at = gemm_tile_at(a, t);
+        const int col = at.n * BN + (int)(CG == 2 ? rank : 0) * T::NB;
+        for (int kb = k_lo; kb < k_hi; kb += KPC, ++pc) {
+          const int p = pc % RING;
+          if (!(alive = gemm_wait(smem_u32(&pempty_bar[p]), ((pc / RING) & 1) ^ 1, abortp))) break;
+          mbar_arrive_expect_tx(&pfull_bar[p], T::CHUNK);
+          gemm_tma_3d<1>(smP + p * T::CHUNK, &map_w, smem_u32(&pfull_bar[p]), kb / KPC * 128, col, 0);
+        }
+        if (SPLIT) break;
+      }
+      if (!alive)
+        for (int w = 0; w < 1000; ++w) __nanosleep(1000);
+    }
+  } else if (QB && warp >= T::W_DEQ) {
+    // ---------------------------------------------------------------- dequantisers: thread = row, group = every GROUPS-th K step
+    const int r = (tid - 32 * T::W_DEQ) & 127, grp = (warp - T::W_DEQ) >> 2;
+    const uint32_t swz = (uint32_t)(r & 7);
+    const int chunks = (k_hi - k_lo + KPC - 1) / KPC;      // of one tile
+    int it0 = 0, pc0 = 0;                                   // K steps and chunks of the tiles before this one
+    bool alive = true;
+    for (int t = first_tile; t < ntiles && alive; t += tile_step, it0 += k_hi - k_lo, pc0 += chunks) {
+      const GemmTileAt at = gemm_tile_at(a, t);
+      const int row = min(at.n * BN + (int)(CG == 2 ? rank : 0) * T::NB + r, a.N - 1);
+      const uint16_t* sp = a.scales + (size_t)row * nk_all;
+      const uint16_t* bp = a.biases + (size_t)row * nk_all;
+      int kb = k_lo + (grp + T::GROUPS - it0 % T::GROUPS) % T::GROUPS;
+      uint4 sv = make_uint4(0, 0, 0, 0), bv = sv, sn = sv, bn = sv;   // scale_vec: eight K steps' values, and the next eight
+      uint32_t s_next = 0, b_next = 0;                      // otherwise: the next step's
+      int have = -1;
+      if (a.scale_vec) {
+        sn = __ldg(reinterpret_cast<const uint4*>(sp + k_lo));
+        bn = __ldg(reinterpret_cast<const uint4*>(bp + k_lo));
+      } else if (kb < k_hi) {
+        s_next = __ldg(sp + kb);
+        b_next = __ldg(bp + kb);
+      }
+      for (; kb < k_hi; kb += T::GROUPS) {
+        const int it = it0 + kb - k_lo, pc = pc0 + (kb - k_lo) / KPC;
+        const int s = it % S, p = pc % RING, j = kb % KPC;
+        uint32_t sc, bi;                                    // bf16 bits
+        if (a.scale_vec) {
+          const int e = kb & 7;
+          if ((kb >> 3) != have) {
+            have = kb >> 3;
+            sv = sn; bv = bn;
+            if (8 * have + 8 < k_hi) {
+              sn = __ldg(reinterpret_cast<const uint4*>(sp + 8 * have + 8));
+              bn = __ldg(reinterpret_cast<const uint4*>(bp + 8 * have + 8));
+            }
+          }
+          const uint32_t sw = e < 4 ? (e < 2 ? sv.x : sv.y) : (e < 6 ? sv.z : sv.w);
+          const uint32_t bw = e < 4 ? (e < 2 ? bv.x : bv.y) : (e < 6 ? bv.z : bv.w);
+          sc = (e & 1) ? sw >> 16 : sw & 0xffffu;
+          bi = (e & 1) ? bw >> 16 : bw & 0xffffu;
+        } else {
+          sc = s_next; bi = b_next;
+          if (kb + T::GROUPS < k_hi) { s_next = __ldg(sp + kb + T::GROUPS); b_next = __ldg(bp + kb + T::GROUPS); }
+        }
+        if (!(alive = gemm_wait_warp(smem_u32(&pfull_bar[p]), (pc / RING) & 1, abortp))) break;
+        const uint32_t src = smP + p * T::CHUNK + r * 128, dst = smB + s * T::B_STAGE + r * 128;
+        uint4 w[QB == 4 ? 2 : 4];
+#pragma unroll
+        for (int c = 0; c < QB / 2; ++c) w[c] = lds128(src + (((uint32_t)(QB / 2 * j + c) ^ swz) << 4));
+        if (!(alive = gemm_wait_warp(smem_u32(&empty_bar[s]), ((it / S) & 1) ^ 1, abortp))) break;
+        if (QB == 4) {
+          const uint32_t s2 = sc | (sc << 16), b2 = bi | (bi << 16);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const uint4 q = w[c >> 2];
+            const uint4 o = gemm_dequant4((c & 3) == 0 ? q.x : (c & 3) == 1 ? q.y : (c & 3) == 2 ? q.z : q.w, s2, b2);
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + (((uint32_t)c ^ swz) << 4)), "r"(o.x), "r"(o.y),
+                         "r"(o.z), "r"(o.w) : "memory");
+          }
+        } else {
+          const float sf = __uint_as_float(sc << 16), bf = __uint_as_float(bi << 16);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const uint4 q = w[c >> 1];
+            const uint2 o0 = gemm_dequant8(c & 1 ? q.z : q.x, sf, bf), o1 = gemm_dequant8(c & 1 ? q.w : q.y, sf, bf);
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + (((uint32_t)c ^ swz) << 4)), "r"(o0.x), "r"(o0.y),
+                         "r"(o1.x), "r"(o1.y) : "memory");
+          }
+        }
+        fence_proxy_async();   // generic-proxy stores -> the tensor core's async proxy
+        __syncwarp();
+        if (lane == 0) {
+          if (CG == 2) mbar_arrive_remote(map_to_rank(smem_u32(&full_bar[s]), lead));
+          else mbar_arrive(&full_bar[s]);
+          mbar_arrive_n(&pempty_bar[p], kb == k_hi - 1 ? KPC - j : 1);   // the last chunk of a tile may hold fewer steps
+        }
+      }
+      if (SPLIT) break;
+    }
+  }
+
+  __syncwarp();
+  if (SPLIT) {
+    // ---- partial tiles meet: the 32-column run g belongs to rank g % ranks, which adds the ranks' parts in rank order.  The
+    // parts lie where the operand stages were (every rank is past its main loop), [run][source][4 columns][row] in 16 bytes.
+    const uint32_t ranks = gridDim.x;
+    cluster_sync_all();
+    if (warp < 4 && !*abortp) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int row_in = warp * 32 + lane;
+#pragma unroll 1
+      for (int g = 0; g < BN / 32; ++g) {
+        uint32_t v[32];
+        tmem_ld32(tmem + (uint32_t)(g * 32) + ((uint32_t)(warp * 32) << 16), v);
+        const uint32_t dst = map_to_rank(base, g % ranks) + ((uint32_t)((g / ranks) * ranks + rank) * 8 * 128 + row_in) * 16;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst + q * 128 * 16), "r"(v[4 * q]), "r"(v[4 * q + 1]),
+                       "r"(v[4 * q + 2]), "r"(v[4 * q + 3]) : "memory");
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    if (warp < T::EPI_WARPS && !*abortp) {
+      const GemmTileAt at = gemm_tile_at(a, first_tile);
+      const int row_in = (warp & 3) * 32 + lane;
+      for (int gi = warp >> 2; gi * (int)ranks + (int)rank < BN / 32; gi += T::EPI_WARPS / 4) {
+        uint32_t v[32];
+        float acc[32];
+#pragma unroll
+        for (int q = 0; q < 32; ++q) acc[q] = 0.f;
+        for (int src = 0; src < (int)ranks; ++src) {
+          const uint32_t p = base + ((uint32_t)(gi * (int)ranks + src) * 8 * 128 + row_in) * 16;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint4 u = lds128(p + q * 128 * 16);
+            acc[4 * q] += __uint_as_float(u.x); acc[4 * q + 1] += __uint_as_float(u.y);
+            acc[4 * q + 2] += __uint_as_float(u.z); acc[4 * q + 3] += __uint_as_float(u.w);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(acc[q]);
+        epi(at.z, at.m * T::BM + row_in, at.n * BN + (gi * (int)ranks + (int)rank) * 32, v);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (CG == 2) cluster_sync_all();   // neither CTA of a pair leaves while the other may still use its memory
+  if (warp == T::W_MMA) {
+    if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(T::TMEM_COLS) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(T::TMEM_COLS) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------- host side
+typedef CUresult (*GemmEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+inline GemmEncodeFn gemm_encode_fn() {
+  static const GemmEncodeFn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                   q == cudaDriverEntryPointSuccess ? (GemmEncodeFn)p : (GemmEncodeFn) nullptr;
+  }();
+  return fn;
+}
+// rows of `inner` elements (2 bytes, or 1: packed words) `pitch` bytes apart, `nb` such matrices `bpitch` bytes apart; boxes of
+// 128 bytes x box_rows, 128-byte swizzle, zeros beyond the ends.  base and pitches are multiples of 16 bytes.
+inline bool gemm_map(CUtensorMap* m, const void* p, int elem_bytes, long long inner, long long rows, long long pitch, int nb,
+                     long long bpitch, int box_rows) {
+  const GemmEncodeFn fn = gemm_encode_fn();
+  if (!fn) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)nb};
+  const cuuint64_t strides[2] = {(cuuint64_t)pitch, (cuuint64_t)(nb > 1 ? bpitch : pitch)};
+  const cuuint32_t box[3] = {(cuuint32_t)(128 / elem_bytes), (cuuint32_t)box_rows, 1}, one[3] = {1, 1, 1};
+  return fn(m, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(p), dims,
+            strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Measured, B200, 4-bit weights, us (TFLOP/s) with the 256 x 256 tile of one CTA, cp.async producers and no overlap of the
+// epilogue that this replaced -> here: 8192 x 14336 x 4096 1590 (605) -> 785 (1226); 1000 rows 290 -> 122; 256 rows -> 40; 77 rows
+// 400 -> 34; 77 x 4096 x 14336 720 -> 35 (four ranks).  bf16 weights: 8192 x 28672 x 4096 -> 1370 (1404).
+// The tile for a shape: the pair's 256 x 256, or a single CTA's 128 x 128 with K over 1..4 ranks of a cluster, whichever the
+// estimate (waves x K steps x SM cycles of a step, and the fixed costs of a wave) says is done first.
+struct GemmChoice { int pair, ranks, k_per, mt, nt; };
+inline GemmChoice gemm_choose(int M, int N, int K, int nb, int sms, double pair_step, double single_step) {
+  auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  const long long nk = K / 64, pair_tiles = up(M, 256) * up(N, 256) * nb, tiles = up(M, 128) * up(N, 128) * nb;
+  GemmChoice best = {1, 1, (int)nk, (int)up(M, 256), (int)up(N, 256)};
+  double cost = (double)up(pair_tiles, sms / 2) * nk * pair_step + 2500;
+  for (int r = 1; r <= 4; ++r) {
+    const long long per = up(up(nk, r), 8) * 8;     // ranks start on 16-byte runs of the scales and on whole packed chunks
+    if (up(nk, per) != r || tiles > 65535) continue;
+    const long long waves = up(tiles * r, sms);
+    const double c = r == 1 ? (double)waves * nk * single_step + 2500 : (double)waves * (per * single_step + 5000);
+    if (c < cost) { cost = c; best = {0, r, (int)per, (int)up(M, 128), (int)up(N, 128)}; }
+  }
+  return best;
+}
+
+template <int CG, int BN, int QB, bool SPLIT, class Epi>
+cudaError_t gemm_launch(const CUtensorMap& mx, const CUtensorMap& mw, const GemmArgs& a, const Epi& epi, int ranks, int sms,
+                        cudaStream_t st) {
+  using T = GemmTile<CG, BN, QB, SPLIT>;
+  auto kern = gemm_kernel<CG, BN, QB, SPLIT, Epi>;
+  static unsigned long long configured = 0;   // per device
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!(configured >> (dev & 63) & 1)) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
+    if (e != cudaSuccess) return e;
+    configured |= 1ull << (dev & 63);
+  }
+  const int tiles = a.mt * a.nt * a.nb, slots = sms / CG;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = SPLIT ? dim3((unsigned)ranks, (unsigned)tiles, 1) : dim3((unsigned)((tiles < slots ? tiles : slots) * CG), 1, 1);
+  cfg.blockDim = dim3(T::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = T::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = SPLIT ? (unsigned)ranks : (unsigned)CG;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CG == 2 || SPLIT ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, mx, mw, a, epi);
+}
+
+}  // namespace pie

@@ -1,0 +1,43 @@
+"""The tcgen05 tile kernels (pie_gemm.cuh: quantized prefill GEMM and dense linear; pie_fa_prefill.cu) against float64, at the
+edges of their tiles and on every route of their dispatch.  The bounds are elementwise and derived: a result rounded once to
+bf16 is off by at most 2^-9 of itself; an fp32 sum of K products by at most K 2^-24 of the sum of their magnitudes (2^-23
+where the tensor core truncates instead of rounding)."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _p(t):
+    return C.c_void_p(t.data_ptr())
+
+
+def _within(got, want, slack):
+    off = (got.double() - want).abs() - slack
+    assert torch.isfinite(got).all() and off.max() <= 0, float(off.max())
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("M,N,K", [(64, 128, 128),        # one tile, one packed chunk that is not full (4 bits)
+                                   (77, 300, 384),        # ragged rows and columns, scales one at a time
+                                   (129, 257, 512),       # one past a tile both ways, scales eight at a time
+                                   (70, 640, 14336),      # K over four ranks of a cluster
+                                   (200, 1024, 1152),     # a last rank with fewer steps
+                                   (513, 4100, 640),      # more tiles than one wave of single CTAs
+                                   (2050, 2056, 1024)])   # CTA pairs, ragged both ways, several tiles a pair
+def test_quantized_gemm_tiles(bits, M, N, K):
+    from proxy_inference_engine_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + K + bits)
+    w = torch.randn((N, K), generator=g, device="cuda").to(torch.bfloat16)
+    wq, s, b = ops.quantize(w, 64, bits)
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    shifts = torch.arange(0, 32, bits, device="cuda", dtype=torch.int32)
+    q = ((wq[:, :, None] >> shifts) & (2 ** bits - 1)).reshape(N, K // 64, 64).double()
+    dense = (q * s.double()[:, :, None] + b.double()[:, :, None]).reshape(N, K).to(torch.bfloat16).double()
+    want, mass = x.double() @ dense.t(), x.double().abs() @ dense.abs().t()
+    # w_hat comes from fp32 (8 bits) or a fused bf16 operation: where the float64 value sits on a rounding boundary it may
+    # differ by an ulp, 2^-8 of the weight, in a few weights of a thousand: allow 2^-9 / 64 of the mass
+    _within(ops.quantized_matmul(x, wq, s, b, group_size=64, bits=bits), want, want.abs() * 2 ** -8.9 + mass * (K * 2 ** -23 + 2 ** -15))
+    assert _lib.load().pie_pipeline_error() == 0
