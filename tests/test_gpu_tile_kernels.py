@@ -41,3 +41,44 @@ def test_quantized_gemm_tiles(bits, M, N, K):
     # differ by an ulp, 2^-8 of the weight, in a few weights of a thousand: allow 2^-9 / 64 of the mass
     _within(ops.quantized_matmul(x, wq, s, b, group_size=64, bits=bits), want, want.abs() * 2 ** -8.9 + mass * (K * 2 ** -23 + 2 ** -15))
     assert _lib.load().pie_pipeline_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 64, 64), (129, 257, 128), (70, 640, 8192), (200, 1024, 1152), (513, 4100, 192), (2050, 2056, 512)])
+def test_dense_gemm_tiles(M, N, K):
+    from proxy_inference_engine_b200 import _lib
+    L = _lib.load_hybrid(build_if_missing=True)
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn((N, K), generator=g, device="cuda").to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    slack = (x.double().abs() @ w.double().abs().t()) * (K * 2 ** -23)
+    for dt, code, rel in ((torch.float32, 1, 0.0), (torch.bfloat16, 0, 2 ** -8.9)):
+        out = torch.full((M, N), float("nan"), device="cuda", dtype=dt)
+        assert L.pieh_linear(_p(out), code, N, _p(x), 0, K, _p(w), 0, None, M, N, K, 0, 0.0, None, None, 0, None) == 0
+        _within(out, want, slack + want.abs() * rel)
+    for S in (1, 2, 3, 4):   # the residual-stream update: one routine for 1, 2 and 4 streams, another for the rest
+        xs = torch.randn((M, S, N), generator=g, device="cuda")
+        mix, ow = torch.randn((S, S), generator=g, device="cuda"), torch.randn((S,), generator=g, device="cuda")
+        ref = torch.einsum("su,msn->mun", mix.double(), xs.double()) + ow.double()[None, :, None] * want[:, None]
+        size = torch.einsum("su,msn->mun", mix.double().abs(), xs.double().abs()) + ow.double().abs()[None, :, None] * want.abs()[:, None]
+        assert L.pieh_linear(_p(xs), 1, 0, _p(x), 0, K, _p(w), 0, None, M, N, K, 3, 0.0, _p(mix), _p(ow), S, None) == 0
+        _within(xs, ref, size * (2 * S * 2 ** -23) + ow.double().abs()[None, :, None] * slack[:, None])
+    assert L.pieh_pipeline_error() == 0
+
+
+@pytest.mark.parametrize("shared", ["", "x", "w"])
+def test_dense_gemm_batched(shared):
+    """Products side by side, head-major columns; an operand stride of zero shares that operand."""
+    from proxy_inference_engine_b200 import _lib
+    L = _lib.load_hybrid(build_if_missing=True)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    M, N, K, nb = 150, 72, 128, 5
+    x = torch.randn((M, nb, K), generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn((nb, N, K), generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((M, nb, N), float("nan"), device="cuda")
+    assert L.pieh_linear_batched(_p(out), 1, nb * N, N, _p(x), 0, nb * K, 0 if shared == "x" else K, _p(w), 0,
+                                 0 if shared == "w" else N * K, nb, M, N, K, 0, None, 0, 0, None) == 0
+    xr = (x[:, :1].expand(M, nb, K) if shared == "x" else x).double()
+    wr = (w[:1].expand(nb, N, K) if shared == "w" else w).double()
+    want = torch.einsum("mzk,znk->mzn", xr, wr)
+    _within(out, want, torch.einsum("mzk,znk->mzn", xr.abs(), wr.abs()) * (K * 2 ** -23))
