@@ -126,8 +126,8 @@ int pie_prefill_attn(void* out, const void* q, const void* kcache, const void* v
                                          (cudaStream_t)stream));
 }
 
-// 1: a pipeline wait of the prefill GEMM expired (the call's results are void); 0: none did
-unsigned int pie_pipeline_error(void) { return qmm_pipeline_error(); }
+// 1: a pipeline wait of the prefill GEMM or of the prefill attention expired (the call's results are void); 0: none did
+unsigned int pie_pipeline_error(void) { return qmm_pipeline_error() | fa_prefill_pipeline_error(); }
 
 int pie_silu_mul(void* out, const void* gate, const void* up, long long n, void* stream) {
   if (n == 0) return PIE_OK;

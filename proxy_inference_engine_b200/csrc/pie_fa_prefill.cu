@@ -1,0 +1,377 @@
+// Prefill attention (L > 1, causal) on the 5th-generation tensor cores (tcgen05 + TMEM), sm_100a.
+//
+// Replaces mx.fast.scaled_dot_product_attention with the additive causal mask of create_attention_mask
+// (PIE/models/base.py:18-53, 92-113; Metal steel_attention, MLX/mlx/backend/metal/scaled_dot_product_attention.cpp:
+// 16-131): out[b, l, h] = softmax(scale * q[b,h,l] . K[b, h / n_rep, :offset+l+1]) . V.  The mask value -1e9 makes
+// masked probabilities exactly 0 in fp32, so masked keys are skipped (tiles beyond the diagonal are never loaded).
+//
+// A CTA owns 256 query rows of one head as two tiles of 128, and walks the keys in tiles of 128.  Per (query tile, key tile)
+// the tensor pipe needs 2 x 128 x 128 x D multiply-adds and the softmax 128 x 128 exponentials; at D = 128 the two take the
+// same ~1000 cycles of an SM, so the kernel is built to keep both going at once:
+//   * warps 0-3 / 4-7: the softmax of query tile 0 / 1, a thread per row.  S comes out of tensor memory (128 columns), is
+//     masked on the diagonal, the running maximum moves only when exceeded by 8 (log2 units; the same sums, and O is rescaled
+//     rarely), p = exp2(s - m) is rounded to bf16 and put back over S as the A operand of the second product.  Row sums are
+//     of the unrounded p, in fp32.
+//   * warp 8: TMA.  Q once; K and V tiles of the contiguous or paged cache into two-deep rings (128-byte swizzle).
+//   * warp 9, one lane: MMAs.  S_g = Q_g K^T (both operands in shared memory), O_g += P_g V (P in tensor memory, V as it lies:
+//     its rows are keys, so it is an MN-major operand).  Order: PV of tile 0, QK^T of tile 0's next keys, then the same for
+//     tile 1: one tile's softmax runs under the other's MMAs.
+// Tensor memory: S/P 2 x 128 columns, O 2 x D.  Longest query tiles are dispatched first (causal: tile i sees i + 1 key tiles).
+// Every wait is bounded (pie_gemm.cuh).
+// Measured, 32 query / 8 kv heads, D 128, us (TFLOP/s) with the mma.sync kernel of pie_fa.cu -> here: 8192 tokens 2190 (251) -> 547
+// (1005); 2 x 3000 tokens 640 (231) -> 190 (774); 1531 behind 517: D 64 92 -> 51.  The exponentials bound it at D 64.
+#include "pie_gemm.cuh"
+#include "pie_internal.h"
+
+namespace pie {
+
+struct FapArgs {
+  uint16_t* out;
+  int Hq, Hkv, L, offset, B;
+  float scale_log2e;
+  const int32_t* page_table;   // paged cache, else nullptr
+  int pt_stride, page_size;
+};
+
+template <int D>
+struct FapTile {
+  static constexpr int CH = D / 64;                     // 64-feature chunks of a row: 128 bytes each
+  static constexpr int TILE = 128 * D * 2;              // bytes of 128 rows
+  static constexpr int SMEM = 1024 + 6 * TILE;          // Q0, Q1, K x 2, V x 2
+  static constexpr int THREADS = 384;
+};
+
+__device__ __forceinline__ void fap_tma_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+// D[128 x N] += A[128 x 16] (tensor memory, bf16 pairs) * B (shared memory)
+__device__ __forceinline__ void fap_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accum) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc),
+      "r"(accum) : "memory");
+}
+// shared-memory descriptor of an MN-major operand in the 128-byte swizzle: rows of 64 features, 8 rows (keys) per atom,
+// atoms 1024 bytes apart along the keys, 64-feature chunks 128 rows apart
+__device__ __forceinline__ uint64_t fap_desc_mn(uint32_t smem_addr) {
+  return (uint64_t)((smem_addr & 0x3FFFF) >> 4) | ((uint64_t)(128 * 128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+// 32 columns of this warp's 32 lanes, not waited for
+__device__ __forceinline__ void fap_tmem_ld(uint32_t taddr, float* v) {
+  uint32_t* u = reinterpret_cast<uint32_t*>(v);
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
+      "%29,%30,%31}, [%32];"
+      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
+        "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]), "=r"(u[16]),
+        "=r"(u[17]), "=r"(u[18]), "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]),
+        "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
+      : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void fap_tmem_st(uint32_t taddr, const uint32_t* u) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
+      "%29,%30,%31};" ::"r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]),
+      "r"(u[9]), "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15]), "r"(u[16]), "r"(u[17]), "r"(u[18]),
+      "r"(u[19]), "r"(u[20]), "r"(u[21]), "r"(u[22]), "r"(u[23]), "r"(u[24]), "r"(u[25]), "r"(u[26]), "r"(u[27]), "r"(u[28]),
+      "r"(u[29]), "r"(u[30]), "r"(u[31]), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void fap_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ float fap_exp2(float x) {   // results below 2^-126 are 0
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ void fap_commit(uint64_t* bar) { gemm_commit<1>(smem_u32(bar)); }
+
+template <int D>
+__global__ void __launch_bounds__(FapTile<D>::THREADS, 1)
+fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ FapArgs a) {
+  using T = FapTile<D>;
+  constexpr uint32_t ID_S = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+  constexpr uint32_t ID_O = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(D >> 3) << 17) | ((128u >> 4) << 24);
+  constexpr int COL_S = 0, COL_O = 256;   // + g * 128, + g * D
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], o_full[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t smQ = base, smK = base + 2 * T::TILE, smV = base + 4 * T::TILE;
+  const int b = blockIdx.x / a.Hq, h = blockIdx.x - b * a.Hq, kvh = h / (a.Hq / a.Hkv);
+  const int q0 = (int)(gridDim.y - 1 - blockIdx.y) * 256;
+  const int keys = a.offset + a.L;
+  // key tiles of query tile g: up to the diagonal of its last live row; none if the tile lies beyond the queries
+  auto tiles_of = [&](int g) { return q0 + g * 128 < a.L ? (a.offset + min(q0 + g * 128 + 128, a.L) - 1) / 128 + 1 : 0; };
+  const int n0 = tiles_of(0), n1 = tiles_of(1), n = max(n0, n1);
+
+  if (tid == 0) {
+    mbar_init(&q_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
+      mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_full[i], 1);
+    }
+    abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "n"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (warp == 8 && lane < 3) tma_prefetch_desc(lane == 0 ? &map_q : lane == 1 ? &map_k : &map_v);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  volatile int* const abortp = &abort_flag;
+
+  if (warp < 8) {
+    // ------------------------------------------------------------------------------------------------ softmax of tile g
+    const int g = warp >> 2, quad = warp & 3, ng = g ? n1 : n0;
+    const int row = q0 + g * 128 + quad * 32 + lane, lim = a.offset + row;   // last key this row sees
+    const uint32_t lanes = (uint32_t)(quad * 32) << 16;
+    const uint32_t tS = tmem + COL_S + g * 128 + lanes, tO = tmem + COL_O + g * D + lanes;
+    const int tail = keys & 127;   // rows of the last key tile that exist
+    float m = -INFINITY, l = 0.f;
+    bool alive = true;
+    for (int j = 0; j < ng; ++j) {
+      if (!(alive = gemm_wait_warp(smem_u32(&s_full[g]), j & 1, abortp))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float s[128];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) fap_tmem_ld(tS + 32 * c, s + 32 * c);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 128; ++i) s[i] *= a.scale_log2e;
+      if (j * 128 + 127 > a.offset + q0 + g * 128 + quad * 32) {   // a key of this tile lies beyond some row of the warp
+        const int last = lim - j * 128;
+#pragma unroll
+        for (int i = 0; i < 128; ++i)
+          if (i > last) s[i] = -INFINITY;
+      }
+      float x0 = s[0], x1 = s[1], x2 = s[2], x3 = s[3];
+#pragma unroll
+      for (int i = 4; i < 128; i += 4) {
+        x0 = fmaxf(x0, s[i]); x1 = fmaxf(x1, s[i + 1]); x2 = fmaxf(x2, s[i + 2]); x3 = fmaxf(x3, s[i + 3]);
+      }
+      const float mx = fmaxf(fmaxf(x0, x1), fmaxf(x2, x3));
+      const bool move = mx > m + 8.f;
+      if (j == 0) {
+        m = mx;
+      } else if (__any_sync(0xffffffffu, move)) {
+        const float c = move ? fap_exp2(m - mx) : 1.f;   // m == -inf: 0, and everything it multiplies is 0
+        if (move) m = mx;
+        l *= c;
+        // O holds the tiles before this one once their product has finished
+        if (!(alive = gemm_wait_warp(smem_u32(&o_full[g]), (j - 1) & 1, abortp))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+        for (int c0 = 0; c0 < D; c0 += 32) {
+          float o[32];
+          fap_tmem_ld(tO + c0, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] *= c;
+          fap_tmem_st(tO + c0, reinterpret_cast<uint32_t*>(o));
+        }
+        fap_tmem_st_wait();
+      }
+      const float ms = m == -INFINITY ? 0.f : m;
+      float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t p[32];
+#pragma unroll
+        for (int i = 0; i < 64; i += 4) {
+          const float* q = s + 64 * hf + i;
+          const float e0 = fap_exp2(q[0] - ms), e1 = fap_exp2(q[1] - ms), e2 = fap_exp2(q[2] - ms), e3 = fap_exp2(q[3] - ms);
+          l0 += e0; l1 += e1; l2 += e2; l3 += e3;
+          p[i / 2] = pack_bf16(e0, e1);
+          p[i / 2 + 1] = pack_bf16(e2, e3);
+        }
+        fap_tmem_st(tS + 32 * hf, p);
+      }
+      l += (l0 + l1) + (l2 + l3);
+      fap_tmem_st_wait();
+      if (a.page_table && tail && j == (keys - 1) / 128) {
+        // the slots behind the last key of a page may hold anything, and 0 * NaN is not 0: clear them
+        if (!(alive = gemm_wait_warp(smem_u32(&v_full[j & 1]), (j >> 1) & 1, abortp))) break;
+        const int r = quad * 32 + lane;
+        if (r >= tail)
+#pragma unroll
+          for (int c = 0; c < 8 * T::CH; ++c)
+            asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(smV + (j & 1) * T::TILE + (c >> 3) * 16384 + r * 128 + (c & 7) * 16),
+                         "r"(0) : "memory");
+        fence_proxy_async();
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[g]);
+    }
+    if (alive && ng > 0 && gemm_wait_warp(smem_u32(&o_full[g]), (ng - 1) & 1, abortp)) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const float inv = 1.f / l;
+      uint16_t* o_row = a.out + (((size_t)b * a.L + row) * a.Hq + h) * D;
+#pragma unroll 1
+      for (int c0 = 0; c0 < D; c0 += 32) {
+        float o[32];
+        fap_tmem_ld(tO + c0, o);
+        tmem_ld_wait();
+        if (row < a.L)
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            *reinterpret_cast<uint4*>(o_row + c0 + 8 * q) =
+                make_uint4(pack_bf16(o[8 * q] * inv, o[8 * q + 1] * inv), pack_bf16(o[8 * q + 2] * inv, o[8 * q + 3] * inv),
+                           pack_bf16(o[8 * q + 4] * inv, o[8 * q + 5] * inv), pack_bf16(o[8 * q + 6] * inv, o[8 * q + 7] * inv));
+      }
+    }
+  } else if (warp == 8) {
+    // ------------------------------------------------------------------------------------------------ TMA
+    if (lane == 0) {
+      const int ntq = n1 > 0 ? 2 : 1;
+      mbar_arrive_expect_tx(&q_full, ntq * T::TILE);
+      for (int g = 0; g < ntq; ++g)
+        for (int c = 0; c < T::CH; ++c)
+          gemm_tma_3d<1>(smQ + g * T::TILE + c * 16384, &map_q, smem_u32(&q_full), c * 64, q0 + g * 128, b * a.Hq + h);
+      bool alive = true;
+      auto fetch = [&](int j, const CUtensorMap* map, uint32_t dst, uint64_t* full) {
+        mbar_arrive_expect_tx(full, T::TILE);
+        for (int r = 0; r < 2; ++r) {   // 64 keys at a time: a page, or half a tile
+          int t = j * 128 + r * 64, c1 = t, c2 = kvh, c3 = b;
+          if (a.page_table) {
+            t = min(t, (keys - 1) / 64 * 64);   // behind the last key: any page that exists
+            c1 = t % a.page_size;
+            c3 = __ldg(a.page_table + (size_t)b * a.pt_stride + t / a.page_size);
+          }
+          for (int c = 0; c < T::CH; ++c) fap_tma_4d(dst + c * 16384 + r * 8192, map, smem_u32(full), c * 64, c1, c2, c3);
+        }
+      };
+      for (int j = 0; j < n && alive; ++j) {
+        const int i = j & 1, ph = (j >> 1) & 1;
+        if (!(alive = gemm_wait(smem_u32(&k_empty[i]), ph ^ 1, abortp))) break;
+        fetch(j, &map_k, smK + i * T::TILE, &k_full[i]);
+        if (!(alive = gemm_wait(smem_u32(&v_empty[i]), ph ^ 1, abortp))) break;
+        fetch(j, &map_v, smV + i * T::TILE, &v_full[i]);
+      }
+      if (!alive)
+        for (int w = 0; w < 1000; ++w) __nanosleep(1000);
+    }
+  } else if (warp == 9) {
+    // ------------------------------------------------------------------------------------------------ MMAs
+    auto qk = [&](int g, int j) {
+      if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+          const uint64_t dq = umma_desc_sw128(smQ + g * T::TILE + (k >> 2) * 16384) + 2 * (k & 3);
+          const uint64_t dk = umma_desc_sw128(smK + (j & 1) * T::TILE + (k >> 2) * 16384) + 2 * (k & 3);
+          umma_bf16(tmem + COL_S + g * 128, dq, dk, ID_S, k > 0 ? 1u : 0u);
+        }
+        fap_commit(&s_full[g]);
+      }
+    };
+    auto pv = [&](int g, int j) {
+      if (lane == 0) {
+        const uint64_t dv = fap_desc_mn(smV + (j & 1) * T::TILE);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)   // 16 keys: 8 columns of P, two 8-key atoms of V
+          fap_mma_ts(tmem + COL_O + g * D, tmem + COL_S + g * 128 + 8 * k, dv + (uint64_t)k * (2048 >> 4), ID_O, (j > 0 || k > 0) ? 1u : 0u);
+        fap_commit(&o_full[g]);
+      }
+    };
+    bool alive = gemm_wait_warp(smem_u32(&q_full), 0, abortp) && gemm_wait_warp(smem_u32(&k_full[0]), 0, abortp);
+    if (alive) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (n0 > 0) qk(0, 0);
+      if (n1 > 0) qk(1, 0);
+      if (lane == 0) fap_commit(&k_empty[0]);
+    }
+    for (int j = 0; j < n && alive; ++j) {
+      const int i = j & 1, i2 = (j + 1) & 1;
+      if (!(alive = gemm_wait_warp(smem_u32(&v_full[i]), (j >> 1) & 1, abortp))) break;
+      if (j + 1 < n && !(alive = gemm_wait_warp(smem_u32(&k_full[i2]), ((j + 1) >> 1) & 1, abortp))) break;
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        const int ng = g ? n1 : n0;
+        if (j < ng) {
+          if (!(alive = gemm_wait_warp(smem_u32(&p_full[g]), j & 1, abortp))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          pv(g, j);
+          if (j + 1 < ng) qk(g, j + 1);
+        }
+      }
+      if (!alive) break;
+      if (lane == 0) {
+        fap_commit(&v_empty[i]);
+        if (j + 1 < n) fap_commit(&k_empty[i2]);
+      }
+      __syncwarp();
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
+}
+
+// What a tiled copy of the cache asks for: 16-byte aligned arrays, positive strides where there is more than one head / row,
+// pages of whole 64-key boxes, and grid limits.
+bool fa_prefill_umma_ok(const uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc, const KvLayout& kv, int B,
+                        int Hq, int Hkv, int L, int D, int offset) {
+  auto off16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
+  if (off16(out) || off16(q) || off16(kc) || off16(vc) || (L + 255) / 256 > 65535 || (long long)B * Hq > (1 << 30)) return false;
+  if (kv.tok_stride <= 0 || (Hkv > 1 && kv.head_stride <= 0)) return false;
+  return kv.page_table ? kv.page_size % 64 == 0 : (B == 1 || kv.batch_stride > 0);
+}
+
+template <int D>
+static cudaError_t launch_fap(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FapArgs& a, cudaStream_t st) {
+  using T = FapTile<D>;
+  cudaError_t e = cudaFuncSetAttribute(fa_prefill_umma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
+  if (e != cudaSuccess) return e;
+  count_launch();
+  fa_prefill_umma_kernel<D><<<dim3((unsigned)(a.B * a.Hq), (unsigned)((a.L + 255) / 256)), T::THREADS, T::SMEM, st>>>(mq, mk, mv, a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fa_prefill_umma(uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc, const KvLayout& kv, int B,
+                                   int Hq, int Hkv, int L, int D, int offset, float scale, cudaStream_t st) {
+  FapArgs a;
+  a.out = out; a.Hq = Hq; a.Hkv = Hkv; a.L = L; a.offset = offset; a.B = B;
+  a.scale_log2e = scale * 1.4426950408889634f;
+  a.page_table = kv.page_table; a.pt_stride = kv.pt_stride; a.page_size = kv.page_size;
+  CUtensorMap mq, maps[2];
+  if (!gemm_map(&mq, q, 2, D, L, (long long)D * 2, B * Hq, (long long)L * D * 2, 128)) return cudaErrorNotSupported;
+  const GemmEncodeFn fn = gemm_encode_fn();
+  const long long tok = kv.tok_stride * 2, head = Hkv > 1 ? kv.head_stride * 2 : tok;
+  for (int i = 0; i < 2; ++i) {
+    // contiguous: [rows][heads][keys][D] with the keys that exist; paged: [pages][heads][slots][D]
+    const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)(kv.page_table ? kv.page_size : offset + L), (cuuint64_t)Hkv,
+                                (cuuint64_t)(kv.page_table ? 0x7fffffff : B)};
+    const cuuint64_t strides[3] = {(cuuint64_t)tok, (cuuint64_t)head,
+                                   (cuuint64_t)(kv.page_table ? kv.page_size * tok : B > 1 ? kv.batch_stride * 2 : tok)};
+    const cuuint32_t box[4] = {64, 64, 1, 1}, one[4] = {1, 1, 1, 1};
+    if (fn(&maps[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<uint16_t*>(i ? vc : kc), dims, strides, box, one,
+           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return cudaErrorNotSupported;
+  }
+  return D == 128 ? launch_fap<128>(mq, maps[0], maps[1], a, st) : launch_fap<64>(mq, maps[0], maps[1], a, st);
+}
+
+unsigned int fa_prefill_pipeline_error() {
+  unsigned int v = 0;
+  cudaMemcpyFromSymbol(&v, g_gemm_error, sizeof(v));
+  return v;
+}
+
+}  // namespace pie

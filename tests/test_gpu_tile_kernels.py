@@ -82,3 +82,45 @@ def test_dense_gemm_batched(shared):
     wr = (w[:1].expand(nb, N, K) if shared == "w" else w).double()
     want = torch.einsum("mzk,znk->mzn", xr, wr)
     _within(out, want, torch.einsum("mzk,znk->mzn", xr.abs(), wr.abs()) * (K * 2 ** -23))
+
+
+@pytest.mark.parametrize("paged", [False, True])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Hq,Hkv,L,offset", [(1, 2, 1, 1, 0),        # one query, one key
+                                               (1, 2, 2, 2, 255),      # two queries across a key tile's end
+                                               (2, 4, 2, 129, 0),      # one row in the second query tile
+                                               (1, 4, 1, 256, 128),    # whole tiles
+                                               (2, 4, 2, 300, 77),     # ragged everywhere
+                                               (1, 2, 1, 1030, 517)])  # several blocks, the ring wraps
+def test_prefill_attention_tiles(paged, D, B, Hq, Hkv, L, offset):
+    from proxy_inference_engine_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(L + offset + D)
+    T, scale = offset + L, D ** -0.5
+    rnd = lambda *s: (1.5 * torch.randn(s, generator=g, device="cuda")).to(torch.bfloat16)
+    q, k, v = rnd(B, Hq, L, D), rnd(B, Hkv, T, D), rnd(B, Hkv, T, D)
+    nan = float("nan")   # slots no token was written to: what is there must not matter
+    if paged:
+        n = (T + 63) // 64
+        kb, vb = (torch.full((B * n + 2, 64, Hkv, D), nan, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        table = torch.full((B, n + 1), -1, device="cuda", dtype=torch.int32)
+        table[:, :n] = torch.randperm(B * n + 2, generator=g, device="cuda")[:B * n].view(B, n)
+        t = torch.arange(T, device="cuda")
+        for b in range(B):
+            kb[table[b, t // 64].long(), t % 64], vb[table[b, t // 64].long(), t % 64] = k[b].transpose(0, 1), v[b].transpose(0, 1)
+        lay = ops.kv_layout(kb, table, 64)
+    else:
+        kb, vb = (torch.full((B, Hkv, T + 70, D), nan, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        kb[:, :, :T], vb[:, :, :T] = k, v
+        lay = ops.kv_layout(kb)
+    got = ops.prefill_attention(q, kb, vb, lay, offset, scale)
+    rep = Hq // Hkv
+    s = torch.einsum("bhld,bhtd->bhlt", q.double(), k.double().repeat_interleave(rep, 1)) * scale
+    i, j = torch.arange(L, device="cuda")[:, None] + offset, torch.arange(T, device="cuda")[None]
+    p = torch.softmax(s.masked_fill(j > i, float("-inf")), -1)
+    vr = v.double().repeat_interleave(rep, 1)
+    want, mass = p @ vr, p @ vr.abs()
+    # each weight rounded to bf16 (2^-9 of it), the result rounded once; scores are fp32 sums of D products of size |s| and the
+    # exponential turns their error into a relative one
+    slack = mass * (2 ** -8.9 + 2 * D * 2 ** -23 * float(s.abs().max())) + want.abs() * 2 ** -8.9
+    _within(got, want, slack)
+    assert _lib.load().pie_pipeline_error() == 0
