@@ -124,3 +124,21 @@ def test_prefill_attention_tiles(paged, D, B, Hq, Hkv, L, offset):
     slack = mass * (2 ** -8 + 2 * D * 2 ** -23 * float(s.abs().max())) + want.abs() * 2 ** -8
     _within(got, want, slack)
     assert _lib.load().pie_pipeline_error() == 0
+
+
+@pytest.mark.parametrize("rows,dims", [(1, 8), (3, 2048), (2, 2056), (5, 4096), (3, 8192), (2, 8200), (3, 100)])
+def test_row_and_elementwise_operators(rows, dims):
+    """RMSNorm at the edges of its register tiles, SwiGLU and the sum with and without 16-byte alignment and a tail."""
+    from proxy_inference_engine_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(dims)
+    rnd = lambda *s: (3 * torch.randn(s, generator=g, device="cuda")).to(torch.bfloat16)
+    x, w = rnd(rows, dims), rnd(dims)
+    n = x.double() * torch.rsqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-5)
+    _within(ops.rms_norm(x, w, 1e-5), n * w.double(), (n * w.double()).abs() * 2.1 * 2 ** -8)      # rounded twice
+    _within(ops.rms_norm(x, None, 1e-5), n, n.abs() * 1.1 * 2 ** -8)
+    a, b = rnd(rows * dims + 5), rnd(rows * dims + 5)
+    for off in (0, 1):   # 1: not 16-byte aligned
+        u, v = a[off:], b[off:]
+        want = u.double() * torch.sigmoid(u.double()) * v.double()
+        _within(ops.silu_mul(u, v), want, want.abs() * 3.1 * 2 ** -8)                              # rounded three times
+        assert torch.equal(ops.add(u, v), u + v)
