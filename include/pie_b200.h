@@ -130,6 +130,14 @@ int pie_rope_kv_append(void* q_out, const void* qkv, void* kcache, void* vcache,
 /* ---- a8  cache.update_and_fetch for L >= 1 (prefill): copy k,v [B, Hkv, L, D] into the cache at offset - */
 int pie_kv_write(void* kcache, void* vcache, const pie_kv_layout* kv_host, const void* k, const void* v, int B,
                  int Hkv, int L, int D, int offset, void* stream);
+/* the same from k, v [B, Hkv, L, D] with any strides (elements) and contiguous features: a projection's rows as they lie */
+int pie_kv_write_strided(void* kcache, void* vcache, const pie_kv_layout* kv_host, const void* k, long long k_stride_b,
+                         long long k_stride_h, long long k_stride_l, const void* v, long long v_stride_b, long long v_stride_h,
+                         long long v_stride_l, int B, int Hkv, int L, int D, int offset, void* stream);
+/* pie_rope with dims == D (64 or 128), halves paired, scale 1 and freqs, from x [B, H, L, D] with any strides that are multiples
+ * of 8 elements (x 16-byte aligned) to a contiguous out; positions offset .. offset + L - 1 */
+int pie_rope_heads(void* out, const void* x, int B, int H, int L, int D, long long stride_b, long long stride_h,
+                   long long stride_l, int offset, const float* freqs, void* stream);
 
 /* ---- a9  mx.fast.scaled_dot_product_attention, L == 1, mask None (PIE/models/base.py:92-113) ----------
  * split-K flash-decode (the scheme of Metal sdpa_vector_2pass, kernels/sdpa_vector.h:168-392).

@@ -90,6 +90,8 @@ SIGNATURES = {
     "pie_rms_norm": (_i, [_vp, _vp, _vp, _ll, _i, _f, _vp]),
     "pie_rope": (_i, [_vp, _vp, _ll, _i, _i, _i, _i, _f, _f, _i, _vp, _vp]),
     "pie_rope_kv_append": (_i, [_vp, _vp, _vp, _vp, C.POINTER(KvLayout), _vp, _vp, _i, _i, _i, _i, _vp]),
+    "pie_kv_write_strided": (_i, [_vp, _vp, C.POINTER(KvLayout), _vp, _ll, _ll, _ll, _vp, _ll, _ll, _ll, _i, _i, _i, _i, _i, _vp]),
+    "pie_rope_heads": (_i, [_vp, _vp, _i, _i, _i, _i, _ll, _ll, _ll, _i, _vp, _vp]),
     "pie_kv_write": (_i, [_vp, _vp, C.POINTER(KvLayout), _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "pie_decode_attn_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "pie_decode_attn_pick_splits": (_i, [_i, _i, _i, _i]),

@@ -10,9 +10,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _lib, ops
-from .ops import _p, _stream
-import ctypes as C
+from . import ops
 
 
 class KVCache:
@@ -43,10 +41,7 @@ class KVCache:
         B, H, L, D = keys.shape
         if self.keys is None or self.offset + L > self.keys.shape[2]:
             self._grow(B, H, D, L, keys.device)
-        lay = ops.kv_layout(self.keys)
-        kc, vc = keys.contiguous(), values.contiguous()  # keep both alive across the launch (no pointer reuse)
-        _lib.check(_lib.load().pie_kv_write(_p(self.keys), _p(self.values), C.byref(lay), _p(kc), _p(vc), B, H, L, D,
-                                            self.offset, _stream()), "update_and_fetch")
+        ops.kv_write(self.keys, self.values, ops.kv_layout(self.keys), keys, values, self.offset)
         self.offset += L
         return self.keys[:, :, : self.offset], self.values[:, :, : self.offset]
 
@@ -81,10 +76,7 @@ class PagedKVCache:
         B, H, L, D = keys.shape
         if self.offset + L > self.page_table.shape[1] * self.page_size:
             raise ValueError("PagedKVCache: page table too small for this many tokens")
-        lay = self.layout()
-        kc, vc = keys.contiguous(), values.contiguous()  # keep both alive across the launch (no pointer reuse)
-        _lib.check(_lib.load().pie_kv_write(_p(self.k_pool), _p(self.v_pool), C.byref(lay), _p(kc), _p(vc), B, H, L, D,
-                                            self.offset, _stream()), "update_and_fetch")
+        ops.kv_write(self.k_pool, self.v_pool, self.layout(), keys, values, self.offset)
         self.offset += L
         return self, self
 

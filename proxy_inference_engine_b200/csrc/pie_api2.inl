@@ -59,14 +59,32 @@ int pie_rope_kv_append(void* q_out, const void* qkv, void* kcache, void* vcache,
                                            (cudaStream_t)stream));
 }
 
-int pie_kv_write(void* kcache, void* vcache, const pie_kv_layout* kv, const void* k, const void* v, int B, int Hkv,
-                 int L, int D, int offset, void* stream) {
+int pie_rope_heads(void* out, const void* x, int B, int H, int L, int D, long long stride_b, long long stride_h,
+                   long long stride_l, int offset, const float* freqs, void* stream) {
+  if (B == 0 || H == 0 || L == 0) return PIE_OK;
+  if (!out || !x || !freqs) return PIE_ENULL;
+  if (B < 0 || H < 0 || L < 0 || (D != 64 && D != 128) || B > 65535) return PIE_EINVAL_SHAPE;
+  if (!aligned16(out) || !aligned16(x) || (stride_b | stride_h | stride_l) % 8) return PIE_EALIGN;
+  return cuda_status(launch_rope_heads((uint16_t*)out, (const uint16_t*)x, B, H, L, D, stride_b, stride_h, stride_l, offset, freqs,
+                                       (cudaStream_t)stream));
+}
+
+int pie_kv_write_strided(void* kcache, void* vcache, const pie_kv_layout* kv, const void* k, long long k_stride_b,
+                         long long k_stride_h, long long k_stride_l, const void* v, long long v_stride_b, long long v_stride_h,
+                         long long v_stride_l, int B, int Hkv, int L, int D, int offset, void* stream) {
   if (B == 0 || L == 0) return PIE_OK;
   if (!kcache || !vcache || !k || !v) return PIE_ENULL;
   if (B < 0 || Hkv <= 0 || L < 0 || D <= 0 || offset < 0) return PIE_EINVAL_SHAPE;
   if (int s = check_kv(kv, D)) return s;
-  return cuda_status(launch_kv_write((uint16_t*)kcache, (uint16_t*)vcache, to_kv(kv), (const uint16_t*)k,
-                                     (const uint16_t*)v, B, Hkv, L, D, offset, (cudaStream_t)stream));
+  const KvSrc ks = {k_stride_b, k_stride_h, k_stride_l}, vs = {v_stride_b, v_stride_h, v_stride_l};
+  return cuda_status(launch_kv_write((uint16_t*)kcache, (uint16_t*)vcache, to_kv(kv), (const uint16_t*)k, (const uint16_t*)v, ks, vs,
+                                     B, Hkv, L, D, offset, (cudaStream_t)stream));
+}
+
+int pie_kv_write(void* kcache, void* vcache, const pie_kv_layout* kv, const void* k, const void* v, int B, int Hkv,
+                 int L, int D, int offset, void* stream) {
+  const long long sl = D, sh = sl * L, sb = sh * Hkv;
+  return pie_kv_write_strided(kcache, vcache, kv, k, sb, sh, sl, v, sb, sh, sl, B, Hkv, L, D, offset, stream);
 }
 
 size_t pie_decode_attn_workspace_bytes(int B, int Hq, int D, int nsplit) {

@@ -98,8 +98,12 @@ cudaError_t launch_rope(uint16_t* out, const uint16_t* x, long long n_batch, int
 cudaError_t launch_rope_kv_append(uint16_t* q_out, const uint16_t* qkv, uint16_t* kc, uint16_t* vc,
                                   const KvLayout& kv, const int32_t* pos, const float* freqs, int B, int Hq,
                                   int Hkv, int D, cudaStream_t st);
-cudaError_t launch_kv_write(uint16_t* kc, uint16_t* vc, const KvLayout& kv, const uint16_t* k,
-                            const uint16_t* v, int B, int Hkv, int L, int D, int offset, cudaStream_t st);
+// strides (elements) of a [B, H, L, D] source with contiguous features
+struct KvSrc { long long sb, sh, sl; };
+cudaError_t launch_kv_write(uint16_t* kc, uint16_t* vc, const KvLayout& kv, const uint16_t* k, const uint16_t* v, const KvSrc& ks,
+                            const KvSrc& vs, int B, int Hkv, int L, int D, int offset, cudaStream_t st);
+cudaError_t launch_rope_heads(uint16_t* out, const uint16_t* x, int B, int H, int L, int D, long long sb, long long sh,
+                              long long sl, int offset, const float* freqs, cudaStream_t st);
 cudaError_t launch_decode_attn(uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc,
                                const KvLayout& kv, const int32_t* pos, int B, int Hq, int Hkv, int D,
                                float scale, int nsplit, float* ws, cudaStream_t st);

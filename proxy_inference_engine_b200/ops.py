@@ -195,14 +195,38 @@ def rope(x, dims: int, *, traditional: bool = False, base: float | None = None, 
         freqs = freqs.to(torch.float32).contiguous()
     if x.dtype != _BF16:
         raise ValueError("[rope] only bfloat16 is built here")
-    x = x.contiguous()
-    out = torch.empty_like(x)
     Lq, D = x.shape[-2], x.shape[-1]
     L = _lib.load()
+    if freqs is not None and not traditional and dims == D and D in (64, 128) and scale == 1.0 and x.dim() == 4 and _heads_ok(x):
+        # the Llama case: every feature rotated, halves paired; heads may lie as the projection wrote them
+        B, H = x.shape[0], x.shape[1]
+        out = torch.empty((B, H, Lq, D), dtype=_BF16, device=x.device)
+        _lib.check(L.pie_rope_heads(_p(out), _p(x), B, H, Lq, D, x.stride(0), x.stride(1), x.stride(2), int(offset), _p(freqs),
+                                    _stream()), "rope")
+        return out
+    x = x.contiguous()
+    out = torch.empty_like(x)
     _lib.check(L.pie_rope(_p(out), _p(x), x.numel() // (Lq * D), Lq, D, dims, int(traditional),
                           0.0 if base is None else float(base), float(scale), int(offset), _p(freqs), _stream()),
                "rope")
     return out
+
+
+def _heads_ok(x) -> bool:
+    """[B, H, L, D] whose rows a kernel can read 16 bytes at a time wherever they lie."""
+    return x.stride(3) == 1 and (x.stride(0) | x.stride(1) | x.stride(2)) % 8 == 0 and x.data_ptr() % 16 == 0 and x.shape[0] <= 65535
+
+
+def kv_write(kbuf, vbuf, lay: "KvLayout", keys, values, offset: int):
+    """keys, values [B, Hkv, L, D] -> cache rows offset .. offset + L - 1, from wherever their rows lie."""
+    B, H, Lq, D = keys.shape
+    if keys.stride(3) != 1:
+        keys = keys.contiguous()
+    if values.stride(3) != 1:
+        values = values.contiguous()
+    _lib.check(_lib.load().pie_kv_write_strided(_p(kbuf), _p(vbuf), C.byref(lay), _p(keys), keys.stride(0), keys.stride(1),
+                                                keys.stride(2), _p(values), values.stride(0), values.stride(1), values.stride(2),
+                                                B, H, Lq, D, offset, _stream()), "update_and_fetch")
 
 
 class CausalMask:

@@ -142,3 +142,29 @@ def test_row_and_elementwise_operators(rows, dims):
         want = u.double() * torch.sigmoid(u.double()) * v.double()
         _within(ops.silu_mul(u, v), want, want.abs() * 3.1 * 2 ** -8)                              # rounded three times
         assert torch.equal(ops.add(u, v), u + v)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,L,offset", [(1, 1, 7), (3, 5, 0), (2, 513, 100)])
+def test_rope_and_cache_write_of_strided_heads(D, B, L, offset):
+    """Heads as the projection wrote them give the same bits as a contiguous copy of them; so does the cache."""
+    from proxy_inference_engine_b200 import ops
+    from proxy_inference_engine_b200.cache import KVCache
+    g = torch.Generator(device="cuda").manual_seed(L + D)
+    H, pad = 3, 8
+    rows = torch.randn((B, L, 2 * H * D + pad), generator=g, device="cuda").to(torch.bfloat16)   # k and v side by side
+    k, v = (rows[..., i * H * D:(i + 1) * H * D].reshape(B, L, H, D).transpose(1, 2) for i in (0, 1))
+    freqs = torch.linspace(1.0, 500.0, D // 2, device="cuda")
+    turned = ops.rope(k, D, freqs=freqs, offset=offset)
+    assert torch.equal(turned, ops.rope(k.contiguous(), D, freqs=freqs, offset=offset))
+    theta = (torch.arange(L, device="cuda") + offset)[:, None] / freqs.double()
+    a, b = k.double().chunk(2, -1)
+    want = torch.cat([a * theta.cos() - b * theta.sin(), a * theta.sin() + b * theta.cos()], -1)
+    _within(turned, want, want.abs() * 2 ** -8 + 1e-5 * (1 + offset + L) ** 0.5)   # angles in fp32
+    cache, plain = KVCache(offset + L), KVCache(offset + L)
+    for c, kk, vv in ((cache, k, v), (plain, k.contiguous(), v.contiguous())):
+        c.update_and_fetch(torch.zeros((B, H, offset, D), device="cuda", dtype=torch.bfloat16),
+                           torch.zeros((B, H, offset, D), device="cuda", dtype=torch.bfloat16)) if offset else None
+        c.update_and_fetch(kk, vv)
+    assert torch.equal(cache.keys, plain.keys) and torch.equal(cache.values, plain.values)
+    assert torch.equal(cache.values[:, :, offset:offset + L], v)
