@@ -137,7 +137,12 @@ class Attention(nn.Module):
 
     def __call__(self, x, mask=None, cache=None):
         B, L, _ = x.shape
-        queries, keys, values = self.q_proj(x), self.k_proj(x), self.v_proj(x)
+        output = self.attend(self.q_proj(x), self.k_proj(x), self.v_proj(x), B, L, mask, cache)
+        # tensor parallel: o_proj holds a K slice; the ranks' partial sums meet in one all-reduce (tp.py)
+        return all_reduce_sum(self.o_proj(output), getattr(self, "tp", None))
+
+    def attend(self, queries, keys, values, B: int, L: int, mask, cache):
+        """Rotation, cache update and attention of projected rows [B, L, heads * D] -> [B, L, Hq * D]."""
         queries = queries.reshape(B, L, self.num_heads, -1).transpose(1, 2)
         keys = keys.reshape(B, L, self.n_kv_heads, -1).transpose(1, 2)
         values = values.reshape(B, L, self.n_kv_heads, -1).transpose(1, 2)
@@ -148,9 +153,7 @@ class Attention(nn.Module):
         else:
             queries, keys = self.rope(queries), self.rope(keys)
         output = scaled_dot_product_attention(queries, keys, values, cache=cache, scale=self.scale, mask=mask)
-        output = output.transpose(1, 2).reshape(B, L, -1)
-        # tensor parallel: o_proj holds a K slice; the ranks' partial sums meet in one all-reduce (tp.py)
-        return all_reduce_sum(self.o_proj(output), getattr(self, "tp", None))
+        return output.transpose(1, 2).reshape(B, L, -1)
 
 
 class MLP(nn.Module):
@@ -162,7 +165,10 @@ class MLP(nn.Module):
         self.up_proj = mk(args.hidden_size, args.intermediate_size)
 
     def __call__(self, x):
-        return all_reduce_sum(self.down_proj(ops.silu_mul(self.gate_proj(x), self.up_proj(x))), getattr(self, "tp", None))
+        act = nn.fused_rows(x, (self.gate_proj, self.up_proj), swiglu=True)
+        if act is None:
+            act = ops.silu_mul(self.gate_proj(x), self.up_proj(x))
+        return all_reduce_sum(self.down_proj(act), getattr(self, "tp", None))
 
 
 class TransformerBlock(nn.Module):
@@ -173,10 +179,35 @@ class TransformerBlock(nn.Module):
         self.post_attention_layernorm = nn.RMSNorm(args.hidden_size, eps=args.rms_norm_eps, device=device)
 
     def __call__(self, x, mask=None, cache=None):
+        y = self._few_rows(x, mask, cache)
+        if y is not None:
+            return y
         r = self.self_attn(self.input_layernorm(x), mask, cache)
         h = ops.add(x, r)
         r = self.mlp(self.post_attention_layernorm(h))
         return ops.add(h, r)
+
+    def _few_rows(self, x, mask, cache):
+        """Up to 32 rows on one GPU: norms, residual sums and SwiGLU ride in the four quantized matmuls (nn.fused_rows).  None
+        where they do not apply."""
+        at, mlp = self.self_attn, self.mlp
+        tp = getattr(at, "tp", None)
+        if type(at) is not Attention or type(mlp) is not MLP or (tp is not None and tp.on) or x.dim() != 3:
+            return None
+        qkv = nn.fused_rows(x, (at.q_proj, at.k_proj, at.v_proj), norm=self.input_layernorm)
+        if qkv is None:
+            return None
+        B, L, _ = x.shape
+        nq, nk = at.q_proj.weight.shape[0], at.k_proj.weight.shape[0]
+        out = at.attend(qkv[..., :nq], qkv[..., nq:nq + nk], qkv[..., nq + nk:], B, L, mask, cache)
+        h = nn.fused_rows(out, (at.o_proj,), residual=x)
+        if h is None:
+            h = ops.add(x, at.o_proj(out))
+        act = nn.fused_rows(h, (mlp.gate_proj, mlp.up_proj), norm=self.post_attention_layernorm, swiglu=True)
+        if act is None:
+            return ops.add(h, mlp(self.post_attention_layernorm(h)))
+        y = nn.fused_rows(act, (mlp.down_proj,), residual=h)
+        return ops.add(h, mlp.down_proj(act)) if y is None else y
 
 
 class LlamaModel(nn.Module):

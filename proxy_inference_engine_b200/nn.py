@@ -106,6 +106,42 @@ class QuantizedEmbedding(Module):
                                     group_size=self.group_size, bits=self.bits)
 
 
+def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
+    """Up to 32 rows through several bias-free QuantizedLinears in ONE launch, with the RMSNorm in front of them, and the
+    residual sum or SwiGLU behind them where asked for -- the arithmetic of the separate calls, rounding for rounding:
+        [..., sum N]  their outputs side by side;   residual: residual + output;   swiglu: silu(first) * second.
+    None where that kernel does not apply (the caller then makes the separate calls, which also report what is wrong)."""
+    K = x.shape[-1]
+    rows = x.numel() // K if K else 0
+    if not 0 < rows <= 32 or x.dtype != torch.bfloat16 or not x.is_contiguous() or x.data_ptr() % 16:
+        return None
+    bits, N = linears[0].bits, 0
+    if bits not in (4, 8) or K % (1024 // bits):
+        return None
+    for lin in linears:
+        w, s, b = lin.weight, lin.scales, lin.biases
+        if (type(lin) is not QuantizedLinear or "bias" in lin.__dict__ or lin.bits != bits or lin.group_size != 64
+                or w.dtype != torch.int32 or w.dim() != 2 or w.shape[1] * 32 != K * bits or s.dtype != torch.bfloat16
+                or b.dtype != torch.bfloat16 or s.shape != b.shape or s.shape != (w.shape[0], K // 64)
+                or not (w.is_contiguous() and s.is_contiguous() and b.is_contiguous())
+                or w.data_ptr() % 16 or s.data_ptr() % 8 or b.data_ptr() % 8):
+            return None
+        N += w.shape[0]
+    if swiglu:
+        if linears[0].weight.shape[0] != linears[1].weight.shape[0]:
+            return None
+        N //= 2
+    if norm is not None:
+        nw = norm.weight
+        if type(norm) is not RMSNorm or nw.dtype != torch.bfloat16 or nw.shape != (K,) or not nw.is_contiguous() or nw.data_ptr() % 16:
+            return None
+    if residual is not None and (residual.shape != x.shape[:-1] + (N,) or residual.dtype != torch.bfloat16
+                                 or not residual.is_contiguous()):
+        return None
+    return ops.qmv_fused(x, linears, rows, K, N, bits, None if norm is None else norm.weight, 0.0 if norm is None else norm.eps,
+                         residual, swiglu)
+
+
 class RMSNorm(Module):
     """nn.RMSNorm(dims, eps) (normalization.py:105-143)."""
 

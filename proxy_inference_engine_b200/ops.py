@@ -8,21 +8,28 @@ Every function is one or two calls into libpie_b200.so on the current CUDA strea
 from __future__ import annotations
 
 import ctypes as C
+import functools
 
 import torch
 
 from . import _lib
-from ._lib import KvLayout, KvqCache, QmvSeg
+from ._lib import EPI_RESADD, EPI_SILUMUL, EPI_STORE, KvLayout, KvqCache, QmvSeg
 
 _BF16 = torch.bfloat16
 
 
 def _p(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+@functools.lru_cache(maxsize=4096)
+def _qmv_workspace_bytes(M: int, N: int, K: int, bits: int, dual: int) -> int:
+    """A pure function of the sizes, asked for at every call."""
+    return _lib.load().pie_qmv_workspace_bytes(M, N, K, bits, dual, 0)
 
 
 def _as_words(w: torch.Tensor) -> torch.Tensor:
@@ -147,12 +154,26 @@ def quantized_matmul(x, w, scales, biases, transpose: bool = True, group_size: i
     M = x2.shape[0]
     y = torch.empty((M, N), dtype=_BF16, device=x.device)
     L = _lib.load()
-    nb = L.pie_qmv_workspace_bytes(min(M, 32) if M else 1, N, K, bits, 0, 0) if bits in (4, 8) and group_size == 64 else 0
+    nb = _qmv_workspace_bytes(min(M, 32) if M else 1, N, K, bits, 0) if bits in (4, 8) and group_size == 64 else 0
     ws = workspaces.get("qmv", nb, x.device)
     fn = L.pie_qmv if M <= 32 else L.pie_qmm
     _lib.check(fn(_p(y), _p(x2), _p(w), _p(scales), _p(biases), M, N, K, group_size, bits, _p(ws), ws.numel(),
                   _stream()), "quantized_matmul")
     return y.reshape(x.shape[:-1] + (N,))
+
+
+def qmv_fused(x, linears, rows: int, K: int, N: int, bits: int, norm_weight, eps: float, residual, swiglu: bool):
+    """pie_qmv_fused on operands nn.fused_rows has checked.  N: output columns."""
+    L = _lib.load()
+    segs = (QmvSeg * len(linears))()
+    for seg, lin in zip(segs, linears):
+        seg.wq, seg.scales, seg.biases, seg.N = lin.weight.data_ptr(), lin.scales.data_ptr(), lin.biases.data_ptr(), lin.weight.shape[0]
+    out = torch.empty(x.shape[:-1] + (N,), dtype=_BF16, device=x.device)
+    ws = workspaces.get("qmv", _qmv_workspace_bytes(rows, N, K, bits, int(swiglu)), x.device)
+    _lib.check(L.pie_qmv_fused(_p(out), N, _p(x), K, rows, K, segs, len(linears), 64, bits, _p(norm_weight), float(eps),
+                               EPI_SILUMUL if swiglu else EPI_STORE if residual is None else EPI_RESADD, _p(residual), 0, _p(ws),
+                               ws.numel(), 0, _stream()), "qmv_fused")
+    return out
 
 
 def rms_norm(x, weight, eps: float):
