@@ -1,13 +1,14 @@
 // Dense linear layers y = x W^T (+ bias) over unquantized weights, with the epilogues of pie_b200_hybrid.h.
 //
-// Three kernels behind pieh_linear:
-//   * linear_rows_kernel  (M <= 32: decode): a CTA streams 1, 2 or 4 weight rows once with 16-byte loads, its warps cutting K
-//     between them, one fp32 accumulator per (activation row, weight row) -- bound by the weight bytes;
-//   * linear_umma_kernel  (bf16 x bf16, M > 32, K % 64 == 0: prefill): tcgen05.mma with the fp32 accumulator in
-//     tensor memory, both operands brought into 128B-swizzled K-major shared memory by cp.async (hyb_umma.cu);
+// Kernels behind pieh_linear:
+//   * linear_rows_mma_kernel (bf16 x bf16, M <= 32: decode): a CTA streams 16 output rows of the matrix once, straight into
+//     mma.sync operands -- bound by the weight bytes;
+//   * linear_rows_kernel  (M <= 32, everything else; grouped products of few slots): a CTA streams 1, 2 or 4 weight rows once with
+//     16-byte loads, its warps cutting K between them, one fp32 accumulator per (activation row, weight row);
+//   * the tcgen05 kernels of hyb_umma.cu (bf16 x bf16, M > 32, K % 64 == 0: prefill);
 //   * linear_tile_kernel  (everything else, and every fp32 product): 64 x 64 tiles, fp32 multiply-add on the CUDA cores.
-// With bf16 weights the activation is rounded to bf16 first, so the three agree up to the order of the fp32 sums.
-#include "hyb_common.cuh"
+// With bf16 weights the activation is rounded to bf16 first, so they agree up to the order of the fp32 sums.
+#include "hyb_mma.cuh"
 
 namespace pieh {
 
@@ -200,6 +201,80 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const LinArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------------------------------
+// bf16 x bf16, M <= 8 NT rows.  A CTA owns 16 output rows; its 8 warps take 64 elements of K in turn.  The weights are the
+// mma.sync m16n8k16 A operand and go from global memory into it directly: which k of a 16-wide step an operand register holds
+// does not matter as long as both operands agree, so a lane loads 8 CONSECUTIVE k of rows g and g + 8 (16 bytes each) and of its
+// activation row, and feeds two MMAs from them.  The tensor core does the sum over k that linear_rows_kernel does with shuffles
+// (16 values x 5 shuffles for every 16 KB of weights at four rows), so a warp keeps eight 16-byte weight loads in flight and
+// little else.  The warps' partial tiles meet in shared memory in warp order.  Four rows, us (GB/s): 28672 x 4096 61.6 (3810) -> 40.9
+// (5750); 4096 x 14336 31 -> 24.6 (4780); 16 rows: 57.6 and 33.3; 32 rows: 92 and 55 (x comes from L2 once per 16 outputs).
+__device__ __forceinline__ uint4 load_stream16(const __nv_bfloat16* p) {   // read once: past L1
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+template <typename OT, int NT>
+__global__ void __launch_bounds__(256) linear_rows_mma_kernel(const LinArgs a) {
+  __shared__ float part[8][16][8 * NT + 1];
+  pdl_sync();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, n0 = blockIdx.x * 16;
+  const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(a.x) + (size_t)blockIdx.z * a.x_bs;
+  const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(a.w) + (size_t)blockIdx.z * a.w_bs;
+  const __nv_bfloat16* w0 = w + (size_t)min(n0 + g, a.N - 1) * a.K;
+  const __nv_bfloat16* w1 = w + (size_t)min(n0 + g + 8, a.N - 1) * a.K;
+  float acc[NT][4];
+#pragma unroll
+  for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+#pragma unroll(NT == 1 ? 4 : 2)
+  for (int kb = warp * 64; kb < a.K; kb += 512) {
+    uint4 wa[2], wb[2], xv[2][NT];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = kb + 32 * h + 8 * t;
+      const bool in = k < a.K;   // K is a multiple of 8: the piece exists or it does not
+      const uint4 zero = make_uint4(0, 0, 0, 0);
+      wa[h] = in ? load_stream16(w0 + k) : zero;
+      wb[h] = in ? load_stream16(w1 + k) : zero;
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+        xv[h][i] = in && 8 * i + g < a.M ? *reinterpret_cast<const uint4*>(x + (size_t)(8 * i + g) * a.x_ld + k) : zero;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        mma_16816(acc[i], wa[h].x, wb[h].x, wa[h].y, wb[h].y, xv[h][i].x, xv[h][i].y);
+        mma_16816(acc[i], wa[h].z, wb[h].z, wa[h].w, wb[h].w, xv[h][i].z, xv[h][i].w);
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < NT; ++i) {
+    part[warp][g][8 * i + 2 * t] = acc[i][0];
+    part[warp][g][8 * i + 2 * t + 1] = acc[i][1];
+    part[warp][g + 8][8 * i + 2 * t] = acc[i][2];
+    part[warp][g + 8][8 * i + 2 * t + 1] = acc[i][3];
+  }
+  __syncthreads();
+  auto sum = [&](int r, int m) {
+    float y = 0.f;
+#pragma unroll
+    for (int wp = 0; wp < 8; ++wp) y += part[wp][r][m];
+    return y;
+  };
+  if (a.epi == PIEH_EPI_GLU) {   // rows (2 r, 2 r + 1) are a (gate, linear) pair
+    for (int e = threadIdx.x; e < 8 * a.M; e += 256) {
+      const int m = e >> 3, r = 2 * (e & 7);
+      if (n0 + r + 1 < a.N) lin_store_glu<OT>(a, m, n0 + r, sum(r, m), sum(r + 1, m));
+    }
+    return;
+  }
+  for (int e = threadIdx.x; e < 16 * a.M; e += 256) {
+    const int m = e >> 4, r = e & 15;
+    if (n0 + r < a.N) lin_store<OT>(a, m, n0 + r, sum(r, m));
+  }
+}
+
+// ------------------------------------------------------------------------------------------------------------------
 // Many rows, few outputs (N <= NMAX <= 32; a router): a warp per activation row, its lanes cutting K in 8-element
 // pieces; the whole weight matrix is a few tens of KB and stays in L1 / L2, so the kernel reads x once -- the tensor-core
 // tiles would spend a 256-column tile on a handful of columns.
@@ -240,6 +315,15 @@ __global__ void __launch_bounds__(256) linear_skinny_kernel(const LinArgs a) {
   }
 }
 
+template <typename OT>
+static cudaError_t launch_rows_mma(const LinArgs& a, cudaStream_t st) {
+  const dim3 grid((unsigned)((a.N + 15) / 16), 1, (unsigned)a.nb);
+  count_launch();
+  if (a.M <= 8) return launch_k(linear_rows_mma_kernel<OT, 1>, grid, dim3(256), 0, st, a);
+  if (a.M <= 16) return launch_k(linear_rows_mma_kernel<OT, 2>, grid, dim3(256), 0, st, a);
+  return launch_k(linear_rows_mma_kernel<OT, 4>, grid, dim3(256), 0, st, a);
+}
+
 template <typename XT, typename WT, typename OT>
 static cudaError_t launch_typed(const LinArgs& a, cudaStream_t st) {
   const bool vec_ok = a.K % 8 == 0 && a.x_ld % 8 == 0 && (reinterpret_cast<uintptr_t>(a.x) & 31) == 0 &&
@@ -264,16 +348,18 @@ static cudaError_t launch_typed(const LinArgs& a, cudaStream_t st) {
       const dim3 grid((a.N + 63) / 64, a.M / 64 + (int)a.S);   // S carries the expert count here: the tile list's bound
       e = launch_k(linear_tile_kernel<XT, WT, OT>, grid, dim3(256), 0, st, t);
     }
-  } else if (a.M <= 32 && vec_ok) {
-    // rows per CTA: enough to amortise the activation loads, few enough that every SM still gets several CTAs
-    const bool wide = (long long)a.N * a.nb >= 4 * 4 * num_sms() || a.epi == PIEH_EPI_GLU;   // a gated pair needs an even row count
+  } else if (sizeof(XT) == 4 && a.M <= 32 && vec_ok) {
+    if constexpr (sizeof(XT) == 4) {   // bf16 activations go to launch_rows_mma
+      // rows per CTA: enough to amortise the activation loads, few enough that every SM still gets several CTAs
+      const bool wide = (long long)a.N * a.nb >= 4 * 4 * num_sms() || a.epi == PIEH_EPI_GLU;   // a gated pair needs an even row count
 #define PIEH_ROWS(MR, R) e = launch_k(linear_rows_kernel<XT, WT, OT, MR, R>, dim3((a.N + R - 1) / R, 1, nb), dim3(256), 0, st, a)
-    if (a.M <= 1) { if (wide) PIEH_ROWS(1, 2); else PIEH_ROWS(1, 1); }
-    else if (a.M <= 4) { if (wide) PIEH_ROWS(4, 4); else PIEH_ROWS(4, 2); }
-    else if (a.M <= 8) { if (wide) PIEH_ROWS(8, 4); else PIEH_ROWS(8, 2); }
-    else if (a.M <= 16) PIEH_ROWS(16, 2);
-    else PIEH_ROWS(32, 2);
+      if (a.M <= 1) { if (wide) PIEH_ROWS(1, 2); else PIEH_ROWS(1, 1); }
+      else if (a.M <= 4) { if (wide) PIEH_ROWS(4, 4); else PIEH_ROWS(4, 2); }
+      else if (a.M <= 8) { if (wide) PIEH_ROWS(8, 4); else PIEH_ROWS(8, 2); }
+      else if (a.M <= 16) PIEH_ROWS(16, 2);
+      else PIEH_ROWS(32, 2);
 #undef PIEH_ROWS
+    }
   } else {
     const dim3 grid((a.N + 63) / 64, (a.M + 63) / 64, nb);
     e = launch_k(linear_tile_kernel<XT, WT, OT>, grid, dim3(256), 0, st, a);
@@ -326,7 +412,10 @@ int run_linear(const LinArgs& a, int out_dtype, int x_dtype, int w_dtype, cudaSt
   }
   typedef __nv_bfloat16 bf;
   cudaError_t e;
-  if (w_dtype == PIE_DTYPE_F32) {
+  if (!a.g_tiles && a.M <= 32 && x_dtype == PIE_DTYPE_BF16 && w_dtype == PIE_DTYPE_BF16 && a.K % 8 == 0 && a.x_ld % 8 == 0 &&
+      a.x_bs % 8 == 0 && a.w_bs % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) & 15) == 0) {
+    e = out_dtype == PIE_DTYPE_F32 ? launch_rows_mma<float>(a, st) : launch_rows_mma<bf>(a, st);
+  } else if (w_dtype == PIE_DTYPE_F32) {
     e = out_dtype == PIE_DTYPE_F32 ? launch_typed<float, float, float>(a, st) : launch_typed<float, float, bf>(a, st);
   } else if (x_dtype == PIE_DTYPE_F32) {
     e = out_dtype == PIE_DTYPE_F32 ? launch_typed<float, bf, float>(a, st) : launch_typed<float, bf, bf>(a, st);

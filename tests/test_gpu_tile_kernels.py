@@ -168,3 +168,25 @@ def test_rope_and_cache_write_of_strided_heads(D, B, L, offset):
         c.update_and_fetch(kk, vv)
     assert torch.equal(cache.keys, plain.keys) and torch.equal(cache.values, plain.values)
     assert torch.equal(cache.values[:, :, offset:offset + L], v)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 16, 8), (4, 17, 72), (8, 300, 520), (9, 40, 1000), (32, 130, 2048)])
+def test_dense_matmul_of_few_rows(M, N, K):
+    """bf16 activations and weights, up to 32 rows (linear_rows_mma_kernel), plain and gated-pair epilogues."""
+    from proxy_inference_engine_b200 import _lib
+    L = _lib.load_hybrid(build_if_missing=True)
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn((M, K + 8), generator=g, device="cuda").to(torch.bfloat16)[:, :K]     # rows further apart than they are long
+    w = torch.randn((N, K), generator=g, device="cuda").to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    slack = (x.double().abs() @ w.double().abs().t()) * (K * 2 ** -23)
+    for dt, code, rel in ((torch.float32, 1, 0.0), (torch.bfloat16, 0, 2 ** -8)):
+        out = torch.full((M, N), float("nan"), device="cuda", dtype=dt)
+        assert L.pieh_linear(_p(out), code, N, _p(x), 0, K + 8, _p(w), 0, None, M, N, K, 0, 0.0, None, None, 0, None) == 0
+        _within(out, want, slack + want.abs() * rel)
+    if N % 2 == 0:
+        out = torch.full((M, N // 2), float("nan"), device="cuda")
+        assert L.pieh_linear_glu(_p(out), 1, N // 2, _p(x), 0, K + 8, _p(w), 0, M, N, K, 1.0, 0.0, 0.0, None) == 0
+        gate, up = want[:, 0::2], want[:, 1::2]
+        silu = gate * torch.sigmoid(gate)
+        _within(out, silu * up, 1.1 * up.abs() * slack[:, 0::2] + silu.abs() * slack[:, 1::2] + (silu * up).abs() * 2 ** -20)
