@@ -319,21 +319,11 @@ static cudaError_t launch_grouped(const LinArgs& a, cudaStream_t st) {
 template <typename OT>
 static cudaError_t launch_dense(const LinArgs& a, cudaStream_t st) {
   pie::GemmArgs g = {};
-  g.M = a.M; g.N = a.N; g.K = a.K; g.nb = a.nb; g.group_m = 8;
-  CUtensorMap mx, mw;
-  // a stride of zero: one operand for all products
-  g.zx = a.x_bs != 0; g.zw = a.w_bs != 0;
-  if (!pie::gemm_map(&mx, a.x, 2, a.K, a.M, a.x_ld * 2, g.zx ? a.nb : 1, a.x_bs * 2, 128) ||
-      !pie::gemm_map(&mw, a.w, 2, a.K, a.N, (long long)a.K * 2, g.zw ? a.nb : 1, a.w_bs * 2, 128))
-    return cudaErrorNotSupported;
+  g.M = a.M; g.N = a.N; g.K = a.K; g.nb = a.nb;
+  g.zx = a.x_bs != 0; g.zw = a.w_bs != 0;   // a stride of zero: one operand for all products
   const DenseEpi<OT> epi = {a};
-  const int sms = num_sms();
-  const pie::GemmChoice c = pie::gemm_choose(a.M, a.N, a.K, a.nb, sms, 560, 300);
   count_launch();
-  g.mt = c.mt; g.nt = c.nt; g.k_per = c.k_per;
-  if (c.pair) return pie::gemm_launch<2, 256, 0, false>(mx, mw, g, epi, 1, sms, st);
-  if (c.ranks == 1) return pie::gemm_launch<1, 128, 0, false>(mx, mw, g, epi, 1, sms, st);
-  return pie::gemm_launch<1, 128, 0, true>(mx, mw, g, epi, c.ranks, sms, st);
+  return pie::gemm_run<0>(g, epi, a.x, a.x_ld * 2, a.x_bs * 2, a.w, a.w_bs * 2, num_sms(), st);
 }
 
 cudaError_t launch_linear_umma(const LinArgs& a, int out_dtype, cudaStream_t st) {

@@ -2,7 +2,7 @@
 // by the prefill quantized GEMM (pie_qmm.cu: w is dequantised into shared memory on the way) and the dense linear of the
 // hybrid families (hyb_umma.cu: w arrives by TMA).  What bounds it is the tensor pipe; the shape of the kernel follows from
 // keeping that pipe fed:
-//   * CG = 2: a CTA pair (two SMs) owns a 256 x 256 tile, cta_group::2.  Each CTA stages 128 rows of x and HALF of the w rows
+//   * CG = 2: a CTA pair (two SMs) owns a 256 x BN tile (BN = 256, or less where fewer columns fill the last wave better).  Each CTA stages 128 rows of x and HALF of the w rows
 //     (128), so a 64-element K step moves 32 KB into each SM for 512 tensor-pipe cycles (64 B / cycle of shared-memory reads
 //     and 64 of writes, the 128 the SM has); a 128 x 256 tile of one CTA would need 192.
 //   * CG = 1: one CTA owns a 128 x BN tile: few rows or few tiles, where the pair would leave SMs idle.  SPLIT cuts K over the
@@ -48,6 +48,11 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
 }
 __device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
+}
+__device__ __forceinline__ bool elect_one() {   // one lane of the (converged) warp
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
 }
 constexpr uint32_t kGemmWaitLimit = 1u << 22;
 // false: the wait expired here or the CTA is already leaving
@@ -129,9 +134,10 @@ struct GemmTile {
   static constexpr int GROUPS = 3;                                // dequantising groups of four warps, a K step each in turn
   static constexpr int THREADS = 32 * (QB ? W_DEQ + 4 * GROUPS : EPI_WARPS + 4);
   static constexpr int SMEM = 1024 + S * (A_STAGE + B_STAGE) + RING * CHUNK;
-  static constexpr int TMEM_COLS = 2 * BN;
-  static_assert(SMEM <= 227 * 1024 && TMEM_COLS <= 512 && BN % 32 == 0, "tile");
-  static_assert(!QB || NB == 128, "the dequantising threads are laid out for 128 rows");
+  static constexpr int ACC = BN > 128 ? 256 : 128;              // columns between the two accumulators
+  static constexpr int TMEM_COLS = 2 * ACC;                      // a power of two
+  static_assert(SMEM <= 227 * 1024 && TMEM_COLS <= 512 && BN % (8 * EPI_WARPS) == 0 && NB % 8 == 0, "tile");
+  static_assert(!QB || NB <= 128, "a dequantising thread per row, 128 threads a group");
   static_assert(!(SPLIT && CG == 2), "K is split over single CTAs");
 };
 
@@ -242,7 +248,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
 #pragma unroll 1
         for (int c = 0; c < RUNS; ++c) {
           uint32_t v[32];
-          tmem_ld32(tmem + (uint32_t)(b * BN + (c_lo + c) * 32) + ((uint32_t)(quad * 32) << 16), v);
+          tmem_ld32(tmem + (uint32_t)(b * T::ACC + (c_lo + c) * 32) + ((uint32_t)(quad * 32) << 16), v);
           if (c == RUNS - 1) {   // the accumulator may be overwritten
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -280,26 +286,31 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     }
   } else if (warp == T::W_MMA) {
     // ---------------------------------------------------------------- MMA issue
+    // The loop's own instructions are on the critical path (a step of four MMAs is 250 to 500 cycles): the whole warp runs it,
+    // so that addresses and descriptors stay warp-uniform, one elected lane issues, and nothing in it brings the lanes together
+    // but the election.  (A lane's own loop with a vote per wait: 8192 x 4096 x 4096, 4 bits, 223 us; this one 197.)
     if (rank == lead) {
-      int it = 0, i = 0;
-      bool alive = true;
-      for (int t = first_tile; t < ntiles && alive; t += tile_step, ++i) {
+      const uint32_t acc = __shfl_sync(0xffffffffu, tmem, 0);
+      const uint64_t da0 = umma_desc_sw128(smA), db0 = umma_desc_sw128(smB);
+      int i = 0, s = 0;
+      uint32_t ph = 0;
+      bool alive = true;   // a lane's own: a wait that expires (and every one after it) only keeps the elected lane from issuing
+      for (int t = first_tile; t < ntiles; t += tile_step, ++i) {
         const int b = i & 1;
-        alive = gemm_wait_warp(smem_u32(&tempty_bar[b]), ((i >> 1) & 1) ^ 1, abortp);
+        alive &= gemm_wait(smem_u32(&tempty_bar[b]), ((i >> 1) & 1) ^ 1, abortp);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int kb = k_lo; kb < k_hi && alive; ++kb, ++it) {
-          const int s = it % S;
-          if (!(alive = gemm_wait_warp(smem_u32(&full_bar[s]), (it / S) & 1, abortp))) break;
+        for (int kb = k_lo; kb < k_hi; ++kb) {
+          alive &= gemm_wait(smem_u32(&full_bar[s]), ph, abortp);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (lane == 0) {
-            const uint64_t da = umma_desc_sw128(smA + s * T::A_STAGE), db = umma_desc_sw128(smB + s * T::B_STAGE);
+          const uint64_t da = da0 + (uint64_t)(s * (T::A_STAGE >> 4)), db = db0 + (uint64_t)(s * (T::B_STAGE >> 4));
+          if (elect_one() && alive) {
 #pragma unroll
             for (int k4 = 0; k4 < 4; ++k4)   // 16 elements of K: 32 bytes inside the swizzle atom
-              gemm_mma<CG>(tmem + b * BN, da + 2 * k4, db + 2 * k4, IDESC, (kb > k_lo || k4 > 0) ? 1u : 0u);
+              gemm_mma<CG>(acc + b * T::ACC, da + 2 * k4, db + 2 * k4, IDESC, (kb > k_lo || k4 > 0) ? 1u : 0u);
             gemm_commit<CG>(smem_u32(&empty_bar[s]));
             if (kb == k_hi - 1) gemm_commit<CG>(smem_u32(&tfull_bar[b]));
           }
-          __syncwarp();
+          if (++s == S) { s = 0; ph ^= 1; }
         }
         if (SPLIT) break;
       }
@@ -332,7 +343,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     bool alive = true;
     for (int t = first_tile; t < ntiles && alive; t += tile_step, it0 += k_hi - k_lo, pc0 += chunks) {
       const GemmTileAt at = gemm_tile_at(a, t);
-      const int row = min(at.n * BN + (int)(CG == 2 ? rank : 0) * T::NB + r, a.N - 1);
+      const int row = min(at.n * BN + (int)(CG == 2 ? rank : 0) * T::NB + min(r, T::NB - 1), a.N - 1);
       const uint16_t* sp = a.scales + (size_t)row * nk_all;
       const uint16_t* bp = a.biases + (size_t)row * nk_all;
       int kb = k_lo + (grp + T::GROUPS - it0 % T::GROUPS) % T::GROUPS;
@@ -369,12 +380,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
           if (kb + T::GROUPS < k_hi) { s_next = __ldg(sp + kb + T::GROUPS); b_next = __ldg(bp + kb + T::GROUPS); }
         }
         if (!(alive = gemm_wait_warp(smem_u32(&pfull_bar[p]), (pc / RING) & 1, abortp))) break;
-        const uint32_t src = smP + p * T::CHUNK + r * 128, dst = smB + s * T::B_STAGE + r * 128;
+        const uint32_t src = smP + p * T::CHUNK + min(r, T::NB - 1) * 128, dst = smB + s * T::B_STAGE + r * 128;
         uint4 w[QB == 4 ? 2 : 4];
 #pragma unroll
         for (int c = 0; c < QB / 2; ++c) w[c] = lds128(src + (((uint32_t)(QB / 2 * j + c) ^ swz) << 4));
         if (!(alive = gemm_wait_warp(smem_u32(&empty_bar[s]), ((it / S) & 1) ^ 1, abortp))) break;
-        if (QB == 4) {
+        if (T::NB < 128 && r >= T::NB) {
+          // (no row of this tile: the thread only keeps the warp's count)
+        } else if (QB == 4) {
           const uint32_t s2 = sc | (sc << 16), b2 = bi | (bi << 16);
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
@@ -489,20 +502,32 @@ inline bool gemm_map(CUtensorMap* m, const void* p, int elem_bytes, long long in
 // Measured, B200, 4-bit weights, us (TFLOP/s) with the 256 x 256 tile of one CTA, cp.async producers and no overlap of the
 // epilogue that this replaced -> here: 8192 x 14336 x 4096 1590 (605) -> 785 (1226); 1000 rows 290 -> 122; 256 rows -> 40; 77 rows
 // 400 -> 34; 77 x 4096 x 14336 720 -> 35 (four ranks).  bf16 weights: 8192 x 28672 x 4096 -> 1370 (1404).
-// The tile for a shape: the pair's 256 x 256, or a single CTA's 128 x 128 with K over 1..4 ranks of a cluster, whichever the
-// estimate (waves x K steps x SM cycles of a step, and the fixed costs of a wave) says is done first.
-struct GemmChoice { int pair, ranks, k_per, mt, nt; };
-inline GemmChoice gemm_choose(int M, int N, int K, int nb, int sms, double pair_step, double single_step) {
+// The tile for a shape: a pair's 256 x {256, 224, 192, 128}, or a single CTA's 128 x 128 with K over 1..4 ranks of a cluster --
+// whichever the estimate (waves x K steps x SM cycles of a step, and the fixed cost of a cluster's reduction) says is done first.
+// The steps' cycles are measured (1.9 GHz; waves x 64 steps of N 14336, M 1000): pairs with bf16 weights 720 / 612 / 575 for BN = 256 /
+// 192 / 128, dequantised 770 / 765 / 680 / 630 for 256 / 224 / 192 / 128, single CTAs 580 and 650.  Over 190 shapes (M 77 to 3000) the
+// choice takes 1.02 times the best tile's time on average.
+struct GemmChoice { int pair, bn, ranks, k_per, mt, nt; };
+inline GemmChoice gemm_choose(int M, int N, int K, int nb, int sms, bool quant) {
   auto up = [](long long a, long long b) { return (a + b - 1) / b; };
-  const long long nk = K / 64, pair_tiles = up(M, 256) * up(N, 256) * nb, tiles = up(M, 128) * up(N, 128) * nb;
-  GemmChoice best = {1, 1, (int)nk, (int)up(M, 256), (int)up(N, 256)};
-  double cost = (double)up(pair_tiles, sms / 2) * nk * pair_step + 2500;
+  const long long nk = K / 64;
+  GemmChoice best = {1, 256, 1, (int)nk, (int)up(M, 256), (int)up(N, 256)};
+  double cost = 1e30;
+  for (int bn : {256, 224, 192, 128}) {
+    if (bn == 224 && !quant) continue;   // (the eight epilogue warps of the dense kernel share 64-column runs)
+    const long long tiles = up(M, 256) * up(N, bn) * nb;
+    const double c = (double)up(tiles, sms / 2) * nk * (quant ? 490 + 280 * bn / 256.0 : 430 + 290 * bn / 256.0);
+    if (c < cost) { cost = c; best = {1, bn, 1, (int)nk, (int)up(M, 256), (int)up(N, bn)}; }
+  }
+  const long long tiles = up(M, 128) * up(N, 128) * nb;
+  const double step = quant ? 650 : 580;
   for (int r = 1; r <= 4; ++r) {
     const long long per = up(up(nk, r), 8) * 8;     // ranks start on 16-byte runs of the scales and on whole packed chunks
     if (up(nk, per) != r || tiles > 65535) continue;
-    const long long waves = up(tiles * r, sms);
-    const double c = r == 1 ? (double)waves * nk * single_step + 2500 : (double)waves * (per * single_step + 5000);
-    if (c < cost) { cost = c; best = {0, r, (int)per, (int)up(M, 128), (int)up(N, 128)}; }
+    // clusters of three or four do not fill every SM: what is resident at once was 128 CTAs and more for four, not 144 for three
+    const long long slots = r == 3 ? sms * 3 / 4 : r == 4 ? sms * 7 / 8 : sms;
+    const double c = (double)up(tiles * r, slots) * (per * step + (r > 1 ? 4500 : 0));
+    if (c < cost) { cost = c; best = {0, 128, r, (int)per, (int)up(M, 128), (int)up(N, 128)}; }
   }
   return best;
 }
@@ -533,6 +558,26 @@ cudaError_t gemm_launch(const CUtensorMap& mx, const CUtensorMap& mw, const Gemm
   cfg.attrs = attr;
   cfg.numAttrs = CG == 2 || SPLIT ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, mx, mw, a, epi);
+}
+
+// One product (or nb of them): picks the tile, describes the operands and launches.  w_inner / w_pitch in bytes: a row of w as it
+// lies (packed words for QB).
+template <int QB, class Epi>
+cudaError_t gemm_run(GemmArgs a, const Epi& epi, const void* x, long long x_pitch, long long x_bpitch, const void* w,
+                     long long w_bpitch, int sms, cudaStream_t st) {
+  GemmChoice c = gemm_choose(a.M, a.N, a.K, a.nb, sms, QB != 0);
+  a.mt = c.mt; a.nt = c.nt; a.k_per = c.k_per; a.group_m = 8;
+  const long long w_row = QB ? (long long)a.K * QB / 8 : (long long)a.K * 2;
+  CUtensorMap mx, mw;
+  if (!gemm_map(&mx, x, 2, a.K, a.M, x_pitch, a.zx ? a.nb : 1, x_bpitch, 128) ||
+      !gemm_map(&mw, w, QB ? 1 : 2, QB ? w_row : a.K, a.N, w_row, a.zw ? a.nb : 1, w_bpitch, c.pair ? c.bn / 2 : c.bn))
+    return cudaErrorNotSupported;
+  if (!c.pair)
+    return c.ranks == 1 ? gemm_launch<1, 128, QB, false>(mx, mw, a, epi, 1, sms, st) : gemm_launch<1, 128, QB, true>(mx, mw, a, epi, c.ranks, sms, st);
+  if (c.bn == 256) return gemm_launch<2, 256, QB, false>(mx, mw, a, epi, 1, sms, st);
+  if constexpr (QB != 0)
+    if (c.bn == 224) return gemm_launch<2, 224, QB, false>(mx, mw, a, epi, 1, sms, st);
+  return c.bn == 192 ? gemm_launch<2, 192, QB, false>(mx, mw, a, epi, 1, sms, st) : gemm_launch<2, 128, QB, false>(mx, mw, a, epi, 1, sms, st);
 }
 
 }  // namespace pie

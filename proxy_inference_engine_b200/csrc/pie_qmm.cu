@@ -36,29 +36,16 @@ struct QmmStore {
   }
 };
 
-template <int QB>
-static cudaError_t launch_bits(const CUtensorMap& mx, const CUtensorMap& mw, GemmArgs& a, const QmmStore& epi, cudaStream_t st) {
-  const int sms = num_sms();
-  GemmChoice c = gemm_choose(a.M, a.N, a.K, 1, sms, 900, 870);
-  a.mt = c.mt; a.nt = c.nt; a.k_per = c.k_per;
-  if (c.pair) return gemm_launch<2, 256, QB, false>(mx, mw, a, epi, 1, sms, st);
-  if (c.ranks == 1) return gemm_launch<1, 128, QB, false>(mx, mw, a, epi, 1, sms, st);
-  return gemm_launch<1, 128, QB, true>(mx, mw, a, epi, c.ranks, sms, st);
-}
-
 cudaError_t launch_qmm_tc(uint16_t* y, const uint16_t* x, const uint32_t* wq, const uint16_t* s, const uint16_t* b,
                           int M, int N, int K, int bits, cudaStream_t st) {
   GemmArgs a = {};
-  a.M = M; a.N = N; a.K = K; a.nb = 1; a.group_m = 8;
+  a.M = M; a.N = N; a.K = K; a.nb = 1;
   a.scales = s; a.biases = b;
   a.scale_vec = K % 512 == 0 && ((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
-  CUtensorMap mx, mw;
-  if (!gemm_map(&mx, x, 2, K, M, (long long)K * 2, 1, 0, 128) ||
-      !gemm_map(&mw, wq, 1, (long long)K * bits / 8, N, (long long)K * bits / 8, 1, 0, 128))
-    return cudaErrorNotSupported;
   const QmmStore epi = {y, M, N};
   count_launch();
-  return bits == 4 ? launch_bits<4>(mx, mw, a, epi, st) : launch_bits<8>(mx, mw, a, epi, st);
+  return bits == 4 ? gemm_run<4>(a, epi, x, (long long)K * 2, 0, wq, 0, num_sms(), st)
+                   : gemm_run<8>(a, epi, x, (long long)K * 2, 0, wq, 0, num_sms(), st);
 }
 
 unsigned int qmm_pipeline_error() {

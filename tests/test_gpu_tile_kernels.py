@@ -26,7 +26,10 @@ def _within(got, want, slack):
                                    (70, 640, 14336),      # K over four ranks of a cluster
                                    (200, 1024, 1152),     # a last rank with fewer steps
                                    (513, 4100, 640),      # more tiles than one wave of single CTAs
-                                   (2050, 2056, 1024)])   # CTA pairs, ragged both ways, several tiles a pair
+                                   (2050, 2056, 1024),    # CTA pairs, ragged both ways, several tiles a pair
+                                   (1000, 14336, 128),    # pairs of 224 columns
+                                   (1500, 2100, 1024),    # pairs of 192
+                                   (400, 3000, 256)])     # pairs of 128
 def test_quantized_gemm_tiles(bits, M, N, K):
     from proxy_inference_engine_b200 import _lib, ops
     g = torch.Generator(device="cuda").manual_seed(M + N + K + bits)
@@ -43,7 +46,8 @@ def test_quantized_gemm_tiles(bits, M, N, K):
     assert _lib.load().pie_pipeline_error() == 0
 
 
-@pytest.mark.parametrize("M,N,K", [(33, 64, 64), (129, 257, 128), (70, 640, 8192), (200, 1024, 1152), (513, 4100, 192), (2050, 2056, 512)])
+@pytest.mark.parametrize("M,N,K", [(33, 64, 64), (129, 257, 128), (70, 640, 8192), (200, 1024, 1152), (513, 4100, 192), (2050, 2056, 512), (1200, 8192, 128),
+                                   (700, 3000, 128)])
 def test_dense_gemm_tiles(M, N, K):
     from proxy_inference_engine_b200 import _lib
     L = _lib.load_hybrid(build_if_missing=True)
