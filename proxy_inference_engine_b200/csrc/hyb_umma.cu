@@ -35,138 +35,187 @@ __device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity, vol
   return true;
 }
 
-// x_u <- sum_s mix[s, u] x_s + outw[u] (y + bias) over the S residual streams of one row, 32 columns.  Columns are read in
-// batches before any is written back: the loads of a batch are in flight together.
-template <int S>
-__device__ __forceinline__ void streams_run(const LinArgs& a, int m, int n0, const uint32_t (&v)[32]) {
-  constexpr int NB = S <= 2 ? 4 : 2;   // batch: 16 columns, 8 for four streams
-  float* xs = reinterpret_cast<float*>(a.out) + (size_t)m * S * a.N;
-#pragma unroll
-  for (int q0 = 0; q0 < 8; q0 += NB) {
-    float4 old[NB][S];
-#pragma unroll
-    for (int j = 0; j < NB; ++j)
-#pragma unroll
-      for (int s = 0; s < S; ++s) old[j][s] = *reinterpret_cast<const float4*>(xs + (size_t)s * a.N + n0 + 4 * (q0 + j));
-#pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      const int n = n0 + 4 * (q0 + j);
-      float y[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) y[e] = __uint_as_float(v[4 * (q0 + j) + e]) + (a.bias ? a.bias[n + e] : 0.f);
-#pragma unroll
-      for (int u = 0; u < S; ++u) {
-        const float ow = a.outw[u];
-        float4 acc = make_float4(ow * y[0], ow * y[1], ow * y[2], ow * y[3]);
-#pragma unroll
-        for (int s = 0; s < S; ++s) {
-          const float mx = a.mix[s * S + u];
-          acc.x = fmaf(mx, old[j][s].x, acc.x); acc.y = fmaf(mx, old[j][s].y, acc.y);
-          acc.z = fmaf(mx, old[j][s].z, acc.z); acc.w = fmaf(mx, old[j][s].w, acc.w);
-        }
-        *reinterpret_cast<float4*>(xs + (size_t)u * a.N + n) = acc;
-      }
-    }
-  }
-}
 // any number of streams up to 8, any alignment, the edge of the matrix: a column at a time
-__device__ __noinline__ void streams_any(const LinArgs& a, int m, int n0, const uint32_t* v) {
+__device__ __noinline__ void streams_any(const LinArgs& a, int m, int n0, const float* y) {
   float* xs = reinterpret_cast<float*>(a.out) + (size_t)m * a.S * a.N;
   for (int q = 0; q < 32 && n0 + q < a.N; ++q) {
     const int n = n0 + q;
-    const float y = __uint_as_float(v[q]) + (a.bias ? a.bias[n] : 0.f);
     float old[8];
     for (int s = 0; s < a.S; ++s) old[s] = xs[(size_t)s * a.N + n];
     for (int u = 0; u < a.S; ++u) {
-      float acc = a.outw[u] * y;
+      float acc = a.outw[u] * y[q];
       for (int s = 0; s < a.S; ++s) acc = fmaf(a.mix[s * a.S + u], old[s], acc);
       xs[(size_t)u * a.N + n] = acc;
     }
   }
 }
-
-template <typename OT>
-__device__ __forceinline__ void umma_store(const LinArgs& a, int z, int m, int n0, const uint32_t (&v)[32]) {
-  if (a.epi == PIEH_EPI_STREAMS) {
-    const bool whole = n0 + 32 <= a.N && (a.N & 3) == 0;   // the run's four-column pieces exist and are 16-byte aligned
-    if (whole && a.S == 1) streams_run<1>(a, m, n0, v);
-    else if (whole && a.S == 2) streams_run<2>(a, m, n0, v);
-    else if (whole && a.S == 4) streams_run<4>(a, m, n0, v);
-    else {
-      uint32_t w[32];
+// x_u <- sum_s mix[s, u] x_s + outw[u] y over S residual streams: this lane's four columns of every fourth row of the warp's tile,
+// read from the staged y.  Rows are taken in batches: the loads of a batch are in flight together.
+template <int S>
+__device__ __forceinline__ void streams_tile(const LinArgs& a, int row0, int m_end, int n, uint32_t buf, int lane) {
+  constexpr int NB = S <= 2 ? 4 : 2;
+  float* xs = reinterpret_cast<float*>(a.out) + n;
 #pragma unroll
-      for (int q = 0; q < 32; ++q) w[q] = v[q];
-      streams_any(a, m, n0, w);
+  for (int i0 = 0; i0 < 8; i0 += NB) {
+    float4 old[NB][S];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      const int m = row0 + 4 * (i0 + j) + (lane >> 3);
+#pragma unroll
+      for (int s = 0; s < S; ++s)
+        if (m < m_end) old[j][s] = *reinterpret_cast<const float4*>(xs + ((size_t)m * S + s) * a.N);
     }
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      const int r = 4 * (i0 + j) + (lane >> 3), m = row0 + r;
+      const uint4 yq = pie::lds128(buf + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+      if (m < m_end)
+#pragma unroll
+        for (int u = 0; u < S; ++u) {
+          const float ow = a.outw[u];
+          float4 acc = make_float4(ow * __uint_as_float(yq.x), ow * __uint_as_float(yq.y), ow * __uint_as_float(yq.z), ow * __uint_as_float(yq.w));
+#pragma unroll
+          for (int s = 0; s < S; ++s) {
+            const float mx = a.mix[s * S + u];
+            acc.x = fmaf(mx, old[j][s].x, acc.x); acc.y = fmaf(mx, old[j][s].y, acc.y);
+            acc.z = fmaf(mx, old[j][s].z, acc.z); acc.w = fmaf(mx, old[j][s].w, acc.w);
+          }
+          *reinterpret_cast<float4*>(xs + ((size_t)m * S + u) * a.N) = acc;
+        }
+    }
+  }
+}
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+// The warp's 32 x C tile (a lane's row in y[0 .. C - 1]) to out, rows row0 .. that are below m_end, columns n0 .. that are below
+// n_end.  Through the warp's 4 KB of shared memory, so that a store instruction writes whole 64- or 128-byte runs of a few rows
+// and not 16 bytes of 32 rows; element by element where rows are not 16-byte aligned.
+template <typename OT, int C>
+__device__ __forceinline__ void tile_out(OT* out, long long ld, int row0, int m_end, int n0, int n_end, const float (&y)[C], uint32_t buf,
+                                         int lane) {
+  constexpr int PER = 16 / sizeof(OT), CH = C / PER;   // elements of a 16-byte piece, pieces of a row (2, 4 or 8)
+  OT* const base = out + (size_t)row0 * ld + n0;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) == 0 && (ld * sizeof(OT)) % 16 == 0) {
+    constexpr int G = 8 / CH;                          // rows of a 128-byte line of the buffer
+    auto at = [&](int r, int c) { return buf + r * (16 * CH) + ((c ^ ((r / G) & (CH - 1))) << 4); };
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      if (sizeof(OT) == 4) {
+        sts128(at(lane, c), __float_as_uint(y[4 * c]), __float_as_uint(y[4 * c + 1]), __float_as_uint(y[4 * c + 2]), __float_as_uint(y[4 * c + 3]));
+      } else {
+        constexpr int P = C >= 8 ? 8 : C;
+        const float* q = y + P * c;
+        sts128(at(lane, c), pie::pack_bf16(q[0], q[1]), pie::pack_bf16(q[2], q[3]), pie::pack_bf16(q[4], q[5]), pie::pack_bf16(q[6], q[7]));
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      const int r = i * (32 / CH) + lane / CH, c = lane % CH, n = n0 + PER * c;
+      const uint4 v = pie::lds128(at(r, c));
+      if (row0 + r < m_end && n < n_end) {
+        OT* dst = base + (size_t)r * ld + PER * c;
+        if (n + PER <= n_end) {
+          *reinterpret_cast<uint4*>(dst) = v;
+        } else {
+          const OT* e = reinterpret_cast<const OT*>(&v);
+#pragma unroll
+          for (int k = 0; k < PER; ++k)
+            if (n + k < n_end) dst[k] = e[k];
+        }
+      }
+    }
+    __syncwarp();
     return;
   }
+  if (row0 + lane < m_end)
+#pragma unroll
+    for (int q = 0; q < C; ++q)
+      if (n0 + q < n_end) elem<OT>::store(base + (size_t)lane * ld + q, y[q]);
+}
+
+// 32 columns (n0 ..) of the warp's 32 rows (row0 ..; lane l holds row l's in v) through pieh_linear's epilogue; the whole warp
+// calls it.  buf: the warp's 4 KB of shared memory.
+template <typename OT>
+__device__ __forceinline__ void umma_store(const LinArgs& a, int z, int row0, int m_end, int n0, const uint32_t (&v)[32], uint32_t buf,
+                                           int lane) {
   if (a.epi == PIEH_EPI_GLU) {   // columns (2 j, 2 j + 1) are a (gate, linear) pair -> output column j
-    OT* dst = reinterpret_cast<OT*>(a.out) + (size_t)m * a.out_ld + (n0 >> 1);
     float y[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) y[q] = glu_pair(a, __uint_as_float(v[2 * q]), __uint_as_float(v[2 * q + 1]));
-    if (n0 + 32 <= a.N && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-      if (sizeof(OT) == 4) {
-        float4* d4 = reinterpret_cast<float4*>(dst);
+    tile_out<OT, 16>(reinterpret_cast<OT*>(a.out), a.out_ld, row0, m_end, n0 >> 1, a.N >> 1, y, buf, lane);
+    return;
+  }
+  float y[32];
+  if (a.bias && n0 + 32 <= a.N) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) d4[q] = make_float4(y[4 * q], y[4 * q + 1], y[4 * q + 2], y[4 * q + 3]);
-      } else {
-        uint4* d4 = reinterpret_cast<uint4*>(dst);
+    for (int q = 0; q < 32; ++q) y[q] = __uint_as_float(v[q]) + __ldg(a.bias + n0 + q);
+  } else {
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
-          d4[q] = make_uint4(pie::pack_bf16(y[8 * q], y[8 * q + 1]), pie::pack_bf16(y[8 * q + 2], y[8 * q + 3]),
-                             pie::pack_bf16(y[8 * q + 4], y[8 * q + 5]), pie::pack_bf16(y[8 * q + 6], y[8 * q + 7]));
+    for (int q = 0; q < 32; ++q) y[q] = __uint_as_float(v[q]) + (a.bias && n0 + q < a.N ? a.bias[n0 + q] : 0.f);
+  }
+  switch (a.epi) {   // (outside the loops over columns)
+    case PIEH_EPI_STREAMS: {
+      if (n0 + 32 <= a.N && (a.N & 3) == 0 && (a.S == 1 || a.S == 2 || a.S == 4)) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          sts128(buf + lane * 128 + ((c ^ (lane & 7)) << 4), __float_as_uint(y[4 * c]), __float_as_uint(y[4 * c + 1]),
+                 __float_as_uint(y[4 * c + 2]), __float_as_uint(y[4 * c + 3]));
+        __syncwarp();
+        const int n = n0 + 4 * (lane & 7);
+        if (a.S == 1) streams_tile<1>(a, row0, m_end, n, buf, lane);
+        else if (a.S == 2) streams_tile<2>(a, row0, m_end, n, buf, lane);
+        else streams_tile<4>(a, row0, m_end, n, buf, lane);
+        __syncwarp();
+      } else if (row0 + lane < m_end) {
+        float w[32];
+#pragma unroll
+        for (int q = 0; q < 32; ++q) w[q] = y[q];
+        streams_any(a, row0 + lane, n0, w);
       }
       return;
     }
+    case PIEH_EPI_RELU2:
 #pragma unroll
-    for (int q = 0; q < 16; ++q)
-      if (n0 + 2 * q + 1 < a.N) elem<OT>::store(dst + q, y[q]);
-    return;
+      for (int q = 0; q < 32; ++q) { y[q] = fmaxf(y[q], 0.f); y[q] = y[q] * y[q]; }
+      break;
+    case PIEH_EPI_SOFTCAP:
+#pragma unroll
+      for (int q = 0; q < 32; ++q) y[q] = a.epi_a * tanhf(y[q] / a.epi_a);
+      break;
+    case PIEH_EPI_TANH:
+#pragma unroll
+      for (int q = 0; q < 32; ++q) y[q] = tanhf(y[q]);
+      break;
+    case PIEH_EPI_XIELU:
+#pragma unroll
+      for (int q = 0; q < 32; ++q) y[q] = xielu_f(y[q], a.epi_a, a.epi_b);
+      break;
+    case PIEH_EPI_GELU:
+#pragma unroll
+      for (int q = 0; q < 32; ++q) y[q] = gelu_f(y[q]);
+      break;
+    case PIEH_EPI_SIGMUL:
+      if (row0 + lane < m_end) {
+        const float* gate = a.gate + (size_t)z * a.gate_bs + (size_t)(row0 + lane) * a.gate_ld + n0;
+        if (n0 + 32 <= a.N && (reinterpret_cast<uintptr_t>(gate) & 15) == 0) {   // the gate logits of a whole run, 16 bytes at a time
+#pragma unroll
+          for (int q4 = 0; q4 < 8; ++q4) {
+            const float4 g = *reinterpret_cast<const float4*>(gate + 4 * q4);
+            y[4 * q4] /= 1.f + __expf(-g.x); y[4 * q4 + 1] /= 1.f + __expf(-g.y);
+            y[4 * q4 + 2] /= 1.f + __expf(-g.z); y[4 * q4 + 3] /= 1.f + __expf(-g.w);
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 32; ++q)
+            if (n0 + q < a.N) y[q] *= 1.f / (1.f + __expf(-gate[q]));
+        }
+      }
+      break;
+    default: break;
   }
-  OT* dst = reinterpret_cast<OT*>(a.out) + (size_t)z * a.out_bs + (size_t)m * a.out_ld;
-  const float* gate = a.epi == PIEH_EPI_SIGMUL ? a.gate + (size_t)z * a.gate_bs + (size_t)m * a.gate_ld : nullptr;
-  float y[32];
-  if (gate && n0 + 32 <= a.N && (reinterpret_cast<uintptr_t>(gate + n0) & 15) == 0) {   // the gate logits of a whole run, 16 bytes at a time
-#pragma unroll
-    for (int q4 = 0; q4 < 8; ++q4) {
-      const float4 gq = *reinterpret_cast<const float4*>(gate + n0 + 4 * q4);
-      const float gl[4] = {gq.x, gq.y, gq.z, gq.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) y[4 * q4 + e] = __uint_as_float(v[4 * q4 + e]) / (1.f + __expf(-gl[e]));
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < 32; ++q) {
-      const int n = n0 + q;
-      float t = __uint_as_float(v[q]);
-      if (a.bias && n < a.N) t += a.bias[n];
-      if (a.epi == PIEH_EPI_RELU2) { t = fmaxf(t, 0.f); t = t * t; }
-      else if (a.epi == PIEH_EPI_SOFTCAP) t = a.epi_a * tanhf(t / a.epi_a);
-      else if (a.epi == PIEH_EPI_TANH) t = tanhf(t);
-      else if (a.epi == PIEH_EPI_XIELU) t = xielu_f(t, a.epi_a, a.epi_b);
-      else if (a.epi == PIEH_EPI_GELU) t = gelu_f(t);
-      else if (a.epi == PIEH_EPI_SIGMUL && n < a.N) t *= 1.f / (1.f + __expf(-gate[n]));
-      y[q] = t;
-    }
-  }
-  if (n0 + 32 <= a.N && (reinterpret_cast<uintptr_t>(dst + n0) & 15) == 0) {
-    if (sizeof(OT) == 4) {
-      float4* d4 = reinterpret_cast<float4*>(dst + n0);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) d4[q] = make_float4(y[4 * q], y[4 * q + 1], y[4 * q + 2], y[4 * q + 3]);
-    } else {
-      uint4* d4 = reinterpret_cast<uint4*>(dst + n0);
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        d4[q] = make_uint4(pie::pack_bf16(y[8 * q], y[8 * q + 1]), pie::pack_bf16(y[8 * q + 2], y[8 * q + 3]),
-                           pie::pack_bf16(y[8 * q + 4], y[8 * q + 5]), pie::pack_bf16(y[8 * q + 6], y[8 * q + 7]));
-    }
-    return;
-  }
-#pragma unroll
-  for (int q = 0; q < 32; ++q)
-    if (n0 + q < a.N) elem<OT>::store(dst + n0 + q, y[q]);
+  tile_out<OT, 32>(reinterpret_cast<OT*>(a.out) + (size_t)z * a.out_bs, a.out_ld, row0, m_end, n0, a.N, y, buf, lane);
 }
 
 // One CTA per SM, four stages.  (Two CTAs per SM with 2 stages each, so that one's epilogue runs under the other's main loop,
@@ -247,12 +296,13 @@ __global__ void __launch_bounds__(kThreads, 1) linear_grouped_kernel(const __gri
     if (alive) {
       const int quad = warp & 3;
       const int c_lo = (warp >> 2) * (kBN / 64), c_hi = c_lo + kBN / 64;
-      const int row = m0 + quad * 32 + lane;
+      // every MMA has read its operands: the stages' memory is free
+      const uint32_t buf = base + warp * 4096;
 #pragma unroll 1
       for (int c = c_lo; c < c_hi; ++c) {
         uint32_t v[32];
         pie::tmem_ld32(tmem + (uint32_t)(c * 32) + ((uint32_t)(quad * 32) << 16), v);
-        if (row < m_end && n0 + c * 32 < a.N) umma_store<OT>(a, 0, row, n0 + c * 32, v);
+        if (n0 + c * 32 < a.N) umma_store<OT>(a, 0, m0 + quad * 32, m_end, n0 + c * 32, v, buf, lane);
       }
     }
   } else {
@@ -282,8 +332,8 @@ __global__ void __launch_bounds__(kThreads, 1) linear_grouped_kernel(const __gri
 template <typename OT>
 struct DenseEpi {
   LinArgs a;
-  __device__ __forceinline__ void operator()(int z, int row, int col, const uint32_t (&v)[32]) const {
-    if (row < a.M && col < a.N) umma_store<OT>(a, z, row, col, v);
+  __device__ __forceinline__ void operator()(int z, int row0, int col, const uint32_t (&v)[32], uint32_t buf, int lane) const {
+    if (row0 < a.M && col < a.N) umma_store<OT>(a, z, row0, a.M, col, v, buf, lane);
   }
 };
 

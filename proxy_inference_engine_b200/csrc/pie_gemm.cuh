@@ -11,6 +11,8 @@
 //   * operands by TMA into an S-deep ring of 128-byte-swizzled stages; one thread issues the MMAs; two accumulator buffers, so
 //     the epilogue of a tile runs under the main loop of the next; a CTA (pair) walks tiles blockIdx, + grid, ... with the row
 //     tiles of a group of `group_m` innermost, so that what is in flight at once shares rows of x and of w in L2.
+//   * an epilogue warp turns 32 x 32 pieces of its tile through 4 KB of shared memory, so that rows are written in runs of 64 or 128
+//     bytes: 16 bytes of 32 rows an instruction took a third of a short-K tile's time.
 //   * QB = 4 / 8: a further TMA warp brings the packed rows of w, 128 bytes each, and groups of four warps turn them into
 //     the stage's bf16 rows, w_hat = bf16(scale q + bias) rounded once (fused bf16x2 / fp32 multiply-add): a thread takes one
 //     row of a K step, the groups take the K steps in turn (one step's chain of wait, load, store and proxy fence is longer
@@ -133,11 +135,16 @@ struct GemmTile {
   static constexpr int W_TMA = EPI_WARPS, W_MMA = EPI_WARPS + 1, W_PACK = EPI_WARPS + 2, W_DEQ = EPI_WARPS + 4;
   static constexpr int GROUPS = 3;                                // dequantising groups of four warps, a K step each in turn
   static constexpr int THREADS = 32 * (QB ? W_DEQ + 4 * GROUPS : EPI_WARPS + 4);
-  static constexpr int SMEM = 1024 + S * (A_STAGE + B_STAGE) + RING * CHUNK;
+  static constexpr int SMEM = 1024 + S * (A_STAGE + B_STAGE) + RING * CHUNK + EPI_WARPS * 4096;
   static constexpr int ACC = BN > 128 ? 256 : 128;              // columns between the two accumulators
   static constexpr int TMEM_COLS = 2 * ACC;                      // a power of two
   static_assert(SMEM <= 227 * 1024 && TMEM_COLS <= 512 && BN % (8 * EPI_WARPS) == 0 && NB % 8 == 0, "tile");
   static_assert(!QB || NB <= 128, "a dequantising thread per row, 128 threads a group");
+  // A group waits only for the packed chunks it reads, by the parity of their ring slot.  That is sound while no chunk it skipped
+  // can still be on its way when it waits for the slot's next one: with these numbers the K step it dequantised last had its
+  // stage freed by an MMA that came after a step of the skipped chunk.  (One slot or four groups break it: a stale chunk is read
+  // and the slot's arrivals overflow.  tests/test_cpu_gemm_schedule.py walks all tile lengths.)
+  static_assert(!QB || (GROUPS == 3 && RING == 3 && S == 5), "see tests/test_cpu_gemm_schedule.py before changing these");
   static_assert(!(SPLIT && CG == 2), "K is split over single CTAs");
 };
 
@@ -169,8 +176,9 @@ __device__ __forceinline__ GemmTileAt gemm_tile_at(const GemmArgs& a, int t) {
   return {z, first + rr % gm, rr / gm};
 }
 
-// Epi: void operator()(int z, int row, int col0, const uint32_t (&v)[32]) for 32 columns of one row (any row / column, the
-// callee checks the bounds).
+// Epi: void operator()(int z, int row0, int col0, const uint32_t (&v)[32], uint32_t buf, int lane), called by whole warps: 32 columns
+// of rows row0 .. row0 + 31, lane l holding row l's; any row and column, the callee checks the bounds.  buf: 4 KB of shared memory
+// of the warp's own, to turn the tile so that rows are written in whole runs.
 template <int CG, int BN, int QB, bool SPLIT, class Epi>
 __global__ void __launch_bounds__(GemmTile<CG, BN, QB, SPLIT>::THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ GemmArgs a,
@@ -234,7 +242,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
 
   if (warp < T::EPI_WARPS) {
     // ---------------------------------------------------------------- epilogue: TMEM lane quadrant warp % 4
-    const int quad = warp & 3, row_in = quad * 32 + lane;
+    const int quad = warp & 3;
+    const uint32_t ebuf = smP + T::RING * T::CHUNK + warp * 4096;
     constexpr int PARTS = T::EPI_WARPS / 4, RUNS = BN / 32 / PARTS;   // 32-column runs of this warp
     const int c_lo = (warp >> 2) * RUNS;
     if (!SPLIT) {
@@ -244,7 +253,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         const int b = i & 1;
         if (!gemm_wait_warp(smem_u32(&tfull_bar[b]), (i >> 1) & 1, abortp)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int row = at.m * T::BM + (int)(CG == 2 ? rank : 0) * 128 + row_in;
+        const int row0 = at.m * T::BM + (int)(CG == 2 ? rank : 0) * 128 + quad * 32;
 #pragma unroll 1
         for (int c = 0; c < RUNS; ++c) {
           uint32_t v[32];
@@ -257,7 +266,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
               else mbar_arrive(&tempty_bar[b]);
             }
           }
-          epi(at.z, row, at.n * BN + (c_lo + c) * 32, v);
+          epi(at.z, row0, at.n * BN + (c_lo + c) * 32, v, ebuf, lane);
         }
       }
     } else {
@@ -459,7 +468,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         }
 #pragma unroll
         for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(acc[q]);
-        epi(at.z, at.m * T::BM + row_in, at.n * BN + (gi * (int)ranks + (int)rank) * 32, v);
+        epi(at.z, at.m * T::BM + (warp & 3) * 32, at.n * BN + (gi * (int)ranks + (int)rank) * 32, v,
+            smP + T::RING * T::CHUNK + warp * 4096, lane);
       }
     }
   }

@@ -11,27 +11,35 @@
 
 namespace pie {
 
-// one rounding to bf16; 32 columns of a row, 16 bytes at a time where rows are 16-byte aligned
+// One rounding to bf16.  Rows that are 16-byte aligned go through the warp's shared memory, so that a store instruction writes
+// 64-byte runs of 8 rows and not 16 bytes of 32.
 struct QmmStore {
   uint16_t* y;
   int M, N;
-  __device__ __forceinline__ void operator()(int, int row, int col, const uint32_t (&v)[32]) const {
-    if (row >= M || col >= N) return;
-    uint16_t* dst = y + (size_t)row * N + col;
-    if (col + 32 <= N && (N & 7) == 0) {
+  __device__ __forceinline__ void operator()(int, int row0, int col, const uint32_t (&v)[32], uint32_t buf, int lane) const {
+    if (row0 >= M || col >= N) return;
+    uint16_t* const base = y + (size_t)row0 * N + col;
+    if ((N & 7) == 0) {
+      auto at = [&](int r, int c) { return buf + r * 64 + ((c ^ ((r >> 1) & 3)) << 4); };
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint4 o;
-        o.x = pack_bf16(__uint_as_float(v[8 * q]), __uint_as_float(v[8 * q + 1]));
-        o.y = pack_bf16(__uint_as_float(v[8 * q + 2]), __uint_as_float(v[8 * q + 3]));
-        o.z = pack_bf16(__uint_as_float(v[8 * q + 4]), __uint_as_float(v[8 * q + 5]));
-        o.w = pack_bf16(__uint_as_float(v[8 * q + 6]), __uint_as_float(v[8 * q + 7]));
-        reinterpret_cast<uint4*>(dst)[q] = o;
+      for (int c = 0; c < 4; ++c) {
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e] = pack_bf16(__uint_as_float(v[8 * c + 2 * e]), __uint_as_float(v[8 * c + 2 * e + 1]));
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at(lane, c)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
       }
-    } else {
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = 8 * i + (lane >> 2), c = lane & 3;
+        const uint4 o = lds128(at(r, c));
+        if (row0 + r < M && col + 8 * c < N) *reinterpret_cast<uint4*>(base + (size_t)r * N + 8 * c) = o;
+      }
+      __syncwarp();
+    } else if (row0 + lane < M) {
 #pragma unroll
       for (int q = 0; q < 32; ++q)
-        if (col + q < N) dst[q] = f2bf(__uint_as_float(v[q]));
+        if (col + q < N) base[(size_t)lane * N + q] = f2bf(__uint_as_float(v[q]));
     }
   }
 };
