@@ -88,7 +88,7 @@ cudaError_t launch_prefill_attn(uint16_t* out, const uint16_t* q, const uint16_t
                                 float scale, cudaStream_t st) {
   if (B == 0 || L == 0) return cudaSuccess;
   static const bool naive = [] { const char* e = getenv("PIE_PREFILL_ATTN_NAIVE"); return e && e[0] == '1'; }();
-  if (!naive && fa_prefill_umma_ok(out, q, kc, vc, kv, B, Hq, Hkv, L, D, offset))
+  if (!naive && fa_prefill_umma_ok(out, q, kc, vc, kv, B, Hq, Hkv, L, D, offset, scale))
     return launch_fa_prefill_umma(out, q, kc, vc, kv, B, Hq, Hkv, L, D, offset, scale, st);
   if (!naive) return launch_prefill_attn_tc(out, q, kc, vc, kv, B, Hq, Hkv, L, D, offset, scale, st);
   const float sl = scale * 1.4426950408889634f;

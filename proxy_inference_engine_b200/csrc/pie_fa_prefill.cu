@@ -10,16 +10,20 @@
 // same ~1000 cycles of an SM, so the kernel is built to keep both going at once:
 //   * warps 0-3 / 4-7: the softmax of query tile 0 / 1, a thread per row.  S comes out of tensor memory (128 columns), is
 //     masked on the diagonal, the running maximum moves only when exceeded by 8 (log2 units; the same sums, and O is rescaled
-//     rarely), p = exp2(s - m) is rounded to bf16 and put back over S as the A operand of the second product.  Row sums are
-//     of the unrounded p, in fp32.
+//     rarely), p = exp2(scale s - m), three quarters of them by the approximation unit (16 a cycle of an SM: at D = 64 that alone
+//     would take twice the MMAs' time) and the rest by a polynomial on the multiply-add pipe, is rounded to bf16 and put back over
+//     S as the A operand of the second product.  Row sums are of the unrounded p, in fp32.
 //   * warp 8: TMA.  Q once; K and V tiles of the contiguous or paged cache into two-deep rings (128-byte swizzle).
-//   * warp 9, one lane: MMAs.  S_g = Q_g K^T (both operands in shared memory), O_g += P_g V (P in tensor memory, V as it lies:
+//   * warp 9: MMAs.  S_g = Q_g K^T (both operands in shared memory), O_g += P_g V (P in tensor memory, V as it lies:
 //     its rows are keys, so it is an MN-major operand).  Order: PV of tile 0, QK^T of tile 0's next keys, then the same for
 //     tile 1: one tile's softmax runs under the other's MMAs.
 // Tensor memory: S/P 2 x 128 columns, O 2 x D.  Longest query tiles are dispatched first (causal: tile i sees i + 1 key tiles).
 // Every wait is bounded (pie_gemm.cuh).
-// Measured, 32 query / 8 kv heads, D 128, us (TFLOP/s) with the mma.sync kernel of pie_fa.cu -> here: 8192 tokens 2190 (251) -> 547
-// (1005); 2 x 3000 tokens 640 (231) -> 190 (774); 1531 behind 517: D 64 92 -> 51.  The exponentials bound it at D 64.
+// Measured, 32 query / 8 kv heads, us (TFLOP/s): the mma.sync kernel of pie_fa.cu -> this one with a lane of its own issuing the MMAs
+// and all exponentials on the approximation unit -> as it is.  D 128: 8192 tokens 2190 (251) -> 547 (1005) -> 460 (1196); 2 x 3000
+// tokens 640 (231) -> 190 (774) -> 164 (901).  D 64: 1531 behind 517 92 -> 51 -> 42; 8192 tokens 485 -> 386 (712).
+// What is left is one tile's chain, which the other tile covers only in part: of about 3000 cycles per pair of tiles, 1700 are a
+// softmax and 1300 the two products and their hand-overs.
 #include "pie_gemm.cuh"
 #include "pie_internal.h"
 
@@ -87,6 +91,50 @@ __device__ __forceinline__ float fap_exp2(float x) {   // results below 2^-126 a
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// two fp32 operations an instruction
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ void f2_unpack(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// 2^x of two values by the multiply-add pipe: x = n + f with f in [-1/2, 1/2] (adding 3 * 2^22 rounds to an integer and leaves it
+// in the low bits), 2^f by its least-squares polynomial of degree 5 in the Chebyshev weight (relative error 2.0e-7 in fp32, against
+// the approximation unit's 2.4e-7), times 2^n.  Arguments of -127 and below (a masked key's -inf) give 0, NaN gives NaN.
+__device__ __forceinline__ void fap_exp2_poly(f32x2 x2, float& ya, float& yb) {
+  float xa, xb;
+  f2_unpack(x2, xa, xb);
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(xa) : "f"(-127.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(xb) : "f"(-127.f));
+  const f32x2 x = f2_pack(xa, xb);
+  const f32x2 r = f2_add(x, f2_pack(12582912.f, 12582912.f));
+  const f32x2 f = f2_fma(f2_add(r, f2_pack(-12582912.f, -12582912.f)), f2_pack(-1.f, -1.f), x);
+  f32x2 p = f2_pack(0.00132669706f, 0.00132669706f);
+  p = f2_fma(p, f, f2_pack(0.00967545994f, 0.00967545994f));
+  p = f2_fma(p, f, f2_pack(0.0555074252f, 0.0555074252f));
+  p = f2_fma(p, f, f2_pack(0.240221217f, 0.240221217f));
+  p = f2_fma(p, f, f2_pack(0.693146944f, 0.693146944f));
+  p = f2_fma(p, f, f2_pack(1.00000012f, 1.00000012f));
+  float ra, rb;
+  f2_unpack(r, ra, rb);
+  f2_unpack(f2_mul(p, f2_pack(__int_as_float((__float_as_int(ra) << 23) + 0x3f800000), __int_as_float((__float_as_int(rb) << 23) + 0x3f800000))), ya, yb);
+}
 __device__ __forceinline__ void fap_commit(uint64_t* bar) { gemm_commit<1>(smem_u32(bar)); }
 
 template <int D>
@@ -135,7 +183,10 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const uint32_t tmem = tmem_slot;
   volatile int* const abortp = &abort_flag;
 
+  // Registers: 384 threads x 168 at launch = 64512; the eight softmax warps hold a row of scores each and take 216, the other
+  // four give theirs up to 64: 8 x 32 x 216 + 4 x 32 x 64 = 63488.
   if (warp < 8) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     // ------------------------------------------------------------------------------------------------ softmax of tile g
     const int g = warp >> 2, quad = warp & 3, ng = g ? n1 : n0;
     const int row = q0 + g * 128 + quad * 32 + lane, lim = a.offset + row;   // last key this row sees
@@ -151,8 +202,6 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #pragma unroll
       for (int c = 0; c < 4; ++c) fap_tmem_ld(tS + 32 * c, s + 32 * c);
       tmem_ld_wait();
-#pragma unroll
-      for (int i = 0; i < 128; ++i) s[i] *= a.scale_log2e;
       if (j * 128 + 127 > a.offset + q0 + g * 128 + quad * 32) {   // a key of this tile lies beyond some row of the warp
         const int last = lim - j * 128;
 #pragma unroll
@@ -164,7 +213,7 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       for (int i = 4; i < 128; i += 4) {
         x0 = fmaxf(x0, s[i]); x1 = fmaxf(x1, s[i + 1]); x2 = fmaxf(x2, s[i + 2]); x3 = fmaxf(x3, s[i + 3]);
       }
-      const float mx = fmaxf(fmaxf(x0, x1), fmaxf(x2, x3));
+      const float mx = fmaxf(fmaxf(x0, x1), fmaxf(x2, x3)) * a.scale_log2e;   // (the scale is positive)
       const bool move = mx > m + 8.f;
       if (j == 0) {
         m = mx;
@@ -187,21 +236,34 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         fap_tmem_st_wait();
       }
       const float ms = m == -INFINITY ? 0.f : m;
-      float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
+      const f32x2 sc2 = f2_pack(a.scale_log2e, a.scale_log2e), ms2 = f2_pack(-ms, -ms);
+      f32x2 l01 = f2_pack(0.f, 0.f), l23 = l01;
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
         uint32_t p[32];
 #pragma unroll
-        for (int i = 0; i < 64; i += 4) {
-          const float* q = s + 64 * hf + i;
-          const float e0 = fap_exp2(q[0] - ms), e1 = fap_exp2(q[1] - ms), e2 = fap_exp2(q[2] - ms), e3 = fap_exp2(q[3] - ms);
-          l0 += e0; l1 += e1; l2 += e2; l3 += e3;
-          p[i / 2] = pack_bf16(e0, e1);
-          p[i / 2 + 1] = pack_bf16(e2, e3);
+        for (int i = 0; i < 32; ++i) {
+          const f32x2 x = f2_fma(f2_pack(s[64 * hf + 2 * i], s[64 * hf + 2 * i + 1]), sc2, ms2);
+          float e0, e1;
+          if (i % 4 == 3) {        // every fourth pair off the approximation unit, which would otherwise bound the tile
+            fap_exp2_poly(x, e0, e1);
+          } else {
+            float x0, x1;
+            f2_unpack(x, x0, x1);
+            e0 = fap_exp2(x0);
+            e1 = fap_exp2(x1);
+          }
+          p[i] = pack_bf16(e0, e1);
+          if (i & 1) l23 = f2_add(l23, f2_pack(e0, e1));
+          else l01 = f2_add(l01, f2_pack(e0, e1));
         }
         fap_tmem_st(tS + 32 * hf, p);
       }
-      l += (l0 + l1) + (l2 + l3);
+      {
+        float l0, l1;
+        f2_unpack(f2_add(l01, l23), l0, l1);
+        l += l0 + l1;
+      }
       fap_tmem_st_wait();
       if (a.page_table && tail && j == (keys - 1) / 128) {
         // the slots behind the last key of a page may hold anything, and 0 * NaN is not 0: clear them
@@ -235,9 +297,10 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                            pack_bf16(o[8 * q + 4] * inv, o[8 * q + 5] * inv), pack_bf16(o[8 * q + 6] * inv, o[8 * q + 7] * inv));
       }
     }
-  } else if (warp == 8) {
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     // ------------------------------------------------------------------------------------------------ TMA
-    if (lane == 0) {
+    if (warp == 8 && lane == 0) {
       const int ntq = n1 > 0 ? 2 : 1;
       mbar_arrive_expect_tx(&q_full, ntq * T::TILE);
       for (int g = 0; g < ntq; ++g)
@@ -266,55 +329,55 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       if (!alive)
         for (int w = 0; w < 1000; ++w) __nanosleep(1000);
     }
-  } else if (warp == 9) {
     // ------------------------------------------------------------------------------------------------ MMAs
-    auto qk = [&](int g, int j) {
-      if (lane == 0) {
+    if (warp == 9) {
+      // The whole warp walks the loop, so that addresses and descriptors stay warp-uniform; one elected lane issues, and nothing
+      // brings the lanes together but the election (a lane's own branch took 80 cycles an MMA; 4096 tokens, D 128: 155 -> 127 us).
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+      const uint64_t dq0 = umma_desc_sw128(smQ), dk0 = umma_desc_sw128(smK), dv0 = fap_desc_mn(smV);
+      auto qk = [&](int g, int j) {
+        const uint64_t dq = dq0 + (uint64_t)(g * (T::TILE >> 4)), dk = dk0 + (uint64_t)((j & 1) * (T::TILE >> 4));
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t dq = umma_desc_sw128(smQ + g * T::TILE + (k >> 2) * 16384) + 2 * (k & 3);
-          const uint64_t dk = umma_desc_sw128(smK + (j & 1) * T::TILE + (k >> 2) * 16384) + 2 * (k & 3);
-          umma_bf16(tmem + COL_S + g * 128, dq, dk, ID_S, k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < D / 16; ++k)
+          umma_bf16(tm + COL_S + g * 128, dq + (k >> 2) * 1024 + 2 * (k & 3), dk + (k >> 2) * 1024 + 2 * (k & 3), ID_S, k > 0 ? 1u : 0u);
         fap_commit(&s_full[g]);
-      }
-    };
-    auto pv = [&](int g, int j) {
-      if (lane == 0) {
-        const uint64_t dv = fap_desc_mn(smV + (j & 1) * T::TILE);
+      };
+      auto pv = [&](int g, int j) {
+        const uint64_t dv = dv0 + (uint64_t)((j & 1) * (T::TILE >> 4));
 #pragma unroll
         for (int k = 0; k < 8; ++k)   // 16 keys: 8 columns of P, two 8-key atoms of V
-          fap_mma_ts(tmem + COL_O + g * D, tmem + COL_S + g * 128 + 8 * k, dv + (uint64_t)k * (2048 >> 4), ID_O, (j > 0 || k > 0) ? 1u : 0u);
+          fap_mma_ts(tm + COL_O + g * D, tm + COL_S + g * 128 + 8 * k, dv + k * (2048 >> 4), ID_O, (j > 0 || k > 0) ? 1u : 0u);
         fap_commit(&o_full[g]);
-      }
-    };
-    bool alive = gemm_wait_warp(smem_u32(&q_full), 0, abortp) && gemm_wait_warp(smem_u32(&k_full[0]), 0, abortp);
-    if (alive) {
+      };
+      bool alive = gemm_wait(smem_u32(&q_full), 0, abortp);   // a lane's own: once a wait expires it only keeps the lane from issuing
+      alive &= gemm_wait(smem_u32(&k_full[0]), 0, abortp);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (n0 > 0) qk(0, 0);
-      if (n1 > 0) qk(1, 0);
-      if (lane == 0) fap_commit(&k_empty[0]);
-    }
-    for (int j = 0; j < n && alive; ++j) {
-      const int i = j & 1, i2 = (j + 1) & 1;
-      if (!(alive = gemm_wait_warp(smem_u32(&v_full[i]), (j >> 1) & 1, abortp))) break;
-      if (j + 1 < n && !(alive = gemm_wait_warp(smem_u32(&k_full[i2]), ((j + 1) >> 1) & 1, abortp))) break;
+      if (elect_one() && alive) {
+        if (n0 > 0) qk(0, 0);
+        if (n1 > 0) qk(1, 0);
+        fap_commit(&k_empty[0]);
+      }
+      for (int j = 0; j < n; ++j) {
+        const int i = j & 1, i2 = (j + 1) & 1;
+        alive &= gemm_wait(smem_u32(&v_full[i]), (j >> 1) & 1, abortp);
+        if (j + 1 < n) alive &= gemm_wait(smem_u32(&k_full[i2]), ((j + 1) >> 1) & 1, abortp);
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        const int ng = g ? n1 : n0;
-        if (j < ng) {
-          if (!(alive = gemm_wait_warp(smem_u32(&p_full[g]), j & 1, abortp))) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          pv(g, j);
-          if (j + 1 < ng) qk(g, j + 1);
+        for (int g = 0; g < 2; ++g) {
+          const int ng = g ? n1 : n0;
+          if (j < ng) {
+            alive &= gemm_wait(smem_u32(&p_full[g]), j & 1, abortp);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one() && alive) {
+              pv(g, j);
+              if (j + 1 < ng) qk(g, j + 1);
+            }
+          }
+        }
+        if (elect_one() && alive) {
+          fap_commit(&v_empty[i]);
+          if (j + 1 < n) fap_commit(&k_empty[i2]);
         }
       }
-      if (!alive) break;
-      if (lane == 0) {
-        fap_commit(&v_empty[i]);
-        if (j + 1 < n) fap_commit(&k_empty[i2]);
-      }
-      __syncwarp();
     }
   }
   __syncwarp();
@@ -326,7 +389,8 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 // What a tiled copy of the cache asks for: 16-byte aligned arrays, positive strides where there is more than one head / row,
 // pages of whole 64-key boxes, and grid limits.
 bool fa_prefill_umma_ok(const uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc, const KvLayout& kv, int B,
-                        int Hq, int Hkv, int L, int D, int offset) {
+                        int Hq, int Hkv, int L, int D, int offset, float scale) {
+  if (!(scale > 0.f)) return false;   // the running maximum is taken before the scale
   auto off16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
   if (off16(out) || off16(q) || off16(kc) || off16(vc) || (L + 255) / 256 > 65535 || (long long)B * Hq > (1 << 30)) return false;
   if (kv.tok_stride <= 0 || (Hkv > 1 && kv.head_stride <= 0)) return false;
@@ -336,8 +400,15 @@ bool fa_prefill_umma_ok(const uint16_t* out, const uint16_t* q, const uint16_t* 
 template <int D>
 static cudaError_t launch_fap(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FapArgs& a, cudaStream_t st) {
   using T = FapTile<D>;
-  cudaError_t e = cudaFuncSetAttribute(fa_prefill_umma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
-  if (e != cudaSuccess) return e;
+  static unsigned long long configured = 0;   // per device
+  if (first_use_on_device(configured)) {
+    cudaFuncAttributes at;
+    cudaError_t e = cudaFuncGetAttributes(&at, fa_prefill_umma_kernel<D>);
+    // the warps' register shares must fit what the block is launched with, or they would wait for registers for good
+    if (e == cudaSuccess && at.numRegs * T::THREADS < 8 * 32 * 216 + 4 * 32 * 64) e = cudaErrorInvalidConfiguration;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_prefill_umma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
+    if (e != cudaSuccess) { configured = 0; return e; }
+  }
   count_launch();
   fa_prefill_umma_kernel<D><<<dim3((unsigned)(a.B * a.Hq), (unsigned)((a.L + 255) / 256)), T::THREADS, T::SMEM, st>>>(mq, mk, mv, a);
   return cudaGetLastError();

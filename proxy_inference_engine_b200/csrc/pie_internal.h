@@ -114,7 +114,7 @@ cudaError_t launch_prefill_attn_tc(uint16_t* out, const uint16_t* q, const uint1
                                    const KvLayout& kv, int B, int Hq, int Hkv, int L, int D, int offset, float scale,
                                    cudaStream_t st);
 bool fa_prefill_umma_ok(const uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc, const KvLayout& kv, int B,
-                        int Hq, int Hkv, int L, int D, int offset);
+                        int Hq, int Hkv, int L, int D, int offset, float scale);
 cudaError_t launch_fa_prefill_umma(uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc, const KvLayout& kv,
                                    int B, int Hq, int Hkv, int L, int D, int offset, float scale, cudaStream_t st);
 unsigned int qmm_pipeline_error();

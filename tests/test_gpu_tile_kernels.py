@@ -130,6 +130,32 @@ def test_prefill_attention_tiles(paged, D, B, Hq, Hkv, L, offset):
     assert _lib.load().pie_pipeline_error() == 0
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("scale", [0.1, 4.0, 0.0, -0.1])   # exponents down to 0 and past the smallest; not positive: the other kernel
+def test_prefill_attention_exponentials(D, scale):
+    """Keys beyond a row weigh exactly nothing whatever lies there, a NaN key reaches every row that sees it and no other."""
+    from proxy_inference_engine_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(D)
+    L = 200
+    rnd = lambda *s: (1.5 * torch.randn(s, generator=g, device="cuda")).to(torch.bfloat16)
+    q, k, v = rnd(1, 1, L, D), rnd(1, 1, L, D), rnd(1, 1, L, D)
+    k[0, 0, 180:188], v[0, 0, 188:] = float("nan"), 3e38
+    rows = ops.prefill_attention(q, k, v, ops.kv_layout(k), 0, scale).reshape(L, D)
+    seen = 180
+    s = (q[0, 0, :seen].double() @ k[0, 0, :seen].double().T) * scale
+    p = torch.softmax(s.masked_fill(torch.ones_like(s).triu(1) > 0, float("-inf")), -1)
+    want, mass = p @ v[0, 0, :seen].double(), p @ v[0, 0, :seen].double().abs()
+    # as above; 200 weights below the smallest fp32 number add nothing that a bound of 2^-100 would not cover
+    slack = mass * (2 ** -8 + 2 * D * 2 ** -23 * float(s.abs().max())) + want.abs() * 2 ** -8 + 2 ** -100
+    _within(rows[:seen], want, slack)
+    for key in range(180, 188):                      # one NaN key alone
+        k1 = k.clone()
+        k1[0, 0, 180:188] = 0
+        k1[0, 0, key] = float("nan")
+        rows = ops.prefill_attention(q, k1, v, ops.kv_layout(k1), 0, scale).reshape(L, D)
+        assert not rows[:key].isnan().any() and rows[key:].isnan().all(), key
+
+
 @pytest.mark.parametrize("rows,dims", [(1, 8), (3, 2048), (2, 2056), (5, 4096), (3, 8192), (2, 8200), (3, 100)])
 def test_row_and_elementwise_operators(rows, dims):
     """RMSNorm at the edges of its register tiles, SwiGLU and the sum with and without 16-byte alignment and a tail."""
