@@ -9,7 +9,7 @@
 //                       scheduler walks a serial chain, so what counts is the chain's length: rows of a column are dealt four
 //                       at a time (a lane reads k and q 16 bytes at a time), a token's k is read while the token before it is
 //                       worked on, and the decay is applied to S beside the shuffles, not in front of the prediction
-//                       (S^T k with the old S, times g).  1200 rows, 16 heads of 128 x 128: 477 -> 369 us.
+//                       (S^T k with the old S, times g).  1200 rows, 16 heads of 128 x 128: 477 -> 244 us.
 // delta_gate_kernel     per-head RMS norm of o, times the norm weight, times silu(gate)
 // Everything that enters the recurrence is fp32; only delta_gate's output takes the act dtype.
 #include "hyb_common.cuh"
@@ -167,13 +167,13 @@ __device__ __forceinline__ void cp_async_f(float* smem_dst, const float* gsrc, i
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(gsrc) : "memory");
 }
 
-template <int RPT>
+template <int RPT, int R>   // rows of a state column in a lane, lanes of a column
 __global__ void __launch_bounds__(kScanThreads, 1) delta_scan_kernel(float* o, const float* q, const float* k, const float* v,
-                                                                  const float* beta, const float* decay,
-                                                                  const pieh_delta d, const pieh_batch b, int R) {
+                                                                     const float* beta, const float* decay,
+                                                                     const pieh_delta d, const pieh_batch b) {
   extern __shared__ __align__(16) float sm[];
   pdl_sync();
-  const int cols = kScanThreads / R;
+  constexpr int cols = kScanThreads / R;
   const int h = blockIdx.y, i = blockIdx.z;
   const int hk = h / (d.H / d.G);
   const int start = b.seq_start[i], n = b.seq_len[i], ctx = b.seq_ctx[i];
@@ -182,8 +182,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_scan_kernel(float* o, c
   const bool col_ok = j < d.dv;
   const int dk = d.dk, dv = d.dv;
   // two chunk buffers: while the recurrence walks one chunk of tokens, cp.async fills the other
-  const int dkp = RPT * R;                        // rows as the lanes hold them: dk and zeros behind
-  const int buf_floats = kScanChunk * (2 * dkp + cols + 2);
+  constexpr int dkp = RPT * R;                    // rows as the lanes hold them: dk and zeros behind
+  constexpr int buf_floats = kScanChunk * (2 * dkp + cols + 2);
   float* S_g = d.state + (((size_t)b.seq_slot[i] * d.H + h) * dk) * dv;
   float S[RPT];
 #pragma unroll
@@ -248,28 +248,30 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_scan_kernel(float* o, c
     const float* vs = qs + kScanChunk * dkp;
     const float* gb = vs + kScanChunk * cols;
     float kk[RPT], vv = vs[cl], g = gb[0], be = gb[1];
-    auto load4 = [&](float* dst, const float* row) {
+    auto load_rows = [&](float* dst, const float* row) {
 #pragma unroll
       for (int r = 0; r < RPT; r += 4) {
         const float4 f = *reinterpret_cast<const float4*>(row + r * R + 4 * rl);
         dst[r] = f.x; dst[r + 1] = f.y; dst[r + 2] = f.z; dst[r + 3] = f.w;
       }
     };
-    load4(kk, ks);
+    load_rows(kk, ks);
+#pragma unroll 2
     for (int tt = 0; tt < nc; ++tt) {
       float pp[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int r = 0; r < RPT; ++r) pp[r & 3] = fmaf(S[r], kk[r], pp[r & 3]);
       float pred = (pp[0] + pp[1]) + (pp[2] + pp[3]);
       float qq[RPT], kn[RPT];
-      load4(qq, qs + tt * dkp);
+      load_rows(qq, qs + tt * dkp);
       const int nx = min(tt + 1, nc - 1);
-      load4(kn, ks + nx * dkp);
+      load_rows(kn, ks + nx * dkp);
       const float vn = vs[nx * cols + cl], gn = gb[2 * nx], bn = gb[2 * nx + 1];
 #pragma unroll
       for (int r = 0; r < RPT; ++r) S[r] *= g;
       // the read-out of the PREVIOUS token is reduced over the R lanes together with this token's prediction: two
       // independent shuffle chains instead of two in a row on the recurrence's critical path
+#pragma unroll
       for (int off = 1; off < R; off <<= 1) {
         pred += __shfl_xor_sync(0xffffffffu, pred, off);
         out_prev += __shfl_xor_sync(0xffffffffu, out_prev, off);
@@ -289,6 +291,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) delta_scan_kernel(float* o, c
     }
     __syncthreads();   // everyone is done with this buffer before the next fill overwrites it
   }
+#pragma unroll
   for (int off = 1; off < R; off <<= 1) out_prev += __shfl_xor_sync(0xffffffffu, out_prev, off);
   if (row_prev >= 0 && rl == 0 && col_ok) o[((size_t)row_prev * d.H + h) * dv + j] = out_prev;
   if (col_ok) {
@@ -315,6 +318,19 @@ __global__ void delta_gate_kernel(OT* out, const float* o, const float* proj, lo
   const float* gate = proj + (size_t)t * ld + gate_off + (size_t)h * d.dv;
   for (int c = lane; c < d.dv; c += 32)
     elem<OT>::store(out + (size_t)w * d.dv + c, src[c] * inv * d.out_norm[c] * silu_f(gate[c]));
+}
+
+template <int RPT, int R>
+static cudaError_t launch_scan(float* o, const float* q, const float* k, const float* v, const float* beta, const float* decay,
+                               const pieh_delta& d, const pieh_batch& b, cudaStream_t st) {
+  constexpr int cols = kScanThreads / R;
+  constexpr size_t smem = (size_t)2 * kScanChunk * (2 * RPT * R + cols + 2) * 4;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<RPT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_k(delta_scan_kernel<RPT, R>, dim3((d.dv + cols - 1) / cols, d.H, b.n_seq), dim3(kScanThreads), smem, st, o, q, k, v,
+                  beta, decay, d, b);
 }
 
 static bool delta_ok(const pieh_delta* d) {
@@ -353,18 +369,14 @@ extern "C" int pieh_delta_scan(float* o, const float* q, const float* k, const f
   // 16 rows of a state column per lane.  Measured on a 4096-row portion (dk = dv = 128, 16 heads, one sequence):
   // 8 rows per lane (16 lanes, 4 shuffle steps) 2.10 ms, 16 rows 1.74 ms, 32 rows (4 lanes, 2 steps, 64 CTAs) 2.62 ms
   constexpr int RPT = 16;
-  int R = 1;
-  while (R * RPT < d->dk) R <<= 1;   // lanes per column, a power of two <= 32
-  const int cols = kScanThreads / R;
-  const size_t smem = (size_t)2 * kScanChunk * (2 * RPT * R + cols + 2) * 4;
-  static bool opted = false;
-  if (smem > 48 * 1024 && !opted) {
-    cudaFuncSetAttribute(delta_scan_kernel<RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    opted = true;
-  }
+  cudaStream_t st = (cudaStream_t)stream;
   count_launch();
-  return status_of(launch_k(delta_scan_kernel<RPT>, dim3((d->dv + cols - 1) / cols, d->H, b->n_seq), dim3(kScanThreads), smem,
-                            (cudaStream_t)stream, o, q, k, v, beta, decay, *d, *b, R));
+  if (d->dk <= RPT) return status_of(launch_scan<RPT, 1>(o, q, k, v, beta, decay, *d, *b, st));
+  if (d->dk <= 2 * RPT) return status_of(launch_scan<RPT, 2>(o, q, k, v, beta, decay, *d, *b, st));
+  if (d->dk <= 4 * RPT) return status_of(launch_scan<RPT, 4>(o, q, k, v, beta, decay, *d, *b, st));
+  if (d->dk <= 8 * RPT) return status_of(launch_scan<RPT, 8>(o, q, k, v, beta, decay, *d, *b, st));
+  if (d->dk <= 16 * RPT) return status_of(launch_scan<RPT, 16>(o, q, k, v, beta, decay, *d, *b, st));
+  return status_of(launch_scan<RPT, 32>(o, q, k, v, beta, decay, *d, *b, st));
 }
 
 extern "C" int pieh_delta_gate(void* out, int out_dtype, const float* o, const float* proj, long long ld,

@@ -12,9 +12,11 @@
 
 namespace pieh {
 
+// by_four: rows in runs of four (a decode step's 4 rows of 4096, mostly, 10.5 -> 4.3 us).  Odd widths and unaligned tables go one
+// element at a time.
 template <typename ET, typename AT>
 __global__ void embed_positions_kernel(float* x, AT* act, const ET* table, const ET* pos_table, const int32_t* tokens,
-                                       const int32_t* positions, int W, int vocab, int max_pos) {
+                                       const int32_t* positions, int W, int vocab, int max_pos, int by_four) {
   pdl_sync();
   const int t = blockIdx.x;
   int id = tokens[t];
@@ -25,6 +27,19 @@ __global__ void embed_positions_kernel(float* x, AT* act, const ET* table, const
     int p = positions[t];
     p = p < 0 ? 0 : (p >= max_pos ? max_pos - 1 : p);
     prow = pos_table + (size_t)p * W;
+  }
+  if (by_four) {
+#pragma unroll 4
+    for (int c = 4 * threadIdx.x; c < W; c += 4 * blockDim.x) {
+      float4 v = load4(row + c);
+      if (prow) {
+        const float4 p = load4(prow + c);
+        v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+      }
+      store4(x + (size_t)t * W + c, v);
+      if (act) store4(act + (size_t)t * W + c, v);
+    }
+    return;
   }
   for (int c = threadIdx.x; c < W; c += blockDim.x) {
     float v = elem<ET>::load(row + c);
@@ -206,7 +221,7 @@ extern "C" int pieh_embed_positions(float* x, void* act, int act_dtype, const vo
   count_launch();
   PIEH_DISPATCH_DTYPE(table_dtype, ET, PIEH_DISPATCH_DTYPE(act_dtype, AT,
       launch_k(embed_positions_kernel<ET, AT>, dim3(T), dim3(256), 0, st, x, (AT*)act, (const ET*)table, (const ET*)pos_table,
-               tokens, positions, W, vocab, max_positions)));
+               tokens, positions, W, vocab, max_positions, (int)rows_of_four(W, x, act, table, pos_table))));
   return status_of(cudaGetLastError());
 }
 

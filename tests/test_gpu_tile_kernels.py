@@ -220,3 +220,23 @@ def test_dense_matmul_of_few_rows(M, N, K):
         gate, up = want[:, 0::2], want[:, 1::2]
         silu = gate * torch.sigmoid(gate)
         _within(out, silu * up, 1.1 * up.abs() * slack[:, 0::2] + silu.abs() * slack[:, 1::2] + (silu * up).abs() * 2 ** -20)
+
+
+@pytest.mark.parametrize("W,shift", [(4, 0), (1028, 0), (4096, 0), (4096, 1), (1030, 0), (7, 0)])
+def test_embedding_rows_by_four_and_by_one(W, shift):
+    """Widths of whole fours, odd ones and a table that is not 16-byte aligned; the sums are of two values, so exact in fp32."""
+    from proxy_inference_engine_b200 import _lib
+    L, T, V, S = _lib.load_hybrid(), 3, 11, 2
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    tok, pos = (torch.tensor(t, dtype=torch.int32, device="cuda") for t in ([10, 0, 4], [2, 0, 6]))
+    for dt, code in ((torch.bfloat16, _lib.DTYPE_BF16), (torch.float32, _lib.DTYPE_F32)):
+        table = torch.randn(V * W + 4, device="cuda").to(dt)[shift:shift + V * W].view(V, W)
+        ptab = torch.randn(V, W, device="cuda").to(dt)
+        xs = torch.empty(T, S, W, device="cuda")
+        _lib.check_hybrid(L.pieh_embed_streams(_p(xs), _p(table), code, _p(tok), T, S, W, V, st), "embed_streams")
+        assert torch.equal(xs, table[tok.long()].float()[:, None].expand(T, S, W))
+        x, act = torch.empty(T, W, device="cuda"), torch.empty(T, W, device="cuda", dtype=torch.bfloat16)
+        _lib.check_hybrid(L.pieh_embed_positions(_p(x), _p(act), _lib.DTYPE_BF16, _p(table), _p(ptab), code, _p(tok), _p(pos), T, W, V,
+                                                 V, st), "embed_positions")
+        want = table[tok.long()].float() + ptab[pos.long()].float()
+        assert torch.equal(x, want) and torch.equal(act, want.to(torch.bfloat16))
