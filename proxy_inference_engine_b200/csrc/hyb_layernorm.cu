@@ -39,9 +39,28 @@ __device__ __forceinline__ void put4(__nv_bfloat16* p, float4 v) {
 }
 __device__ __forceinline__ float4 get4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
+// a norm's weight and bias on their way before the reductions that they wait for (a few rows), or read behind them (many rows: the
+// registers are worth more as resident CTAs)
+template <int NV, bool AHEAD>
+struct LnWeights {
+  const float *w, *b;
+  float4 wv[AHEAD ? NV : 1], bv[AHEAD ? NV : 1];
+  __device__ __forceinline__ LnWeights(const float* w_, const float* b_, int W) : w(w_), b(b_) {
+    if (AHEAD && w) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int c = (threadIdx.x + i * blockDim.x) * 4;
+        if (c < W) { wv[AHEAD ? i : 0] = get4(w + c); bv[AHEAD ? i : 0] = get4(b + c); }
+      }
+    }
+  }
+  __device__ __forceinline__ float4 weight(int i, int c) const { return AHEAD ? wv[AHEAD ? i : 0] : get4(w + c); }
+  __device__ __forceinline__ float4 bias(int i, int c) const { return AHEAD ? bv[AHEAD ? i : 0] : get4(b + c); }
+};
+
 // v <- (v - mean(v)) / sqrt(mean((v - mean)^2) + eps) * w + b, the row spread over the CTA's registers
-template <int NV>
-__device__ __forceinline__ void ln_rows(float4 (&v)[NV], const float* w, const float* b, float eps, int W, float* red) {
+template <int NV, bool AHEAD>
+__device__ __forceinline__ void ln_rows(float4 (&v)[NV], const LnWeights<NV, AHEAD>& wb, float eps, int W, float* red) {
   float s = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);   // what lies past the row is zero
@@ -59,14 +78,16 @@ __device__ __forceinline__ void ln_rows(float4 (&v)[NV], const float* w, const f
   for (int i = 0; i < NV; ++i) {
     const int c = (threadIdx.x + i * blockDim.x) * 4;
     if (c < W) {
-      const float4 g = get4(w + c), o = get4(b + c);
+      const float4 g = wb.weight(i, c), o = wb.bias(i, c);
       v[i].x = fmaf(v[i].x * inv, g.x, o.x); v[i].y = fmaf(v[i].y * inv, g.y, o.y);
       v[i].z = fmaf(v[i].z * inv, g.z, o.z); v[i].w = fmaf(v[i].w * inv, g.w, o.w);
     }
   }
 }
 
-template <typename AT, int NV>   // NV runs of 4 elements a thread
+// Of a few rows nothing but the chain of loads and reductions takes time, so AHEAD has every load on its way at once: 4 rows of
+// 4096 with weights from memory 6.9 -> 4.0 us, 148 rows 7.4 -> 4.9, 4 rows of 8192 11.2 -> 5.8.
+template <typename AT, int NV, bool AHEAD>   // NV runs of 4 elements a thread
 __global__ void __launch_bounds__(256) layernorm_add_kernel(const LnAdd a) {
   __shared__ float red[4][8];
   pdl_sync();
@@ -88,7 +109,8 @@ __global__ void __launch_bounds__(256) layernorm_add_kernel(const LnAdd a) {
       }
     }
   }
-  if (yr && !replace) ln_rows<NV>(u, a.post_w, a.post_b, a.eps, W, red[0]);
+  const LnWeights<NV, AHEAD> post(replace || !yr ? nullptr : a.post_w, a.post_b, W), next(a.h ? a.next_w : nullptr, a.next_b, W);
+  if (yr && !replace) ln_rows<NV>(u, post, a.eps, W, red[0]);
   const bool changed = yr || a.add_rows || a.add_vec;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
@@ -106,7 +128,7 @@ __global__ void __launch_bounds__(256) layernorm_add_kernel(const LnAdd a) {
     if (changed && !a.rows) put4(xr + c, v[i]);
   }
   if (!a.h) return;
-  if (a.next_w) ln_rows<NV>(v, a.next_w, a.next_b, a.eps, W, red[2]);
+  if (a.next_w) ln_rows<NV>(v, next, a.eps, W, red[2]);
   AT* hr = reinterpret_cast<AT*>(a.h) + (size_t)blockIdx.x * W;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
@@ -154,6 +176,10 @@ __global__ void __launch_bounds__(256) layernorm_add_any_kernel(const LnAdd a) {
   for (int c = threadIdx.x; c < W; c += blockDim.x) elem<AT>::store(hr + c, row[c]);
 }
 
+// One CTA on every SM: up to here a row has its SM's registers to itself.  Beyond it rows share an SM and hide each other's loads, and
+// the registers of AHEAD cost resident rows (behind / ahead, us: 592 rows of 4096 10.0 / 11.0, 1542 rows 22.6 / 24.2, 4 TB/s; 1542 of
+// 1024 9.4 / 9.9; between 149 and 400 rows of 4096 AHEAD would still win, 8.1 / 6.2 at 296, at other widths it does not).
+constexpr int kLnFewRows = 148;
 template <typename AT>
 static cudaError_t launch_ln(const LnAdd& a, int n, cudaStream_t st) {
   const void* ptrs[] = {a.x, a.y, a.post_w, a.post_b, a.add_rows, a.add_vec, a.h, a.next_w, a.next_b};
@@ -161,7 +187,8 @@ static cudaError_t launch_ln(const LnAdd& a, int n, cudaStream_t st) {
   for (const void* p : ptrs) vec = vec && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
   if (vec) {
     const int runs = a.W / 4, threads = runs >= 256 ? 256 : (runs + 31) / 32 * 32, nv = (runs + threads - 1) / threads;
-#define PIEH_LN(NV) launch_k(layernorm_add_kernel<AT, NV>, dim3(n), dim3(threads), 0, st, a)
+#define PIEH_LN(NV) (n <= kLnFewRows ? launch_k(layernorm_add_kernel<AT, NV, true>, dim3(n), dim3(threads), 0, st, a) \
+                                     : launch_k(layernorm_add_kernel<AT, NV, false>, dim3(n), dim3(threads), 0, st, a))
     return nv <= 1 ? PIEH_LN(1) : nv <= 2 ? PIEH_LN(2) : nv <= 4 ? PIEH_LN(4) : PIEH_LN(8);
 #undef PIEH_LN
   }

@@ -240,3 +240,23 @@ def test_embedding_rows_by_four_and_by_one(W, shift):
                                                  V, st), "embed_positions")
         want = table[tok.long()].float() + ptab[pos.long()].float()
         assert torch.equal(x, want) and torch.equal(act, want.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("W", [4, 1020, 2052, 4096, 8192])
+@pytest.mark.parametrize("rows", [148, 149])   # weights read ahead of the reductions, or behind them
+def test_layer_norms_of_few_and_many_rows(rows, W):
+    from proxy_inference_engine_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(W)
+    x, y = (torch.randn(rows, W, generator=g, device="cuda") for _ in range(2))
+    pw, pb, nw, nb = (torch.randn(W, generator=g, device="cuda") for _ in range(4))
+    ln = lambda v, w, b: (v - v.mean(-1, keepdim=True)) / (v.var(-1, unbiased=False, keepdim=True) + 1e-5).sqrt() * w.double() + b.double()
+    new = x.double() + ln(y.double(), pw, pb)
+    want, h = ln(new, nw, nb), torch.empty(rows, W, device="cuda")
+    _lib.check_hybrid(_lib.load_hybrid().pieh_layernorm_add(_p(x), _p(y), W, _p(pw), _p(pb), None, 0, None, _p(h), _lib.DTYPE_F32, _p(nw),
+                                                            _p(nb), None, 1e-5, rows, W, C.c_void_p(torch.cuda.current_stream().cuda_stream)),
+                      "layernorm_add")
+    # sums in runs of at most 64 values and then pairwise; a row of 4 may be nearly constant, and its norm then enlarges the error
+    # of the mean by 1 / sigma
+    sd = new.std(-1, unbiased=False, keepdim=True) if W > 1 else 1.0
+    size = new.abs().amax(-1, keepdim=True) * (1 + 1 / y.double().std(-1, unbiased=False, keepdim=True))
+    _within(h, want, 2 ** -24 * 80 * (size / sd) * (1 + (want - nb.double()).abs() + nw.double().abs()) + 2 ** -23 * want.abs())
