@@ -206,11 +206,16 @@ __global__ void __launch_bounds__(kRunWarps * 32) attn_run_kernel(OT* out, const
 }
 
 // ---- prompt portions on the tensor cores ---------------------------------------------------------------------------
-// A CTA of 4 warps owns one 64-row query tile (consecutive positions of ONE sequence) of one query head; key tiles are
-// whole pages (64 keys) from the first page the window reaches to the page of the tile's last row, double-buffered in
-// XOR-swizzled shared memory by cp.async.  Per map: S = Q_m K_m^T on mma.sync.m16n8k16 (bf16 in, fp32 out), scale,
-// soft cap, causal and window mask, online softmax in fp32 (exp2 domain), P rounded to bf16, O_m += P V.  Both maps walk
-// the same V tile.  The end combines the maps, normalises each row over its dv values and stores bf16.
+// A CTA owns one 64-row query tile (consecutive positions of ONE sequence) of one query head; key tiles are whole pages (64
+// keys) from the first page the window reaches to the page of the tile's last row, double-buffered in XOR-swizzled shared
+// memory by cp.async.  Warps 0-3 have the first map, warps 4-7 the second, 16 rows each: S = Q_m K_m^T on mma.sync.m16n8k16
+// (bf16 in, fp32 out), scale, soft cap, causal and window mask (only where some row does not see the whole page), online softmax
+// in fp32 (exp2 domain), P rounded to bf16, O_m += P V, both maps on the same V tile.  The end combines the maps through shared
+// memory, normalises each row over its dv values and stores bf16.
+// What bounds it is the latency of a warp's chain (products, softmax, products) per key tile: a warp with both maps needed 255
+// registers, which left two warps to a scheduler, and walked the maps one behind the other; with one map a warp and the query
+// fragments in shared memory it is four.  Tiles are dispatched last position first: the longest walks do not start last.
+// 1200 rows, 16 heads, d 64 per map, dv 128, window 1024: 139 -> 65 us.
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr) : "memory");
@@ -234,16 +239,32 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
 template <int ROWB>   // bytes of a tile row; 16-byte chunk c of row r sits at chunk c ^ (r & 7)
 __device__ __forceinline__ uint32_t tile_off(int r, int c) { return (uint32_t)(r * ROWB + ((c ^ (r & 7)) << 4)); }
 
+__device__ __forceinline__ float exp2_ftz(float x) {   // results below 2^-126 are 0
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+constexpr int kTileThreads = 256;
 template <int D, int DV>
-__global__ void __launch_bounds__(128) attn_tile_kernel(__nv_bfloat16* out, const float* q, const pieh_attn a,
-                                                        const pieh_batch b) {
-  constexpr int KC = D / 16, NT = 8, DT = DV / 8;
-  constexpr int KROWB = 2 * D * 2, VROWB = DV * 2;
-  constexpr int KTILE = 64 * KROWB, VTILE = 64 * VROWB;
+struct TileSmem {
+  static constexpr int KROWB = 2 * D * 2, VROWB = DV * 2, K = 64 * KROWB, V = 64 * VROWB;
+  static constexpr int Q = 2 * (K + V);                 // behind two stages of keys and values
+  static constexpr int BYTES = Q + 64 * KROWB;
+  static constexpr int COMB_LD = DV + 8;                // the second map's rows, over the stages at the end
+  static_assert(64 * COMB_LD * 4 <= BYTES, "");
+};
+
+template <int D, int DV>
+__global__ void __launch_bounds__(kTileThreads, 2) attn_tile_kernel(__nv_bfloat16* out, const float* q, const pieh_attn a,
+                                                                    const pieh_batch b) {
+  using T = TileSmem<D, DV>;
+  constexpr int KC = D / 16, NT = 8, DT = DV / 8, KROWB = T::KROWB, VROWB = T::VROWB;
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_sync();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-  const int tile = blockIdx.x, h = blockIdx.y;
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  const int mp = tid >> 7, warp = (tid >> 5) & 3;
+  const int h = blockIdx.x % a.H, tile = b.n_tiles - 1 - blockIdx.x / a.H;
   const int i = b.tile_seq[tile], row0 = b.tile_row[tile];
   const int nrows = min(64, b.seq_start[i] + b.seq_len[i] - row0);
   const int pos0 = b.tok_pos[row0];
@@ -254,17 +275,17 @@ __global__ void __launch_bounds__(128) attn_tile_kernel(__nv_bfloat16* out, cons
   const int32_t* table = b.block_table + (size_t)i * b.bt_stride;
   const __nv_bfloat16* kpool = reinterpret_cast<const __nv_bfloat16*>(a.k_pages);
   const __nv_bfloat16* vpool = reinterpret_cast<const __nv_bfloat16*>(a.v_pages);
-  const uint32_t sK = (uint32_t)__cvta_generic_to_shared(smem), sV = sK + 2 * KTILE;
+  const uint32_t sK = (uint32_t)__cvta_generic_to_shared(smem), sV = sK + 2 * T::K, sQ = sK + T::Q;
 
   auto issue = [&](int j) {
     const size_t page = (size_t)table[j] * kPage;
-    const uint32_t dk = sK + ((j - j_lo) & 1) * KTILE, dvv = sV + ((j - j_lo) & 1) * VTILE;
+    const uint32_t dk = sK + ((j - j_lo) & 1) * T::K, dvv = sV + ((j - j_lo) & 1) * T::V;
     constexpr int CK = KROWB / 16, CV = VROWB / 16;
-    for (int e = tid; e < 64 * CK; e += 128) {
+    for (int e = tid; e < 64 * CK; e += kTileThreads) {
       const int r = e / CK, c = e - r * CK;
       cp16(dk + tile_off<KROWB>(r, c), kpool + ((page + r) * a.G + kvh) * (2 * D) + c * 8);
     }
-    for (int e = tid; e < 64 * CV; e += 128) {
+    for (int e = tid; e < 64 * CV; e += kTileThreads) {
       const int r = e / CV, c = e - r * CV;
       cp16(dvv + tile_off<VROWB>(r, c), vpool + ((page + r) * a.G + kvh) * DV + c * 8);
     }
@@ -272,129 +293,138 @@ __global__ void __launch_bounds__(128) attn_tile_kernel(__nv_bfloat16* out, cons
   };
   issue(j_lo);
 
-  // Q fragments of both maps: rows 16 warp + g and + 8 of the tile (rows past the tile's end repeat its last row)
-  const int r0 = warp * 16 + g, r1 = r0 + 8;
-  uint32_t qf[2][KC][4];
-#pragma unroll
-  for (int mp = 0; mp < 2; ++mp) {
-    const float* q0 = q + (((size_t)(row0 + min(r0, nrows - 1)) * a.H + h) * 2 + mp) * D;
-    const float* q1 = q + (((size_t)(row0 + min(r1, nrows - 1)) * a.H + h) * 2 + mp) * D;
-#pragma unroll
-    for (int kc = 0; kc < KC; ++kc) {
-      const float2 x0 = *reinterpret_cast<const float2*>(q0 + kc * 16 + 2 * t4);
-      const float2 x1 = *reinterpret_cast<const float2*>(q1 + kc * 16 + 2 * t4);
-      const float2 x2 = *reinterpret_cast<const float2*>(q0 + kc * 16 + 8 + 2 * t4);
-      const float2 x3 = *reinterpret_cast<const float2*>(q1 + kc * 16 + 8 + 2 * t4);
-      qf[mp][kc][0] = pack2(x0.x, x0.y); qf[mp][kc][1] = pack2(x1.x, x1.y);
-      qf[mp][kc][2] = pack2(x2.x, x2.y); qf[mp][kc][3] = pack2(x3.x, x3.y);
-    }
+  // Q of both maps as bf16 (rows past the tile's end repeat its last row); the fragments are read again for every key tile
+  for (int e = tid; e < 64 * (2 * D / 8); e += kTileThreads) {
+    const int r = e / (2 * D / 8), c = e - r * (2 * D / 8);
+    const float* src = q + ((size_t)(row0 + min(r, nrows - 1)) * a.H + h) * 2 * D + c * 8;
+    const float2 x0 = *reinterpret_cast<const float2*>(src), x1 = *reinterpret_cast<const float2*>(src + 2);
+    const float2 x2 = *reinterpret_cast<const float2*>(src + 4), x3 = *reinterpret_cast<const float2*>(src + 6);
+    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(sQ + tile_off<KROWB>(r, c)), "r"(pack2(x0.x, x0.y)), "r"(pack2(x1.x, x1.y)),
+                 "r"(pack2(x2.x, x2.y)), "r"(pack2(x3.x, x3.y)) : "memory");
   }
-  float o[2][DT][4];
+  const int r0 = warp * 16 + g, r1 = r0 + 8;
+  float o[DT][4];
 #pragma unroll
-  for (int mp = 0; mp < 2; ++mp)
-#pragma unroll
-    for (int x = 0; x < DT; ++x) o[mp][x][0] = o[mp][x][1] = o[mp][x][2] = o[mp][x][3] = 0.f;
-  float mrun[2][2] = {{-INFINITY, -INFINITY}, {-INFINITY, -INFINITY}}, lrun[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+  for (int x = 0; x < DT; ++x) o[x][0] = o[x][1] = o[x][2] = o[x][3] = 0.f;
+  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
   const int p0 = pos0 + min(r0, nrows - 1), p1 = pos0 + min(r1, nrows - 1);   // positions of this thread's two rows
   const int w0 = a.window > 0 ? p0 - a.window + 1 : 0, w1 = a.window > 0 ? p1 - a.window + 1 : 0;
   constexpr float kLog2e = 1.4426950408889634f;
+  // scores in log2 units: cap tanh(v / cap) = cap (1 - 2 / (exp(2 v / cap) + 1)), absolute error ~1e-7 of cap
+  const float lin = a.scale * kLog2e, cap = a.softcap * kLog2e, arg = a.softcap > 0.f ? 2.f * lin / a.softcap : 0.f;
+  const uint32_t q_row = warp * 16 + (lane & 15), q_chunk = mp * (D / 8) + (lane >> 4);
 
   for (int j = j_lo; j <= j_hi; ++j) {
     if (j < j_hi) { issue(j + 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
     else asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    const uint32_t tk = sK + ((j - j_lo) & 1) * KTILE, tv = sV + ((j - j_lo) & 1) * VTILE;
+    const uint32_t tk = sK + ((j - j_lo) & 1) * T::K, tv = sV + ((j - j_lo) & 1) * T::V;
+    float s[NT][4];
 #pragma unroll
-    for (int mp = 0; mp < 2; ++mp) {
-      float s[NT][4];
+    for (int n = 0; n < NT; ++n) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; }
 #pragma unroll
-      for (int n = 0; n < NT; ++n) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; }
-#pragma unroll
-      for (int n = 0; n < NT; ++n) {
-#pragma unroll
-        for (int kc = 0; kc < KC; kc += 2) {
-          uint32_t b0, b1, b2, b3;
-          ldsm_x4(tk + tile_off<KROWB>(n * 8 + (lane & 7), mp * (D / 8) + kc * 2 + (lane >> 3)), b0, b1, b2, b3);
-          mma_16816(s[n], qf[mp][kc][0], qf[mp][kc][1], qf[mp][kc][2], qf[mp][kc][3], b0, b1);
-          mma_16816(s[n], qf[mp][kc + 1][0], qf[mp][kc + 1][1], qf[mp][kc + 1][2], qf[mp][kc + 1][3], b2, b3);
-        }
-      }
-      const int key0 = j * kPage + 2 * t4;
-      float mx0 = -INFINITY, mx1 = -INFINITY;
+    for (int kc = 0; kc < KC; kc += 2) {
+      uint32_t a0, a1, a2, a3, c0, c1, c2, c3;
+      ldsm_x4(sQ + tile_off<KROWB>(q_row, q_chunk + 2 * kc), a0, a1, a2, a3);
+      ldsm_x4(sQ + tile_off<KROWB>(q_row, q_chunk + 2 * kc + 2), c0, c1, c2, c3);
 #pragma unroll
       for (int n = 0; n < NT; ++n) {
-        const int k = key0 + n * 8;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float v = s[n][e] * a.scale;
-          if (a.softcap > 0.f) v = a.softcap * (1.f - __fdividef(2.f, __expf(2.f * v / a.softcap) + 1.f));   // tanh, abs error ~1e-7
-          const int key = k + (e & 1), pr = e < 2 ? p0 : p1, wl = e < 2 ? w0 : w1;
-          s[n][e] = (key <= pr && key >= wl) ? v * kLog2e : -INFINITY;
-        }
-        mx0 = fmaxf(mx0, fmaxf(s[n][0], s[n][1]));
-        mx1 = fmaxf(mx1, fmaxf(s[n][2], s[n][3]));
-      }
-      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-      if (mx0 > mrun[mp][0]) {
-        const float c = exp2f(mrun[mp][0] - mx0);   // running maximum -inf: 0, and everything it multiplies is 0
-        lrun[mp][0] *= c;
-#pragma unroll
-        for (int x = 0; x < DT; ++x) { o[mp][x][0] *= c; o[mp][x][1] *= c; }
-        mrun[mp][0] = mx0;
-      }
-      if (mx1 > mrun[mp][1]) {
-        const float c = exp2f(mrun[mp][1] - mx1);
-        lrun[mp][1] *= c;
-#pragma unroll
-        for (int x = 0; x < DT; ++x) { o[mp][x][2] *= c; o[mp][x][3] *= c; }
-        mrun[mp][1] = mx1;
-      }
-      const float ms0 = mrun[mp][0] == -INFINITY ? 0.f : mrun[mp][0], ms1 = mrun[mp][1] == -INFINITY ? 0.f : mrun[mp][1];
-      float ps0 = 0.f, ps1 = 0.f;
-      uint32_t pf[NT][2];
-#pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        const float e0 = exp2f(s[n][0] - ms0), e1 = exp2f(s[n][1] - ms0);
-        const float e2 = exp2f(s[n][2] - ms1), e3 = exp2f(s[n][3] - ms1);
-        ps0 += e0 + e1; ps1 += e2 + e3;
-        pf[n][0] = pack2(e0, e1);
-        pf[n][1] = pack2(e2, e3);
-      }
-      lrun[mp][0] += ps0; lrun[mp][1] += ps1;
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        const uint32_t a0 = pf[2 * kk][0], a1 = pf[2 * kk][1], a2 = pf[2 * kk + 1][0], a3 = pf[2 * kk + 1][1];
-#pragma unroll
-        for (int dj = 0; dj < DT; dj += 2) {
-          uint32_t b0, b1, b2, b3;
-          ldsm_x4_trans(tv + tile_off<VROWB>(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, dj + (lane >> 4)), b0, b1, b2, b3);
-          mma_16816(o[mp][dj], a0, a1, a2, a3, b0, b1);
-          mma_16816(o[mp][dj + 1], a0, a1, a2, a3, b2, b3);
-        }
+        uint32_t b0, b1, b2, b3;
+        ldsm_x4(tk + tile_off<KROWB>(n * 8 + (lane & 7), mp * (D / 8) + kc * 2 + (lane >> 3)), b0, b1, b2, b3);
+        mma_16816(s[n], a0, a1, a2, a3, b0, b1);
+        mma_16816(s[n], c0, c1, c2, c3, b2, b3);
       }
     }
+    if (a.softcap > 0.f) {
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[n][e] = cap * (1.f - __fdividef(2.f, exp2_ftz(s[n][e] * arg) + 1.f));
+    } else {
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[n][e] *= lin;
+    }
+    if (j * kPage + kPage - 1 > pos0 || (a.window > 0 && j * kPage < last_key - a.window + 1)) {   // some row does not see all keys
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int key = j * kPage + n * 8 + 2 * t4 + (e & 1);
+          if (key > (e < 2 ? p0 : p1) || key < (e < 2 ? w0 : w1)) s[n][e] = -INFINITY;
+        }
+    }
+    float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      mx0 = fmaxf(mx0, fmaxf(s[n][0], s[n][1]));
+      mx1 = fmaxf(mx1, fmaxf(s[n][2], s[n][3]));
+    }
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+    if (mx0 > m0) {
+      const float c = exp2_ftz(m0 - mx0);   // running maximum -inf: 0, and everything it multiplies is 0
+      l0 *= c;
+#pragma unroll
+      for (int x = 0; x < DT; ++x) { o[x][0] *= c; o[x][1] *= c; }
+      m0 = mx0;
+    }
+    if (mx1 > m1) {
+      const float c = exp2_ftz(m1 - mx1);
+      l1 *= c;
+#pragma unroll
+      for (int x = 0; x < DT; ++x) { o[x][2] *= c; o[x][3] *= c; }
+      m1 = mx1;
+    }
+    const float ms0 = m0 == -INFINITY ? 0.f : m0, ms1 = m1 == -INFINITY ? 0.f : m1;
+    float ps0 = 0.f, ps1 = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      uint32_t pf[2][2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float e0 = exp2_ftz(s[2 * kk + u][0] - ms0), e1 = exp2_ftz(s[2 * kk + u][1] - ms0);
+        const float e2 = exp2_ftz(s[2 * kk + u][2] - ms1), e3 = exp2_ftz(s[2 * kk + u][3] - ms1);
+        ps0 += e0 + e1; ps1 += e2 + e3;
+        pf[u][0] = pack2(e0, e1);
+        pf[u][1] = pack2(e2, e3);
+      }
+#pragma unroll
+      for (int dj = 0; dj < DT; dj += 2) {
+        uint32_t b0, b1, b2, b3;
+        ldsm_x4_trans(tv + tile_off<VROWB>(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, dj + (lane >> 4)), b0, b1, b2, b3);
+        mma_16816(o[dj], pf[0][0], pf[0][1], pf[1][0], pf[1][1], b0, b1);
+        mma_16816(o[dj + 1], pf[0][0], pf[0][1], pf[1][0], pf[1][1], b2, b3);
+      }
+    }
+    l0 += ps0; l1 += ps1;
     __syncthreads();   // the stage is refilled two iterations from now
   }
   // ---- combine the maps, unit rms over the row's dv values, store --------------------------------------------------
-  float inv[2][2];
+  l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+  l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+  const float inv0 = 1.f / l0, inv1 = 1.f / l1;
+  float* const other = reinterpret_cast<float*>(smem);
+  if (mp == 1) {
 #pragma unroll
-  for (int mp = 0; mp < 2; ++mp)
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-      float l = lrun[mp][rr];
-      l += __shfl_xor_sync(0xffffffffu, l, 1); l += __shfl_xor_sync(0xffffffffu, l, 2);
-      inv[mp][rr] = 1.f / l;
+    for (int x = 0; x < DT; ++x) {
+      const int c = x * 8 + 2 * t4;
+      *reinterpret_cast<float2*>(other + r0 * T::COMB_LD + c) = make_float2(a.lambda * o[x][0] * inv0, a.lambda * o[x][1] * inv0);
+      *reinterpret_cast<float2*>(other + r1 * T::COMB_LD + c) = make_float2(a.lambda * o[x][2] * inv1, a.lambda * o[x][3] * inv1);
     }
+  }
+  __syncthreads();
+  if (mp == 1) return;
   float ss0 = 0.f, ss1 = 0.f;
 #pragma unroll
   for (int x = 0; x < DT; ++x) {
-    o[0][x][0] = o[0][x][0] * inv[0][0] - a.lambda * o[1][x][0] * inv[1][0];
-    o[0][x][1] = o[0][x][1] * inv[0][0] - a.lambda * o[1][x][1] * inv[1][0];
-    o[0][x][2] = o[0][x][2] * inv[0][1] - a.lambda * o[1][x][2] * inv[1][1];
-    o[0][x][3] = o[0][x][3] * inv[0][1] - a.lambda * o[1][x][3] * inv[1][1];
-    ss0 += o[0][x][0] * o[0][x][0] + o[0][x][1] * o[0][x][1];
-    ss1 += o[0][x][2] * o[0][x][2] + o[0][x][3] * o[0][x][3];
+    const int c = x * 8 + 2 * t4;
+    const float2 u0 = *reinterpret_cast<const float2*>(other + r0 * T::COMB_LD + c), u1 = *reinterpret_cast<const float2*>(other + r1 * T::COMB_LD + c);
+    o[x][0] = o[x][0] * inv0 - u0.x; o[x][1] = o[x][1] * inv0 - u0.y;
+    o[x][2] = o[x][2] * inv1 - u1.x; o[x][3] = o[x][3] * inv1 - u1.y;
+    ss0 += o[x][0] * o[x][0] + o[x][1] * o[x][1];
+    ss1 += o[x][2] * o[x][2] + o[x][3] * o[x][3];
   }
   ss0 += __shfl_xor_sync(0xffffffffu, ss0, 1); ss0 += __shfl_xor_sync(0xffffffffu, ss0, 2);
   ss1 += __shfl_xor_sync(0xffffffffu, ss1, 1); ss1 += __shfl_xor_sync(0xffffffffu, ss1, 2);
@@ -402,14 +432,14 @@ __global__ void __launch_bounds__(128) attn_tile_kernel(__nv_bfloat16* out, cons
 #pragma unroll
   for (int x = 0; x < DT; ++x) {
     const int c = x * 8 + 2 * t4;
-    if (r0 < nrows) *reinterpret_cast<uint32_t*>(out + ((size_t)(row0 + r0) * a.H + h) * DV + c) = pack2(o[0][x][0] * n0, o[0][x][1] * n0);
-    if (r1 < nrows) *reinterpret_cast<uint32_t*>(out + ((size_t)(row0 + r1) * a.H + h) * DV + c) = pack2(o[0][x][2] * n1, o[0][x][3] * n1);
+    if (r0 < nrows) *reinterpret_cast<uint32_t*>(out + ((size_t)(row0 + r0) * a.H + h) * DV + c) = pack2(o[x][0] * n0, o[x][1] * n0);
+    if (r1 < nrows) *reinterpret_cast<uint32_t*>(out + ((size_t)(row0 + r1) * a.H + h) * DV + c) = pack2(o[x][2] * n1, o[x][3] * n1);
   }
 }
 
 template <int D, int DV>
 static cudaError_t launch_tile(__nv_bfloat16* out, const float* q, const pieh_attn& a, const pieh_batch& b, cudaStream_t st) {
-  constexpr int smem = 2 * (64 * 2 * D * 2 + 64 * DV * 2);
+  constexpr int smem = TileSmem<D, DV>::BYTES;
   static unsigned long long configured = 0;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -418,14 +448,14 @@ static cudaError_t launch_tile(__nv_bfloat16* out, const float* q, const pieh_at
     if (e != cudaSuccess) return e;
     configured |= 1ull << (dev & 63);
   }
-  return launch_k(attn_tile_kernel<D, DV>, dim3(b.n_tiles, a.H), dim3(128), smem, st, out, q, a, b);
+  return launch_k(attn_tile_kernel<D, DV>, dim3((unsigned)(a.H * b.n_tiles)), dim3(kTileThreads), smem, st, out, q, a, b);
 }
 
 // the tile kernel serves steps that are mostly prompt portions, over bf16 pages, at the head sizes it is built for
 static bool tile_ok(const pieh_attn& a, const pieh_batch& b, int out_dtype) {
   static const bool off = [] { const char* e = getenv("PIE_HYBRID_NO_TILE_ATTN"); return e && e[0] == '1'; }();
   return !off && a.kv_dtype == PIE_DTYPE_BF16 && out_dtype == PIE_DTYPE_BF16 && (a.d == 32 || a.d == 64) &&
-         (a.dv == 64 || a.dv == 128) && b.n_tiles > 0 && b.tile_seq && b.tile_row && a.H <= 65535 &&
+         (a.dv == 64 || a.dv == 128) && b.n_tiles > 0 && b.tile_seq && b.tile_row && (long long)a.H * b.n_tiles <= 0x7fffffff &&
          (long long)b.T >= 16LL * b.n_seq;
 }
 
