@@ -101,6 +101,11 @@ int pie_qmv_fused(void* out, int out_ld, const void* x, int x_ld, int M, int K, 
  * Same contraction and workspace contract as pie_qmv.  x bf16 [M, K] row-major, y bf16 [M, N].           */
 int pie_qmm(void* y, const void* x, const uint32_t* wq, const void* scales, const void* biases, int M, int N,
             int K, int group_size, int bits, void* workspace, size_t workspace_bytes, void* stream);
+/* y = silu(x gate^T) * (x up^T), each product, the sigmoid, silu and y rounded to bf16: pie_qmm twice and pie_silu_mul in one launch.
+ * gate_up: two matrices of the same N.  PIE_EUNSUPPORTED (nothing launched) where those three calls serve the shape better (_pays
+ * says 0) or alone. */
+int pie_qmm_swiglu_pays(int M, int N, int K, int group_size, int bits);
+int pie_qmm_swiglu(void* y, const void* x, const pie_qmv_seg* gate_up, int M, int K, int group_size, int bits, void* stream);
 
 /* ---- a6  mx.fast.rms_norm (MLX/mlx/fast.cpp:56-123; kernels/rms_norm.metal:13-81) -------------------- */
 int pie_rms_norm(void* out, const void* x, const void* weight, long long rows, int dims, float eps,

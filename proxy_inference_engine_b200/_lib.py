@@ -16,6 +16,7 @@ CSRC = os.path.join(_HERE, "csrc")
 PIE_OK = 0
 STATUS = {1: "EINVAL_SHAPE", 2: "EINVAL_DTYPE", 3: "EUNSUPPORTED", 4: "ECUDA", 5: "ENULL", 6: "EALIGN",
           7: "EWORKSPACE", 8: "ESTATIC_LIMIT"}
+EUNSUPPORTED = 3
 EPI_STORE, EPI_RESADD, EPI_SILUMUL = 0, 1, 2
 DTYPE_BF16, DTYPE_F32 = 0, 1
 
@@ -86,6 +87,8 @@ SIGNATURES = {
     "pie_qmv": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _sz, _vp]),
     "pie_qmv_fused": (_i, [_vp, _i, _vp, _i, _i, _i, C.POINTER(QmvSeg), _i, _i, _i, _vp, _f, _i, _vp, _i, _vp,
                            _sz, _i, _vp]),
+    "pie_qmm_swiglu_pays": (_i, [_i, _i, _i, _i, _i]),
+    "pie_qmm_swiglu": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "pie_qmm": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _sz, _vp]),
     "pie_rms_norm": (_i, [_vp, _vp, _vp, _ll, _i, _f, _vp]),
     "pie_rope": (_i, [_vp, _vp, _ll, _i, _i, _i, _i, _f, _f, _i, _vp, _vp]),

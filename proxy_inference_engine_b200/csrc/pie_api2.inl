@@ -30,6 +30,29 @@ int pie_qmm(void* y, const void* x, const uint32_t* wq, const void* scales, cons
   return pie_qmv(y, x, wq, scales, biases, M, N, K, group_size, bits, workspace, workspace_bytes, stream);
 }
 
+int pie_qmm_swiglu_pays(int M, int N, int K, int group_size, int bits) {
+  return M >= 64 && N > 0 && K > 0 && K % 128 == 0 && quant_supported(group_size, bits) && qmm_swiglu_pays(M, N, K);
+}
+// silu(x w_gate^T) * (x w_up^T) on the same tile kernel.  Another status than PIE_OK: nothing was launched.
+int pie_qmm_swiglu(void* y, const void* x, const pie_qmv_seg* gate_up, int M, int K, int group_size, int bits, void* stream) {
+  if (!y || !x || !gate_up || !gate_up[0].wq || !gate_up[1].wq || !gate_up[0].scales || !gate_up[1].scales || !gate_up[0].biases ||
+      !gate_up[1].biases)
+    return PIE_ENULL;
+  const int N = gate_up[0].N;
+  if (M < 0 || N < 0 || K <= 0 || gate_up[1].N != N) return PIE_EINVAL_SHAPE;
+  if (M == 0 || N == 0) return PIE_OK;
+  if (M < 64 || !quant_supported(group_size, bits) || K % 128 || !aligned16(x) || !aligned16(y) || env_int("PIE_QMM_TC", 1) == 0)
+    return PIE_EUNSUPPORTED;
+  const uint32_t* wq[2];
+  const uint16_t *s[2], *b[2];
+  for (int i = 0; i < 2; ++i) {
+    wq[i] = gate_up[i].wq; s[i] = (const uint16_t*)gate_up[i].scales; b[i] = (const uint16_t*)gate_up[i].biases;
+    if (!aligned16(wq[i]) || ((reinterpret_cast<uintptr_t>(s[i]) | reinterpret_cast<uintptr_t>(b[i])) & 3)) return PIE_EUNSUPPORTED;
+  }
+  const cudaError_t e = launch_qmm_swiglu((uint16_t*)y, (const uint16_t*)x, wq, s, b, M, N, K, bits, (cudaStream_t)stream);
+  return e == cudaErrorNotSupported ? PIE_EUNSUPPORTED : cuda_status(e);
+}
+
 int pie_rms_norm(void* out, const void* x, const void* weight, long long rows, int dims, float eps, void* stream) {
   if (rows == 0) return PIE_OK;
   if (!out || !x) return PIE_ENULL;

@@ -51,11 +51,6 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
 __device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
 }
-__device__ __forceinline__ bool elect_one() {   // one lane of the (converged) warp
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
-  return p != 0;
-}
 constexpr uint32_t kGemmWaitLimit = 1u << 22;
 // false: the wait expired here or the CTA is already leaving
 __device__ __forceinline__ bool gemm_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
@@ -176,6 +171,12 @@ __device__ __forceinline__ GemmTileAt gemm_tile_at(const GemmArgs& a, int t) {
   return {z, first + rr % gm, rr / gm};
 }
 
+// An epilogue with a member PAIRED works on two products of one x: CTA 0 of a pair stages rows of w, CTA 1 the same rows of a second
+// matrix (map_up, s_up, b_up), so a tile's accumulator holds BN / 2 columns of the one and behind them the same columns of the other.
+// It is called as gate(v, t) on 32 columns of the first product and then, t in hand, on those of the second.
+template <class E, class = void> struct gemm_paired { static constexpr bool value = false; };
+template <class E> struct gemm_paired<E, decltype((void)E::PAIRED)> { static constexpr bool value = true; };
+
 // Epi: void operator()(int z, int row0, int col0, const uint32_t (&v)[32], uint32_t buf, int lane), called by whole warps: 32 columns
 // of rows row0 .. row0 + 31, lane l holding row l's; any row and column, the callee checks the bounds.  buf: 4 KB of shared memory
 // of the warp's own, to turn the tile so that rows are written in whole runs.
@@ -184,6 +185,9 @@ __global__ void __launch_bounds__(GemmTile<CG, BN, QB, SPLIT>::THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ GemmArgs a,
             const __grid_constant__ Epi epi) {
   using T = GemmTile<CG, BN, QB, SPLIT>;
+  constexpr bool PAIRED = gemm_paired<Epi>::value;
+  static_assert(!PAIRED || (CG == 2 && QB && T::NB % 32 == 0), "each CTA of a pair stages one matrix, in whole runs");
+  constexpr int COLS = PAIRED ? T::NB : BN;   // columns of y in a tile
   constexpr int S = T::S, RING = T::RING > 0 ? T::RING : 1, KPC = QB == 4 ? 4 : 2;   // K steps per packed chunk
   constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(T::BM >> 4) << 24);
   extern __shared__ uint8_t smem_raw[];
@@ -255,10 +259,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int row0 = at.m * T::BM + (int)(CG == 2 ? rank : 0) * 128 + quad * 32;
 #pragma unroll 1
-        for (int c = 0; c < RUNS; ++c) {
-          uint32_t v[32];
-          tmem_ld32(tmem + (uint32_t)(b * T::ACC + (c_lo + c) * 32) + ((uint32_t)(quad * 32) << 16), v);
-          if (c == RUNS - 1) {   // the accumulator may be overwritten
+        for (int c = 0; c < (PAIRED ? RUNS / 2 : RUNS); ++c) {
+          uint32_t v[32], t[PAIRED ? 16 : 1];
+          const uint32_t run = tmem + (uint32_t)(b * T::ACC + (c_lo + c) * 32) + ((uint32_t)(quad * 32) << 16);
+          tmem_ld32(run, v);
+          if constexpr (PAIRED) {
+            epi.gate(v, t);
+            tmem_ld32(run + T::NB, v);
+          }
+          if (c == (PAIRED ? RUNS / 2 : RUNS) - 1) {   // the accumulator may be overwritten
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) {
@@ -266,7 +275,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
               else mbar_arrive(&tempty_bar[b]);
             }
           }
-          epi(at.z, row0, at.n * BN + (c_lo + c) * 32, v, ebuf, lane);
+          if constexpr (PAIRED) epi(row0, at.n * COLS + c * 32, t, v, ebuf, lane);
+          else epi(at.z, row0, at.n * BN + (c_lo + c) * 32, v, ebuf, lane);
         }
       }
     } else {
@@ -331,12 +341,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
       bool alive = true;
       for (int t = first_tile; t < ntiles && alive; t += tile_step) {
         const GemmTileAt at = gemm_tile_at(a, t);
-        const int col = at.n * BN + (int)(CG == 2 ? rank : 0) * T::NB;
+        const int col = at.n * COLS + (int)(CG == 2 && !PAIRED ? rank : 0) * T::NB;
         for (int kb = k_lo; kb < k_hi; kb += KPC, ++pc) {
           const int p = pc % RING;
           if (!(alive = gemm_wait(smem_u32(&pempty_bar[p]), ((pc / RING) & 1) ^ 1, abortp))) break;
           mbar_arrive_expect_tx(&pfull_bar[p], T::CHUNK);
-          gemm_tma_3d<1>(smP + p * T::CHUNK, &map_w, smem_u32(&pfull_bar[p]), kb / KPC * 128, col, 0);
+          const CUtensorMap* map = &map_w;
+          if constexpr (PAIRED) map = rank ? &epi.map_up : &map_w;
+          gemm_tma_3d<1>(smP + p * T::CHUNK, map, smem_u32(&pfull_bar[p]), kb / KPC * 128, col, 0);
         }
         if (SPLIT) break;
       }
@@ -352,9 +364,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     bool alive = true;
     for (int t = first_tile; t < ntiles && alive; t += tile_step, it0 += k_hi - k_lo, pc0 += chunks) {
       const GemmTileAt at = gemm_tile_at(a, t);
-      const int row = min(at.n * BN + (int)(CG == 2 ? rank : 0) * T::NB + min(r, T::NB - 1), a.N - 1);
-      const uint16_t* sp = a.scales + (size_t)row * nk_all;
-      const uint16_t* bp = a.biases + (size_t)row * nk_all;
+      const int row = min(at.n * COLS + (int)(CG == 2 && !PAIRED ? rank : 0) * T::NB + min(r, T::NB - 1), a.N - 1);
+      const uint16_t *sp = a.scales, *bp = a.biases;
+      if constexpr (PAIRED)
+        if (rank) { sp = epi.s_up; bp = epi.b_up; }
+      sp += (size_t)row * nk_all;
+      bp += (size_t)row * nk_all;
       int kb = k_lo + (grp + T::GROUPS - it0 % T::GROUPS) % T::GROUPS;
       uint4 sv = make_uint4(0, 0, 0, 0), bv = sv, sn = sv, bn = sv;   // scale_vec: eight K steps' values, and the next eight
       uint32_t s_next = 0, b_next = 0;                      // otherwise: the next step's
@@ -468,8 +483,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         }
 #pragma unroll
         for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(acc[q]);
-        epi(at.z, at.m * T::BM + (warp & 3) * 32, at.n * BN + (gi * (int)ranks + (int)rank) * 32, v,
-            smP + T::RING * T::CHUNK + warp * 4096, lane);
+        if constexpr (!PAIRED)
+          epi(at.z, at.m * T::BM + (warp & 3) * 32, at.n * BN + (gi * (int)ranks + (int)rank) * 32, v,
+              smP + T::RING * T::CHUNK + warp * 4096, lane);
       }
     }
   }
@@ -510,24 +526,24 @@ inline bool gemm_map(CUtensorMap* m, const void* p, int elem_bytes, long long in
 }
 
 // Measured, B200, 4-bit weights, us (TFLOP/s) with the 256 x 256 tile of one CTA, cp.async producers and no overlap of the
-// epilogue that this replaced -> here: 8192 x 14336 x 4096 1590 (605) -> 785 (1226); 1000 rows 290 -> 122; 256 rows -> 40; 77 rows
-// 400 -> 34; 77 x 4096 x 14336 720 -> 35 (four ranks).  bf16 weights: 8192 x 28672 x 4096 -> 1370 (1404).
+// epilogue that this replaced -> here: 8192 x 14336 x 4096 1590 (605) -> 676 (1424); 1000 rows 290 -> 97; 200 rows 29; 77 rows 400 -> 27;
+// 77 x 4096 x 14336 720 -> 29 (a cluster's ranks).  8 bits, 1000 rows: 280 -> 111.  bf16 weights: 8192 x 4096 x 4096 179 (1537).
 // The tile for a shape: a pair's 256 x {256, 224, 192, 128}, or a single CTA's 128 x 128 with K over 1..4 ranks of a cluster --
 // whichever the estimate (waves x K steps x SM cycles of a step, and the fixed cost of a cluster's reduction) says is done first.
 // The steps' cycles are measured (1.9 GHz; waves x 64 steps of N 14336, M 1000): pairs with bf16 weights 720 / 612 / 575 for BN = 256 /
 // 192 / 128, dequantised 770 / 765 / 680 / 630 for 256 / 224 / 192 / 128, single CTAs 580 and 650.  Over 190 shapes (M 77 to 3000) the
 // choice takes 1.02 times the best tile's time on average.
-struct GemmChoice { int pair, bn, ranks, k_per, mt, nt; };
+struct GemmChoice { int pair, bn, ranks, k_per, mt, nt; double cycles; };
+inline double gemm_pair_step(int bn, bool quant) { return quant ? 490 + 280 * bn / 256.0 : 430 + 290 * bn / 256.0; }
 inline GemmChoice gemm_choose(int M, int N, int K, int nb, int sms, bool quant) {
   auto up = [](long long a, long long b) { return (a + b - 1) / b; };
   const long long nk = K / 64;
-  GemmChoice best = {1, 256, 1, (int)nk, (int)up(M, 256), (int)up(N, 256)};
-  double cost = 1e30;
+  GemmChoice best = {1, 256, 1, (int)nk, (int)up(M, 256), (int)up(N, 256), 1e30};
   for (int bn : {256, 224, 192, 128}) {
     if (bn == 224 && !quant) continue;   // (the eight epilogue warps of the dense kernel share 64-column runs)
     const long long tiles = up(M, 256) * up(N, bn) * nb;
-    const double c = (double)up(tiles, sms / 2) * nk * (quant ? 490 + 280 * bn / 256.0 : 430 + 290 * bn / 256.0);
-    if (c < cost) { cost = c; best = {1, bn, 1, (int)nk, (int)up(M, 256), (int)up(N, bn)}; }
+    const double c = (double)up(tiles, sms / 2) * nk * gemm_pair_step(bn, quant);
+    if (c < best.cycles) best = {1, bn, 1, (int)nk, (int)up(M, 256), (int)up(N, bn), c};
   }
   const long long tiles = up(M, 128) * up(N, 128) * nb;
   const double step = quant ? 650 : 580;
@@ -537,7 +553,7 @@ inline GemmChoice gemm_choose(int M, int N, int K, int nb, int sms, bool quant) 
     // clusters of three or four do not fill every SM: what is resident at once was 128 CTAs and more for four, not 144 for three
     const long long slots = r == 3 ? sms * 3 / 4 : r == 4 ? sms * 7 / 8 : sms;
     const double c = (double)up(tiles * r, slots) * (per * step + (r > 1 ? 4500 : 0));
-    if (c < cost) { cost = c; best = {0, 128, r, (int)per, (int)up(M, 128), (int)up(N, 128)}; }
+    if (c < best.cycles) best = {0, 128, r, (int)per, (int)up(M, 128), (int)up(N, 128), c};
   }
   return best;
 }
@@ -587,6 +603,29 @@ cudaError_t gemm_run(GemmArgs a, const Epi& epi, const void* x, long long x_pitc
   if (c.bn == 256) return gemm_launch<2, 256, QB, false>(mx, mw, a, epi, 1, sms, st);
   if constexpr (QB != 0)
     if (c.bn == 224) return gemm_launch<2, 224, QB, false>(mx, mw, a, epi, 1, sms, st);
+  return c.bn == 192 ? gemm_launch<2, 192, QB, false>(mx, mw, a, epi, 1, sms, st) : gemm_launch<2, 128, QB, false>(mx, mw, a, epi, 1, sms, st);
+}
+
+// Two products of one x in pairs' tiles (an Epi with PAIRED), of 256, 192 or 128 columns.  bn = 0: not worth it.
+inline GemmChoice gemm_choose_paired(int M, int N, int K, int sms, double apart) {
+  auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  const long long nk = K / 64;
+  GemmChoice best = {1, 0, 1, (int)nk, 0, 0, apart};
+  for (int bn : {256, 192, 128}) {
+    const double c = (double)up(up(M, 256) * up(N, bn / 2), sms / 2) * nk * gemm_pair_step(bn, true);
+    if (c < best.cycles) best = {1, bn, 1, (int)nk, (int)up(M, 256), (int)up(N, bn / 2), c};
+  }
+  return best;
+}
+template <int QB, class Epi>
+cudaError_t gemm_run_paired(GemmArgs a, Epi epi, const GemmChoice& c, const void* x, const void* w, const void* w_up, int sms, cudaStream_t st) {
+  a.mt = c.mt; a.nt = c.nt; a.k_per = c.k_per; a.group_m = 8;
+  const long long w_row = (long long)a.K * QB / 8;
+  CUtensorMap mx, mw;
+  if (!gemm_map(&mx, x, 2, a.K, a.M, (long long)a.K * 2, 1, 0, 128) || !gemm_map(&mw, w, 1, w_row, a.N, w_row, 1, 0, c.bn / 2) ||
+      !gemm_map(&epi.map_up, w_up, 1, w_row, a.N, w_row, 1, 0, c.bn / 2))
+    return cudaErrorNotSupported;
+  if (c.bn == 256) return gemm_launch<2, 256, QB, false>(mx, mw, a, epi, 1, sms, st);
   return c.bn == 192 ? gemm_launch<2, 192, QB, false>(mx, mw, a, epi, 1, sms, st) : gemm_launch<2, 128, QB, false>(mx, mw, a, epi, 1, sms, st);
 }
 

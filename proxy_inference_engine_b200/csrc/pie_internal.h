@@ -117,6 +117,9 @@ bool fa_prefill_umma_ok(const uint16_t* out, const uint16_t* q, const uint16_t* 
                         int Hq, int Hkv, int L, int D, int offset, float scale);
 cudaError_t launch_fa_prefill_umma(uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc, const KvLayout& kv,
                                    int B, int Hq, int Hkv, int L, int D, int offset, float scale, cudaStream_t st);
+cudaError_t launch_qmm_swiglu(uint16_t* y, const uint16_t* x, const uint32_t* const* wq, const uint16_t* const* s, const uint16_t* const* b,
+                              int M, int N, int K, int bits, cudaStream_t st);
+bool qmm_swiglu_pays(int M, int N, int K);
 unsigned int qmm_pipeline_error();
 unsigned int fa_prefill_pipeline_error();
 cudaError_t launch_prefill_attn(uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc,

@@ -94,7 +94,7 @@ cudaError_t launch_dequantize(uint16_t* out, const uint32_t* wq, const uint16_t*
 // fp32 sum of squares; out = bf16( bf16(x * inv) * w ): the cast to T comes BEFORE the weight multiply.  HBM-bound over many
 // rows, one L2 round trip and a barrier over few: a CTA per row, the row held in registers between the two passes in 16-byte
 // pieces, NV per thread (rms_norm_rows_kernel); rows that do not fit or are not aligned are read twice, element by element.
-// 8192 rows of 4096: 39.0 -> 25.4 us (5.3 TB/s); 1531 of 2048: 8.7 -> 4.3; 32 of 4096: 7.7 -> 2.9.
+// 8192 rows of 4096: 39.0 -> 25.4 us (5.3 TB/s); 1531 of 2048: 8.7 -> 4.3.
 __device__ __forceinline__ float rms_row_scale(float ss, int dims, float eps) {
   __shared__ float red[8];
   ss = warp_sum(ss);
@@ -176,12 +176,7 @@ cudaError_t launch_rms_norm(uint16_t* out, const uint16_t* x, const uint16_t* w,
 // (the last n % 8 elements, and arrays that are not, one element at a time).  8192 x 14336, us: SwiGLU 406 -> 111 (6.3 TB/s; it was
 // bound by two-byte accesses and a full-range division), 8192 x 4096 sum 73 -> 28.
 struct SiluMul {   // bf16 after every operator: sigmoid, gate * sigmoid, * up
-  static __device__ __forceinline__ uint32_t pair(uint32_t g, uint32_t u) {
-    const float a = bf16lo(g), b = bf16hi(g);
-    const uint32_t s = pack_bf16(__fdividef(1.f, 1.f + __expf(-a)), __fdividef(1.f, 1.f + __expf(-b)));
-    const uint32_t t = pack_bf16(a * bf16lo(s), b * bf16hi(s));
-    return pack_bf16(bf16lo(t) * bf16lo(u), bf16hi(t) * bf16hi(u));
-  }
+  static __device__ __forceinline__ uint32_t pair(uint32_t g, uint32_t u) { return mul_bf16x2_rn(silu_bf16x2(g), u); }
 };
 struct Add {
   static __device__ __forceinline__ uint32_t pair(uint32_t a, uint32_t b) {

@@ -44,6 +44,47 @@ struct QmmStore {
   }
 };
 
+// silu(x . w) * (x . w_up), rounded where the separate operators round: both products, the sigmoid, silu, the result.  It saves the two
+// products' way to memory and back and a launch: 8192 x 14336 x 4096 (4 bits)
+// 2 x 676 + 113 -> 1275 us, 1531 x 8192 x 2048 87 + 12 -> 83.
+struct QmmSwiglu {
+  static constexpr bool PAIRED = true;
+  CUtensorMap map_up;
+  const uint16_t *s_up, *b_up;
+  uint16_t* y;
+  int M, N;
+  __device__ __forceinline__ void gate(const uint32_t (&v)[32], uint32_t (&t)[16]) const {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) t[e] = silu_bf16x2(pack_bf16(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])));
+  }
+  __device__ __forceinline__ void operator()(int row0, int col, const uint32_t (&t)[16], const uint32_t (&v)[32], uint32_t buf, int lane) const {
+    if (row0 >= M || col >= N) return;
+    uint32_t o[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) o[e] = mul_bf16x2_rn(t[e], pack_bf16(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])));
+    uint16_t* const base = y + (size_t)row0 * N + col;
+    if ((N & 7) == 0) {   // as QmmStore
+      auto at = [&](int r, int c) { return buf + r * 64 + ((c ^ ((r >> 1) & 3)) << 4); };
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at(lane, c)), "r"(o[4 * c]), "r"(o[4 * c + 1]), "r"(o[4 * c + 2]),
+                     "r"(o[4 * c + 3]) : "memory");
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = 8 * i + (lane >> 2), c = lane & 3;
+        const uint4 w = lds128(at(r, c));
+        if (row0 + r < M && col + 8 * c < N) *reinterpret_cast<uint4*>(base + (size_t)r * N + 8 * c) = w;
+      }
+      __syncwarp();
+    } else if (row0 + lane < M) {
+#pragma unroll
+      for (int q = 0; q < 32; ++q)
+        if (col + q < N) base[(size_t)lane * N + q] = (uint16_t)(o[q >> 1] >> (16 * (q & 1)));
+    }
+  }
+};
+
 cudaError_t launch_qmm_tc(uint16_t* y, const uint16_t* x, const uint32_t* wq, const uint16_t* s, const uint16_t* b,
                           int M, int N, int K, int bits, cudaStream_t st) {
   GemmArgs a = {};
@@ -54,6 +95,31 @@ cudaError_t launch_qmm_tc(uint16_t* y, const uint16_t* x, const uint32_t* wq, co
   count_launch();
   return bits == 4 ? gemm_run<4>(a, epi, x, (long long)K * 2, 0, wq, 0, num_sms(), st)
                    : gemm_run<8>(a, epi, x, (long long)K * 2, 0, wq, 0, num_sms(), st);
+}
+
+// bn = 0 where two products and the elementwise operator are estimated to be done sooner (its 6 bytes an element at 6 TB/s and two
+// launches in cycles of 1.9 GHz beside the products' own estimate), as they are where one wave of single CTAs holds a product: 77 rows of
+// 14336 x 4096 take 27 + 27 + 3 us, in pairs' tiles two waves.
+static GemmChoice qmm_swiglu_choice(int M, int N, int K, int sms) {
+  const double apart = 2 * gemm_choose(M, N, K, 1, sms, true).cycles + (double)M * N * 6 / 3158 + 4000;
+  return gemm_choose_paired(M, N, K, sms, apart);
+}
+bool qmm_swiglu_pays(int M, int N, int K) { return qmm_swiglu_choice(M, N, K, num_sms()).bn != 0; }
+cudaError_t launch_qmm_swiglu(uint16_t* y, const uint16_t* x, const uint32_t* const* wq, const uint16_t* const* s, const uint16_t* const* b,
+                              int M, int N, int K, int bits, cudaStream_t st) {
+  const int sms = num_sms();
+  const GemmChoice c = qmm_swiglu_choice(M, N, K, sms);
+  if (!c.bn) return cudaErrorNotSupported;
+  GemmArgs a = {};
+  a.M = M; a.N = N; a.K = K; a.nb = 1;
+  a.scales = s[0]; a.biases = b[0];
+  uintptr_t at = 0;
+  for (int i = 0; i < 2; ++i) at |= reinterpret_cast<uintptr_t>(s[i]) | reinterpret_cast<uintptr_t>(b[i]);
+  a.scale_vec = K % 512 == 0 && (at & 15) == 0;
+  QmmSwiglu epi = {};
+  epi.s_up = s[1]; epi.b_up = b[1]; epi.y = y; epi.M = M; epi.N = N;
+  count_launch();
+  return bits == 4 ? gemm_run_paired<4>(a, epi, c, x, wq[0], wq[1], sms, st) : gemm_run_paired<8>(a, epi, c, x, wq[0], wq[1], sms, st);
 }
 
 unsigned int qmm_pipeline_error() {

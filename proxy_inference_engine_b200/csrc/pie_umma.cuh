@@ -1,4 +1,5 @@
-// tcgen05 / TMEM helpers shared by the prefill GEMM (pie_qmm.cu) and the batched-decode GEMM (pie_qmd.cu).
+// tcgen05 / TMEM helpers shared by the GEMM core (pie_gemm.cuh), the prefill attention and the batched-decode GEMMs (pie_qmd.cu,
+// pie_qmi.cu).
 #pragma once
 #include "pie_ptx.cuh"
 
@@ -19,6 +20,11 @@ constexpr uint32_t umma_idesc_bf16_m128(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
+__device__ __forceinline__ bool elect_one() {   // one lane of the (converged) warp
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accum) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"

@@ -106,6 +106,29 @@ class QuantizedEmbedding(Module):
                                     group_size=self.group_size, bits=self.bits)
 
 
+def _plain(lin, bits: int, K: int) -> bool:
+    """A bias-free QuantizedLinear whose arrays the kernels can take as they lie."""
+    w, s, b = lin.weight, lin.scales, lin.biases
+    return not (type(lin) is not QuantizedLinear or "bias" in lin.__dict__ or lin.bits != bits or lin.group_size != 64
+                or w.dtype != torch.int32 or w.dim() != 2 or w.shape[1] * 32 != K * bits or s.dtype != torch.bfloat16
+                or b.dtype != torch.bfloat16 or s.shape != b.shape or s.shape != (w.shape[0], K // 64)
+                or not (w.is_contiguous() and s.is_contiguous() and b.is_contiguous())
+                or w.data_ptr() % 16 or s.data_ptr() % 8 or b.data_ptr() % 8)
+
+
+def fused_swiglu(x, gate, up):
+    """silu(gate(x)) * up(x) of a prompt's rows in ONE launch, rounding for rounding the separate calls.  None where that does not
+    apply or does not pay (the caller then makes the separate calls, which also report what is wrong)."""
+    K = x.shape[-1]
+    if x.dtype != torch.bfloat16 or not x.is_contiguous() or gate.bits not in (4, 8) or K == 0 or x.numel() < 64 * K:
+        return None
+    if not ops.qmm_swiglu_pays(x.numel() // K, gate.weight.shape[0], K, gate.bits):
+        return None
+    if not _plain(gate, gate.bits, K) or not _plain(up, gate.bits, K) or gate.weight.shape != up.weight.shape:
+        return None
+    return ops.qmm_swiglu(x, gate, up, x.numel() // K, K)
+
+
 def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
     """Up to 32 rows through several bias-free QuantizedLinears in ONE launch, with the RMSNorm in front of them, and the
     residual sum or SwiGLU behind them where asked for -- the arithmetic of the separate calls, rounding for rounding:
@@ -119,14 +142,9 @@ def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
     if bits not in (4, 8) or K % (1024 // bits):
         return None
     for lin in linears:
-        w, s, b = lin.weight, lin.scales, lin.biases
-        if (type(lin) is not QuantizedLinear or "bias" in lin.__dict__ or lin.bits != bits or lin.group_size != 64
-                or w.dtype != torch.int32 or w.dim() != 2 or w.shape[1] * 32 != K * bits or s.dtype != torch.bfloat16
-                or b.dtype != torch.bfloat16 or s.shape != b.shape or s.shape != (w.shape[0], K // 64)
-                or not (w.is_contiguous() and s.is_contiguous() and b.is_contiguous())
-                or w.data_ptr() % 16 or s.data_ptr() % 8 or b.data_ptr() % 8):
+        if not _plain(lin, bits, K):
             return None
-        N += w.shape[0]
+        N += lin.weight.shape[0]
     if swiglu:
         if linears[0].weight.shape[0] != linears[1].weight.shape[0]:
             return None

@@ -176,6 +176,24 @@ def qmv_fused(x, linears, rows: int, K: int, N: int, bits: int, norm_weight, eps
     return out
 
 
+@functools.lru_cache(maxsize=4096)
+def qmm_swiglu_pays(rows: int, N: int, K: int, bits: int) -> bool:
+    return bool(_lib.load().pie_qmm_swiglu_pays(rows, N, K, 64, bits))
+
+
+def qmm_swiglu(x, gate, up, rows: int, K: int):
+    """pie_qmm_swiglu on operands nn.fused_swiglu has checked; None where the library leaves the shape to the separate calls."""
+    segs = (QmvSeg * 2)()
+    for seg, lin in zip(segs, (gate, up)):
+        seg.wq, seg.scales, seg.biases, seg.N = lin.weight.data_ptr(), lin.scales.data_ptr(), lin.biases.data_ptr(), lin.weight.shape[0]
+    out = torch.empty(x.shape[:-1] + (segs[0].N,), dtype=_BF16, device=x.device)
+    status = _lib.load().pie_qmm_swiglu(_p(out), _p(x), segs, rows, K, 64, gate.bits, _stream())
+    if status == _lib.EUNSUPPORTED:
+        return None
+    _lib.check(status, "qmm_swiglu")
+    return out
+
+
 def rms_norm(x, weight, eps: float):
     """mx.fast.rms_norm (MLX/mlx/fast.cpp:56-123): bf16(bf16(x * rsqrt(mean(x^2) + eps)) * weight)."""
     if x.dim() < 1:

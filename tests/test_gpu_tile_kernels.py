@@ -46,6 +46,28 @@ def test_quantized_gemm_tiles(bits, M, N, K):
     assert _lib.load().pie_pipeline_error() == 0
 
 
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("M,N,K", [(64, 128, 128),        # 128 columns a tile pair, 64 of y; one tile
+                                   (300, 1100, 384),      # the same, ragged
+                                   (1500, 2100, 1024),    # 192
+                                   (777, 4100, 640),      # 256, rows of y off 16 bytes, scales one at a time
+                                   (2050, 2056, 1024)])   # several tiles a pair
+def test_swiglu_in_the_gemm_is_the_separate_operators(bits, M, N, K):
+    """Both products sum K in the order of the separate ones and every rounding is kept: the same bits."""
+    from proxy_inference_engine_b200 import _lib, nn, ops
+    g = torch.Generator(device="cuda").manual_seed(M + N + K + bits)
+    lins = []
+    for _ in range(2):
+        lin = nn.QuantizedLinear(K, N, bias=False, group_size=64, bits=bits)
+        lin.weight, lin.scales, lin.biases = ops.quantize(torch.randn((N, K), generator=g, device="cuda").to(torch.bfloat16), 64, bits)
+        lins.append(lin)
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    got = nn.fused_swiglu(x, *lins)
+    assert got is not None and torch.equal(got, ops.silu_mul(lins[0](x), lins[1](x)))
+    assert nn.fused_swiglu(x[:63], *lins) is None and nn.fused_swiglu(x.float(), *lins) is None
+    assert _lib.load().pie_pipeline_error() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(33, 64, 64), (129, 257, 128), (70, 640, 8192), (200, 1024, 1152), (513, 4100, 192), (2050, 2056, 512), (1200, 8192, 128),
                                    (700, 3000, 128)])
 def test_dense_gemm_tiles(M, N, K):
