@@ -633,7 +633,7 @@ def prefill_figure(margs, bits, M=8192):
         peak, src = 1400.0, "fallback (B200_PROFILING.md)"
     tf = flops / ms / 1e9
     return {"workload": f"one transformer layer's 7 quantized matmuls, M = {M} (8k-token prefill), q{bits}",
-            "kernel": f"qmm_tc_kernel<{bits}> (tcgen05.mma kind::f16, TMEM accumulators)", "ms_per_layer": round(ms, 3),
+            "kernel": f"gemm_kernel, {bits}-bit weights (tcgen05.mma kind::f16, TMEM accumulators)", "ms_per_layer": round(ms, 3),
             "achieved": round(tf, 1), "unit": "TFLOP/s", "peak": peak, "peak_source": src, "frac": round(tf / peak, 4),
             "bound": "tensor"}
 

@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const LinArgs a) {
 // activation row, and feeds two MMAs from them.  The tensor core does the sum over k that linear_rows_kernel does with shuffles
 // (16 values x 5 shuffles for every 16 KB of weights at four rows), so a warp keeps eight 16-byte weight loads in flight and
 // little else.  The warps' partial tiles meet in shared memory in warp order.  Four rows, us (GB/s): 28672 x 4096 61.6 (3810) -> 40.9
-// (5750); 4096 x 14336 31 -> 24.6 (4780); 16 rows: 57.6 and 33.3; 32 rows: 92 and 55 (x comes from L2 once per 16 outputs).
+// (5750); 4096 x 14336 24.6 (4780); 16 rows: 57.6 and 33.3; 32 rows: 92 and 55 (x comes from L2 once per 16 outputs).
 __device__ __forceinline__ uint4 load_stream16(const __nv_bfloat16* p) {   // read once: past L1
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));

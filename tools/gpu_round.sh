@@ -22,7 +22,7 @@ timeout 600 $CMD > $OUT/plain2.log 2>&1 &&
 timeout 900 ncu --set full --clock-control none --import-source on --kernel-name-base demangled -k regex:qmv_kernel -s 400 -c 6 \
     -o $OUT/prof_qmv $CMD > $OUT/ncu_full.log 2>&1
 timeout 300 python tools/bench_qmm.py --iters 1 > /dev/null 2>&1 &&
-timeout 600 ncu --set full --clock-control none --import-source on --kernel-name-base demangled -k regex:qmm_tc_kernel -s 8 -c 2 \
+timeout 600 ncu --set full --clock-control none --import-source on --kernel-name-base demangled -k regex:gemm_kernel -s 8 -c 2 \
     -o $OUT/prof_qmm python tools/bench_qmm.py --iters 1 > $OUT/ncu_qmm.log 2>&1
 # BASELINE configs 3 and 4 + captures of the kernels that dominate them
 ( timeout 400 python bench.py --bits 8 --batch 32 --prompt 2048 --paged --steps 32 --warmup 4 --no-cpu-baseline --no-kernel-timing --no-prefill ) > $OUT/config3.log 2> $OUT/config3.err
