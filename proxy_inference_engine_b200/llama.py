@@ -152,6 +152,7 @@ class Attention(nn.Module):
             keys, values = cache.update_and_fetch(keys, values)
         else:
             queries, keys = self.rope(queries), self.rope(keys)
+            values = values.contiguous()   # in the layout of the rotated keys; a cache would have copied both
         output = scaled_dot_product_attention(queries, keys, values, cache=cache, scale=self.scale, mask=mask)
         return output.transpose(1, 2).reshape(B, L, -1)
 

@@ -326,7 +326,8 @@ def scaled_dot_product_attention(q, k, v, *, scale: float, mask=None):
         raise ValueError("[scaled_dot_product_attention] n_heads must be a multiple of n_kv_heads")
     if q.dtype != _BF16 or k.dtype != _BF16 or v.dtype != _BF16:
         raise ValueError("[scaled_dot_product_attention] only bfloat16 is built here")
-    if k.stride() != v.stride():
+    # (the stride of a dimension of one element says nothing: a view of projected rows and a rotated copy of one differ there)
+    if any(a != b and (n != 1 or m != 1) for n, m, a, b in zip(k.shape, v.shape, k.stride(), v.stride())):
         raise ValueError("[scaled_dot_product_attention] keys and values must share one layout")
     lay = kv_layout(k)
     L = _lib.load()
