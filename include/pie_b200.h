@@ -54,8 +54,11 @@ const char* pie_last_cuda_error(void);
 /* number of kernels this library has launched since load (the bench's gpu_launches claim) */
 unsigned long long pie_launch_count(void);
 /* 1: a bounded wait inside the prefill GEMM (pie_qmm) or the prefill attention (pie_prefill_attn) expired since the library was
- * loaded, and that call's results are void; 0: none did.  Reads a device word: synchronises. */
+ * loaded or pie_pipeline_error_clear() was called, and that call's results are void; 0: none did.  Reads a device word: synchronises. */
 unsigned int pie_pipeline_error(void);
+int pie_pipeline_error_clear(void);
+/* the same without waiting: words[0 .. 1] (page-locked memory, or the copy waits) become non-zero, in stream order, if it holds */
+int pie_pipeline_words(unsigned int* words, void* stream);
 
 /* ---- a1  mx.quantize  (MLX/mlx/ops.cpp:4023-4029 -> MLX/mlx/backend/cpu/quantized.cpp:603-661) -------
  * w [rows, K] (dtype) -> wq [rows, K*bits/32] u32, scales/biases [rows, K/group_size] (dtype). Bit-exact. */

@@ -28,9 +28,11 @@ extern "C" {
 int pieh_abi_version(void);
 const char* pieh_last_cuda_error(void);
 unsigned long long pieh_launch_count(void);
-/* non-zero after a tensor-core pipeline gave up a bounded wait (the kernel returned early; its output is invalid).
- * Synchronises the device. */
+/* non-zero after a tensor-core pipeline gave up a bounded wait (the kernel returned early; its output is invalid), until it is
+ * cleared.  Synchronises the device; pieh_pipeline_words does not (as pie_pipeline_words; words[1] stays as it is). */
 unsigned int pieh_pipeline_error(void);
+int pieh_pipeline_error_clear(void);
+int pieh_pipeline_words(unsigned int* words, void* stream);
 /* on: every operator is launched as a programmatic dependent of the launch before it on its stream (its blocks may become
  * resident early and wait at their top); captured into CUDA graphs as such.  Off by default. */
 void pieh_set_pdl(int on);

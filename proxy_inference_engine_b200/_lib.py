@@ -81,6 +81,8 @@ SIGNATURES = {
     "pie_last_cuda_error": (C.c_char_p, []),
     "pie_launch_count": (C.c_ulonglong, []),
     "pie_pipeline_error": (C.c_uint, []),
+    "pie_pipeline_error_clear": (_i, []),
+    "pie_pipeline_words": (_i, [_vp, _vp]),
     "pie_quantize": (_i, [_vp, _i, _vp, _vp, _vp, _ll, _i, _i, _i, _vp]),
     "pie_dequantize": (_i, [_vp, _vp, _vp, _vp, _vp, _ll, _ll, _i, _i, _i, _vp]),
     "pie_qmv_workspace_bytes": (_sz, [_i, _ll, _i, _i, _i, _i]),
@@ -240,6 +242,8 @@ HYBRID_SIGNATURES = {
     "pieh_last_cuda_error": (C.c_char_p, []),
     "pieh_launch_count": (C.c_ulonglong, []),
     "pieh_pipeline_error": (C.c_uint, []),
+    "pieh_pipeline_error_clear": (_i, []),
+    "pieh_pipeline_words": (_i, [_vp, _vp]),
     "pieh_set_pdl": (None, [_i]),
     "pieh_linear": (_i, [_vp, _i, _ll, _vp, _i, _ll, _vp, _i, _vp, _i, _i, _i, _i, _f, _vp, _vp, _i, _vp]),
     "pieh_embed_streams": (_i, [_vp, _vp, _i, _vp, _i, _i, _i, _i, _vp]),

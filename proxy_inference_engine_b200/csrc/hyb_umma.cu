@@ -21,14 +21,12 @@ constexpr int kBN = 256, kBK = 64, kProducers = 256, kThreads = kProducers + 32;
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr uint32_t IDESC = pie::umma_idesc_bf16_m128(kBN);
 
-__device__ unsigned int g_umma_error = 0;   // 1: a pipeline wait expired
-
 __device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   uint32_t spins = 0;
   while (!pie::mbar_try_wait(bar, parity)) {
     if (++spins > kWaitLimit || *abort_flag) {
       *abort_flag = 1;
-      atomicExch(&g_umma_error, 1u);
+      atomicExch(&pie::g_gemm_error, 1u);
       return false;
     }
   }
@@ -383,9 +381,8 @@ cudaError_t launch_linear_umma(const LinArgs& a, int out_dtype, cudaStream_t st)
 
 }  // namespace pieh
 
-extern "C" unsigned int pieh_pipeline_error(void) {
-  unsigned int v = 0, g = 0;
-  cudaMemcpyFromSymbol(&v, pieh::g_umma_error, sizeof(v));
-  cudaMemcpyFromSymbol(&g, pie::g_gemm_error, sizeof(g));
-  return v | g;
+extern "C" unsigned int pieh_pipeline_error(void) { return pie::gemm_error_now(); }
+extern "C" int pieh_pipeline_error_clear(void) { return pieh::status_of(pie::gemm_error_clear()); }
+extern "C" int pieh_pipeline_words(unsigned int* words, void* stream) {
+  return words ? pieh::status_of(pie::gemm_error_post(words, (cudaStream_t)stream)) : PIE_ENULL;
 }

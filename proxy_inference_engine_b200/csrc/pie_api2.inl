@@ -169,6 +169,15 @@ int pie_prefill_attn(void* out, const void* q, const void* kcache, const void* v
 
 // 1: a pipeline wait of the prefill GEMM or of the prefill attention expired (the call's results are void); 0: none did
 unsigned int pie_pipeline_error(void) { return qmm_pipeline_error() | fa_prefill_pipeline_error(); }
+int pie_pipeline_error_clear(void) {
+  if (int s = cuda_status(qmm_pipeline_clear())) return s;
+  return cuda_status(fa_prefill_pipeline_clear());
+}
+int pie_pipeline_words(unsigned int* words, void* stream) {
+  if (!words) return PIE_ENULL;
+  if (int s = cuda_status(qmm_pipeline_post(words, (cudaStream_t)stream))) return s;
+  return cuda_status(fa_prefill_pipeline_post(words + 1, (cudaStream_t)stream));
+}
 
 int pie_silu_mul(void* out, const void* gate, const void* up, long long n, void* stream) {
   if (n == 0) return PIE_OK;

@@ -439,10 +439,8 @@ cudaError_t launch_fa_prefill_umma(uint16_t* out, const uint16_t* q, const uint1
   return D == 128 ? launch_fap<128>(mq, maps[0], maps[1], a, st) : launch_fap<64>(mq, maps[0], maps[1], a, st);
 }
 
-unsigned int fa_prefill_pipeline_error() {
-  unsigned int v = 0;
-  cudaMemcpyFromSymbol(&v, g_gemm_error, sizeof(v));
-  return v;
-}
+unsigned int fa_prefill_pipeline_error() { return gemm_error_now(); }
+cudaError_t fa_prefill_pipeline_post(unsigned int* host, cudaStream_t st) { return gemm_error_post(host, st); }
+cudaError_t fa_prefill_pipeline_clear() { return gemm_error_clear(); }
 
 }  // namespace pie

@@ -29,7 +29,20 @@
 
 namespace pie {
 
-static __device__ unsigned int g_gemm_error = 0;   // 1: a pipeline wait of this library's GEMM expired
+static __device__ unsigned int g_gemm_error = 0;   // 1: a pipeline wait of a kernel of this source file expired
+// the word on the host: now (waits for the device), behind what is queued on a stream, and set back
+static inline unsigned int gemm_error_now() {
+  unsigned int v = 0;
+  cudaMemcpyFromSymbol(&v, g_gemm_error, sizeof(v));
+  return v;
+}
+static inline cudaError_t gemm_error_post(unsigned int* host, cudaStream_t st) {
+  return cudaMemcpyFromSymbolAsync(host, g_gemm_error, sizeof(*host), 0, cudaMemcpyDeviceToHost, st);
+}
+static inline cudaError_t gemm_error_clear() {
+  const unsigned int v = 0;
+  return cudaMemcpyToSymbol(g_gemm_error, &v, sizeof(v));
+}
 
 // ---------------------------------------------------------------------------------------------------- cluster / mbarrier
 __device__ __forceinline__ uint32_t cluster_rank() {

@@ -121,7 +121,11 @@ cudaError_t launch_qmm_swiglu(uint16_t* y, const uint16_t* x, const uint32_t* co
                               int M, int N, int K, int bits, cudaStream_t st);
 bool qmm_swiglu_pays(int M, int N, int K);
 unsigned int qmm_pipeline_error();
+cudaError_t qmm_pipeline_post(unsigned int* host, cudaStream_t st);
+cudaError_t qmm_pipeline_clear();
 unsigned int fa_prefill_pipeline_error();
+cudaError_t fa_prefill_pipeline_post(unsigned int* host, cudaStream_t st);
+cudaError_t fa_prefill_pipeline_clear();
 cudaError_t launch_prefill_attn(uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc,
                                 const KvLayout& kv, int B, int Hq, int Hkv, int L, int D, int offset,
                                 float scale, cudaStream_t st);

@@ -122,10 +122,8 @@ cudaError_t launch_qmm_swiglu(uint16_t* y, const uint16_t* x, const uint32_t* co
   return bits == 4 ? gemm_run_paired<4>(a, epi, c, x, wq[0], wq[1], sms, st) : gemm_run_paired<8>(a, epi, c, x, wq[0], wq[1], sms, st);
 }
 
-unsigned int qmm_pipeline_error() {
-  unsigned int v = 0;
-  cudaMemcpyFromSymbol(&v, g_gemm_error, sizeof(v));
-  return v;
-}
+unsigned int qmm_pipeline_error() { return gemm_error_now(); }
+cudaError_t qmm_pipeline_post(unsigned int* host, cudaStream_t st) { return gemm_error_post(host, st); }
+cudaError_t qmm_pipeline_clear() { return gemm_error_clear(); }
 
 }  // namespace pie

@@ -155,6 +155,7 @@ class DecodeEngine:
             self.vbuf = [c.values for c in self.cache]
         L = _lib.load()
         self.L = L
+        self.watch = ops.PipelineWatch(L, "pie")
         self.nsplit = (L.pie_decode_attn_q8_pick_splits if kv_bits is not None else L.pie_decode_attn_pick_splits)(
             B, self.Hq, self.Hkv, max_context)
         # Two forms of decode attention.  Latency form: rope + KV append + SIMT flash-decode in ONE launch
@@ -417,6 +418,7 @@ class DecodeEngine:
     # ------------------------------------------------------------------------------------------------
     def prefill(self, prompt_ids: torch.Tensor):
         """Whole prompt in ONE forward (inference_engine.py:278), B rows of equal length; samples the first token."""
+        self.watch.check()
         ids = prompt_ids.to(self.dev).to(torch.int32).reshape(self.B, -1)
         Lp = ids.shape[1]
         if Lp + 1 > self.max_context:
@@ -439,6 +441,7 @@ class DecodeEngine:
         last = logits[:, -1, :].contiguous()
         self.logits.copy_(last)
         self._sample(self.logits)
+        self.watch.post()   # the prompt's matrices and attention have waits that can expire, the steps have not
         return self.tokens
 
     def step(self, n: int = 1):
@@ -448,6 +451,7 @@ class DecodeEngine:
         because the captured graph holds their addresses)."""
         if getattr(self, "_next_pos", None) is None:
             raise ValueError("DecodeEngine.step() before prefill()")
+        self.watch.check()
         if self._next_pos + n > self.max_context:
             raise ValueError(f"decode step past max_context: position {self._next_pos} + {n} steps > {self.max_context}")
         self._next_pos += n
@@ -465,6 +469,7 @@ class DecodeEngine:
     def generated(self) -> torch.Tensor:
         """Tokens sampled so far, [B, n] (device -> host copy: the sync point, inference_engine.py:202)."""
         end = int(self.positions[0].item()) + 1
+        self.watch.check()
         return self.seq[:, self.prompt_len:end].cpu()
 
     def generate(self, prompt_ids, n_steps: int) -> torch.Tensor:

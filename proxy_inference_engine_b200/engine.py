@@ -18,6 +18,7 @@ import os
 
 import torch
 
+from .ops import PipelineWatch
 from .ragged import BatchDetails
 
 
@@ -110,12 +111,23 @@ class HybridEngine:
         self.use_graph = use_graph and str(self.device).startswith("cuda")
         self.use_pdl = os.environ.get("PIE_HYBRID_PDL", "0") == "1"
         self._graphs = {}
+        self.watch = PipelineWatch(model.L, "pieh") if str(self.device).startswith("cuda") and hasattr(model, "L") else None
+
+    def check(self) -> None:
+        """Raises if a kernel of a finished step gave up a wait: for callers of ``forward`` that have read its logits."""
+        if self.watch is not None:
+            self.watch.check()
+
+    def _post(self) -> None:
+        if self.watch is not None:
+            self.watch.post()
 
     # ---- one step ----------------------------------------------------------------------------------
     def forward(self, entries, trace=None) -> torch.Tensor:
         """entries: [(seq_id, new_token_ids, wanted)] with ``wanted`` the indices into new_token_ids whose logits are
         asked for (None: the last one).  Unknown ids are admitted.  Returns fp32 logits [total wanted, vocab] in entry
         order (an empty tensor if nothing is wanted; the step still runs and advances every sequence)."""
+        self.check()
         seqs, rows, row0 = [], [], 0
         for sid, toks, want in entries:
             toks = [int(t) for t in toks]
@@ -139,6 +151,7 @@ class HybridEngine:
             if dg.graph is None:
                 dg.snapshot()
             logits = dg.run([(toks, ctx, pages, slot) for _, toks, ctx, pages, slot in seqs])
+            self._post()
             for sid, toks, *_ in seqs:
                 self.cache.seqs[sid]["length"] += 1
             if not rows:
@@ -149,6 +162,7 @@ class HybridEngine:
         # with nothing wanted the head still needs a row: take the last and drop the result
         idx = torch.tensor(rows if rows else [row0 - 1], dtype=torch.int32).to(self.device)
         logits = self.model.step(batch, self.cache, rows=idx, trace=trace)
+        self._post()
         for sid, toks, *_ in seqs:
             self.cache.seqs[sid]["length"] += len(toks)
         return logits if rows else logits[:0]
@@ -195,6 +209,7 @@ class HybridEngine:
             logits = self.forward(entries)
             if takers:
                 toks = sampler(logits.to(torch.bfloat16)).tolist()
+                self.check()
                 for i, tok in zip(takers, toks):
                     out[i].append(int(tok))
                     live[i]["next"] = int(tok)

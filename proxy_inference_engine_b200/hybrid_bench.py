@@ -185,7 +185,7 @@ class _Timed:
 
     def __getattr__(self, name):
         fn = getattr(self._lib, name)
-        if not name.startswith("pieh_") or name in ("pieh_launch_count", "pieh_pipeline_error"):
+        if not name.startswith("pieh_") or name in ("pieh_launch_count", "pieh_pipeline_error", "pieh_pipeline_error_clear", "pieh_pipeline_words"):
             return fn
 
         def call(*args):

@@ -479,5 +479,43 @@ def sample(logits, temp: float, top_p: float = 0.0, min_p: float = 0.0, min_toke
     return (out, logprobs_out) if return_logprobs else out
 
 
+_VOID = ("a bounded wait inside a tensor-core pipeline expired: results since the last check that passed are void "
+         "(and every check fails until {}_pipeline_error_clear())")
+
+
+class PipelineWatch:
+    """Whether a kernel gave up a wait, without a wait for it: post() behind a step's launches queues a copy of the library's word
+    on the current stream, check() raises once a copy that said so has landed -- where the host has waited for the step anyway
+    (its tokens are there), and before the next step."""
+
+    def __init__(self, lib, prefix: str, page_locked: bool = True):
+        self._words_fn, self._prefix = getattr(lib, prefix + "_pipeline_words"), prefix
+        self.words = torch.zeros(2, dtype=torch.int32, pin_memory=page_locked)
+        self._seen = self.words.numpy()
+        self._posted = torch.cuda.Event() if page_locked else None
+
+    def post(self) -> None:
+        if self._words_fn(self.words.data_ptr(), _stream()):
+            raise RuntimeError("[pipeline_words] CUDA error")
+        if self._posted is not None:
+            self._posted.record()
+
+    def __del__(self):
+        # torch hands the words to someone else once they are dropped: not while a copy is on its way to them
+        if getattr(self, "_posted", None) is not None and not self._posted.query():
+            self._posted.synchronize()
+
+    def check(self) -> None:
+        if self._seen[0] or self._seen[1]:
+            self._seen[:] = 0   # the library's word is what lasts: the next copy brings it again unless it was cleared
+            raise RuntimeError(_VOID.format(self._prefix))
+
+
+def check_pipeline() -> None:
+    """The same for calls outside an engine (a layer, a model, attention): waits for the device."""
+    if _lib.load().pie_pipeline_error():
+        raise RuntimeError(_VOID.format("pie"))
+
+
 def launch_count() -> int:
     return int(_lib.load().pie_launch_count())

@@ -54,6 +54,7 @@ def main(argv=None) -> int:
             logits = eng.forward(entries)
             if logits.shape[0]:
                 data = logits.to(torch.float32).contiguous().cpu().numpy().astype("<f4")
+                eng.check()
                 tmp = os.path.join(a.out, f".{step['step']}.f32.part")
                 with open(tmp, "wb") as f:
                     f.write(data.tobytes())

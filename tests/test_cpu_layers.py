@@ -1,4 +1,6 @@
 """Host side of the Llama layers' calls: what reaches the library and what is refused, on CPU tensors with the library stubbed."""
+import ctypes
+
 import pytest
 import torch
 
@@ -24,3 +26,101 @@ def test_one_key_may_be_a_view_and_a_copy(monkeypatch):
         ops.scaled_dot_product_attention(q, k, view(3, 3 * H * D), scale=1.0)
     with pytest.raises(ValueError, match="one layout"):
         ops.scaled_dot_product_attention(_bf16(1, H, 1, D), _bf16(1, H, 5, D), _bf16(1, 5, H, D).transpose(1, 2), scale=1.0)
+
+
+class _Expired:
+    """A library one of whose waits has expired: its word reaches the host as the real one's does, once the copy has landed."""
+
+    def __init__(self):
+        self.word, self.posts = 0, []
+
+    def pie_pipeline_words(self, words, stream):
+        self.posts.append(ctypes.cast(words, ctypes.POINTER(ctypes.c_uint)))
+        return 0
+    pieh_pipeline_words = pie_pipeline_words
+
+    def pie_pipeline_error(self):
+        return self.word
+
+    def land(self):
+        for p in self.posts:
+            p[0] = self.word
+        self.posts.clear()
+
+
+@pytest.fixture
+def expired(monkeypatch):
+    lib = _Expired()
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops._lib, "load", lambda: lib)
+    return lib
+
+
+def test_an_expired_wait_is_raised_once_its_copy_has_landed(expired):
+    watch = ops.PipelineWatch(expired, "pie", page_locked=False)
+    watch.check()
+    expired.word = 1
+    watch.post()
+    watch.check()                       # nothing is waited for
+    expired.land()
+    with pytest.raises(RuntimeError, match="expired"):
+        watch.check()
+    watch.post(), expired.land()        # the word lasts until it is cleared
+    with pytest.raises(RuntimeError, match="expired"):
+        watch.check()
+    expired.word = 0
+    watch.post(), expired.land()
+    watch.check()
+    ops.check_pipeline()
+    expired.word = 1
+    with pytest.raises(RuntimeError, match="expired"):
+        ops.check_pipeline()
+
+
+def test_the_decode_engine_raises_instead_of_handing_out_void_tokens(expired):
+    from proxy_inference_engine_b200.decode import DecodeEngine
+    eng = object.__new__(DecodeEngine)
+    eng.watch = ops.PipelineWatch(expired, "pie", page_locked=False)
+    eng.positions, eng.seq, eng.prompt_len = torch.tensor([3]), torch.arange(8)[None], 2
+    eng._next_pos, eng.max_context = 3, 8
+    eng.watch.post(), expired.land()
+    assert eng.generated().tolist() == [[2, 3]]
+    for call in (eng.generated, eng.step, lambda: eng.prefill(torch.zeros(1, 4))):
+        expired.word = 1
+        eng.watch.post(), expired.land()
+        with pytest.raises(RuntimeError, match="expired"):
+            call()
+
+
+def test_the_hybrid_engine_raises_at_the_end_of_a_step_and_before_the_next(expired):
+    from proxy_inference_engine_b200.engine import HybridEngine
+
+    class Model:
+        device, layers = "cpu", []
+
+        def make_cache(self, max_tokens, max_seqs):
+            from proxy_inference_engine_b200.cache import HybridCache
+            return HybridCache([], max_tokens, max_seqs, device="cpu", lib=ops._lib.load_hybrid(build_if_missing=True))
+
+        def step(self, batch, cache, rows=None, trace=None):
+            expired.word = int(batch.total_tokens_in_step > 2)
+            return torch.zeros(len(rows), 5)
+
+    def sampler(logits):
+        expired.land()                  # the host waits for the step
+        return logits.argmax(-1)
+
+    eng = HybridEngine(Model(), max_tokens=256, max_seqs=1, use_graph=False)
+    eng.watch = ops.PipelineWatch(expired, "pieh", page_locked=False)
+    assert eng.generate([[1, 2]], max_new_tokens=2, sampler=sampler) == [[0, 0]]
+    with pytest.raises(RuntimeError, match="expired"):
+        eng.generate([[1, 2, 3]], max_new_tokens=2, sampler=sampler)
+    eng.finish(("gen", 0))
+    eng.forward([("a", [1, 2, 3], None)])
+    expired.land()
+    with pytest.raises(RuntimeError, match="expired"):
+        eng.check()
+    eng.forward([("a", [1, 2, 3], None)])
+    expired.land()
+    with pytest.raises(RuntimeError, match="expired"):
+        eng.forward([("a", [4], None)])

@@ -15,3 +15,19 @@ def test_a_model_without_a_cache_is_the_one_with_an_empty_cache(head_dim, B, L):
     model = build_model(args, random_weights(args, seed=0, device="cuda"))
     ids = torch.randint(0, args.vocab_size, (B, L), generator=torch.Generator().manual_seed(L)).cuda().to(torch.int32)
     assert torch.equal(model(ids), model(ids, cache=model.make_cache()))
+
+
+def test_the_engines_bring_the_pipelines_word_to_the_host():
+    """Whatever the words hold, a prompt overwrites them with the library's own (0: no wait expired) by the time its tokens are read."""
+    from proxy_inference_engine_b200.checkpoint import build_model, random_weights
+    from proxy_inference_engine_b200.decode import DecodeEngine
+    args = tiny_args(bits=4)
+    eng = DecodeEngine(build_model(args, random_weights(args, seed=0, device="cuda")), batch=1, max_context=128)
+    eng.prefill(torch.arange(70))
+    torch.cuda.synchronize()
+    eng.watch.words.fill_(-1)
+    with pytest.raises(RuntimeError, match="expired"):
+        eng.generated()
+    eng.watch.words.fill_(-1)
+    eng.watch.post()
+    assert eng.generated().shape == (1, 1) and eng.watch.words.tolist() == [0, 0]
