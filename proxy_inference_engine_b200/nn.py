@@ -107,9 +107,12 @@ class QuantizedEmbedding(Module):
 
 
 def _plain(lin, bits: int, K: int) -> bool:
-    """A bias-free QuantizedLinear whose arrays the kernels can take as they lie."""
+    """A bias-free QuantizedLinear whose arrays the kernels can take as they lie.  (Anything that can be called may stand in a
+    layer's place: nothing of it is read before its type is known.)"""
+    if type(lin) is not QuantizedLinear:
+        return False
     w, s, b = lin.weight, lin.scales, lin.biases
-    return not (type(lin) is not QuantizedLinear or "bias" in lin.__dict__ or lin.bits != bits or lin.group_size != 64
+    return not ("bias" in lin.__dict__ or lin.bits != bits or lin.group_size != 64
                 or w.dtype != torch.int32 or w.dim() != 2 or w.shape[1] * 32 != K * bits or s.dtype != torch.bfloat16
                 or b.dtype != torch.bfloat16 or s.shape != b.shape or s.shape != (w.shape[0], K // 64)
                 or not (w.is_contiguous() and s.is_contiguous() and b.is_contiguous())
@@ -120,7 +123,9 @@ def fused_swiglu(x, gate, up):
     """silu(gate(x)) * up(x) of a prompt's rows in ONE launch, rounding for rounding the separate calls.  None where that does not
     apply or does not pay (the caller then makes the separate calls, which also report what is wrong)."""
     K = x.shape[-1]
-    if x.dtype != torch.bfloat16 or not x.is_contiguous() or gate.bits not in (4, 8) or K == 0 or x.numel() < 64 * K:
+    if x.dtype != torch.bfloat16 or not x.is_contiguous() or K == 0 or x.numel() < 64 * K:
+        return None
+    if type(gate) is not QuantizedLinear or gate.bits not in (4, 8):
         return None
     if not ops.qmm_swiglu_pays(x.numel() // K, gate.weight.shape[0], K, gate.bits):
         return None
@@ -138,7 +143,7 @@ def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
     rows = x.numel() // K if K else 0
     if not 0 < rows <= 32 or x.dtype != torch.bfloat16 or not x.is_contiguous() or x.data_ptr() % 16:
         return None
-    bits, N = linears[0].bits, 0
+    bits, N = getattr(linears[0], "bits", None), 0
     if bits not in (4, 8) or K % (1024 // bits):
         return None
     for lin in linears:

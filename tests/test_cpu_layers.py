@@ -124,3 +124,24 @@ def test_the_hybrid_engine_raises_at_the_end_of_a_step_and_before_the_next(expir
     expired.land()
     with pytest.raises(RuntimeError, match="expired"):
         eng.forward([("a", [4], None)])
+
+
+@pytest.mark.parametrize("rows", [1, 70])
+@pytest.mark.parametrize("swapped", ["gate_proj", "up_proj", "both"])
+def test_any_callable_may_stand_for_a_projection(monkeypatch, rows, swapped):
+    """The fused calls step aside for a projection that is no QuantizedLinear, whatever it has or lacks."""
+    from proxy_inference_engine_b200 import llama, nn
+    K, N = 512, 256
+    plain = object.__new__(nn.QuantizedLinear)
+    plain.group_size, plain.bits = 64, 4
+    plain.weight, plain.scales, plain.biases = torch.zeros((N, K // 8), dtype=torch.int32), _bf16(N, K // 64), _bf16(N, K // 64)
+    monkeypatch.setattr(nn.QuantizedLinear, "__call__", lambda self, x: x[..., :N])
+    monkeypatch.setattr(ops, "qmm_swiglu_pays", lambda *a: True)
+    monkeypatch.setattr(ops, "silu_mul", lambda a, b: a + b)
+    mlp = object.__new__(llama.MLP)
+    mlp.down_proj = lambda a: a
+    other = lambda x: x[..., :N]
+    mlp.gate_proj = plain if swapped == "up_proj" else other
+    mlp.up_proj = plain if swapped == "gate_proj" else other
+    x = torch.ones((rows, K), dtype=torch.bfloat16)
+    assert torch.equal(mlp(x), 2 * x[..., :N])
