@@ -185,16 +185,24 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 __device__ __forceinline__ uint16_t f2bf(float f) { return (uint16_t)(pack_bf16(f, 0.f) & 0xffffu); }
 __device__ __forceinline__ float bfround(float f) { return __uint_as_float(pack_bf16(0.f, f) & 0xffff0000u); }
-// bf16x2 fused multiply-add (HFMA2.BF16, FMA pipe): fp32-exact product and sum, ONE rounding per lane
-// silu of two bf16 values, bf16 after every operator: sigmoid, gate * sigmoid
+__device__ __forceinline__ float rcp_approx(float x) {   // subnormal results too, which __fdividef(1, x) makes 0
+  float y;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// silu of two bf16 values, bf16 after every operator: sigmoid, gate * sigmoid.  The approximations are off by a few units of fp32's
+// last place and the sigmoid is rounded to bf16 at once: for all 65536 gates the bits are those of 1 / (1 + expf(-g)) with a full
+// division, which the layers of up to 32 rows use and which the memory-bound kernel over a prompt's rows has no time for
+// (8192 x 14336: 2-byte accesses and full division 406 us, 16-byte accesses and this 111).
 __device__ __forceinline__ uint32_t silu_bf16x2(uint32_t g) {
   const float a = __uint_as_float(g << 16), b = __uint_as_float(g & 0xffff0000u);
-  const uint32_t s = pack_bf16(__fdividef(1.f, 1.f + __expf(-a)), __fdividef(1.f, 1.f + __expf(-b)));
+  const uint32_t s = pack_bf16(rcp_approx(1.f + __expf(-a)), rcp_approx(1.f + __expf(-b)));
   return pack_bf16(a * __uint_as_float(s << 16), b * __uint_as_float(s & 0xffff0000u));
 }
 __device__ __forceinline__ uint32_t mul_bf16x2_rn(uint32_t t, uint32_t u) {   // products in fp32, one rounding
   return pack_bf16(__uint_as_float(t << 16) * __uint_as_float(u << 16), __uint_as_float(t & 0xffff0000u) * __uint_as_float(u & 0xffff0000u));
 }
+// bf16x2 fused multiply-add (HFMA2.BF16, FMA pipe): fp32-exact product and sum, ONE rounding per lane
 __device__ __forceinline__ uint32_t fma_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;
   asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));

@@ -31,3 +31,14 @@ def test_the_engines_bring_the_pipelines_word_to_the_host():
     eng.watch.words.fill_(-1)
     eng.watch.post()
     assert eng.generated().shape == (1, 1) and eng.watch.words.tolist() == [0, 0]
+
+
+def test_silu_of_every_gate():
+    """All bf16 gates: the bits of sigmoid and product in full fp32, rounded to bf16 after each (subnormal sigmoids among them)."""
+    from proxy_inference_engine_b200 import ops
+    g = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    sig = (1 / (1 + torch.exp(-g.float()))).to(torch.bfloat16)
+    want = (g.float() * sig.float()).to(torch.bfloat16)
+    got = ops.silu_mul(g.cuda(), torch.ones_like(g).cuda()).cpu()
+    nan = want.isnan()
+    assert torch.equal(nan, got.isnan()) and torch.equal(got[~nan].view(torch.int16), want[~nan].view(torch.int16))
