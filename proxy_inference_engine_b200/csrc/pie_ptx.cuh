@@ -185,10 +185,13 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 __device__ __forceinline__ uint16_t f2bf(float f) { return (uint16_t)(pack_bf16(f, 0.f) & 0xffffu); }
 __device__ __forceinline__ float bfround(float f) { return __uint_as_float(pack_bf16(0.f, f) & 0xffff0000u); }
-__device__ __forceinline__ float rcp_approx(float x) {   // subnormal results too, which __fdividef(1, x) makes 0
-  float y;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
+// 1 / (1 + e^-a), approximately, in six instructions.  Divisors beyond 2^126, whose reciprocal is subnormal (__fdividef makes it 0),
+// are taken a quarter at a time; rcp.approx.f32, which handles them itself, cost the whole kernel 28 % of its time.
+__device__ __forceinline__ float sigmoid_approx(float a) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(a * -1.4426950408889634f));   // (e^-a below 2^-126 adds nothing to 1)
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(e, 0.25f, 0.25f)));
+  return r * 0.25f;
 }
 // silu of two bf16 values, bf16 after every operator: sigmoid, gate * sigmoid.  The approximations are off by a few units of fp32's
 // last place and the sigmoid is rounded to bf16 at once: for all 65536 gates the bits are those of 1 / (1 + expf(-g)) with a full
@@ -196,7 +199,7 @@ __device__ __forceinline__ float rcp_approx(float x) {   // subnormal results to
 // (8192 x 14336: 2-byte accesses and full division 406 us, 16-byte accesses and this 111).
 __device__ __forceinline__ uint32_t silu_bf16x2(uint32_t g) {
   const float a = __uint_as_float(g << 16), b = __uint_as_float(g & 0xffff0000u);
-  const uint32_t s = pack_bf16(rcp_approx(1.f + __expf(-a)), rcp_approx(1.f + __expf(-b)));
+  const uint32_t s = pack_bf16(sigmoid_approx(a), sigmoid_approx(b));
   return pack_bf16(a * __uint_as_float(s << 16), b * __uint_as_float(s & 0xffff0000u));
 }
 __device__ __forceinline__ uint32_t mul_bf16x2_rn(uint32_t t, uint32_t u) {   // products in fp32, one rounding
