@@ -440,14 +440,11 @@ __global__ void __launch_bounds__(kTileThreads, 2) attn_tile_kernel(__nv_bfloat1
 template <int D, int DV>
 static cudaError_t launch_tile(__nv_bfloat16* out, const float* q, const pieh_attn& a, const pieh_batch& b, cudaStream_t st) {
   constexpr int smem = TileSmem<D, DV>::BYTES;
-  static unsigned long long configured = 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!(configured >> (dev & 63) & 1)) {
-    cudaError_t e = cudaFuncSetAttribute(attn_tile_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    configured |= 1ull << (dev & 63);
-  }
+  static std::atomic<unsigned long long> served{0};
+  const cudaError_t set = pie::once_per_device(served, [] {
+    return cudaFuncSetAttribute(attn_tile_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  });
+  if (set != cudaSuccess) return set;
   return launch_k(attn_tile_kernel<D, DV>, dim3((unsigned)(a.H * b.n_tiles)), dim3(kTileThreads), smem, st, out, q, a, b);
 }
 

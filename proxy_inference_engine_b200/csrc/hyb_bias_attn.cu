@@ -517,14 +517,11 @@ template <int D, int DV, bool SHARED>
 static cudaError_t launch_tile(__nv_bfloat16* out, const float* q, const float* proj, long long ld, const pieh_bias_attn& a,
                                const pieh_batch& b, cudaStream_t st) {
   constexpr int smem = 2 * 64 * ((D * 2 + 127) / 128 * 128 + (SHARED ? 0 : DV * 2));
-  static unsigned long long configured = 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!(configured >> (dev & 63) & 1)) {
-    cudaError_t e = cudaFuncSetAttribute(bias_tile_kernel<D, DV, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    configured |= 1ull << (dev & 63);
-  }
+  static std::atomic<unsigned long long> served{0};
+  const cudaError_t set = pie::once_per_device(served, [] {
+    return cudaFuncSetAttribute(bias_tile_kernel<D, DV, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  });
+  if (set != cudaSuccess) return set;
   return launch_k(bias_tile_kernel<D, DV, SHARED>, dim3(b.n_tiles, a.H), dim3(128), smem, st, out, q, proj, ld, a, b);
 }
 

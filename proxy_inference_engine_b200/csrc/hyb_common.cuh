@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "../../include/pie_b200_hybrid.h"
+#include "pie_once.h"
 
 namespace pieh {
 

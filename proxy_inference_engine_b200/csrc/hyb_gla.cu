@@ -484,13 +484,12 @@ static cudaError_t launch_gla(float* o, const float* proj, long long ld, const f
                               const pieh_batch& b, const GlaSeg& sg, cudaStream_t st) {
   constexpr int NT = R * (kGlaCols / CPT);
   constexpr size_t smem = (size_t)2 * kGlaChunk * (3 * R * RPT + kGlaCols) * 4;
-  static unsigned long long configured = 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (smem > 48 * 1024 && !(configured >> (dev & 63) & 1)) {
-    cudaError_t e = cudaFuncSetAttribute(gla_scan_kernel<R, RPT, CPT, PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    configured |= 1ull << (dev & 63);
+  if (smem > 48 * 1024) {
+    static std::atomic<unsigned long long> served{0};
+    const cudaError_t set = pie::once_per_device(served, [] {
+      return cudaFuncSetAttribute(gla_scan_kernel<R, RPT, CPT, PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    });
+    if (set != cudaSuccess) return set;
   }
   count_launch();
   return launch_k(gla_scan_kernel<R, RPT, CPT, PASS>, dim3((d.dv + kGlaCols - 1) / kGlaCols, d.H, PASS == 0 ? b.n_seq : b.n_tiles),

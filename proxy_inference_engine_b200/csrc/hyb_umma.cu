@@ -349,14 +349,11 @@ bool linear_umma_ok(const LinArgs& a, int x_dtype, int w_dtype) {
 template <typename OT>
 static cudaError_t launch_grouped(const LinArgs& a, cudaStream_t st) {
   constexpr size_t smem = (size_t)4 * (128 * kBK * 2 + kBN * kBK * 2) + 1024;
-  static unsigned long long configured = 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!(configured >> (dev & 63) & 1)) {
-    cudaError_t e = cudaFuncSetAttribute(linear_grouped_kernel<OT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    configured |= 1ull << (dev & 63);
-  }
+  static std::atomic<unsigned long long> served{0};
+  const cudaError_t set = pie::once_per_device(served, [] {
+    return cudaFuncSetAttribute(linear_grouped_kernel<OT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
+  if (set != cudaSuccess) return set;
   // blockIdx.y walks the list of <= 128-slot tiles, whose length is only known on the device (S = experts)
   const dim3 grid((a.N + kBN - 1) / kBN, a.M / 128 + a.S, 1);
   count_launch();

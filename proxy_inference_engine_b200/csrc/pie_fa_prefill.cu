@@ -400,15 +400,16 @@ bool fa_prefill_umma_ok(const uint16_t* out, const uint16_t* q, const uint16_t* 
 template <int D>
 static cudaError_t launch_fap(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FapArgs& a, cudaStream_t st) {
   using T = FapTile<D>;
-  static unsigned long long configured = 0;   // per device
-  if (first_use_on_device(configured)) {
+  static std::atomic<unsigned long long> served{0};
+  const cudaError_t set = once_per_device(served, [] {
     cudaFuncAttributes at;
-    cudaError_t e = cudaFuncGetAttributes(&at, fa_prefill_umma_kernel<D>);
+    const cudaError_t e = cudaFuncGetAttributes(&at, fa_prefill_umma_kernel<D>);
+    if (e != cudaSuccess) return e;
     // the warps' register shares must fit what the block is launched with, or they would wait for registers for good
-    if (e == cudaSuccess && at.numRegs * T::THREADS < 8 * 32 * 216 + 4 * 32 * 64) e = cudaErrorInvalidConfiguration;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fa_prefill_umma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
-    if (e != cudaSuccess) { configured = 0; return e; }
-  }
+    if (at.numRegs * T::THREADS < 8 * 32 * 216 + 4 * 32 * 64) return cudaErrorInvalidConfiguration;
+    return cudaFuncSetAttribute(fa_prefill_umma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
+  });
+  if (set != cudaSuccess) return set;
   count_launch();
   fa_prefill_umma_kernel<D><<<dim3((unsigned)(a.B * a.Hq), (unsigned)((a.L + 255) / 256)), T::THREADS, T::SMEM, st>>>(mq, mk, mv, a);
   return cudaGetLastError();

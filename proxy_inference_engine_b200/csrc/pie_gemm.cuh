@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "pie_once.h"
 #include "pie_ptx.cuh"
 #include "pie_umma.cuh"
 
@@ -576,14 +577,9 @@ cudaError_t gemm_launch(const CUtensorMap& mx, const CUtensorMap& mw, const Gemm
                         cudaStream_t st) {
   using T = GemmTile<CG, BN, QB, SPLIT>;
   auto kern = gemm_kernel<CG, BN, QB, SPLIT, Epi>;
-  static unsigned long long configured = 0;   // per device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!(configured >> (dev & 63) & 1)) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
-    if (e != cudaSuccess) return e;
-    configured |= 1ull << (dev & 63);
-  }
+  static std::atomic<unsigned long long> served{0};
+  const cudaError_t set = once_per_device(served, [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM); });
+  if (set != cudaSuccess) return set;
   const int tiles = a.mt * a.nt * a.nb, slots = sms / CG;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = SPLIT ? dim3((unsigned)ranks, (unsigned)tiles, 1) : dim3((unsigned)((tiles < slots ? tiles : slots) * CG), 1, 1);

@@ -20,12 +20,11 @@ int num_sms() {
 template <int BITS, int MT, bool ONECOL>
 static cudaError_t launch_qmv_t(const QmvArgs& a, int warps, int grid, bool pdl, cudaStream_t st) {
   const size_t smem = qmv_smem_bytes(a.M, a.kslice, BITS, warps, MT);
-  static unsigned long long configured = 0;  // opt in to the full 227 KB of dynamic shared memory, once per device
-  if (first_use_on_device(configured)) {
-    cudaError_t e = cudaFuncSetAttribute(qmv_kernel<BITS, MT, ONECOL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kQmvMaxSmem);
-    if (e != cudaSuccess) return e;
-  }
+  static std::atomic<unsigned long long> served{0};   // opt in to the full 227 KB of dynamic shared memory
+  const cudaError_t set = once_per_device(served, [] {
+    return cudaFuncSetAttribute(qmv_kernel<BITS, MT, ONECOL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQmvMaxSmem);
+  });
+  if (set != cudaSuccess) return set;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid, 1, 1);
   cfg.blockDim = dim3((unsigned)warps * 32, 1, 1);
@@ -42,12 +41,11 @@ static cudaError_t launch_qmv_t(const QmvArgs& a, int warps, int grid, bool pdl,
 
 static cudaError_t launch_qmv_smemargs(const QmvArgs& a, int warps, int grid, bool pdl, cudaStream_t st) {
   const size_t smem = qmv_smem_bytes(a.M, a.kslice, 4, warps, 1) + (size_t)warps * 32 * kQmvProdWords * 4;
-  static unsigned long long configured = 0;
-  if (first_use_on_device(configured)) {
-    cudaError_t e = cudaFuncSetAttribute(qmv_kernel_smemargs<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kQmvMaxSmem - 1024);
-    if (e != cudaSuccess) return e;
-  }
+  static std::atomic<unsigned long long> served{0};
+  const cudaError_t set = once_per_device(served, [] {
+    return cudaFuncSetAttribute(qmv_kernel_smemargs<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQmvMaxSmem - 1024);
+  });
+  if (set != cudaSuccess) return set;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid, 1, 1);
   cfg.blockDim = dim3((unsigned)warps * 32, 1, 1);
