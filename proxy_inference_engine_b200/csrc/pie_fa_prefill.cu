@@ -326,8 +326,6 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (!(alive = gemm_wait(smem_u32(&v_empty[i]), ph ^ 1, abortp))) break;
         fetch(j, &map_v, smV + i * T::TILE, &v_full[i]);
       }
-      if (!alive)
-        for (int w = 0; w < 1000; ++w) __nanosleep(1000);
     }
     // ------------------------------------------------------------------------------------------------ MMAs
     if (warp == 9) {
@@ -383,6 +381,7 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (*abortp) gemm_drain();
   if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
 }
 

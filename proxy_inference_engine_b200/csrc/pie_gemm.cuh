@@ -17,8 +17,8 @@
 //     the stage's bf16 rows, w_hat = bf16(scale q + bias) rounded once (fused bf16x2 / fp32 multiply-add): a thread takes one
 //     row of a K step, the groups take the K steps in turn (one step's chain of wait, load, store and proxy fence is longer
 //     than its MMAs).
-// No wait is unbounded: one that expires raises g_gemm_error and a CTA-wide flag, every role leaves its loop, copies in flight
-// are given time to land, tensor memory is freed and the kernel returns.
+// No wait is unbounded: one that expires raises g_gemm_error and a CTA-wide flag, every role leaves its loop, copies and MMAs in
+// flight are given time to land, tensor memory is freed and the kernel returns.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -84,7 +84,13 @@ __device__ __forceinline__ bool gemm_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
-// the same for a whole warp whose lanes go on together: one lane's expiry takes the warp out
+// A wait of some role expired: the roles that issue have left their loops, what they asked for lands within microseconds, and nothing
+// of it may outlive the CTA's shared and tensor memory.  (The issuing role need not be the one whose wait expired, and may have come to
+// its end: the whole CTA waits, behind its last barrier.)
+__device__ __forceinline__ void gemm_drain() {
+  for (int w = 0; w < 1000; ++w) __nanosleep(1000);
+}
+// gemm_wait for a whole warp whose lanes go on together: one lane's expiry takes the warp out
 __device__ __forceinline__ bool gemm_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return __all_sync(0xffffffffu, gemm_wait(bar, parity, abort_flag));
 }
@@ -314,8 +320,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         }
         if (SPLIT) break;
       }
-      if (!alive)   // copies that were requested land within microseconds; nothing of them may outlive the CTA
-        for (int w = 0; w < 1000; ++w) __nanosleep(1000);
     }
   } else if (warp == T::W_MMA) {
     // ---------------------------------------------------------------- MMA issue
@@ -366,8 +370,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         }
         if (SPLIT) break;
       }
-      if (!alive)
-        for (int w = 0; w < 1000; ++w) __nanosleep(1000);
     }
   } else if (QB && warp >= T::W_DEQ) {
     // ---------------------------------------------------------------- dequantisers: thread = row, group = every GROUPS-th K step
@@ -505,6 +507,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (*abortp) gemm_drain();
   if (CG == 2) cluster_sync_all();   // neither CTA of a pair leaves while the other may still use its memory
   if (warp == T::W_MMA) {
     if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(T::TMEM_COLS) : "memory");
