@@ -342,6 +342,8 @@ bool linear_umma_ok(const LinArgs& a, int x_dtype, int w_dtype) {
       (reinterpret_cast<uintptr_t>(a.x) & 31) == 0 && a.epi != PIEH_EPI_GLU)
     return false;   // a handful of output columns: linear_skinny_kernel reads x once instead of filling 256-column tiles
   if (a.x_bs % 8 || a.w_bs % 8 || a.x_bs < 0 || a.w_bs < 0) return false;   // every product's operands start on a 16-byte boundary
+  // what a tiled copy can describe: rows that go forward, strides below 2^40 bytes (rows that repeat or go backward: linear_tile_kernel)
+  if (!a.g_tiles && (a.x_ld <= 0 || ((a.x_ld | a.x_bs | a.w_bs) >> 39) != 0)) return false;
   return x_dtype == PIE_DTYPE_BF16 && w_dtype == PIE_DTYPE_BF16 && a.M > 32 && a.K % kBK == 0 && a.x_ld % 8 == 0 &&
          (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.w) & 15) == 0;
 }

@@ -92,6 +92,20 @@ def test_dense_gemm_tiles(M, N, K):
     assert L.pieh_pipeline_error() == 0
 
 
+@pytest.mark.parametrize("step", [0, -1])   # rows that repeat, rows that go backward
+def test_dense_rows_a_tiled_copy_cannot_describe(step):
+    from proxy_inference_engine_b200 import _lib
+    L = _lib.load_hybrid(build_if_missing=True)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    M, N, K = 70, 130, 128
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn((N, K), generator=g, device="cuda").to(torch.bfloat16)
+    rows = x.flip(0) if step else x[-1:].expand(M, K)
+    out = torch.full((M, N), float("nan"), device="cuda")
+    assert L.pieh_linear(_p(out), 1, N, _p(x[-1]), 0, step * K, _p(w), 0, None, M, N, K, 0, 0.0, None, None, 0, None) == 0
+    _within(out, rows.double() @ w.double().t(), (rows.double().abs() @ w.double().abs().t()) * (K * 2 ** -23))
+
+
 @pytest.mark.parametrize("shared", ["", "x", "w"])
 def test_dense_gemm_batched(shared):
     """Products side by side, head-major columns; an operand stride of zero shares that operand."""
