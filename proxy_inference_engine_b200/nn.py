@@ -136,8 +136,11 @@ def fused_swiglu(x, gate, up):
 
 def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
     """Up to 32 rows through several bias-free QuantizedLinears in ONE launch, with the RMSNorm in front of them, and the
-    residual sum or SwiGLU behind them where asked for -- the arithmetic of the separate calls, rounding for rounding:
+    residual sum or SwiGLU behind them where asked for:
         [..., sum N]  their outputs side by side;   residual: residual + output;   swiglu: silu(first) * second.
+    Results are rounded where the separate calls round them.  One matrix, with or without a residual, gives their bits; a norm's
+    sum of squares and the sums over K of several matrices are taken in another order, so that a value near a rounding boundary
+    may fall on its other side.
     None where that kernel does not apply (the caller then makes the separate calls, which also report what is wrong)."""
     K = x.shape[-1]
     rows = x.numel() // K if K else 0
@@ -155,8 +158,10 @@ def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
             return None
         N //= 2
     if norm is not None:
+        if type(norm) is not RMSNorm:
+            return None
         nw = norm.weight
-        if type(norm) is not RMSNorm or nw.dtype != torch.bfloat16 or nw.shape != (K,) or not nw.is_contiguous() or nw.data_ptr() % 16:
+        if nw.dtype != torch.bfloat16 or nw.shape != (K,) or not nw.is_contiguous() or nw.data_ptr() % 16:
             return None
     if residual is not None and (residual.shape != x.shape[:-1] + (N,) or residual.dtype != torch.bfloat16
                                  or not residual.is_contiguous()):

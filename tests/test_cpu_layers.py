@@ -145,3 +145,55 @@ def test_any_callable_may_stand_for_a_projection(monkeypatch, rows, swapped):
     mlp.up_proj = plain if swapped == "gate_proj" else other
     x = torch.ones((rows, K), dtype=torch.bfloat16)
     assert torch.equal(mlp(x), 2 * x[..., :N])
+
+
+def _plain(N=256, K=512, bits=4):
+    from proxy_inference_engine_b200 import nn
+    lin = object.__new__(nn.QuantizedLinear)
+    lin.group_size, lin.bits = 64, bits
+    lin.weight, lin.scales, lin.biases = torch.zeros((N, K * bits // 32), dtype=torch.int32), _bf16(N, K // 64), _bf16(N, K // 64)
+    return lin
+
+
+def _with(lin, **fields):
+    for name, value in fields.items():
+        setattr(lin, name, value)
+    return lin
+
+
+def test_fused_rows_takes_what_its_kernel_takes_and_nothing_else(monkeypatch):
+    from proxy_inference_engine_b200 import nn
+    monkeypatch.setattr(ops, "qmv_fused", lambda *a: "fused")
+    norm = object.__new__(nn.RMSNorm)
+    norm.weight, norm.eps = _bf16(512), 1e-5
+    x = _bf16(32, 512)
+    takes = lambda x=x, lins=(_plain(),), **kw: nn.fused_rows(x, lins, **kw) == "fused"
+    assert takes() and takes(_bf16(1, 1, 512)) and takes(lins=(_plain(7), _plain(300)), norm=norm)
+    assert takes(residual=_bf16(32, 256)) and takes(lins=(_plain(), _plain()), swiglu=True)
+    assert takes(_bf16(4, 384), (_plain(K=384, bits=8),))
+    assert not takes(_bf16(33, 512)) and not takes(_bf16(0, 512))                       # rows
+    assert not takes(x.float()) and not takes(_bf16(32, 1024)[:, ::2]) and not takes(_bf16(513)[1:].view(1, 512))   # type, stride, alignment
+    assert not takes(_bf16(4, 384), (_plain(K=384),))                                   # K in whole stages: 256 at 4 bits, 128 at 8
+    assert not takes(_bf16(4, 1024))                                                    # K of x and of the matrix
+    assert not takes(lins=(_plain(), _plain(bits=8))) and not takes(lins=(_with(_plain(), group_size=32),))
+    assert not takes(lins=(_with(_plain(), bias=_bf16(256)),)) and not takes(lins=(_with(_plain(), scales=torch.zeros(256, 8)),))
+    other = object.__new__(type("Other", (nn.QuantizedLinear,), {}))
+    other.__dict__.update(vars(_plain()))
+    assert not takes(lins=(other,)) and not takes(lins=(_plain(), lambda x: x))         # a subclass may compute something else
+    assert not takes(lins=(_plain(128), _plain(256)), swiglu=True)                      # halves of one width
+    assert not takes(residual=_bf16(32, 255)) and not takes(residual=torch.zeros(32, 256))
+    norm.weight = torch.zeros(512)
+    assert not takes(norm=norm) and not takes(norm=lambda x: x)
+
+
+def test_a_tensor_parallel_block_takes_the_separate_calls(monkeypatch):
+    from types import SimpleNamespace
+    from proxy_inference_engine_b200 import llama, nn
+    monkeypatch.setattr(nn, "fused_rows", lambda *a, **k: pytest.fail("fused"))
+    block = object.__new__(llama.TransformerBlock)
+    block.self_attn, block.mlp = object.__new__(llama.Attention), object.__new__(llama.MLP)
+    block.self_attn.tp = SimpleNamespace(on=True)
+    assert block._few_rows(_bf16(1, 1, 512), None, None) is None
+    block.self_attn.tp = None
+    block.mlp = lambda x: x
+    assert block._few_rows(_bf16(1, 1, 512), None, None) is None
