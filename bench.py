@@ -1,4 +1,4 @@
-"""bench.py -- decode tok/s of the B200 quantized-Llama path (BASELINE.json configs[1]: Llama-3.1-8B, MLX q4 gs64,
+"""bench.py -- decode tok/s of the B200 quantized-Llama path (Llama-3.1-8B, MLX q4 gs64,
 bs1 decode) with the HBM roofline of its dominant kernel and the reference's CPU path timed beside it.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference] [--model llama-3.1-8b] [--bits 4] [--batch 1]
@@ -36,8 +36,8 @@ def parse():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-kernel-timing", action="store_true")
     ap.add_argument("--no-70b", action="store_true", help="N > 1: skip the Llama-3.1-70B tensor-parallel sub-records")
-    ap.add_argument("--no-config3", action="store_true", help="skip the 8-bit / batch-32 / paged-KV sub-record (BASELINE configs[2])")
-    ap.add_argument("--no-prefill", action="store_true", help="skip the prefill GEMM figure (BASELINE config 4 shapes)")
+    ap.add_argument("--no-config3", action="store_true", help="skip the 8-bit / batch-32 / paged-KV sub-record (Llama-3.1-8B)")
+    ap.add_argument("--no-prefill", action="store_true", help="skip the prefill GEMM figure (an 8192-token prompt)")
     ap.add_argument("--family", default="llama", choices=("llama", "golitar", "babodra", "maginex", "zelinex", "dudurax",
                                                               "vokusun"),
                     help="golitar: prefill / decode throughput and per-operator rooflines of the Golitar family at --size, "
@@ -50,7 +50,7 @@ def parse():
 
 
 def model_numbers(args, bits):
-    """Algorithmic bytes per decode step (SURVEY.md 8d): packed W + bf16 scales + bf16 biases, read once per step."""
+    """Algorithmic bytes per decode step: packed W + bf16 scales + bf16 biases, read once per step."""
     h, f, L, V = args.hidden_size, args.intermediate_size, args.num_hidden_layers, args.vocab_size
     nh, nkv = args.num_attention_heads, args.num_key_value_heads
     d = args.head_dim
@@ -66,7 +66,7 @@ def model_numbers(args, bits):
 # ------------------------------------------------------------------------------------------ CPU baseline
 def host_threads():
     """Threads the CPU arm uses: the cores this process may run on.  NOT omp_get_max_threads(): torchrun exports
-    OMP_NUM_THREADS=1 to its workers, which made round 1's N>1 reference arms 15-20x slower than its N=1 arm."""
+    OMP_NUM_THREADS=1 to its workers, which makes an N>1 reference arm 15-20x slower than an N=1 arm."""
     try:
         return max(1, len(os.sched_getaffinity(0)))
     except Exception:
@@ -76,13 +76,13 @@ def host_threads():
 def cpu_baseline(margs, bits, steps=1, warmup=0, budget_s=20.0, config1=True):
     """The reference's own `_qmm_t<float, bits, 64>` (MLX/mlx/backend/cpu/quantized.cpp:96-153, compiled where it lies
     into oracle/_ref) on the decode shapes of this model, M = 1; falls back to the oracle port when oracle/_ref is
-    absent.  Reported figures (SURVEY 8d / BASELINE.md section 4):
+    absent.  Reported figures:
       value          all host cores (rows sliced over `cores` threads, each thread runs the untouched reference loop);
       single_thread  1 thread -- MLX's CPU stream is one worker thread (MLX/mlx/scheduler.h:22-35) and `_qmm_t` has no
                      intra-op threading: this is what the reference itself would do on this host;
       bf16_exact     one matrix through `_qmm_t<bfloat16_t>` (what MLX-CPU really executes for a bf16 checkpoint on x86:
                      every product and sum rounded to bf16 -- low precision, time only);
-      config1        BASELINE config 1 (Llama-3.2-1B q4, 128-token prefill, greedy decode) through the WHOLE oracle
+      config1        Llama-3.2-1B q4, 128-token prefill, greedy decode through the WHOLE oracle
                      (attention, norms, rope, head), prefill and decode tok/s separately.
     Sample: `n_layers_sample` transformer layers' seven matmuls, tok/s extrapolated by parameter count."""
     import numpy as np
@@ -162,7 +162,7 @@ def cpu_baseline(margs, bits, steps=1, warmup=0, budget_s=20.0, config1=True):
 
 
 def cpu_config1(nthreads, prompt_len=128, decode_steps=3):
-    """BASELINE config 1 through the whole CPU oracle (fp32 mode A = MLX-CPU on fp32 inputs): Llama-3.2-1B q4 gs64,
+    """The 1B model through the whole CPU oracle (fp32 mode A = MLX-CPU on fp32 inputs): Llama-3.2-1B q4 gs64,
     bs1, 128-token prompt in ONE forward (inference_engine.py:278), then greedy decode steps.  Random packed weights
     (the path is data-independent).  Bounded: the prefill plus `decode_steps` steps."""
     import numpy as np
@@ -257,7 +257,7 @@ def measured_peaks():
             p = json.load(f)
         return float(p["hbm_gbs"]), "measured (MEASURED_PEAKS.json)"
     except Exception:
-        return 6650.0, "fallback (B200_PROFILING.md)"
+        return 6650.0, "fallback"
 
 
 def time_qmv_launches(eng, n_steps=3):
@@ -344,7 +344,7 @@ def time_exchanges_in_graph(eng, replays=20):
 
 
 def tp_subrecord(model_name, bits, batches, rank, world, prompt=128, steps=32):
-    """north_star's tensor-parallel curve: Llama-3.1-70B q4 at bs1 and bs16 on this many GPUs.
+    """The tensor-parallel curve: Llama-3.1-70B q4 at bs1 and bs16 on this many GPUs.
     One sharded random-init model (every rank draws the full tensors with the same seed and keeps its slice), one
     engine per batch size; device-timed like the headline value (barrier, CUDA events, max over ranks)."""
     import torch
@@ -383,7 +383,7 @@ def tp_subrecord(model_name, bits, batches, rank, world, prompt=128, steps=32):
 
 
 def config3_subrecord(model_name, steps=24, warmup=4, batch=32, prompt=2048, kv_bits=None):
-    """BASELINE configs[2]: 8-bit weights, batch 32, paged KV cache, 2k context on one GPU -- the other end of the metric's
+    """8-bit weights, batch 32, paged KV cache, 2k context on one GPU -- the other end of the metric's
     "bs 1/32".  Random-init model of its own (the headline model is 4-bit), device-timed like the headline value."""
     import torch
     from proxy_inference_engine_b200.checkpoint import build_model, preset_args, random_weights
@@ -422,7 +422,7 @@ def ncu_traffic_per_launch(alg_bytes_per_launch, bits):
     average launch.  None if the capture is absent or was taken at another bit width."""
     import csv
     pdir = os.path.join(os.path.dirname(os.path.abspath(__file__)), "profiles")
-    path = os.path.join(pdir, "r02c_prof_qmv_ncu_full_summary.csv")   # this round's capture (both GEMV kernels)
+    path = os.path.join(pdir, "r02c_prof_qmv_ncu_full_summary.csv")    # both GEMV kernels
     if not os.path.exists(path):
         path = os.path.join(pdir, "r01e_prof_qmv_ncu_full_summary.csv")
     if bits != 4 or not os.path.exists(path):
@@ -434,7 +434,7 @@ def ncu_traffic_per_launch(alg_bytes_per_launch, bits):
         wr = sum(float(x) for x in rows["dram__bytes_write.sum"][2:6]) * unit[rows["dram__bytes_write.sum"][1]]
     except (KeyError, ValueError):
         return None, "ncu summary not readable"
-    alg = 66.10e6 + 33.07e6 + 14.18e6 + 9.45e6  # weights + scales + biases of gate+up, down, qkv, o (DESIGN.md section 4)
+    alg = 66.10e6 + 33.07e6 + 14.18e6 + 9.45e6  # weights + scales + biases of gate+up, down, qkv, o
     ratio = (rd + wr) / alg
     return int(alg_bytes_per_launch * ratio), (f"{os.path.basename(path)}: committed ncu --set full capture of the step's GEMV "
                                                 f"launches (traffic / algorithmic = {ratio:.4f}); NOT measured in this run")
@@ -596,7 +596,7 @@ def run_b200(a):
 
 
 def prefill_figure(margs, bits, M=8192):
-    """Tensor-pipe figure of the prefill contraction (8k-token prompt): one layer's seven quantized
+    """Tensor-pipe figure of the prefill contraction (an 8192-token prompt): one layer's seven quantized
     matmuls at M = 8192 through pie_qmm (tcgen05), useful flops 2*M*N*K, against the measured bf16 sustained peak."""
     import torch
     from proxy_inference_engine_b200 import ops
@@ -630,7 +630,7 @@ def prefill_figure(margs, bits, M=8192):
             peak = float(json.load(fh)["bf16_tflops_sustained"])
         src = "measured sustained (MEASURED_PEAKS.json)"
     except Exception:
-        peak, src = 1400.0, "fallback (B200_PROFILING.md)"
+        peak, src = 1400.0, "fallback"
     tf = flops / ms / 1e9
     return {"workload": f"one transformer layer's 7 quantized matmuls, M = {M} (8k-token prefill), q{bits}",
             "kernel": f"gemm_kernel, {bits}-bit weights (tcgen05.mma kind::f16, TMEM accumulators)", "ms_per_layer": round(ms, 3),

@@ -5,12 +5,12 @@ Python face of ``oracle/pie_oracle.c`` (plain-C restatement of the reference alg
 Only ``tests/``, ``__graft_entry__.smoke()`` and ``bench.py``'s ``cpu_baseline`` /
 ``--impl reference`` legs may import this module.  The product package never does.
 
-Citations: MLX = /root/reference/src/pie_core/external/mlx, PIE = /root/reference/src/proxy_inference_engine.
+Citations: MLX = src/pie_core/external/mlx, PIE = src/proxy_inference_engine.
 
 Tensors are numpy float32; a "bf16 tensor" is float32 with bf16-representable values.
 ``mode='A'``: every op in float32 (exactly what MLX's CPU backend computes for float32 inputs).
 ``mode='B'``: fp32 inside each op, bf16 rounding at every MLX op boundary (what the Metal
-kernels compute for a bf16 checkpoint; SURVEY.md section 7 / Appendix A) -- the parity target
+kernels compute for a bf16 checkpoint) -- the parity target
 of the CUDA path.
 """
 from __future__ import annotations
@@ -33,7 +33,7 @@ _u8p = np.ctypeslib.ndpointer(np.uint8, flags="C_CONTIGUOUS")
 
 
 def build(force: bool = False) -> None:
-    """Compile the restatement (always possible: gcc) and, if /root/reference is mounted, _ref."""
+    """Compile the restatement (always possible: gcc) and, if the reference is mounted, _ref."""
     if force or not os.path.exists(_LIB) or (
         os.path.getmtime(_LIB) < os.path.getmtime(os.path.join(_HERE, "pie_oracle.c"))
     ):
@@ -524,7 +524,7 @@ class QuantizedKVCache:
 class LlamaOracle:
     """Model.__call__ (PIE/models/llama/language.py:199-210) over MLX-layout quantized weights.
 
-    ``weights``: dict of numpy arrays keyed as the checkpoint schema (SURVEY.md 8(a13)):
+    ``weights``: dict of numpy arrays keyed as the checkpoint schema:
     ``model.layers.{i}.self_attn.q_proj.{weight,scales,biases}`` ... (uint32 / float32 holding
     bf16 values), ``model.embed_tokens.*``, ``model.norm.weight``, ``lm_head.*``.
     """

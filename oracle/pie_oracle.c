@@ -5,11 +5,11 @@
  * load this library; the product path never does and fails loudly without its CUDA library.
  *
  * Parity status: PINNED.  orc_quantize / orc_qmm_t_seq are checked bit-for-bit against the
- * reference's own code compiled from /root/reference (oracle/ref_harness.cpp -> oracle/_ref),
+ * reference's own code compiled where it lies (oracle/ref_harness.cpp -> oracle/_ref),
  * and every routine is checked against the MLX property tests it restates
  * (tests/test_oracle_*.py; MLX/python/tests/test_quantized.py, test_fast.py, test_fast_sdpa.py).
  *
- * Citations: MLX = /root/reference/src/pie_core/external/mlx, PIE = /root/reference/src/proxy_inference_engine.
+ * Citations: MLX = src/pie_core/external/mlx, PIE = src/proxy_inference_engine.
  *
  * Conventions.  Every float tensor crosses this ABI as float32.  A "bf16 tensor" is a float32
  * array whose values are bf16-representable; "mode B" entry points take `round_out` and round

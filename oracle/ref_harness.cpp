@@ -2,14 +2,14 @@
 //
 // Thin C-ABI harness around the reference's OWN CPU code for the quantized path.  It does not
 // copy any reference source: the single translation unit below #includes the vendored MLX file
-// where it lies under /root/reference and re-exports its anonymous-namespace templates
+// where it lies and re-exports its anonymous-namespace templates
 //   quantize<T,U>            MLX/mlx/backend/cpu/quantized.cpp:603-661
 //   _qmm_t<T,bits,gs>        MLX/mlx/backend/cpu/quantized.cpp:96-153   (the x86 path: simd::max_size==1,
 //                            MLX/mlx/backend/cpu/simd/base_simd.h:13-14 -> dispatch at quantized.cpp:240-244)
 //   _qmm<T,bits,gs>          MLX/mlx/backend/cpu/quantized.cpp:38-94    (transpose=False: the values product of
 //                            quantized_scaled_dot_product_attention, PIE/models/base.py:81-83)
-// (MLX = /root/reference/src/pie_core/external/mlx).  Built by oracle/Makefile into
-// oracle/_ref/libpie_ref.so (git-ignored, NOT gpurun-ignored).  Unreferenced eval_cpu bodies that need
+// (MLX = src/pie_core/external/mlx).  Built by oracle/Makefile into
+// oracle/_ref/libpie_ref.so (git-ignored).  Unreferenced eval_cpu bodies that need
 // libmlx symbols are discarded with -ffunction-sections/--gc-sections.
 //
 // The row-sliced *_mt variants call the very same reference template on disjoint row ranges from

@@ -3,7 +3,7 @@
 ``KVCache`` keeps the semantics of PIE's default cache (ReusableKVCache.update_and_fetch,
 PIE/cache/kv_cache/reusable.py:96-142; KVCache, cache.py:28-68): buffers ``[B, n_kv, cap, D]`` growing in steps
 of 256 tokens, a scalar ``offset``, ``update_and_fetch(k, v)`` returning views of the first ``offset`` tokens.
-``PagedKVCache`` is the layout BASELINE config 3 names (64-token pages as CORE/include/engine/page.hpp:14,29-30,
+``PagedKVCache`` is the paged layout (64-token pages as CORE/include/engine/page.hpp:14,29-30,
 bf16): a page pool ``[n_pages, 64, n_kv, D]`` per layer plus an int32 page table ``[B, max_pages]``.
 """
 from __future__ import annotations

@@ -1,9 +1,9 @@
-"""Checkpoint boundary of the path: MLX-layout quantized Llama checkpoints (SURVEY.md 8(a13)).
+"""Checkpoint boundary of the path: MLX-layout quantized Llama checkpoints.
 
 ``load_model`` mirrors PIE/models/utils.py:51-125: read ``config.json`` + every ``model*.safetensors``, build
 ``Model(ModelArgs)``, ``sanitize``, and assign ``weight`` (U32 words) / ``scales`` / ``biases`` (BF16) to the
 quantized layers named by ``config["quantization"]``.  ``random_weights`` is the synthetic-checkpoint generator
-of the benchmarks (SURVEY.md 8d): nn.Linear / nn.Embedding initialisers, bf16, quantized with the library's
+of the benchmarks: nn.Linear / nn.Embedding initialisers, bf16, quantized with the library's
 bit-exact ``quantize``.
 """
 from __future__ import annotations
@@ -19,7 +19,7 @@ from . import ops
 from .llama import Model, ModelArgs
 
 LLAMA_PRESETS = {
-    # SURVEY.md section 8 header; defaults of PIE/models/llama/language.py:13-29
+    # the models' published sizes; defaults of PIE/models/llama/language.py:13-29
     "llama-3.2-1b": dict(hidden_size=2048, num_hidden_layers=16, intermediate_size=8192, num_attention_heads=32,
                          num_key_value_heads=8, head_dim=64, vocab_size=128256, tie_word_embeddings=True,
                          rope_scaling={"factor": 32.0, "low_freq_factor": 1.0, "high_freq_factor": 4.0}),

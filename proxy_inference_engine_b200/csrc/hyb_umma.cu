@@ -16,7 +16,6 @@ namespace pieh {
 
 using pie::smem_u32;
 
-
 constexpr int kBN = 256, kBK = 64, kProducers = 256, kThreads = kProducers + 32;
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr uint32_t IDESC = pie::umma_idesc_bf16_m128(kBN);

@@ -253,7 +253,7 @@ int pie_qmv_fused_tp(void* out, int out_ld, const void* x, int x_ld, int M, int 
     if (tp) return PIE_EUNSUPPORTED;  // the fused exchange lives in the TMA GEMV (one row, 4-bit, K % 512 == 0)
     // Batched-decode GEMM on tcgen05 (pie_qmd.cu).  PIE_QMD: 0 never, 1 where it measured faster than the GEMV at 32
     // rows (B200, 8B shapes, us GEMV / tcgen05: q8 gate+up 121 / 98, q8 head 417 / 290, q4 head 233 / 217; the narrow
-    // matrices and 4-bit gate+up / down are still faster on the GEMV: DESIGN.md section 4.6), 2 wherever it is supported.
+    // matrices and 4-bit gate+up / down are still faster on the GEMV), 2 wherever it is supported.
     // 8-bit weights, more than 8 rows: the integer tensor cores take the packed weights as they are (pie_qmi.cu).
     // PIE_QMI=0 keeps the bf16 forms below, 2 also routes 1..8 rows here.
     const int qmi_mode = env_int("PIE_QMI", 1);

@@ -145,7 +145,7 @@ struct GemmTile {
   static constexpr int BM = 128 * CG, NB = BN / CG;              // tile rows; w rows staged by one CTA
   static constexpr int A_STAGE = 128 * 128, B_STAGE = NB * 128;  // bytes of one 64-element K step
   static constexpr int CHUNK = NB * 128, RING = QB ? 3 : 0;      // packed rows: 128 bytes each, 256 (4-bit) / 128 (8-bit) of K
-  static constexpr int S = QB ? 5 : (CG == 2 ? 6 : 6);
+  static constexpr int S = QB ? 5 : 6;
   static constexpr int EPI_WARPS = QB ? 4 : 8;
   static constexpr int W_TMA = EPI_WARPS, W_MMA = EPI_WARPS + 1, W_PACK = EPI_WARPS + 2, W_DEQ = EPI_WARPS + 4;
   static constexpr int GROUPS = 3;                                // dequantising groups of four warps, a K step each in turn

@@ -1,4 +1,4 @@
-// Quantised KV cache (SURVEY §8 f3): QuantizedKVCache.update_and_fetch (PIE/cache/kv_cache/quantized.py:38-108:
+// Quantised KV cache: QuantizedKVCache.update_and_fetch (PIE/cache/kv_cache/quantized.py:38-108:
 // mx.quantize of the new keys / values, 8 bits, groups of 64 along head_dim) and quantized_scaled_dot_product_attention
 // for L == 1 (PIE/models/base.py:56-89: scores = quantized_matmul(q * scale, K, transpose=True), softmax,
 // out = quantized_matmul(scores, V, transpose=False)).

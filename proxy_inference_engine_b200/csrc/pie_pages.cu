@@ -1,4 +1,4 @@
-// Page allocator of the paged KV cache (SURVEY 8(f2)): fixed pool of 64-token pages, per-page reference counts, lock-free
+// Page allocator of the paged KV cache: fixed pool of 64-token pages, per-page reference counts, lock-free
 // LIFO free list.  Host code (the pages themselves live in ONE pool tensor per layer in HBM -- cache.PagedKVCache -- and a
 // page id is an index into it; the reference's KVPage owns an MLX array per page, CORE/include/engine/page.hpp:18-123).
 //

@@ -175,7 +175,7 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 // ------------------------------------------------------------------ bf16 helpers
 __device__ __forceinline__ float bf16lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
-// fp32 -> bf16, round to nearest even, NaN -> 0x7FFF canonical (see DESIGN.md).  Always through the PACKED conversion
+// fp32 -> bf16, round to nearest even, NaN -> 0x7FFF canonical.  Always through the PACKED conversion
 // (F2FP.BF16.F32.PACK_AB, full-rate ALU pipe): the scalar F2F.BF16.F32 issues on the quarter-rate XU pipe and was the top
 // stall in the dequantising producers.
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {

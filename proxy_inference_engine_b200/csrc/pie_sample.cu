@@ -1,4 +1,4 @@
-// Device-side sampler of the decode loop (SURVEY 8(f1)): log-probabilities + temperature / top-k / top-p / min-p /
+// Device-side sampler of the decode loop: log-probabilities + temperature / top-k / top-p / min-p /
 // categorical sampling in ONE launch per step, token ids never leave the GPU.
 //
 // Replaces, per step of generate_step (PIE/engine/inference_engine.py:268-271):

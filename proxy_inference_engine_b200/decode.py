@@ -85,7 +85,7 @@ class DecodeEngine:
             self.logits_local = torch.empty((B, a.vocab_size // w), dtype=bf, device=dev)
             self.logits_gather = torch.empty((w * B, a.vocab_size // w), dtype=bf, device=dev)  # rank-major rows
             # exchange steps: one-shot pushes over NVLink peer memory (tp.TPExchange, csrc/pie_comm.cu) unless
-            # PIE_TP_ONESHOT=0 or symmetric memory cannot be set up (then NCCL collectives, as in round 1)
+            # PIE_TP_ONESHOT=0 or symmetric memory cannot be set up (then NCCL collectives)
             self.xch = None
             self.xch_f = None
             self.part = torch.empty((B, h), dtype=bf, device=dev)
@@ -160,7 +160,7 @@ class DecodeEngine:
             B, self.Hq, self.Hkv, max_context)
         # Two forms of decode attention.  Latency form: rope + KV append + SIMT flash-decode in ONE launch
         # (pie_decode_attn_fused).  Throughput form: pie_rope_kv_append + the tensor-core kernel of pie_fa.cu, which
-        # reads K/V once per kv head.  Measured per layer on B200 (tools/run_attn_compare.sh; 8B shapes, us):
+        # reads K/V once per kv head.  Measured per layer on B200 (8B shapes, us):
         #   bs1 ctx500 10.8 / 12.9, bs1 ctx2048 16.9 / 17.4, bs1 ctx8000 40.5 / 22.2, bs4 ctx2048 32.6 / 23.1,
         #   bs32 ctx2048 203 / 77  ->  the latency form while batch x context stays within 4096 keys.
         self.attn_fused = (batch * max_context <= 4096) if attn_fused is None else attn_fused
@@ -197,8 +197,8 @@ class DecodeEngine:
         self.graph = None
         self._next_pos = None
         self.launches_per_step = 0
-        # fused=True: one cooperative launch per step (pie_decode_step), B <= 8.  Round-1 status: parity-green but
-        # slower than the per-operator launches, hence opt-in
+        # fused=True: one cooperative launch per step (pie_decode_step), B <= 8: slower than the per-operator launches (3.68
+        # against 2.13 ms a step of the 8B model), hence opt-in
         self.fused = bool(fused)
         self.trace = trace
         if self.fused:

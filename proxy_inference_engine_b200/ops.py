@@ -1,5 +1,5 @@
 """Operator surface of the path, with the names, argument meaning and error behaviour of the MLX operators
-PIE's Llama model reaches (SURVEY.md 8b): ``quantize``, ``dequantize``, ``quantized_matmul``, ``rms_norm``,
+PIE's Llama model reaches: ``quantize``, ``dequantize``, ``quantized_matmul``, ``rms_norm``,
 ``rope``, ``scaled_dot_product_attention``.  Tensors are torch CUDA tensors; activations, scales, biases and
 norm weights are bf16; packed weights are MLX ``uint32`` words held as ``torch.int32`` (same bits).
 

@@ -1,4 +1,4 @@
-"""Paged KV cache management (SURVEY 8(f2)): the page allocator and prefix reuse.
+"""Paged KV cache management: the page allocator and prefix reuse.
 
     PageAllocator      -- CORE/include/engine/page_allocator.hpp:17-72 (same method names and failure behaviour) over the
                           lock-free C++ allocator of csrc/pie_pages.cu.

@@ -1,4 +1,4 @@
-"""Ragged continuous batching (SURVEY 8 f4): one model step over a mix of prefill chunks and decode rows.
+"""Ragged continuous batching: one model step over a mix of prefill chunks and decode rows.
 
 ``BatchDetails`` carries the fields of the reference's descriptor (CORE/include/engine/batch_details.hpp:10-90): the
 concatenated ``token_ids`` / ``positions`` of the step, per-sequence ``input_lengths`` / ``context_lengths``, the

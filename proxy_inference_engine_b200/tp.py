@@ -1,4 +1,4 @@
-"""Tensor parallelism of the quantized Llama path over one NVSwitch box (SURVEY.md 8e).
+"""Tensor parallelism of the quantized Llama path over one NVSwitch box.
 
 The partition is MLX's own (``QuantizedAllToShardedLinear`` / ``QuantizedShardedToAllLinear``,
 MLX/python/mlx/nn/layers/distributed.py:355-566): q/k/v_proj and gate/up_proj are split by output rows (whole
@@ -103,7 +103,7 @@ class TPExchange:
     """One-shot exchanges over NVLink peer memory for the decode step (csrc/pie_comm.cu): every rank pushes its partial
     row into a slot of every peer's SYMMETRIC buffer and reduces the `world` slots locally -- one small kernel per
     exchange instead of an NCCL collective (8-16 KB messages are pure latency: ~11 us per ncclAllReduce at 2 GPUs,
-    ~26 us at 8, measured in round 1).  NCCL / torch.distributed stay for the rendezvous and for the prefill path.
+    ~26 us at 8, measured).  NCCL / torch.distributed stay for the rendezvous and for the prefill path.
     The buffer comes from torch.distributed._symmetric_memory (CUDA IPC / fabric handles mapped into every peer)."""
 
     def __init__(self, tp: TPInfo, max_elems: int, gather_rows: int, gather_width: int, device):

@@ -1,4 +1,4 @@
-"""On-disk format of the path (SURVEY 8 f4 / a13): MLX-layout safetensors, single file or sharded with
+"""On-disk format of the path: MLX-layout safetensors, single file or sharded with
 model.safetensors.index.json, read back the way PIE's loader globs them (PIE/models/utils.py:62-66)."""
 import json
 import os

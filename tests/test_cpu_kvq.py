@@ -1,4 +1,4 @@
-"""Quantised KV cache (SURVEY 8 f3), CPU side: the oracle's restatement of QuantizedKVCache.update_and_fetch
+"""Quantised KV cache, CPU side: the oracle's restatement of QuantizedKVCache.update_and_fetch
 (PIE/cache/kv_cache/quantized.py:38-108) and quantized_scaled_dot_product_attention (PIE/models/base.py:56-89) against
 tests/golden/ref_kvq.npz -- outputs of the reference's own compiled quantize / _qmm_t / _qmm kernels
 (tools/make_golden_kvq.py)."""
@@ -45,7 +45,7 @@ def test_attention_matches_the_reference_kernels(ci):
     out_a = O.quantized_scaled_dot_product_attention(g("q"), keys, vals, D ** -0.5, None, 64, 8, mode="A")
     np.testing.assert_allclose(out_a, g("out_f32"), rtol=2e-5, atol=2e-5)  # float kernels (summation order differs)
     # (the two reference precisions themselves differ by up to ~0.8 here: the x86 scalar bf16 kernels round the running
-    # sum to bf16 after every term; SURVEY appendix A -- the GPU path follows the fp32-accumulate semantics)
+    # sum to bf16 after every term -- the GPU path follows the fp32-accumulate semantics)
 
 
 def test_attention_with_mask_and_grouped_heads():

@@ -69,7 +69,7 @@ def test_arange_case_of_ops_tests(bits):
 
 
 def test_reference_takes_scalar_path_on_x86():
-    # SURVEY.md section 7: simd::max_size<float> == 1 off Apple -> _qmm_t (not _qmm_t_simd) is what MLX-CPU runs here
+    # simd::max_size<float> == 1 off Apple -> _qmm_t (not _qmm_t_simd) is what MLX-CPU runs here
     assert int(GOLD["simd_max_size_f32"][0]) == 1
 
 

@@ -1,4 +1,4 @@
-"""Page allocator (SURVEY 8(f2)) -- the reference's own test cases (tests/cpp/test_page_allocator.cpp:60-330) on
+"""Page allocator -- the reference's own test cases (tests/cpp/test_page_allocator.cpp:60-330) on
 csrc/pie_pages.cu through the C ABI, plus prefix-length logic of PromptCache.reuse_cache (prompt_cache.py:52-76).
 Host code: runs without a GPU."""
 import threading

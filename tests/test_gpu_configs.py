@@ -1,9 +1,9 @@
-"""GPU parity on the BASELINE.json configurations themselves (not a toy model), against the CPU oracle (mode B = fp32
-inside every MLX op, bf16 at the op boundaries: what MLX computes for a bf16 checkpoint, SURVEY Appendix A).
+"""GPU parity on the benchmark's own configurations (not a toy model), against the CPU oracle (mode B = fp32
+inside every MLX op, bf16 at the op boundaries: what MLX computes for a bf16 checkpoint).
 
-north_star's definition of correct: per-layer bf16 activations within 2e-2 relative error and identical greedy tokens
+Correct means: per-layer bf16 activations within 2e-2 relative error and identical greedy tokens
 over 128 steps.  On random-init weights the logits over 128 256 classes are nearly flat, so a greedy token can flip on a
-near-tie from fp32 summation order alone (SURVEY section 7): tokens are compared teacher-forced, a mismatch only counts when
+near-tie from fp32 summation order alone: tokens are compared teacher-forced, a mismatch only counts when
 the oracle's own gap between the two candidates exceeds twice the largest logit difference seen on that step, and the
 exact-match run length (= how far a free-running decode stays identical) is reported.
 Reference loop: PIE/engine/inference_engine.py:228-297 -> PIE/models/llama/language.py:199-210."""
@@ -60,7 +60,7 @@ def greedy_parity(args, prompt_len, steps, seed=0, max_context=None, engine_kw=N
 
 
 def test_config1_llama_3_2_1b_q4_128_prompt_128_greedy_steps():
-    """BASELINE config 1: Llama-3.2-1B random-init, MLX q4 gs64, bs1, 128-token prompt + 128 greedy steps."""
+    """Llama-3.2-1B random-init, MLX q4 gs64, bs1, 128-token prompt + 128 greedy steps."""
     from proxy_inference_engine_b200.checkpoint import preset_args
     args = preset_args("llama-3.2-1b", bits=4)
     rep = greedy_parity(args, prompt_len=128, steps=128)

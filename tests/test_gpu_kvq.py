@@ -1,4 +1,4 @@
-"""Quantised KV cache on the GPU (SURVEY 8 f3): pie_kvq_write / pie_kvq_append / pie_decode_attn_q8 through the C ABI
+"""Quantised KV cache on the GPU: pie_kvq_write / pie_kvq_append / pie_decode_attn_q8 through the C ABI
 against tests/golden/ref_kvq.npz (outputs of the reference's own compiled quantize / _qmm_t / _qmm kernels,
 tools/make_golden_kvq.py) and against the oracle's restatement of PIE/cache/kv_cache/quantized.py +
 PIE/models/base.py:56-89.  Cache contents: bit-exact.  Attention output: 2e-2 of the float kernels (one bf16 rounding

@@ -8,7 +8,7 @@ from parity_util import make_oracle, rel_l2, run_decode_parity, tiny_args
 
 pytestmark = pytest.mark.gpu
 
-TOL = 2e-2  # north_star: per-layer bf16 activations within 2e-2 relative error
+TOL = 2e-2  # per-layer bf16 activations within 2e-2 relative error
 
 
 def test_model_forward_matches_oracle_per_layer():

@@ -1,4 +1,4 @@
-"""Prefix reuse over the paged KV cache (SURVEY 8(f2)): a prompt that shares a prefix with a cached one re-uses the
+"""Prefix reuse over the paged KV cache: a prompt that shares a prefix with a cached one re-uses the
 prefix's pages by reference count (PromptCache.reuse_cache, PIE/cache/prompt_cache.py:52-76; ReusableKVCache.reuse,
 reusable.py:44-94) and computes only what follows -- same logits as computing the whole prompt on fresh pages."""
 import numpy as np

@@ -1,4 +1,4 @@
-"""Ragged step (SURVEY 8 f4): a mix of prefill chunks and decode rows in ONE model step must give every sequence the
+"""Ragged step: a mix of prefill chunks and decode rows in ONE model step must give every sequence the
 logits it gets when it runs alone through Model.__call__ over its own paged cache (the parity-tested per-sequence path,
 PIE/models/llama/language.py:199-210), and the oracle's."""
 import numpy as np

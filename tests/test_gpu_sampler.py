@@ -1,4 +1,4 @@
-"""Device-side sampler (SURVEY 8(f1)) against the numpy restatement of PIE/samplers/*.py + inference_engine.py:268-271.
+"""Device-side sampler against the numpy restatement of PIE/samplers/*.py + inference_engine.py:268-271.
 The kernel and the restatement are given the SAME uniforms, so the sampled tokens must be identical (not just equal in
 distribution); the Philox path is checked for reproducibility, graph replay and its distribution."""
 import numpy as np

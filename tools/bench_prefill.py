@@ -1,4 +1,4 @@
-"""BASELINE config 4: Llama-3.1-8B q4, one 8192-token prefill (whole prompt in one forward, as
+"""Llama-3.1-8B q4, one 8192-token prefill (whole prompt in one forward, as
 PIE/engine/inference_engine.py:278): time to first token and achieved TFLOP/s (2*M*N*K of the quantized matmuls,
 lm_head on the last position only, + causal attention 4*L^2*h*layers/2)."""
 import argparse, json, os, sys, time

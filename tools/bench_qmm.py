@@ -1,4 +1,4 @@
-"""Prefill quantized GEMM micro-benchmark (BASELINE config 4 shapes: Llama-3.1-8B, M = 8192): achieved TFLOP/s of
+"""Prefill quantized GEMM micro-benchmark (Llama-3.1-8B shapes, M = 8192): achieved TFLOP/s of
 pie_qmm per matrix (CUDA events; 2*M*N*K useful flops, dequant ALU work not counted)."""
 import argparse, json, os, sys
 import torch

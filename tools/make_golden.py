@@ -1,5 +1,5 @@
 """Generate tests/golden/*.npz from the REFERENCE's own code (oracle/_ref/libpie_ref.so = MLX's
-mlx/backend/cpu/quantized.cpp compiled where it lies under /root/reference, see oracle/Makefile).
+mlx/backend/cpu/quantized.cpp compiled where it lies, see oracle/Makefile).
 
 Run in the build container (the reference tree is not on the GPU box):   python tools/make_golden.py
 The fixtures pin (a) quantize<T,U> bytes (cpu/quantized.cpp:603-661) and (b) _qmm_t<float,bits,gs> outputs
