@@ -417,14 +417,14 @@ def config3_subrecord(model_name, steps=24, warmup=4, batch=32, prompt=2048, kv_
 
 def ncu_traffic_per_launch(alg_bytes_per_launch, bits):
     """dram__bytes_read.sum + dram__bytes_write.sum of the GEMV per launch, from the committed `ncu --set full` capture
-    (profiles/r01e_prof_qmv_ncu_full_summary.csv: the q4 gate+up, down, qkv and o launches of one 8B layer).  The capture
+    (profiles/llama_1e_prof_qmv_ncu_full_summary.csv: the q4 gate+up, down, qkv and o launches of one 8B layer).  The capture
     holds four of the five shapes, so the measured traffic / algorithmic ratio of those launches scales this run's
     average launch.  None if the capture is absent or was taken at another bit width."""
     import csv
     pdir = os.path.join(os.path.dirname(os.path.abspath(__file__)), "profiles")
-    path = os.path.join(pdir, "r02c_prof_qmv_ncu_full_summary.csv")    # both GEMV kernels
+    path = os.path.join(pdir, "llama_2c_prof_qmv_ncu_full_summary.csv")   # both GEMV kernels
     if not os.path.exists(path):
-        path = os.path.join(pdir, "r01e_prof_qmv_ncu_full_summary.csv")
+        path = os.path.join(pdir, "llama_1e_prof_qmv_ncu_full_summary.csv")
     if bits != 4 or not os.path.exists(path):
         return None, "no ncu capture for this configuration"
     rows = {r[0]: r for r in csv.reader(open(path)) if r}
