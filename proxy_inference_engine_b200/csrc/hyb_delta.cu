@@ -132,12 +132,15 @@ __global__ void __launch_bounds__(256) delta_prepare_warp_kernel(float* q, float
     }
   }
 }
-// rows, channels and units that warps of four-channel lanes can take; a head's keys in one warp's pass (the norm is over them)
+// rows, channels and units that warps of four-channel lanes can take; a head's keys in one warp's pass (the norm is over them).  Few
+// (row, unit) pairs are one or two waves of the other kernel's CTAs, and a warp's four rows in a row are a longer chain than that (16
+// heads of 128, us, by CTAs / by warps: 4 rows 6.2 / 12.7, 57 rows 8.5 / 11.3, 300 rows 23.3 / 15.0; 8 heads of 16: 57 rows 6.0 / 10.3, 300
+// rows 11.8 / 10.7).  Four taps are what the configurations have; another length takes the other kernel.
 static bool delta_prepare_by_warps(const float* q, const float* k, const float* v, const float* proj, long long ld,
-                                   const pieh_delta& d) {
+                                   const pieh_delta& d, int T) {
   const uintptr_t p = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
                       reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(d.conv_state);
-  return d.taps == 4 && d.dk <= 128 && d.dk % 4 == 0 && d.dv % 4 == 0 && ld % 4 == 0 && (p & 15) == 0;
+  return (long long)T * (2 * d.G + d.H) >= 6144 && d.taps == 4 && d.dk <= 128 && d.dk % 4 == 0 && d.dv % 4 == 0 && ld % 4 == 0 && (p & 15) == 0;
 }
 
 __global__ void conv_advance_kernel(const float* proj, long long ld, const pieh_delta d, const pieh_batch b) {
@@ -349,7 +352,7 @@ extern "C" int pieh_delta_prepare(float* q, float* k, float* v, float* beta, flo
   if (b->T == 0) return PIE_OK;
   cudaStream_t st = (cudaStream_t)stream;
   count_launch(2);
-  if (delta_prepare_by_warps(q, k, v, proj, ld, *d))
+  if (delta_prepare_by_warps(q, k, v, proj, ld, *d, b->T))
     launch_k(delta_prepare_warp_kernel<4>, dim3((b->T + 3) / 4, (2 * d->G + d->H + 7) / 8), dim3(256), 0, st, q, k, v, beta, decay, proj,
              ld, *d, *b);
   else

@@ -296,3 +296,40 @@ def test_layer_norms_of_few_and_many_rows(rows, W):
     sd = new.std(-1, unbiased=False, keepdim=True) if W > 1 else 1.0
     size = new.abs().amax(-1, keepdim=True) * (1 + 1 / y.double().std(-1, unbiased=False, keepdim=True))
     _within(h, want, 2 ** -24 * 80 * (size / sd) * (1 + (want - nb.double()).abs() + nw.double().abs()) + 2 ** -23 * want.abs())
+
+
+@pytest.mark.parametrize("H,G,dk,dv", [(16, 16, 128, 128), (8, 8, 16, 36), (8, 4, 32, 64)])
+def test_delta_rule_of_one_portion_and_of_small_ones(H, G, dk, dv):
+    """A portion prepared by warps and one scanned with registers to spare, against the same rows in small portions (prepared by CTAs)
+    and single tokens (scanned with four CTAs on an SM).  The norms' sums are of other order: a few 2^-24 of a unit vector's size, and
+    the recurrence, whose keys have length one, carries that on without enlarging it."""
+    from proxy_inference_engine_b200 import _lib
+    from proxy_inference_engine_b200.ragged import BatchDetails
+    L = _lib.load_hybrid(build_if_missing=True)
+    g = torch.Generator(device="cuda").manual_seed(dk)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    T, taps, nq = 400, 4, G * dk
+    C_ = 2 * nq + H * dv
+    ld = (C_ + H * dv + 2 * H + 3) // 4 * 4
+    assert T * (2 * G + H) >= 6144 > 120 * (2 * G + H)      # either side of the rule between the two preparations
+    conv_w, A, dt, norm, proj = rnd(C_, taps) * 0.3, rnd(H), rnd(H), torch.ones(dv, device="cuda"), rnd(T, ld)
+    results = []
+    for parts in ([T], [100, 120, 20, 110, 1, 1, 48]):
+        conv, state = torch.zeros(1, taps - 1, C_, device="cuda"), torch.zeros(1, H, dk, dv, device="cuda")
+        d = _lib.HybDelta(H, G, dk, dv, taps, conv_w.data_ptr(), A.data_ptr(), dt.data_ptr(), norm.data_ptr(), 1e-6, conv.data_ptr(),
+                          state.data_ptr())
+        outs, at = [], 0
+        for n in parts:
+            b = BatchDetails.build([("s", [1] * n, at, list(range(8)), 0)])
+            desc, keep = b.hybrid_descriptor()
+            q, k, v = (torch.full((n, w), float("nan"), device="cuda") for w in (nq, nq, H * dv))
+            beta, decay, o = (torch.full((n, w), float("nan"), device="cuda") for w in (H, H, H * dv))
+            rows = proj[at:at + n]
+            assert L.pieh_delta_prepare(_p(q), _p(k), _p(v), _p(beta), _p(decay), _p(rows), ld, C.byref(d), C.byref(desc), None) == 0
+            assert L.pieh_delta_scan(_p(o), _p(q), _p(k), _p(v), _p(beta), _p(decay), C.byref(d), C.byref(desc), None) == 0
+            outs.append((q, k, v, beta, decay, o))
+            at += n
+        results.append([torch.cat(t) for t in zip(*outs)] + [conv, state])
+        torch.cuda.synchronize()
+    for name, a, b in zip(("q", "k", "v", "beta", "decay", "o", "conv", "state"), *results):
+        assert torch.isfinite(a).all() and (a.double() - b.double()).norm() <= 1e-6 * b.double().norm(), name
