@@ -170,8 +170,8 @@ __device__ __forceinline__ void cp_async_f(float* smem_dst, const float* gsrc, i
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(gsrc) : "memory");
 }
 
-template <int RPT, int R>   // rows of a state column in a lane, lanes of a column
-__global__ void __launch_bounds__(kScanThreads, 1) delta_scan_kernel(float* o, const float* q, const float* k, const float* v,
+template <int RPT, int R, int CTAS>   // rows of a state column in a lane, lanes of a column, CTAs of an SM
+__global__ void __launch_bounds__(kScanThreads, CTAS) delta_scan_kernel(float* o, const float* q, const float* k, const float* v,
                                                                      const float* beta, const float* decay,
                                                                      const pieh_delta d, const pieh_batch b) {
   extern __shared__ __align__(16) float sm[];
@@ -328,11 +328,14 @@ static cudaError_t launch_scan(float* o, const float* q, const float* k, const f
                                const pieh_delta& d, const pieh_batch& b, cudaStream_t st) {
   constexpr int cols = kScanThreads / R;
   constexpr size_t smem = (size_t)2 * kScanChunk * (2 * RPT * R + cols + 2) * 4;
+  // One token a sequence (decode) is reading and writing the state: registers are worth most as CTAs in flight.  16 heads of 128 x 128,
+  // 4 / 32 sequences, us: 162 registers 6.2 / 28.3, 124 registers 4.8 / 23.6.
+  auto* kern = b.T == b.n_seq ? delta_scan_kernel<RPT, R, 4> : delta_scan_kernel<RPT, R, 1>;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<RPT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  return launch_k(delta_scan_kernel<RPT, R>, dim3((d.dv + cols - 1) / cols, d.H, b.n_seq), dim3(kScanThreads), smem, st, o, q, k, v,
+  return launch_k(kern, dim3((d.dv + cols - 1) / cols, d.H, b.n_seq), dim3(kScanThreads), smem, st, o, q, k, v,
                   beta, decay, d, b);
 }
 
