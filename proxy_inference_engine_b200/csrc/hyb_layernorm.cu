@@ -45,8 +45,8 @@ template <int NV, bool AHEAD>
 struct LnWeights {
   const float *w, *b;
   float4 wv[AHEAD ? NV : 1], bv[AHEAD ? NV : 1];
-  __device__ __forceinline__ LnWeights(const float* w_, const float* b_, int W) : w(w_), b(b_) {
-    if (AHEAD && w) {
+  __device__ __forceinline__ LnWeights(const float* w_, const float* b_, int W, bool use) : w(w_), b(b_) {
+    if (AHEAD && use) {
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
         const int c = (threadIdx.x + i * blockDim.x) * 4;
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(256) layernorm_add_kernel(const LnAdd a) {
       }
     }
   }
-  const LnWeights<NV, AHEAD> post(replace || !yr ? nullptr : a.post_w, a.post_b, W), next(a.h ? a.next_w : nullptr, a.next_b, W);
+  const LnWeights<NV, AHEAD> post(a.post_w, a.post_b, W, yr && !replace), next(a.next_w, a.next_b, W, a.h && a.next_w);
   if (yr && !replace) ln_rows<NV>(u, post, a.eps, W, red[0]);
   const bool changed = yr || a.add_rows || a.add_vec;
 #pragma unroll
