@@ -2,12 +2,14 @@
 //
 // Kernels behind pieh_linear:
 //   * linear_rows_mma_kernel (bf16 x bf16, M <= 32: decode): a CTA streams 16 output rows of the matrix once, straight into
-//     mma.sync operands -- bound by the weight bytes;
+//     mma.sync operands -- bound by the weight bytes (one or two rows times a small matrix stay with the next kernel);
 //   * linear_rows_kernel  (M <= 32, everything else; grouped products of few slots): a CTA streams 1, 2 or 4 weight rows once with
 //     16-byte loads, its warps cutting K between them, one fp32 accumulator per (activation row, weight row);
 //   * the tcgen05 kernels of hyb_umma.cu (bf16 x bf16, M > 32, K % 64 == 0: prefill);
 //   * linear_tile_kernel  (everything else, and every fp32 product): 64 x 64 tiles, fp32 multiply-add on the CUDA cores.
 // With bf16 weights the activation is rounded to bf16 first, so they agree up to the order of the fp32 sums.
+#include <type_traits>
+
 #include "hyb_mma.cuh"
 
 namespace pieh {
@@ -205,48 +207,80 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const LinArgs a) {
 // mma.sync m16n8k16 A operand and go from global memory into it directly: which k of a 16-wide step an operand register holds
 // does not matter as long as both operands agree, so a lane loads 8 CONSECUTIVE k of rows g and g + 8 (16 bytes each) and of its
 // activation row, and feeds two MMAs from them.  The tensor core does the sum over k that linear_rows_kernel does with shuffles
-// (16 values x 5 shuffles for every 16 KB of weights at four rows), so a warp keeps eight 16-byte weight loads in flight and
-// little else.  The warps' partial tiles meet in shared memory in warp order.  Four rows, us (GB/s): 28672 x 4096 61.6 (3810) -> 40.9
-// (5750); 4096 x 14336 24.6 (4780); 16 rows: 57.6 and 33.3; 32 rows: 92 and 55 (x comes from L2 once per 16 outputs).
+// (16 values x 5 shuffles for every 16 KB of weights at four rows), so a warp has the loads of U steps in flight and little else to do.
+// The tensor core cuts every sum it returns to 24 bits, towards zero (measured), so that a chain of MMAs is off by a multiple of what
+// fp32 additions are (K 14336, rms against float64: 1.8e-6, and 4.5e-6 if all products are positive; linear_rows_kernel 9.6e-8 and
+// 5.2e-8).  Each MMA therefore starts from zero, the four of a step are added as a tree in fp32, four steps make a run, runs are
+// added, and the eight warps' sums meet in double precision in shared memory: 8.3e-8 and 3.9e-8, and at every K from 256 less than
+// linear_rows_kernel is off by.  SHORT (K < 256, where that kernel adds only a few numbers itself): every sum of MMAs in double precision.
+// Weights from memory, us (GB/s), linear_rows_kernel -> this one.  4 rows: 28672 x 4096 61.9 -> 38.2 (6150), 4096 x 14336 33.0 -> 20.5;
+// 16 rows: 225 -> 53.7 and 147 -> 23.9; 32 rows: 817 -> 81 and 375 -> 37 (x comes from L2 once per 16 outputs).
 __device__ __forceinline__ uint4 load_stream16(const __nv_bfloat16* p) {   // read once: past L1
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
-template <typename OT, int NT>
-__global__ void __launch_bounds__(256) linear_rows_mma_kernel(const LinArgs a) {
-  __shared__ float part[8][16][8 * NT + 1];
+template <typename OT, int NT, int CTAS, int U, bool SHORT>   // U: steps whose loads are in flight together
+__global__ void __launch_bounds__(256, CTAS) linear_rows_mma_kernel(const LinArgs a) {
+  using Sum = std::conditional_t<SHORT, double, float>;
+  constexpr bool RUNS = !SHORT && !(NT == 4 && CTAS == 3);   // (there the registers are not; a warp's K / 512 steps in a row, rms 9.1e-8 at most)
+  __shared__ Sum part[8][16][8 * NT + 1];
   pdl_sync();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, n0 = blockIdx.x * 16;
   const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(a.x) + (size_t)blockIdx.z * a.x_bs;
   const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(a.w) + (size_t)blockIdx.z * a.w_bs;
   const __nv_bfloat16* w0 = w + (size_t)min(n0 + g, a.N - 1) * a.K;
   const __nv_bfloat16* w1 = w + (size_t)min(n0 + g + 8, a.N - 1) * a.K;
-  float acc[NT][4];
+  Sum acc[NT][4];
+  float run[NT][4];
 #pragma unroll
-  for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-#pragma unroll(NT == 1 ? 4 : 2)
-  for (int kb = warp * 64; kb < a.K; kb += 512) {
-    uint4 wa[2], wb[2], xv[2][NT];
+  for (int i = 0; i < NT; ++i)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int k = kb + 32 * h + 8 * t;
-      const bool in = k < a.K;   // K is a multiple of 8: the piece exists or it does not
-      const uint4 zero = make_uint4(0, 0, 0, 0);
-      wa[h] = in ? load_stream16(w0 + k) : zero;
-      wb[h] = in ? load_stream16(w1 + k) : zero;
+    for (int e = 0; e < 4; ++e) acc[i][e] = run[i][e] = 0.f;
+  int in_run = 0;
+  auto flush = [&] {
 #pragma unroll
-      for (int i = 0; i < NT; ++i)
-        xv[h][i] = in && 8 * i + g < a.M ? *reinterpret_cast<const uint4*>(x + (size_t)(8 * i + g) * a.x_ld + k) : zero;
-    }
+    for (int i = 0; i < NT; ++i)
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+      for (int e = 0; e < 4; ++e) { acc[i][e] += run[i][e]; run[i][e] = 0.f; }
+  };
+#pragma unroll 1
+  for (int kb = warp * 64; kb < a.K; kb += 512 * U) {
+    uint4 wa[U][2], wb[U][2], xv[U][2][NT];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int k = kb + 512 * u + 32 * h + 8 * t;
+        const bool in = k < a.K;   // K is a multiple of 8: the piece exists or it does not
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        wa[u][h] = in ? load_stream16(w0 + k) : zero;
+        wb[u][h] = in ? load_stream16(w1 + k) : zero;
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+          xv[u][h][i] = in && 8 * i + g < a.M ? *reinterpret_cast<const uint4*>(x + (size_t)(8 * i + g) * a.x_ld + k) : zero;
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (u > 0 && kb + 512 * u >= a.K) break;   // the whole warp
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
-        mma_16816(acc[i], wa[h].x, wb[h].x, wa[h].y, wb[h].y, xv[h][i].x, xv[h][i].y);
-        mma_16816(acc[i], wa[h].z, wb[h].z, wa[h].w, wb[h].w, xv[h][i].z, xv[h][i].w);
+        float p[4][4] = {};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          mma_16816(p[2 * h], wa[u][h].x, wb[u][h].x, wa[u][h].y, wb[u][h].y, xv[u][h][i].x, xv[u][h][i].y);
+          mma_16816(p[2 * h + 1], wa[u][h].z, wb[u][h].z, wa[u][h].w, wb[u][h].w, xv[u][h][i].z, xv[u][h][i].w);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if constexpr (RUNS) run[i][e] += (p[0][e] + p[1][e]) + (p[2][e] + p[3][e]);
+          else acc[i][e] += ((Sum)p[0][e] + p[1][e]) + ((Sum)p[2][e] + p[3][e]);
+        }
       }
+    }
+    if (RUNS && ++in_run == 4 / U) { flush(); in_run = 0; }
   }
+  if (RUNS) flush();
 #pragma unroll
   for (int i = 0; i < NT; ++i) {
     part[warp][g][8 * i + 2 * t] = acc[i][0];
@@ -255,11 +289,11 @@ __global__ void __launch_bounds__(256) linear_rows_mma_kernel(const LinArgs a) {
     part[warp][g + 8][8 * i + 2 * t + 1] = acc[i][3];
   }
   __syncthreads();
+  const int warps = min(8, (a.K + 63) / 64);   // that had a step
   auto sum = [&](int r, int m) {
-    float y = 0.f;
-#pragma unroll
-    for (int wp = 0; wp < 8; ++wp) y += part[wp][r][m];
-    return y;
+    double y = 0.0;
+    for (int wp = 0; wp < warps; ++wp) y += (double)part[wp][r][m];
+    return (float)y;
   };
   if (a.epi == PIEH_EPI_GLU) {   // rows (2 r, 2 r + 1) are a (gate, linear) pair
     for (int e = threadIdx.x; e < 8 * a.M; e += 256) {
@@ -317,11 +351,20 @@ __global__ void __launch_bounds__(256) linear_skinny_kernel(const LinArgs a) {
 
 template <typename OT>
 static cudaError_t launch_rows_mma(const LinArgs& a, cudaStream_t st) {
+  const long long tiles = (long long)((a.N + 15) / 16) * a.nb;
   const dim3 grid((unsigned)((a.N + 15) / 16), 1, (unsigned)a.nb);
   count_launch();
-  if (a.M <= 8) return launch_k(linear_rows_mma_kernel<OT, 1>, grid, dim3(256), 0, st, a);
-  if (a.M <= 16) return launch_k(linear_rows_mma_kernel<OT, 2>, grid, dim3(256), 0, st, a);
-  return launch_k(linear_rows_mma_kernel<OT, 4>, grid, dim3(256), 0, st, a);
+#define PIEH_MMA(NT, CTAS, U, SHORT) launch_k(linear_rows_mma_kernel<OT, NT, CTAS, U, SHORT>, grid, dim3(256), 0, st, a)
+  if (a.K < 256) return a.M <= 8 ? PIEH_MMA(1, 4, 1, true) : a.M <= 16 ? PIEH_MMA(2, 2, 1, true) : PIEH_MMA(4, 2, 1, true);
+  // Up to two steps a warp there is nothing to load ahead of, and more CTAs hide more (16384 x 512, 4 rows: 8.0 us with two CTAs of four
+  // steps ahead, 5.9 with four of one; 16 rows 8.9 and 8.0; at 32 rows two are sooner).  Otherwise two CTAs to an SM with as many loads as
+  // their registers hold; three, with fewer, where that saves the second wave (6368 x 4096, 16 rows: 17.7 -> 13.1 us; 4096 x 14336 is
+  // 23.9 for 34.4 the other way).
+  const bool few_steps = a.K <= 1024, three = tiles > 2LL * num_sms() && tiles <= 3LL * num_sms();
+  if (a.M <= 8) return few_steps ? PIEH_MMA(1, 4, 1, false) : PIEH_MMA(1, 2, 4, false);
+  if (a.M <= 16) return few_steps || three ? PIEH_MMA(2, 3, 1, false) : PIEH_MMA(2, 2, 2, false);
+  return three ? PIEH_MMA(4, 3, 1, false) : PIEH_MMA(4, 2, 1, false);
+#undef PIEH_MMA
 }
 
 template <typename XT, typename WT, typename OT>
@@ -348,18 +391,16 @@ static cudaError_t launch_typed(const LinArgs& a, cudaStream_t st) {
       const dim3 grid((a.N + 63) / 64, a.M / 64 + (int)a.S);   // S carries the expert count here: the tile list's bound
       e = launch_k(linear_tile_kernel<XT, WT, OT>, grid, dim3(256), 0, st, t);
     }
-  } else if (sizeof(XT) == 4 && a.M <= 32 && vec_ok) {
-    if constexpr (sizeof(XT) == 4) {   // bf16 activations go to launch_rows_mma
-      // rows per CTA: enough to amortise the activation loads, few enough that every SM still gets several CTAs
-      const bool wide = (long long)a.N * a.nb >= 4 * 4 * num_sms() || a.epi == PIEH_EPI_GLU;   // a gated pair needs an even row count
+  } else if (a.M <= 32 && vec_ok) {
+    // rows per CTA: enough to amortise the activation loads, few enough that every SM still gets several CTAs
+    const bool wide = (long long)a.N * a.nb >= 4 * 4 * num_sms() || a.epi == PIEH_EPI_GLU;   // a gated pair needs an even row count
 #define PIEH_ROWS(MR, R) e = launch_k(linear_rows_kernel<XT, WT, OT, MR, R>, dim3((a.N + R - 1) / R, 1, nb), dim3(256), 0, st, a)
-      if (a.M <= 1) { if (wide) PIEH_ROWS(1, 2); else PIEH_ROWS(1, 1); }
-      else if (a.M <= 4) { if (wide) PIEH_ROWS(4, 4); else PIEH_ROWS(4, 2); }
-      else if (a.M <= 8) { if (wide) PIEH_ROWS(8, 4); else PIEH_ROWS(8, 2); }
-      else if (a.M <= 16) PIEH_ROWS(16, 2);
-      else PIEH_ROWS(32, 2);
+    if (a.M <= 1) { if (wide) PIEH_ROWS(1, 2); else PIEH_ROWS(1, 1); }
+    else if (a.M <= 4) { if (wide) PIEH_ROWS(4, 4); else PIEH_ROWS(4, 2); }
+    else if (a.M <= 8) { if (wide) PIEH_ROWS(8, 4); else PIEH_ROWS(8, 2); }
+    else if (a.M <= 16) PIEH_ROWS(16, 2);
+    else PIEH_ROWS(32, 2);
 #undef PIEH_ROWS
-    }
   } else {
     const dim3 grid((a.N + 63) / 64, (a.M + 63) / 64, nb);
     e = launch_k(linear_tile_kernel<XT, WT, OT>, grid, dim3(256), 0, st, a);
@@ -400,6 +441,13 @@ extern "C" int pieh_linear_act(void* out, int out_dtype, long long out_ld, const
 }
 
 namespace pieh {
+// A row or two times a matrix of so few outputs that 16 to a CTA leave half the SMs without one, up to four rows where it is three quarters:
+// linear_rows_kernel, with an output or two to a CTA (256 x 4096 from memory, us: 1 row 2.7 / 4.7, 2 rows 4.2 / 4.8, 4 rows 5.0 / 5.2, 8
+// rows 6.9 / 5.1; 1024 x 4096, 4 rows: 5.8 / 5.4; 2048 x 2048, 1 row: 4.4 / 3.9).
+static bool rows_one_by_one(const LinArgs& a) {
+  return a.M <= 4 && (a.M <= 2 ? 2LL : 4LL) * ((a.N + 15) / 16) * a.nb <= num_sms() && a.K % 8 == 0 && a.x_ld % 8 == 0 && a.x_bs % 8 == 0 && a.w_bs % 8 == 0 &&
+         ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) & 31) == 0;
+}
 int run_linear(const LinArgs& a, int out_dtype, int x_dtype, int w_dtype, cudaStream_t st) {
   if (w_dtype == PIE_DTYPE_F32 && x_dtype != PIE_DTYPE_F32) return PIE_EINVAL_DTYPE;   // exact mode is fp32 end to end
   // grouped products go to the tensor cores once an expert's run averages a few rows of a 128-slot tile
@@ -412,7 +460,7 @@ int run_linear(const LinArgs& a, int out_dtype, int x_dtype, int w_dtype, cudaSt
   }
   typedef __nv_bfloat16 bf;
   cudaError_t e;
-  if (!a.g_tiles && a.M <= 32 && x_dtype == PIE_DTYPE_BF16 && w_dtype == PIE_DTYPE_BF16 && a.K % 8 == 0 && a.x_ld % 8 == 0 &&
+  if (!a.g_tiles && a.M <= 32 && !rows_one_by_one(a) && x_dtype == PIE_DTYPE_BF16 && w_dtype == PIE_DTYPE_BF16 && a.K % 8 == 0 && a.x_ld % 8 == 0 &&
       a.x_bs % 8 == 0 && a.w_bs % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) & 15) == 0) {
     e = out_dtype == PIE_DTYPE_F32 ? launch_rows_mma<float>(a, st) : launch_rows_mma<bf>(a, st);
   } else if (w_dtype == PIE_DTYPE_F32) {
