@@ -83,12 +83,36 @@ __global__ void __launch_bounds__(128) prefill_attn_kernel(uint16_t* out, const 
   }
 }
 
+// Few keys: the tcgen05 kernel sets up tensor memory, barriers and 256 query rows for what the mma.sync kernel, with 64 rows to a CTA and
+// several CTAs to an SM, has done by then.  Both are estimated (us) as the longer of one CTA's walk and the SMs' share of all walks; the
+// constants are fitted to 552 measured shapes (1 to 32 sequences, 8 to 32 heads, 1 to 1000 rows behind 0 to 8000 keys) to 4 to 9 %
+// rms, and the choice takes 1.003 (D 64) and 1.001 (D 128) times the sooner kernel's time on average, at most 1.15.  mma.sync /
+// tcgen05: one sequence of 64 rows, 32 heads 3.6 / 5.6 (D 64), 5.4 / 6.4 (D 128); 32 sequences of 8 rows behind 128 keys 17 / 39, 36 / 46.
+// Beyond 1024 keys the tcgen05 kernel was sooner everywhere.
+static bool prefill_mma_sync_sooner(int B, int Hq, int L, int D, int offset) {
+  if ((long long)offset + L > 1024 || B > 65535 || Hq > 65535) return false;   // (its grid has them in y and z)
+  struct Cost { double walk, tile, share_tile, share_cta, set_up, cta, keys128, second; };
+  static constexpr Cost d64 = {2.5, 0.985, 0.69, 0.73, 1.28, 3.06, 1.29, 0.35}, d128 = {3.38, 1.91, 1.41, 1.38, 1.25, 3.72, 1.65, 0.27};
+  const Cost& c = D == 64 ? d64 : d128;
+  const double per_sm = (double)B * Hq / num_sms();
+  int tiles = 0, rows64 = 0, rows256 = 0;
+  for (int q = 0; q < L; q += 64, ++rows64) tiles += (offset + (q + 64 < L ? q + 64 : L) + 63) / 64;
+  double all = 0, longest = 0;
+  for (int q = 0; q < L; q += 256, ++rows256) {
+    const double cta = c.cta + (offset + (q + 256 < L ? q + 256 : L) + 127) / 128 * (c.keys128 + (q + 128 < L ? c.second : 0));
+    all += cta;
+    longest = cta > longest ? cta : longest;
+  }
+  const double one = c.walk + c.tile * ((offset + L + 63) / 64), share = c.walk / 2 + (c.share_tile * tiles + c.share_cta * rows64) * per_sm;
+  const double ctas = rows256 * per_sm, waves = (ctas < 6 ? ceil(ctas) : ctas) * all / rows256;
+  return (one > share ? one : share) < c.set_up + (longest > waves ? longest : waves);
+}
 cudaError_t launch_prefill_attn(uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc,
                                 const KvLayout& kv, int B, int Hq, int Hkv, int L, int D, int offset,
                                 float scale, cudaStream_t st) {
   if (B == 0 || L == 0) return cudaSuccess;
   static const bool naive = [] { const char* e = getenv("PIE_PREFILL_ATTN_NAIVE"); return e && e[0] == '1'; }();
-  if (!naive && fa_prefill_umma_ok(out, q, kc, vc, kv, B, Hq, Hkv, L, D, offset, scale))
+  if (!naive && !prefill_mma_sync_sooner(B, Hq, L, D, offset) && fa_prefill_umma_ok(out, q, kc, vc, kv, B, Hq, Hkv, L, D, offset, scale))
     return launch_fa_prefill_umma(out, q, kc, vc, kv, B, Hq, Hkv, L, D, offset, scale, st);
   if (!naive) return launch_prefill_attn_tc(out, q, kc, vc, kv, B, Hq, Hkv, L, D, offset, scale, st);
   const float sl = scale * 1.4426950408889634f;

@@ -1,5 +1,6 @@
 // Prefill attention (L > 1, causal) on tensor cores, sm_100a, for what the tcgen05 kernel of pie_fa_prefill.cu does not take: caches
-// that a tiled copy cannot describe (unaligned arrays, pages that are no multiple of 64 keys) and scales that are not positive.
+// that a tiled copy cannot describe (unaligned arrays, pages that are no multiple of 64 keys), scales that are not positive, and calls
+// over few keys, which are done here before that kernel has set itself up (prefill_mma_sync_sooner, pie_attn_launch.inl).
 //
 // Replaces mx.fast.scaled_dot_product_attention with the additive causal mask of create_attention_mask
 // (PIE/models/base.py:18-53, 92-113; Metal steel_attention, MLX/mlx/backend/metal/scaled_dot_product_attention.cpp:

@@ -166,6 +166,42 @@ def test_prefill_attention_tiles(paged, D, B, Hq, Hkv, L, offset):
     assert _lib.load().pie_pipeline_error() == 0
 
 
+@pytest.mark.parametrize("page", [0, 64, 128, 192, 48])    # 0: contiguous; 48: no whole 64-key boxes, the mma.sync kernel's
+@pytest.mark.parametrize("D,B,Hq,L,offset", [(64, 1, 2, 65, 63), (64, 1, 2, 128, 190),      # either side of the rule between them: one
+                                             (64, 1, 2, 128, 255), (64, 1, 2, 100, 1000),    # query tile,
+                                             (64, 1, 2, 129, 511), (64, 1, 2, 129, 639),     # two,
+                                             (64, 2, 64, 129, 0), (64, 2, 32, 300, 77),      # more than one wave,
+                                             (64, 40, 32, 8, 128), (64, 40, 32, 128, 256),
+                                             (128, 1, 2, 64, 0), (128, 1, 2, 60, 5), (128, 2, 4, 200, 121)])
+def test_prefill_attention_routes_and_pages(page, D, B, Hq, L, offset):
+    """Both kernels at the edges of the rule between them, over pages of one, two and three 64-key boxes and of none; what slots without
+    a token hold must not matter."""
+    from proxy_inference_engine_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(L + offset + D)
+    T, scale, Hkv = offset + L, D ** -0.5, 2
+    rnd = lambda *s: (1.5 * torch.randn(s, generator=g, device="cuda")).to(torch.bfloat16)
+    q, k, v = rnd(B, Hq, L, D), rnd(B, Hkv, T, D), rnd(B, Hkv, T, D)
+    if page:
+        n = (T + page - 1) // page
+        kb, vb = (torch.full((B * n + 2, page, Hkv, D), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        table = torch.full((B, n + 1), -1, device="cuda", dtype=torch.int32)
+        table[:, :n] = torch.randperm(B * n + 2, generator=g, device="cuda")[:B * n].view(B, n)
+        t = torch.arange(T, device="cuda")
+        for b in range(B):
+            kb[table[b, t // page].long(), t % page], vb[table[b, t // page].long(), t % page] = k[b].transpose(0, 1), v[b].transpose(0, 1)
+        got = ops.prefill_attention(q, kb, vb, ops.kv_layout(kb, table, page), offset, scale)
+    else:
+        got = ops.prefill_attention(q, k, v, ops.kv_layout(k), offset, scale)
+    s = torch.einsum("bhld,bhtd->bhlt", q.double(), k.double().repeat_interleave(Hq // Hkv, 1)) * scale
+    i, j = torch.arange(L, device="cuda")[:, None] + offset, torch.arange(T, device="cuda")[None]
+    p = torch.softmax(s.masked_fill(j > i, float("-inf")), -1)
+    vr = v.double().repeat_interleave(Hq // Hkv, 1)
+    want, mass = p @ vr, p @ vr.abs()
+    # the bound of test_prefill_attention_tiles
+    _within(got, want, mass * (2 ** -8 + 2 * D * 2 ** -23 * float(s.abs().max())) + want.abs() * 2 ** -8)
+    assert _lib.load().pie_pipeline_error() == 0
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("scale", [0.1, 4.0, 0.0, -0.1])   # exponents down to 0 and past the smallest; not positive: the other kernel
 def test_prefill_attention_exponentials(D, scale):
