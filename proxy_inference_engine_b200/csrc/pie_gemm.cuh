@@ -38,7 +38,16 @@ static inline unsigned int gemm_error_now() {
   return v;
 }
 static inline cudaError_t gemm_error_post(unsigned int* host, cudaStream_t st) {
-  return cudaMemcpyFromSymbolAsync(host, g_gemm_error, sizeof(*host), 0, cudaMemcpyDeviceToHost, st);
+  static std::atomic<void*> at[64];   // per device: every step asks
+  int dev = 0;
+  cudaGetDevice(&dev);
+  void* p = at[dev & 63].load(std::memory_order_acquire);
+  if (!p || dev > 63) {
+    const cudaError_t e = cudaGetSymbolAddress(&p, g_gemm_error);
+    if (e != cudaSuccess) return e;
+    at[dev & 63].store(p, std::memory_order_release);
+  }
+  return cudaMemcpyAsync(host, p, sizeof(*host), cudaMemcpyDeviceToHost, st);
 }
 static inline cudaError_t gemm_error_clear() {
   const unsigned int v = 0;

