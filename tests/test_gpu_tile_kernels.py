@@ -172,6 +172,7 @@ def test_prefill_attention_tiles(paged, D, B, Hq, Hkv, L, offset):
                                              (64, 1, 2, 129, 511), (64, 1, 2, 129, 639),     # two,
                                              (64, 2, 64, 129, 0), (64, 2, 32, 300, 77),      # more than one wave,
                                              (64, 40, 32, 8, 128), (64, 40, 32, 128, 256),
+                                             (64, 1, 2, 1, 1030), (64, 1, 2, 129, 900), (64, 1, 4, 256, 896),   # past the rule: tile edges at D 64
                                              (128, 1, 2, 64, 0), (128, 1, 2, 60, 5), (128, 2, 4, 200, 121)])
 def test_prefill_attention_routes_and_pages(page, D, B, Hq, L, offset):
     """Both kernels at the edges of the rule between them, over pages of one, two and three 64-key boxes and of none; what slots without
