@@ -223,7 +223,7 @@ __device__ __forceinline__ uint4 load_stream16(const __nv_bfloat16* p) {   // re
 template <typename OT, int NT, int CTAS, int U, bool SHORT>   // U: steps whose loads are in flight together
 __global__ void __launch_bounds__(256, CTAS) linear_rows_mma_kernel(const LinArgs a) {
   using Sum = std::conditional_t<SHORT, double, float>;
-  constexpr bool RUNS = !SHORT && !(NT == 4 && CTAS == 3);   // (there the registers are not; a warp's K / 512 steps in a row, rms 9.1e-8 at most)
+  constexpr bool RUNS = !SHORT && !(NT == 4 && CTAS == 3);   // (there the registers are not: up to eight steps of a warp in a row, 7.5e-8)
   __shared__ Sum part[8][16][8 * NT + 1];
   pdl_sync();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, n0 = blockIdx.x * 16;
@@ -358,12 +358,13 @@ static cudaError_t launch_rows_mma(const LinArgs& a, cudaStream_t st) {
   if (a.K < 256) return a.M <= 8 ? PIEH_MMA(1, 4, 1, true) : a.M <= 16 ? PIEH_MMA(2, 2, 1, true) : PIEH_MMA(4, 2, 1, true);
   // Up to two steps a warp there is nothing to load ahead of, and more CTAs hide more (16384 x 512, 4 rows: 8.0 us with two CTAs of four
   // steps ahead, 5.9 with four of one; 16 rows 8.9 and 8.0; at 32 rows two are sooner).  Otherwise two CTAs to an SM with as many loads as
-  // their registers hold; three, with fewer, where that saves the second wave (6368 x 4096, 16 rows: 17.7 -> 13.1 us; 4096 x 14336 is
-  // 23.9 for 34.4 the other way).
+  // their registers hold; three, with fewer, where that saves the second wave (6368 x 4096, 16 rows: 17.7 -> 13.1 us, 32 rows 25 -> 21;
+  // 4096 x 14336 is 23.9 for 34.4 the other way).  At 32 rows three have no registers for runs: beyond K 4096 their error would be larger
+  // than linear_rows_kernel's (K 8192 9.2e-8 for 9.0e-8, K 4096 7.5e-8 for 8.4e-8).
   const bool few_steps = a.K <= 1024, three = tiles > 2LL * num_sms() && tiles <= 3LL * num_sms();
   if (a.M <= 8) return few_steps ? PIEH_MMA(1, 4, 1, false) : PIEH_MMA(1, 2, 4, false);
   if (a.M <= 16) return few_steps || three ? PIEH_MMA(2, 3, 1, false) : PIEH_MMA(2, 2, 2, false);
-  return three ? PIEH_MMA(4, 3, 1, false) : PIEH_MMA(4, 2, 1, false);
+  return three && a.K <= 4096 ? PIEH_MMA(4, 3, 1, false) : PIEH_MMA(4, 2, 1, false);
 #undef PIEH_MMA
 }
 

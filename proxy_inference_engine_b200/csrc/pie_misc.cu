@@ -173,7 +173,7 @@ cudaError_t launch_rms_norm(uint16_t* out, const uint16_t* x, const uint16_t* w,
 
 // ---- a11 glue (PIE/models/llama/language.py:126-127,150-154; nn.silu activations.py:125-132) ----------------
 // Both read two arrays and write one: HBM-bound.  A thread takes 16 bytes of each per round where the arrays are 16-byte aligned
-// (the last n % 8 elements, and arrays that are not, one element at a time).  8192 x 14336, us: SwiGLU 406 -> 111 (6.3 TB/s; it was
+// (the last n % 8 elements, and arrays that are not, one element at a time).  8192 x 14336, us: SwiGLU 408 -> 130 (5.4 TB/s; it was
 // bound by two-byte accesses and a full-range division), 8192 x 4096 sum 73 -> 28.
 struct SiluMul {   // bf16 after every operator: sigmoid, gate * sigmoid, * up
   static __device__ __forceinline__ uint32_t pair(uint32_t g, uint32_t u) { return mul_bf16x2_rn(silu_bf16x2(g), u); }

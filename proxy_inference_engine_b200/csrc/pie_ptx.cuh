@@ -196,7 +196,7 @@ __device__ __forceinline__ float sigmoid_approx(float a) {
 // silu of two bf16 values, bf16 after every operator: sigmoid, gate * sigmoid.  The approximations are off by a few units of fp32's
 // last place and the sigmoid is rounded to bf16 at once: for all 65536 gates the bits are those of 1 / (1 + expf(-g)) with a full
 // division, which the layers of up to 32 rows use and which the memory-bound kernel over a prompt's rows has no time for
-// (8192 x 14336: 2-byte accesses and full division 406 us, 16-byte accesses and this 111).
+// (8192 x 14336: 2-byte accesses and full division 408 us, 16-byte accesses and this 130; 123 with __fdividef).
 __device__ __forceinline__ uint32_t silu_bf16x2(uint32_t g) {
   const float a = __uint_as_float(g << 16), b = __uint_as_float(g & 0xffff0000u);
   const uint32_t s = pack_bf16(sigmoid_approx(a), sigmoid_approx(b));

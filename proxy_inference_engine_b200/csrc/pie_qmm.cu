@@ -46,7 +46,7 @@ struct QmmStore {
 
 // silu(x . w) * (x . w_up), rounded where the separate operators round: both products, the sigmoid, silu, the result.  It saves the two
 // products' way to memory and back and a launch: 8192 x 14336 x 4096 (4 bits)
-// 2 x 676 + 113 -> 1275 us, 1531 x 8192 x 2048 87 + 12 -> 83.
+// 2 x 676 + 130 -> 1275 us, 1531 x 8192 x 2048 87 + 12 -> 83.
 struct QmmSwiglu {
   static constexpr bool PAIRED = true;
   CUtensorMap map_up;

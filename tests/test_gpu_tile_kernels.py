@@ -298,13 +298,13 @@ def test_dense_matmul_of_few_rows(M, N, K):
 @pytest.mark.parametrize("positive", [False, True])
 @pytest.mark.parametrize("M,N,K", [(1, 1200, 64), (4, 300, 128), (16, 300, 248),        # less than 256: the cut is added back
                                    (1, 1200, 256), (8, 300, 4096), (9, 2048, 4096),     # runs of four steps, loads of four, two and one ahead
-                                   (16, 5200, 1032), (32, 5200, 1032), (32, 130, 14336),   # 325 tiles: three CTAs to an SM
+                                   (16, 5200, 1032), (32, 5200, 4096), (32, 5200, 4104), (32, 130, 14336),   # 325 tiles: three CTAs to an SM
                                    (1, 1184, 4096), (2, 16, 520), (2, 1185, 4096),      # either side of the rule for few outputs
                                    (4, 592, 1024), (4, 593, 1024)])
 def test_dense_matmul_of_few_rows_sums_like_fp32(M, N, K, positive):
     """fp32 results with the error of fp32 additions, not the tensor core's truncated ones.  A sum of K numbers by a tree or in short runs is off
-    by a few 2^-25 of itself (rms, positive terms) and by a few 2^-25 of the root of K times a term (signs at random); a chain of
-    truncated sums would be off by K / 512 * 2^-24 and more, always towards zero."""
+    by up to three 2^-25 of itself (rms; signs at random, K 14336: the additions of 7 runs, of 4 steps and of a tree, each 2^-25 of its own
+    result or less); a chain of truncated sums would be off by K / 512 * 2^-24 and more, always towards zero."""
     from proxy_inference_engine_b200 import _lib
     L = _lib.load_hybrid(build_if_missing=True)
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
@@ -316,7 +316,7 @@ def test_dense_matmul_of_few_rows_sums_like_fp32(M, N, K, positive):
     out = torch.full((M, N), float("nan"), device="cuda")
     assert L.pieh_linear(_p(out), 1, N, _p(x), 0, K, _p(w), 0, None, M, N, K, 0, 0.0, None, None, 0, None) == 0
     off = out.double() - want
-    assert off.norm() <= 4 * 2 ** -25 * want.norm(), float(off.norm() / want.norm())
+    assert off.norm() <= 3 * 2 ** -25 * want.norm(), float(off.norm() / want.norm())
     if positive and M * N >= 300:      # the mean of as many independent errors: no bias
         assert abs(float((off / want).mean())) <= 2 * 2 ** -25, float((off / want).mean())
     x[:, 3], w[0, 3] = float("inf"), 1.0      # an infinite product stays one
