@@ -100,6 +100,14 @@ int pie_qmv_fused(void* out, int out_ld, const void* x, int x_ld, int M, int K, 
                   const void* residual, int ksplit_hint, void* workspace, size_t workspace_bytes, int pdl,
                   void* stream);
 
+/* The same product for some dozens of rows, weights through tensor memory.  scratch: pie_qmt_scratch_bytes() bytes (0: the call would
+ * not be served, or is sooner done by the others), 16-byte aligned, contents of no matter before and after, not shared by launches that may
+ * overlap.  PIE_EUNSUPPORTED (nothing launched): operands it cannot take.  pie_qmv_fused and pie_qmv make these calls
+ * themselves with a workspace that has room for it. */
+size_t pie_qmt_scratch_bytes(int M, long long n_total, int K, int group_size, int bits, int dual);
+int pie_qmt(void* out, int out_ld, const void* x, int x_ld, int M, int K, const pie_qmv_seg* segs_host, int nseg, int group_size, int bits,
+            const void* norm_weight, float eps, int epilogue, const void* residual, void* scratch, size_t scratch_bytes, void* stream);
+
 /* ---- a3  mx.quantized_matmul for prefill-sized M (replaces Metal qmm_t, kernels/quantized.h:954-1078) -
  * Same contraction and workspace contract as pie_qmv.  x bf16 [M, K] row-major, y bf16 [M, N].           */
 int pie_qmm(void* y, const void* x, const uint32_t* wq, const void* scales, const void* biases, int M, int N,

@@ -150,6 +150,38 @@ static size_t qmd_total_bytes(int M, long long rows_total, int K, int dual, int 
   }
   return qmd_cnt_bytes(rows_total) + worst;
 }
+
+// The tensor-memory form (pie_qmt.cuh): what it needs behind the counter region of a workspace, 0 where it does not apply.
+static size_t qmt_scratch(int M, long long n_total, int K, int group_size, int bits, int dual) {
+  if (n_total <= 0 || !qmt_shape_ok(M, K, group_size, bits)) return 0;
+  return qmt_ws_bytes(M, dual ? (n_total + 63) / 64 : (n_total + 127) / 128 + kMaxSeg, K, bits);
+}
+// Whether a call is sooner done by it.  Measured, 4 bits, B200, us before / with it (graphs of calls, the preparing kernel included): 16 rows
+// 4096 x 4096 10.9 / 11.5, 6144 x 4096 16.4 / 13.1, 2 x 14336 x 4096 with SwiGLU 42.5 / 26.6, 4096 x 14336 27.6 / 17.8, 128256 x 4096 147 / 72;
+// 32 rows 2048 x 2048 11.2 / 13.1, 3072 x 2048 11.8 / 13.2, 4096 x 4096 18.3 / 14.0, 128256 x 4096 198 / 79; 40 rows (two passes of the
+// GEMV before) 2048 x 2048 16.9 / 14.7, 4096 x 14336 54.6 / 24.2.  So up to 32 rows the line is drawn by the work, in stages of 128 rows of
+// 256 codes, that covers the 8 to 10 us a call takes at the least; 33 to 63 rows are sooner done here but for the smallest matrices (8 bits: 4096 x 4096 23.9 / 18.1,
+// 4096 x 14336 44.0 / 34.6), and from 64 on the estimates of both kernels decide (rows: 64 4096 x 4096 13.9 / 17.6, 2 x 14336 x 4096 54.2 / 41.5).
+// 8-bit calls of up to 32 rows stay with pie_qmi.cu (4096 x 14336, 32 rows 25.3 / 31.2).  PIE_QMT: 0 never, 2 always
+static bool qmt_pays(int M, long long n_total, int K, int bits, int dual) {
+  const int mode = env_int("PIE_QMT", 1);
+  if (mode != 1) return mode == 2;
+  const long long tiles = dual ? (n_total + 63) / 64 : (n_total + 127) / 128, work = tiles * ((long long)K * bits / 1024);
+  if (M <= 8) return false;
+  if (M <= 32) return bits == 4 && work >= (M <= 16 ? 700 : 400);
+  if (M < 64) return work >= 100;
+  if (work < 700) return false;
+  const int sms = num_sms(), np = (M + 15) & ~15;
+  const double mine = 6 + 0.13 * np + (double)((work + sms - 1) / sms) * (0.6 + 0.008 * np);
+  return mine < (n_total > 0x7fffffff ? 1e30 : qmm_estimate_us(M, (int)n_total, K, dual));
+}
+// the operands it can read by TMA, validated as build_qmv_args does
+static bool qmt_takes(int M, int K, int x_ld, const pie_qmv_seg* segs, int nseg, int group_size, int bits) {
+  if (!qmt_shape_ok(M, K, group_size, bits) || x_ld % 8 != 0 || x_ld < K) return false;
+  for (int i = 0; i < nseg; ++i)
+    if (!aligned16(segs[i].wq) || !aligned16(segs[i].scales) || !aligned16(segs[i].biases)) return false;
+  return true;
+}
 }  // namespace pie
 
 using namespace pie;
@@ -213,6 +245,10 @@ size_t pie_qmv_workspace_bytes(int M, long long n_total, int K, int bits, int du
     }
     if (kWsCntBytes + worst > need) need = kWsCntBytes + worst;
   }
+  if (M <= kQmtRows && qmt_pays(M, n_total, K, bits, dual)) {
+    const size_t q = qmt_scratch(M, n_total, K, kGroup, bits, dual);
+    if (q && kWsCntBytes + q > need) need = kWsCntBytes + q;
+  }
   return need;
 }
 
@@ -236,6 +272,14 @@ int pie_qmv_fused_tp(void* out, int out_ld, const void* x, int x_ld, int M, int 
     const int st0 = build_qmv_args(a, p, out, out_ld, x, x_ld, m0, mb, K, segs, nseg, group_size, bits, norm_weight, eps,
                                    epilogue, residual, ksplit_hint, workspace, workspace_bytes, 0);
     if (st0 != PIE_OK) return st0;
+    if (m0 == 0 && !tp && qmt_takes(M, K, x_ld, segs, nseg, group_size, bits)) {
+      long long n_total = 0;
+      for (int i = 0; i < nseg; ++i) n_total += segs[i].N;
+      if (a.dual) n_total = segs[0].N;
+      if (workspace && qmt_pays(M, n_total, K, bits, a.dual) && kWsCntBytes + qmt_scratch(M, n_total, K, group_size, bits, a.dual) <= workspace_bytes)
+        return cuda_status(launch_qmt(out, out_ld, x, x_ld, M, K, segs, nseg, bits, norm_weight, eps, epilogue, residual,
+                                      (uint8_t*)workspace + kWsCntBytes, (cudaStream_t)stream));
+    }
     // TMA-fed GEMV (pie_qmv2.cu): 4-bit weights, up to 8 rows, K a multiple of 512 -- every matrix of a Llama decode
     // step.  PIE_QMV2=0 keeps the cp.async kernel below (B200, 8B shapes, one row, us cp.async / TMA: q/k/v 7.8 / 7.7,
     // o 5.5 / 5.3, gate+up 18.9 / 16.5, down 13.1 / 11.5, head 64.2 / 49.7).
@@ -301,6 +345,33 @@ int pie_qmv_fused_tp(void* out, int out_ld, const void* x, int x_ld, int M, int 
     if (st != PIE_OK) return st;
   }
   return PIE_OK;
+}
+
+size_t pie_qmt_scratch_bytes(int M, long long n_total, int K, int group_size, int bits, int dual) {
+  return n_total > 0 && qmt_pays(M, n_total, K, bits, dual) ? qmt_scratch(M, n_total, K, group_size, bits, dual) : 0;
+}
+
+int pie_qmt(void* out, int out_ld, const void* x, int x_ld, int M, int K, const pie_qmv_seg* segs, int nseg, int group_size, int bits,
+            const void* norm_weight, float eps, int epilogue, const void* residual, void* scratch, size_t scratch_bytes, void* stream) {
+  if (M == 0) return PIE_OK;
+  if (!out || !x || !segs || !scratch) return PIE_ENULL;
+  if (nseg < 1 || nseg > kMaxSeg || epilogue < PIE_EPI_STORE || epilogue > PIE_EPI_SILUMUL) return PIE_EINVAL_SHAPE;
+  if (epilogue == PIE_EPI_RESADD && !residual) return PIE_ENULL;
+  const int dual = epilogue == PIE_EPI_SILUMUL;
+  if (dual && (nseg != 2 || segs[0].N != segs[1].N)) return PIE_EINVAL_SHAPE;
+  long long n_total = 0;
+  for (int i = 0; i < nseg; ++i) {
+    if (!segs[i].wq || !segs[i].scales || !segs[i].biases) return PIE_ENULL;
+    if (segs[i].N <= 0) return PIE_EINVAL_SHAPE;
+    n_total += segs[i].N;
+  }
+  if (dual) n_total = segs[0].N;
+  if (out_ld < n_total) return PIE_EINVAL_SHAPE;
+  if (!qmt_takes(M, K, x_ld, segs, nseg, group_size, bits) || !aligned16(x) || (norm_weight && !aligned16(norm_weight)) || !aligned16(scratch))
+    return PIE_EUNSUPPORTED;
+  if (qmt_scratch(M, n_total, K, group_size, bits, dual) > scratch_bytes) return PIE_EWORKSPACE;
+  const cudaError_t e = launch_qmt(out, out_ld, x, x_ld, M, K, segs, nseg, bits, norm_weight, eps, epilogue, residual, scratch, (cudaStream_t)stream);
+  return e == cudaErrorNotSupported ? PIE_EUNSUPPORTED : cuda_status(e);
 }
 
 int pie_qmv(void* y, const void* x, const uint32_t* wq, const void* scales, const void* biases, int M, int N,

@@ -14,10 +14,10 @@ static int check_kv(const pie_kv_layout* k, int D) {
 
 extern "C" {
 
-// M >= 64: the tcgen05 / TMEM tile kernel (pie_qmm.cu), weights dequantised once to bf16 into shared memory.
-// Smaller M, or shapes off its grid (K % 128, unaligned pointers): the decode GEMV in passes of <= 32 rows.  33 .. 63 rows take
-// longer there than on the tile kernel (14336 x 4096, 40 rows in two passes / 64 rows as tiles, us: 52 / 26 at 4 bits, 46 / 29 at 8), but
-// the GEMV multiplies the exact codes and the tile kernel weights rounded to bf16: those calls keep the precision they have.
+// M >= 64: the tcgen05 / TMEM tile kernel (pie_qmm.cu), weights dequantised once to bf16 into shared memory; up to 128 rows the kernel
+// of pie_qmt.cuh where it is sooner done and the workspace has room for it (pie_qmv finds that out).
+// Smaller M, or shapes off its grid (K % 128, unaligned pointers): pie_qmv.  (33 .. 63 rows do not go to the tile kernel, which multiplies weights
+// rounded to bf16, where the others multiply the exact codes.)
 int pie_qmm(void* y, const void* x, const uint32_t* wq, const void* scales, const void* biases, int M, int N,
             int K, int group_size, int bits, void* workspace, size_t workspace_bytes, void* stream) {
   if (M == 0 || N == 0) return PIE_OK;
@@ -26,6 +26,12 @@ int pie_qmm(void* y, const void* x, const uint32_t* wq, const void* scales, cons
   const bool tc = M >= 64 && quant_supported(group_size, bits) && K % 128 == 0 && aligned16(x) && aligned16(wq) &&
                   aligned16(y) && !(reinterpret_cast<uintptr_t>(scales) & 3) &&
                   !(reinterpret_cast<uintptr_t>(biases) & 3) && env_int("PIE_QMM_TC", 1) != 0;
+  if (tc && workspace && M <= kQmtRows && qmt_pays(M, N, K, bits, 0)) {
+    pie_qmv_seg seg = {wq, scales, biases, N};
+    if (qmt_takes(M, K, K, &seg, 1, group_size, bits) && kWsCntBytes + qmt_scratch(M, N, K, group_size, bits, 0) <= workspace_bytes)
+      return cuda_status(launch_qmt(y, N, x, K, M, K, &seg, 1, bits, nullptr, 0.f, PIE_EPI_STORE, nullptr, (uint8_t*)workspace + kWsCntBytes,
+                                    (cudaStream_t)stream));
+  }
   if (tc)
     return cuda_status(launch_qmm_tc((uint16_t*)y, (const uint16_t*)x, wq, (const uint16_t*)scales,
                                      (const uint16_t*)biases, M, N, K, bits, (cudaStream_t)stream));

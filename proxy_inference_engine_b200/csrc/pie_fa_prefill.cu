@@ -50,13 +50,6 @@ __device__ __forceinline__ void fap_tma_4d(uint32_t dst, const CUtensorMap* map,
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
 }
-// D[128 x N] += A[128 x 16] (tensor memory, bf16 pairs) * B (shared memory)
-__device__ __forceinline__ void fap_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accum) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc),
-      "r"(accum) : "memory");
-}
 // shared-memory descriptor of an MN-major operand in the 128-byte swizzle: rows of 64 features, 8 rows (keys) per atom,
 // atoms 1024 bytes apart along the keys, 64-feature chunks 128 rows apart
 __device__ __forceinline__ uint64_t fap_desc_mn(uint32_t smem_addr) {
@@ -76,16 +69,6 @@ __device__ __forceinline__ void fap_tmem_ld(uint32_t taddr, float* v) {
         "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
       : "r"(taddr) : "memory");
 }
-__device__ __forceinline__ void fap_tmem_st(uint32_t taddr, const uint32_t* u) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
-      "%29,%30,%31};" ::"r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]),
-      "r"(u[9]), "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15]), "r"(u[16]), "r"(u[17]), "r"(u[18]),
-      "r"(u[19]), "r"(u[20]), "r"(u[21]), "r"(u[22]), "r"(u[23]), "r"(u[24]), "r"(u[25]), "r"(u[26]), "r"(u[27]), "r"(u[28]),
-      "r"(u[29]), "r"(u[30]), "r"(u[31]), "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void fap_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ float fap_exp2(float x) {   // results below 2^-126 are 0
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -231,9 +214,9 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[i] *= c;
-          fap_tmem_st(tO + c0, reinterpret_cast<uint32_t*>(o));
+          tmem_st32(tO + c0, reinterpret_cast<uint32_t*>(o));
         }
-        fap_tmem_st_wait();
+        tmem_st_wait();
       }
       const float ms = m == -INFINITY ? 0.f : m;
       const f32x2 sc2 = f2_pack(a.scale_log2e, a.scale_log2e), ms2 = f2_pack(-ms, -ms);
@@ -257,14 +240,14 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           if (i & 1) l23 = f2_add(l23, f2_pack(e0, e1));
           else l01 = f2_add(l01, f2_pack(e0, e1));
         }
-        fap_tmem_st(tS + 32 * hf, p);
+        tmem_st32(tS + 32 * hf, p);
       }
       {
         float l0, l1;
         f2_unpack(f2_add(l01, l23), l0, l1);
         l += l0 + l1;
       }
-      fap_tmem_st_wait();
+      tmem_st_wait();
       if (a.page_table && tail && j == (keys - 1) / 128) {
         // the slots behind the last key of a page may hold anything, and 0 * NaN is not 0: clear them
         if (!(alive = gemm_wait_warp(smem_u32(&v_full[j & 1]), (j >> 1) & 1, abortp))) break;
@@ -344,7 +327,7 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const uint64_t dv = dv0 + (uint64_t)((j & 1) * (T::TILE >> 4));
 #pragma unroll
         for (int k = 0; k < 8; ++k)   // 16 keys: 8 columns of P, two 8-key atoms of V
-          fap_mma_ts(tm + COL_O + g * D, tm + COL_S + g * 128 + 8 * k, dv + k * (2048 >> 4), ID_O, (j > 0 || k > 0) ? 1u : 0u);
+          umma_f16_ts(tm + COL_O + g * D, tm + COL_S + g * 128 + 8 * k, dv + k * (2048 >> 4), ID_O, (j > 0 || k > 0) ? 1u : 0u);
         fap_commit(&o_full[g]);
       };
       bool alive = gemm_wait(smem_u32(&q_full), 0, abortp);   // a lane's own: once a wait expires it only keeps the lane from issuing

@@ -121,6 +121,13 @@ cudaError_t launch_fa_prefill_umma(uint16_t* out, const uint16_t* q, const uint1
 cudaError_t launch_qmm_swiglu(uint16_t* y, const uint16_t* x, const uint32_t* const* wq, const uint16_t* const* s, const uint16_t* const* b,
                               int M, int N, int K, int bits, cudaStream_t st);
 bool qmm_swiglu_pays(int M, int N, int K);
+double qmm_estimate_us(int M, int N, int K, int dual);
+// some dozens of activation rows, weights through tensor memory (pie_qmt.cuh, compiled with pie_qmm.cu, whose pipeline word it shares)
+constexpr int kQmtRows = 128;   // the most it takes
+bool qmt_shape_ok(int M, int K, int group_size, int bits);
+size_t qmt_ws_bytes(int M, long long ntiles, int K, int bits);
+cudaError_t launch_qmt(void* out, int out_ld, const void* x, int x_ld, int M, int K, const pie_qmv_seg* segs, int nseg, int bits,
+                       const void* norm_w, float eps, int epi, const void* residual, void* ws, cudaStream_t st);
 unsigned int qmm_pipeline_error();
 cudaError_t qmm_pipeline_post(unsigned int* host, cudaStream_t st);
 cudaError_t qmm_pipeline_clear();

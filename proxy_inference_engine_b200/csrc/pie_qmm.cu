@@ -8,6 +8,7 @@
 // dequantising warps; this file holds the store and the choice of tile.
 #include "pie_gemm.cuh"
 #include "pie_internal.h"
+#include "pie_qmt.cuh"
 
 namespace pie {
 
@@ -120,6 +121,16 @@ cudaError_t launch_qmm_swiglu(uint16_t* y, const uint16_t* x, const uint32_t* co
   epi.s_up = s[1]; epi.b_up = b[1]; epi.y = y; epi.M = M; epi.N = N;
   count_launch();
   return bits == 4 ? gemm_run_paired<4>(a, epi, c, x, wq[0], wq[1], sms, st) : gemm_run_paired<8>(a, epi, c, x, wq[0], wq[1], sms, st);
+}
+
+// what a product takes (dual: two of them and the elementwise operator, or both in one launch); 4 us besides the main loop's cycles
+double qmm_estimate_us(int M, int N, int K, int dual) {
+  const int sms = num_sms();
+  const double one = gemm_choose(M, N, K, 1, sms, true).cycles / 1900 + 4;
+  if (!dual) return one;
+  const GemmChoice c = qmm_swiglu_choice(M, N, K, sms);
+  const double apart = 2 * one + 2 + (double)M * N * 6 / 6e6;
+  return c.bn && c.cycles / 1900 + 4 < apart ? c.cycles / 1900 + 4 : apart;
 }
 
 unsigned int qmm_pipeline_error() { return gemm_error_now(); }

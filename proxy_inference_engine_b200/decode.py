@@ -441,7 +441,7 @@ class DecodeEngine:
         last = logits[:, -1, :].contiguous()
         self.logits.copy_(last)
         self._sample(self.logits)
-        self.watch.post()   # the prompt's matrices and attention have waits that can expire, the steps have not
+        self.watch.post()   # the prompt's matrices and attention have waits that can expire
         return self.tokens
 
     def step(self, n: int = 1):
@@ -463,6 +463,8 @@ class DecodeEngine:
                 n0 = ops.launch_count()
                 self._step_kernels()
                 self.launches_per_step = ops.launch_count() - n0
+        if self.B > 8:
+            self.watch.post()   # as a prompt's (steps of fewer rows have no such waits)
         for c in self.cache:
             c.offset += n
 

@@ -191,8 +191,8 @@ class TransformerBlock(nn.Module):
         return ops.add(h, r)
 
     def _few_rows(self, x, mask, cache):
-        """Up to 32 rows on one GPU: norms, residual sums and SwiGLU ride in the four quantized matmuls (nn.fused_rows).  None
-        where they do not apply."""
+        """Few rows on one GPU: norms, residual sums and SwiGLU ride in the four quantized matmuls (nn.fused_rows).  None where
+        they do not apply."""
         at, mlp = self.self_attn, self.mlp
         tp = getattr(at, "tp", None)
         if type(at) is not Attention or type(mlp) is not MLP or (tp is not None and tp.on) or x.dim() != 3:

@@ -135,8 +135,8 @@ def fused_swiglu(x, gate, up):
 
 
 def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
-    """Up to 32 rows through several bias-free QuantizedLinears in ONE launch, with the RMSNorm in front of them, and the
-    residual sum or SwiGLU behind them where asked for:
+    """Up to 32 rows, and up to 128 where that is sooner done, through several bias-free QuantizedLinears in ONE pass over their weights, with
+    the RMSNorm in front of them, and the residual sum or SwiGLU behind them where asked for:
         [..., sum N]  their outputs side by side;   residual: residual + output;   swiglu: silu(first) * second.
     Results are rounded where the separate calls round them.  One matrix, with or without a residual, gives their bits; a norm's
     sum of squares and the sums over K of several matrices are taken in another order, so that a value near a rounding boundary
@@ -144,7 +144,7 @@ def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
     None where that kernel does not apply (the caller then makes the separate calls, which also report what is wrong)."""
     K = x.shape[-1]
     rows = x.numel() // K if K else 0
-    if not 0 < rows <= 32 or x.dtype != torch.bfloat16 or not x.is_contiguous() or x.data_ptr() % 16:
+    if not 0 < rows <= 128 or x.dtype != torch.bfloat16 or not x.is_contiguous() or x.data_ptr() % 16:
         return None
     bits, N = getattr(linears[0], "bits", None), 0
     if bits not in (4, 8) or K % (1024 // bits):
@@ -157,6 +157,8 @@ def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
         if linears[0].weight.shape[0] != linears[1].weight.shape[0]:
             return None
         N //= 2
+    if rows > 32 and not ops.qmt_scratch_bytes(rows, N, K, bits, int(swiglu)):
+        return None
     if norm is not None:
         if type(norm) is not RMSNorm:
             return None

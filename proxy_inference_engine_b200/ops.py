@@ -32,6 +32,26 @@ def _qmv_workspace_bytes(M: int, N: int, K: int, bits: int, dual: int) -> int:
     return _lib.load().pie_qmv_workspace_bytes(M, N, K, bits, dual, 0)
 
 
+@functools.lru_cache(maxsize=4096)
+def qmt_scratch_bytes(M: int, N: int, K: int, bits: int, dual: int) -> int:
+    """0: the call is not for pie_qmt.  (A pure function of the sizes.)"""
+    return _lib.load().pie_qmt_scratch_bytes(M, N, K, 64, bits, dual) if 0 < M <= 128 else 0
+
+
+def _qmt(out, x, segs, nseg, M: int, K: int, N: int, bits: int, norm_weight, eps, epilogue, residual, dual: int) -> bool:
+    """pie_qmt where it serves the call.  Its scratch lives until the launch is queued and is reused in stream order, as any tensor."""
+    nb = qmt_scratch_bytes(M, N, K, bits, dual)
+    if not nb:
+        return False
+    scratch = torch.empty(nb, dtype=torch.uint8, device=x.device)
+    status = _lib.load().pie_qmt(_p(out), N, _p(x), K, M, K, segs, nseg, 64, bits, _p(norm_weight), eps, epilogue, _p(residual),
+                                 _p(scratch), nb, _stream())
+    if status == _lib.EUNSUPPORTED:
+        return False
+    _lib.check(status, "qmt")
+    return True
+
+
 def _as_words(w: torch.Tensor) -> torch.Tensor:
     if w.dtype == torch.int32:
         return w
@@ -154,6 +174,11 @@ def quantized_matmul(x, w, scales, biases, transpose: bool = True, group_size: i
     M = x2.shape[0]
     y = torch.empty((M, N), dtype=_BF16, device=x.device)
     L = _lib.load()
+    if group_size == 64 and bits in (4, 8) and qmt_scratch_bytes(M, N, K, bits, 0):
+        seg = (QmvSeg * 1)()
+        seg[0].wq, seg[0].scales, seg[0].biases, seg[0].N = w.data_ptr(), scales.data_ptr(), biases.data_ptr(), N
+        if _qmt(y, x2, seg, 1, M, K, N, bits, None, 0.0, EPI_STORE, None, 0):
+            return y.reshape(x.shape[:-1] + (N,))
     nb = _qmv_workspace_bytes(min(M, 32) if M else 1, N, K, bits, 0) if bits in (4, 8) and group_size == 64 else 0
     ws = workspaces.get("qmv", nb, x.device)
     fn = L.pie_qmv if M <= 32 else L.pie_qmm
@@ -163,16 +188,20 @@ def quantized_matmul(x, w, scales, biases, transpose: bool = True, group_size: i
 
 
 def qmv_fused(x, linears, rows: int, K: int, N: int, bits: int, norm_weight, eps: float, residual, swiglu: bool):
-    """pie_qmv_fused on operands nn.fused_rows has checked.  N: output columns."""
+    """pie_qmt or pie_qmv_fused on operands nn.fused_rows has checked.  N: output columns.  None: more than 32 rows that pie_qmt does not serve."""
     L = _lib.load()
     segs = (QmvSeg * len(linears))()
     for seg, lin in zip(segs, linears):
         seg.wq, seg.scales, seg.biases, seg.N = lin.weight.data_ptr(), lin.scales.data_ptr(), lin.biases.data_ptr(), lin.weight.shape[0]
     out = torch.empty(x.shape[:-1] + (N,), dtype=_BF16, device=x.device)
+    epilogue = EPI_SILUMUL if swiglu else EPI_STORE if residual is None else EPI_RESADD
+    if _qmt(out, x, segs, len(linears), rows, K, N, bits, norm_weight, float(eps), epilogue, residual, int(swiglu)):
+        return out
+    if rows > 32:
+        return None
     ws = workspaces.get("qmv", _qmv_workspace_bytes(rows, N, K, bits, int(swiglu)), x.device)
-    _lib.check(L.pie_qmv_fused(_p(out), N, _p(x), K, rows, K, segs, len(linears), 64, bits, _p(norm_weight), float(eps),
-                               EPI_SILUMUL if swiglu else EPI_STORE if residual is None else EPI_RESADD, _p(residual), 0, _p(ws),
-                               ws.numel(), 0, _stream()), "qmv_fused")
+    _lib.check(L.pie_qmv_fused(_p(out), N, _p(x), K, rows, K, segs, len(linears), 64, bits, _p(norm_weight), float(eps), epilogue,
+                               _p(residual), 0, _p(ws), ws.numel(), 0, _stream()), "qmv_fused")
     return out
 
 

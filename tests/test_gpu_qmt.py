@@ -1,0 +1,112 @@
+"""pie_qmt (csrc/pie_qmt.cuh), some dozens of rows with the weights through tensor memory, against float64 at the edges of its rows, tiles and
+shares.  Operands are exact and sums are fp32, so what is left is the rounding of the result to bf16: 2^-9 of a value at the most, in the
+2-norm 2^-9 / sqrt(3) = 1.13e-3 to 1.95e-3 as the values lie in their binade."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(g, n, k, bits):
+    words = torch.randint(-(1 << 31), 1 << 31, (n, k * bits // 32), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    spread = 1 - 0.1 * torch.rand((n, k // 64), generator=g, device="cuda")
+    return [words, (2 / k ** 0.5 / (2 ** bits - 1) * spread).bfloat16(), (-spread / k ** 0.5).bfloat16()]
+
+
+def _dense(m, bits):
+    words, s, b = m
+    q = ((words[:, :, None] >> torch.arange(0, 32, bits, device="cuda", dtype=torch.int32)) & (2 ** bits - 1)).reshape(s.shape + (64,)).double()
+    return (q * s.double()[:, :, None] + b.double()[:, :, None]).flatten(1)
+
+
+def _call(x, mats, bits, norm=None, residual=None, swiglu=False):
+    from proxy_inference_engine_b200 import _lib
+    L = _lib.load()
+    segs = (_lib.QmvSeg * len(mats))()
+    for seg, (w, s, b) in zip(segs, mats):
+        seg.wq, seg.scales, seg.biases, seg.N = w.data_ptr(), s.data_ptr(), b.data_ptr(), w.shape[0]
+    M, K = x.shape
+    N = sum(m[0].shape[0] for m in mats) // (2 if swiglu else 1)
+    nb = L.pie_qmt_scratch_bytes(M, N, K, 64, bits, int(swiglu))
+    scratch = torch.full((nb,), 255, dtype=torch.uint8, device="cuda")            # its contents do not matter
+    out = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    p = lambda t: None if t is None else t.data_ptr()
+    n0 = L.pie_launch_count()
+    _lib.check(L.pie_qmt(p(out), N, p(x), K, M, K, segs, len(mats), 64, bits, p(norm), 1e-5, 2 if swiglu else 0 if residual is None else 1,
+                         p(residual), p(scratch), nb, torch.cuda.current_stream().cuda_stream), "qmt")
+    assert L.pie_launch_count() - n0 == 2 and L.pie_pipeline_error() == 0
+    return out
+
+
+def _rel(y, ref):
+    return float((y.double() - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 512), (16, 129, 1536), (17, 2048, 2048), (32, 19200, 512), (33, 300, 8192), (48, 1000, 28672),
+                                   (49, 4096, 4096), (64, 6144, 512), (80, 257, 4608), (97, 512, 512), (128, 22000, 1024)])
+def test_products_match_float64(bits, M, N, K, monkeypatch):
+    monkeypatch.setenv("PIE_QMT", "2")
+    g = torch.Generator(device="cuda").manual_seed(M + N + K + bits)
+    m, x = _matrix(g, N, K, bits), torch.randn((M, K), generator=g, device="cuda").bfloat16()
+    if M > 3:
+        x[1] *= 1e-30
+        x[2, : K // 2] *= 2.0 ** -12          # half of a row far below its largest values
+        x[3] = 0
+    y, ref = _call(x, [m], bits), x.double() @ _dense(m, bits).t()
+    assert _rel(y, ref) < 2e-3
+    for r in {0, 1, 2, M - 1} & set(range(M)):
+        assert _rel(y[r], ref[r]) < 2.5e-3
+    assert M <= 3 or not y[3].any()
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("M", [23, 70])
+def test_norm_segments_residual_and_swiglu(bits, M, monkeypatch):
+    from proxy_inference_engine_b200 import ops
+    monkeypatch.setenv("PIE_QMT", "2")
+    K = 2048
+    g = torch.Generator(device="cuda").manual_seed(M + bits)
+    x, nw = (3 * torch.randn((M, K), generator=g, device="cuda")).bfloat16(), (1 + 0.1 * torch.randn(K, generator=g, device="cuda")).bfloat16()
+    mats = [_matrix(g, n, K, bits) for n in (520, 128, 130)]
+    xn = ops.rms_norm(x, nw, 1e-5).double()
+    # (the norm's sum of squares has another order: a normalised value may fall on the other side of a rounding boundary)
+    assert _rel(_call(x, mats, bits, norm=nw), torch.cat([xn @ _dense(m, bits).t() for m in mats], 1)) < 2.2e-3
+    res = torch.randn((M, 520), generator=g, device="cuda").bfloat16()
+    assert _rel(_call(x, mats[:1], bits, residual=res), res.double() + x.double() @ _dense(mats[0], bits).t()) < 2.6e-3    # two roundings
+    gate, up = _matrix(g, 9500, K, bits), _matrix(g, 9500, K, bits)
+    a, b = x.double() @ _dense(gate, bits).t(), x.double() @ _dense(up, bits).t()
+    assert _rel(_call(x, [gate, up], bits, swiglu=True), torch.nn.functional.silu(a) * b) < 4.5e-3                           # five roundings
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+def test_scales_no_operand_holds_and_values_that_are_no_numbers(bits, monkeypatch):
+    monkeypatch.setenv("PIE_QMT", "2")
+    M, N, K = 19, 300, 4096
+    g = torch.Generator(device="cuda").manual_seed(bits)
+    m, x = _matrix(g, N, K, bits), torch.randn((M, K), generator=g, device="cuda").bfloat16()
+    w, s, b = m
+    s[5, 3], s[77, 0], b[200, 10], b[131] = 1e-12, 50.0, 1e5, 1e-9
+    s[130] *= 1e20
+    b[130] *= 1e20
+    s[299], b[299] = 0, 0
+    s[140], b[140] = 1e-7, 0                                     # what a group of zeros quantizes to
+    y, ref = _call(x, [m], bits), x.double() @ _dense(m, bits).t()
+    for n in list(range(0, 299, 13)) + [5, 77, 130, 131, 140, 200]:
+        assert _rel(y[:, n], ref[:, n]) < 4e-3, n
+    assert not y[:, 299].any()
+    x[2, 5], x[7, 9] = float("inf"), float("nan")
+    z = _call(x, [m], bits)
+    keep = [r for r in range(M) if r not in (2, 7)]
+    assert torch.equal(z[keep], y[keep]) and z[7].isnan().all() and not z[2].isfinite().any()
+
+
+def test_few_rows_share_their_bits_with_any_batch(monkeypatch):
+    """A row's result does not depend on the rows beside it, nor a call's on the one before it."""
+    monkeypatch.setenv("PIE_QMT", "2")
+    g = torch.Generator(device="cuda").manual_seed(3)
+    m, x = _matrix(g, 4096, 4096, 4), torch.randn((32, 4096), generator=g, device="cuda").bfloat16()
+    y = _call(x, [m], 4)
+    assert torch.equal(_call(x[:20].contiguous(), [m], 4), y[:20]) and torch.equal(_call(x, [m], 4), y)
