@@ -19,7 +19,7 @@ import os
 import torch
 
 from .ops import PipelineWatch
-from .ragged import BatchDetails
+from .ragged import BatchDetails, to_device
 
 
 class _DecodeGraph:
@@ -160,7 +160,7 @@ class HybridEngine:
             return logits.clone() if rows == list(range(n)) else logits[torch.tensor(rows, device=self.device)]
         batch = BatchDetails.build(seqs, device=self.device)
         # with nothing wanted the head still needs a row: take the last and drop the result
-        idx = torch.tensor(rows if rows else [row0 - 1], dtype=torch.int32).to(self.device)
+        idx = to_device(torch.tensor(rows if rows else [row0 - 1], dtype=torch.int32), self.device)
         logits = self.model.step(batch, self.cache, rows=idx, trace=trace)
         self._post()
         for sid, toks, *_ in seqs:

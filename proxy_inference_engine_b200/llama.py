@@ -167,8 +167,10 @@ class MLP(nn.Module):
 
     def __call__(self, x):
         act = nn.fused_rows(x, (self.gate_proj, self.up_proj), swiglu=True)
-        if act is None:
-            act = nn.fused_swiglu(x, self.gate_proj, self.up_proj)
+        if act is not None:
+            y = nn.fused_rows(act, (self.down_proj,))
+            return all_reduce_sum(self.down_proj(act) if y is None else y, getattr(self, "tp", None))
+        act = nn.fused_swiglu(x, self.gate_proj, self.up_proj)
         if act is None:
             act = ops.silu_mul(self.gate_proj(x), self.up_proj(x))
         return all_reduce_sum(self.down_proj(act), getattr(self, "tp", None))

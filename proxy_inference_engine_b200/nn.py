@@ -142,6 +142,10 @@ def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
     sum of squares and the sums over K of several matrices are taken in another order, so that a value near a rounding boundary
     may fall on its other side.
     None where that kernel does not apply (the caller then makes the separate calls, which also report what is wrong)."""
+    if x.is_cuda:
+        y = ops.native_fused_rows()(x, linears, norm, residual, swiglu, QuantizedLinear, RMSNorm, ops.qmv_workspace)
+        if y is not None:
+            return y
     K = x.shape[-1]
     rows = x.numel() // K if K else 0
     if not 0 < rows <= 128 or x.dtype != torch.bfloat16 or not x.is_contiguous() or x.data_ptr() % 16:

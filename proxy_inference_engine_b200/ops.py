@@ -9,6 +9,8 @@ from __future__ import annotations
 
 import ctypes as C
 import functools
+import importlib.util
+import os
 
 import torch
 
@@ -88,6 +90,10 @@ class _Workspaces:
 
 
 workspaces = _Workspaces()
+
+
+def qmv_workspace(nbytes: int, device) -> torch.Tensor:
+    return workspaces.get("qmv", nbytes, device)
 
 
 def quantize(w: torch.Tensor, group_size: int = 64, bits: int = 4):
@@ -180,7 +186,7 @@ def quantized_matmul(x, w, scales, biases, transpose: bool = True, group_size: i
         if _qmt(y, x2, seg, 1, M, K, N, bits, None, 0.0, EPI_STORE, None, 0):
             return y.reshape(x.shape[:-1] + (N,))
     nb = _qmv_workspace_bytes(min(M, 32) if M else 1, N, K, bits, 0) if bits in (4, 8) and group_size == 64 else 0
-    ws = workspaces.get("qmv", nb, x.device)
+    ws = qmv_workspace(nb, x.device)
     fn = L.pie_qmv if M <= 32 else L.pie_qmm
     _lib.check(fn(_p(y), _p(x2), _p(w), _p(scales), _p(biases), M, N, K, group_size, bits, _p(ws), ws.numel(),
                   _stream()), "quantized_matmul")
@@ -199,10 +205,25 @@ def qmv_fused(x, linears, rows: int, K: int, N: int, bits: int, norm_weight, eps
         return out
     if rows > 32:
         return None
-    ws = workspaces.get("qmv", _qmv_workspace_bytes(rows, N, K, bits, int(swiglu)), x.device)
+    ws = qmv_workspace(_qmv_workspace_bytes(rows, N, K, bits, int(swiglu)), x.device)
     _lib.check(L.pie_qmv_fused(_p(out), N, _p(x), K, rows, K, segs, len(linears), 64, bits, _p(norm_weight), float(eps), epilogue,
                                _p(residual), 0, _p(ws), ws.numel(), 0, _stream()), "qmv_fused")
     return out
+
+
+@functools.cache
+def native_fused_rows():
+    """csrc/pie_host.cpp's form of nn.fused_rows, which takes the common calls and answers None to the others; where it was not built: None to
+    every call."""
+    path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_pie_host.so")
+    if not os.path.exists(path):
+        return lambda *args: None
+    spec = importlib.util.spec_from_file_location("_pie_host", path)
+    host = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(host)
+    L = _lib.load()
+    host.bind(*(C.cast(fn, C.c_void_p).value for fn in (L.pie_qmv_fused, L.pie_qmv_workspace_bytes, L.pie_qmt, L.pie_qmt_scratch_bytes)))
+    return host.fused_rows
 
 
 @functools.lru_cache(maxsize=4096)

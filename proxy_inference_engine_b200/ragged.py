@@ -29,6 +29,13 @@ from .ops import _p, _stream
 PAGE_TOKENS = 64
 
 
+def to_device(t: torch.Tensor, device) -> torch.Tensor:
+    """A host tensor on the device, in stream order and without a wait: a copy from pageable memory holds the caller until everything queued
+    before it has run, so that no step was prepared under the one before (a prompt of 1200 tokens: 300 of 1150 us idle).  torch keeps the
+    page-locked copy until the device has read it."""
+    return t.pin_memory().to(device, non_blocking=True) if torch.device(device).type == "cuda" else t.to(device)
+
+
 @dataclass
 class BatchDetails:
     token_ids: torch.Tensor                     # int32 [total_tokens_in_step]
@@ -72,8 +79,10 @@ class BatchDetails:
             raise ValueError("empty batch")
         width = max(1, max(len(r) for r in rows))
         table = torch.tensor([r + [0] * (width - len(r)) for r in rows], dtype=torch.int32)
-        return cls(torch.tensor(ids, dtype=torch.int32).to(device), torch.tensor(pos, dtype=torch.int32).to(device), sids,
-                   ins, ctxs, table.to(device), n_pre, n_dec, len(ids), slots)
+        # tokens | positions | block table: one copy
+        T = len(ids)
+        dev = to_device(torch.cat([torch.tensor(ids + pos, dtype=torch.int32), table.flatten()]), device)
+        return cls(dev[:T], dev[T:2 * T], sids, ins, ctxs, dev[2 * T:].view(table.shape), n_pre, n_dec, T, slots)
 
     def validate(self) -> None:
         n = len(self.sequence_ids)
@@ -120,7 +129,7 @@ class BatchDetails:
         nt = len(tile_seq)
         host = torch.tensor(tok_seq + starts + list(self.input_lengths) + list(self.context_lengths) + slots + tile_seq
                             + tile_row, dtype=torch.int32)
-        dev = host.to(self.token_ids.device)
+        dev = to_device(host, self.token_ids.device)
         ptr = lambda off: dev.data_ptr() + 4 * off
         d = HybBatch(T, n, ptr(0), self.positions.data_ptr(), ptr(T), ptr(T + n), ptr(T + 2 * n), ptr(T + 3 * n),
                      self.consolidated_block_table.data_ptr(), self.consolidated_block_table.stride(0), nt,

@@ -110,3 +110,42 @@ def test_few_rows_share_their_bits_with_any_batch(monkeypatch):
     m, x = _matrix(g, 4096, 4096, 4), torch.randn((32, 4096), generator=g, device="cuda").bfloat16()
     y = _call(x, [m], 4)
     assert torch.equal(_call(x[:20].contiguous(), [m], 4), y[:20]) and torch.equal(_call(x, [m], 4), y)
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+def test_the_native_host_form_is_the_python_one(bits, monkeypatch):
+    """csrc/pie_host.cpp against nn.fused_rows without it: the same bits where it answers, and no answer where that has none."""
+    from proxy_inference_engine_b200 import nn, ops
+    assert ops.native_fused_rows().__name__ == "fused_rows"
+    g = torch.Generator(device="cuda").manual_seed(bits)
+    K = 2048
+
+    def layer(n):
+        lin = object.__new__(nn.QuantizedLinear)
+        lin.group_size, lin.bits = 64, bits
+        lin.weight, lin.scales, lin.biases = _matrix(g, n, K, bits)
+        return lin
+
+    lins, norm = (layer(6144), layer(6144)), object.__new__(nn.RMSNorm)
+    norm.weight, norm.eps = torch.ones(K, dtype=torch.bfloat16, device="cuda"), 1e-5
+    native = lambda x, ls=lins, n=None, r=None, s=False: ops.native_fused_rows()(x, ls, n, r, s, nn.QuantizedLinear, nn.RMSNorm, ops.qmv_workspace)
+    for shape in ((1, K), (2, 1, K), (20, K), (3, 13, K), (100, K), (0, K)):
+        x = torch.randn(shape, generator=g, device="cuda").bfloat16()
+        for kw in (dict(), dict(norm=norm), dict(swiglu=True), dict(residual=torch.randn(shape[:-1] + (6144,), generator=g, device="cuda").bfloat16())):
+            ls = lins if "residual" not in kw else lins[:1]
+            mine = native(x, ls, kw.get("norm"), kw.get("residual"), kw.get("swiglu", False))
+            with monkeypatch.context() as m:
+                m.setattr(ops, "native_fused_rows", lambda: lambda *a: None)
+                want = nn.fused_rows(x, ls, **kw)
+            assert (mine is None) == (want is None) and (mine is None or (mine.shape == want.shape and torch.equal(mine, want)))
+    x = torch.randn((4, K), generator=g, device="cuda").bfloat16()
+    biased, other, strided, wide = layer(256), layer(256), layer(256), layer(256)
+    biased.bias = torch.zeros(256, device="cuda")
+    other.group_size = 32
+    strided.scales = strided.scales.t().contiguous().t()
+    wide.scales = wide.scales.float()
+    for bad in (biased, other, strided, wide, lambda v: v):
+        assert native(x, (bad,)) is None
+    assert native(x.float()) is None and native(x[:, ::2]) is None and native(x.t()) is None and native(x[:, :1024].contiguous()) is None
+    assert native(x, lins[:1], None, x) is None and native(x, lins, lambda v: v) is None and native(x, list(lins)) is None
+    assert torch.func.vmap(lambda v: torch.zeros(()) if native(v) is None else torch.ones(()))(x[:, None]).sum() == 0
