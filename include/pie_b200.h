@@ -118,6 +118,11 @@ int pie_qmm(void* y, const void* x, const uint32_t* wq, const void* scales, cons
 int pie_qmm_swiglu_pays(int M, int N, int K, int group_size, int bits);
 int pie_qmm_swiglu(void* y, const void* x, const pie_qmv_seg* gate_up, int M, int K, int group_size, int bits, void* stream);
 
+/* 64 rows and more: the products of up to three matrices of one K side by side in rows of y (y_ld elements apart), and residual (as y lies; may be
+ * y; NULL: none) added to them: the bits of pie_qmm on each and pie_add.  PIE_EUNSUPPORTED (nothing launched): operands it cannot take. */
+int pie_qmm_rows(void* y, int y_ld, const void* x, const pie_qmv_seg* segs_host, int nseg, const void* residual, int M, int K, int group_size,
+                 int bits, void* stream);
+
 /* ---- a6  mx.fast.rms_norm (MLX/mlx/fast.cpp:56-123; kernels/rms_norm.metal:13-81) -------------------- */
 int pie_rms_norm(void* out, const void* x, const void* weight, long long rows, int dims, float eps,
                  void* stream);

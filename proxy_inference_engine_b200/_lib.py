@@ -93,6 +93,7 @@ SIGNATURES = {
     "pie_qmt": (_i, [_vp, _i, _vp, _i, _i, _i, C.POINTER(QmvSeg), _i, _i, _i, _vp, _f, _i, _vp, _vp, _sz, _vp]),
     "pie_qmm_swiglu_pays": (_i, [_i, _i, _i, _i, _i]),
     "pie_qmm_swiglu": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp]),
+    "pie_qmm_rows": (_i, [_vp, _i, _vp, C.POINTER(QmvSeg), _i, _vp, _i, _i, _i, _i, _vp]),
     "pie_qmm": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _sz, _vp]),
     "pie_rms_norm": (_i, [_vp, _vp, _vp, _ll, _i, _f, _vp]),
     "pie_rope": (_i, [_vp, _vp, _ll, _i, _i, _i, _i, _f, _f, _i, _vp, _vp]),

@@ -61,6 +61,27 @@ int pie_qmm_swiglu(void* y, const void* x, const pie_qmv_seg* gate_up, int M, in
   return e == cudaErrorNotSupported ? PIE_EUNSUPPORTED : cuda_status(e);
 }
 
+// Another status than PIE_OK: nothing was launched.
+int pie_qmm_rows(void* y, int y_ld, const void* x, const pie_qmv_seg* segs, int nseg, const void* residual, int M, int K, int group_size, int bits,
+                 void* stream) {
+  if (!y || !x || !segs) return PIE_ENULL;
+  if (M < 0 || K <= 0 || nseg < 1 || nseg > kMaxSeg) return PIE_EINVAL_SHAPE;
+  long long n = 0;
+  bool ok = M >= 64 && quant_supported(group_size, bits) && K % 128 == 0 && aligned16(x) && aligned16(y) && aligned16(residual) &&
+            env_int("PIE_QMM_TC", 1) != 0;
+  for (int i = 0; i < nseg; ++i) {
+    if (!segs[i].wq || !segs[i].scales || !segs[i].biases) return PIE_ENULL;
+    if (segs[i].N <= 0) return PIE_EINVAL_SHAPE;
+    n += segs[i].N;
+    ok = ok && aligned16(segs[i].wq) && !((reinterpret_cast<uintptr_t>(segs[i].scales) | reinterpret_cast<uintptr_t>(segs[i].biases)) & 3);
+  }
+  if (y_ld < n) return PIE_EINVAL_SHAPE;
+  if (M == 0) return PIE_OK;
+  if (!ok || n > 0x7fffffff) return PIE_EUNSUPPORTED;
+  const cudaError_t e = launch_qmm_rows((uint16_t*)y, y_ld, (const uint16_t*)x, segs, nseg, (const uint16_t*)residual, M, K, bits, (cudaStream_t)stream);
+  return e == cudaErrorNotSupported ? PIE_EUNSUPPORTED : cuda_status(e);
+}
+
 int pie_rms_norm(void* out, const void* x, const void* weight, long long rows, int dims, float eps, void* stream) {
   if (rows == 0) return PIE_OK;
   if (!out || !x) return PIE_ENULL;

@@ -207,6 +207,11 @@ __device__ __forceinline__ GemmTileAt gemm_tile_at(const GemmArgs& a, int t) {
 template <class E, class = void> struct gemm_paired { static constexpr bool value = false; };
 template <class E> struct gemm_paired<E, decltype((void)E::PAIRED)> { static constexpr bool value = true; };
 
+// An epilogue with a member SEGMENTS has the rows of up to three matrices of one K side by side for w: column tiles [tile0[i], tile0[i + 1]) are
+// matrix i's, whose packed rows are map_w's or map_more[i - 1]'s and whose scales are s[i], b[i].  It is told the matrix and the column in it.
+template <class E, class = void> struct gemm_segments { static constexpr bool value = false; };
+template <class E> struct gemm_segments<E, decltype((void)E::SEGMENTS)> { static constexpr bool value = true; };
+
 // Epi: void operator()(int z, int row0, int col0, const uint32_t (&v)[32], uint32_t buf, int lane), called by whole warps: 32 columns
 // of rows row0 .. row0 + 31, lane l holding row l's; any row and column, the callee checks the bounds.  buf: 4 KB of shared memory
 // of the warp's own, to turn the tile so that rows are written in whole runs.
@@ -215,8 +220,9 @@ __global__ void __launch_bounds__(GemmTile<CG, BN, QB, SPLIT>::THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ GemmArgs a,
             const __grid_constant__ Epi epi) {
   using T = GemmTile<CG, BN, QB, SPLIT>;
-  constexpr bool PAIRED = gemm_paired<Epi>::value;
+  constexpr bool PAIRED = gemm_paired<Epi>::value, SEGMENTS = gemm_segments<Epi>::value;
   static_assert(!PAIRED || (CG == 2 && QB && T::NB % 32 == 0), "each CTA of a pair stages one matrix, in whole runs");
+  static_assert(!SEGMENTS || (QB && !PAIRED), "matrices side by side are dequantised ones");
   constexpr int COLS = PAIRED ? T::NB : BN;   // columns of y in a tile
   constexpr int S = T::S, RING = T::RING > 0 ? T::RING : 1, KPC = QB == 4 ? 4 : 2;   // K steps per packed chunk
   constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(T::BM >> 4) << 24);
@@ -306,6 +312,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
             }
           }
           if constexpr (PAIRED) epi(row0, at.n * COLS + c * 32, t, v, ebuf, lane);
+          else if constexpr (SEGMENTS) { const int g = epi.segment(at.n); epi(g, row0, (at.n - epi.tile0[g]) * BN + (c_lo + c) * 32, v, ebuf, lane); }
           else epi(at.z, row0, at.n * BN + (c_lo + c) * 32, v, ebuf, lane);
         }
       }
@@ -369,13 +376,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
       bool alive = true;
       for (int t = first_tile; t < ntiles && alive; t += tile_step) {
         const GemmTileAt at = gemm_tile_at(a, t);
-        const int col = at.n * COLS + (int)(CG == 2 && !PAIRED ? rank : 0) * T::NB;
+        int col = at.n * COLS + (int)(CG == 2 && !PAIRED ? rank : 0) * T::NB;
+        if constexpr (SEGMENTS) col -= epi.tile0[epi.segment(at.n)] * BN;
         for (int kb = k_lo; kb < k_hi; kb += KPC, ++pc) {
           const int p = pc % RING;
           if (!(alive = gemm_wait(smem_u32(&pempty_bar[p]), ((pc / RING) & 1) ^ 1, abortp))) break;
           mbar_arrive_expect_tx(&pfull_bar[p], T::CHUNK);
           const CUtensorMap* map = &map_w;
           if constexpr (PAIRED) map = rank ? &epi.map_up : &map_w;
+          if constexpr (SEGMENTS) { const int g = epi.segment(at.n); map = g == 0 ? &map_w : &epi.map_more[g - 1]; }
           gemm_tma_3d<1>(smP + p * T::CHUNK, map, smem_u32(&pfull_bar[p]), kb / KPC * 128, col, 0);
         }
         if (SPLIT) break;
@@ -390,8 +399,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
     bool alive = true;
     for (int t = first_tile; t < ntiles && alive; t += tile_step, it0 += k_hi - k_lo, pc0 += chunks) {
       const GemmTileAt at = gemm_tile_at(a, t);
-      const int row = min(at.n * COLS + (int)(CG == 2 && !PAIRED ? rank : 0) * T::NB + min(r, T::NB - 1), a.N - 1);
+      int row = at.n * COLS + (int)(CG == 2 && !PAIRED ? rank : 0) * T::NB + min(r, T::NB - 1);
       const uint16_t *sp = a.scales, *bp = a.biases;
+      if constexpr (SEGMENTS) {
+        const int g = epi.segment(at.n);
+        row = min(row - epi.tile0[g] * BN, epi.N[g] - 1);
+        sp = epi.s[g]; bp = epi.b[g];
+      } else {
+        row = min(row, a.N - 1);
+      }
       if constexpr (PAIRED)
         if (rank) { sp = epi.s_up; bp = epi.b_up; }
       sp += (size_t)row * nk_all;
@@ -509,9 +525,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ C
         }
 #pragma unroll
         for (int q = 0; q < 32; ++q) v[q] = __float_as_uint(acc[q]);
-        if constexpr (!PAIRED)
+        if constexpr (SEGMENTS) {
+          const int g = epi.segment(at.n);
+          epi(g, at.m * T::BM + (warp & 3) * 32, (at.n - epi.tile0[g]) * BN + (gi * (int)ranks + (int)rank) * 32, v,
+              smP + T::RING * T::CHUNK + warp * 4096, lane);
+        } else if constexpr (!PAIRED) {
           epi(at.z, at.m * T::BM + (warp & 3) * 32, at.n * BN + (gi * (int)ranks + (int)rank) * 32, v,
               smP + T::RING * T::CHUNK + warp * 4096, lane);
+        }
       }
     }
   }
@@ -562,17 +583,18 @@ inline bool gemm_map(CUtensorMap* m, const void* p, int elem_bytes, long long in
 // choice takes 1.02 times the best tile's time on average.
 struct GemmChoice { int pair, bn, ranks, k_per, mt, nt; double cycles; };
 inline double gemm_pair_step(int bn, bool quant) { return quant ? 490 + 280 * bn / 256.0 : 430 + 290 * bn / 256.0; }
-inline GemmChoice gemm_choose(int M, int N, int K, int nb, int sms, bool quant) {
+inline GemmChoice gemm_choose(int M, int N, int K, int nb, int sms, bool quant, int N1 = 0, int N2 = 0) {   // N1, N2: matrices beside it
   auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  auto cols = [&](int bn) { return up(N, bn) + up(N1, bn) + up(N2, bn); };
   const long long nk = K / 64;
-  GemmChoice best = {1, 256, 1, (int)nk, (int)up(M, 256), (int)up(N, 256), 1e30};
+  GemmChoice best = {1, 256, 1, (int)nk, (int)up(M, 256), (int)cols(256), 1e30};
   for (int bn : {256, 224, 192, 128}) {
     if (bn == 224 && !quant) continue;   // (the eight epilogue warps of the dense kernel share 64-column runs)
-    const long long tiles = up(M, 256) * up(N, bn) * nb;
+    const long long tiles = up(M, 256) * cols(bn) * nb;
     const double c = (double)up(tiles, sms / 2) * nk * gemm_pair_step(bn, quant);
-    if (c < best.cycles) best = {1, bn, 1, (int)nk, (int)up(M, 256), (int)up(N, bn), c};
+    if (c < best.cycles) best = {1, bn, 1, (int)nk, (int)up(M, 256), (int)cols(bn), c};
   }
-  const long long tiles = up(M, 128) * up(N, 128) * nb;
+  const long long tiles = up(M, 128) * cols(128) * nb;
   const double step = quant ? 650 : 580;
   for (int r = 1; r <= 4; ++r) {
     const long long per = up(up(nk, r), 8) * 8;     // ranks start on 16-byte runs of the scales and on whole packed chunks
@@ -580,7 +602,7 @@ inline GemmChoice gemm_choose(int M, int N, int K, int nb, int sms, bool quant) 
     // clusters of three or four do not fill every SM: what is resident at once was 128 CTAs and more for four, not 144 for three
     const long long slots = r == 3 ? sms * 3 / 4 : r == 4 ? sms * 7 / 8 : sms;
     const double c = (double)up(tiles * r, slots) * (per * step + (r > 1 ? 4500 : 0));
-    if (c < best.cycles) best = {0, 128, r, (int)per, (int)up(M, 128), (int)up(N, 128), c};
+    if (c < best.cycles) best = {0, 128, r, (int)per, (int)up(M, 128), (int)cols(128), c};
   }
   return best;
 }
@@ -626,6 +648,28 @@ cudaError_t gemm_run(GemmArgs a, const Epi& epi, const void* x, long long x_pitc
   if constexpr (QB != 0)
     if (c.bn == 224) return gemm_launch<2, 224, QB, false>(mx, mw, a, epi, 1, sms, st);
   return c.bn == 192 ? gemm_launch<2, 192, QB, false>(mx, mw, a, epi, 1, sms, st) : gemm_launch<2, 128, QB, false>(mx, mw, a, epi, 1, sms, st);
+}
+
+// One x, up to three matrices of N[i] rows side by side (an Epi with SEGMENTS, whose maps and tile0 are filled in here).
+template <int QB, class Epi>
+cudaError_t gemm_run_segments(GemmArgs a, Epi epi, int n, const void* x, const uint32_t* const* w, int sms, cudaStream_t st) {
+  const GemmChoice c = gemm_choose(a.M, epi.N[0], a.K, 1, sms, true, n > 1 ? epi.N[1] : 0, n > 2 ? epi.N[2] : 0);
+  a.mt = c.mt; a.nt = c.nt; a.k_per = c.k_per; a.group_m = 8;
+  const int bn = c.pair ? c.bn : 128;
+  const long long w_row = (long long)a.K * QB / 8;
+  CUtensorMap mx, mw;
+  if (!gemm_map(&mx, x, 2, a.K, a.M, (long long)a.K * 2, 1, 0, 128)) return cudaErrorNotSupported;
+  for (int i = 0, t = 0; i < 3; ++i) {
+    epi.tile0[i] = i < n ? t : 0x7fffffff;
+    if (i >= n) continue;
+    if (!gemm_map(i == 0 ? &mw : &epi.map_more[i - 1], w[i], 1, w_row, epi.N[i], w_row, 1, 0, c.pair ? bn / 2 : bn)) return cudaErrorNotSupported;
+    t += (epi.N[i] + bn - 1) / bn;
+  }
+  if (!c.pair)
+    return c.ranks == 1 ? gemm_launch<1, 128, QB, false>(mx, mw, a, epi, 1, sms, st) : gemm_launch<1, 128, QB, true>(mx, mw, a, epi, c.ranks, sms, st);
+  if (bn == 256) return gemm_launch<2, 256, QB, false>(mx, mw, a, epi, 1, sms, st);
+  if (bn == 224) return gemm_launch<2, 224, QB, false>(mx, mw, a, epi, 1, sms, st);
+  return bn == 192 ? gemm_launch<2, 192, QB, false>(mx, mw, a, epi, 1, sms, st) : gemm_launch<2, 128, QB, false>(mx, mw, a, epi, 1, sms, st);
 }
 
 // Two products of one x in pairs' tiles (an Epi with PAIRED), of 256, 192 or 128 columns.  bn = 0: not worth it.

@@ -120,6 +120,8 @@ cudaError_t launch_fa_prefill_umma(uint16_t* out, const uint16_t* q, const uint1
                                    int B, int Hq, int Hkv, int L, int D, int offset, float scale, cudaStream_t st);
 cudaError_t launch_qmm_swiglu(uint16_t* y, const uint16_t* x, const uint32_t* const* wq, const uint16_t* const* s, const uint16_t* const* b,
                               int M, int N, int K, int bits, cudaStream_t st);
+cudaError_t launch_qmm_rows(uint16_t* y, int ld, const uint16_t* x, const pie_qmv_seg* segs, int n, const uint16_t* residual, int M, int K, int bits,
+                            cudaStream_t st);
 bool qmm_swiglu_pays(int M, int N, int K);
 double qmm_estimate_us(int M, int N, int K, int dual);
 // some dozens of activation rows, weights through tensor memory (pie_qmt.cuh, compiled with pie_qmm.cu, whose pipeline word it shares)

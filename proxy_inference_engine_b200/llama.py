@@ -141,6 +141,12 @@ class Attention(nn.Module):
         # tensor parallel: o_proj holds a K slice; the ranks' partial sums meet in one all-reduce (tp.py)
         return all_reduce_sum(self.o_proj(output), getattr(self, "tp", None))
 
+    def attend_beside(self, qkv, x, mask, cache):
+        """attend() of projections that lie side by side in rows."""
+        B, L, _ = x.shape
+        nq, nk = self.q_proj.weight.shape[0], self.k_proj.weight.shape[0]
+        return self.attend(qkv[..., :nq], qkv[..., nq:nq + nk], qkv[..., nq + nk:], B, L, mask, cache)
+
     def attend(self, queries, keys, values, B: int, L: int, mask, cache):
         """Rotation, cache update and attention of projected rows [B, L, heads * D] -> [B, L, Hq * D]."""
         queries = queries.reshape(B, L, self.num_heads, -1).transpose(1, 2)
@@ -166,14 +172,17 @@ class MLP(nn.Module):
         self.up_proj = mk(args.hidden_size, args.intermediate_size)
 
     def __call__(self, x):
-        act = nn.fused_rows(x, (self.gate_proj, self.up_proj), swiglu=True)
+        act, y = nn.fused_rows(x, (self.gate_proj, self.up_proj), swiglu=True), None
         if act is not None:
             y = nn.fused_rows(act, (self.down_proj,))
-            return all_reduce_sum(self.down_proj(act) if y is None else y, getattr(self, "tp", None))
+        else:
+            act = self.activations(x)
+        return all_reduce_sum(self.down_proj(act) if y is None else y, getattr(self, "tp", None))
+
+    def activations(self, x):
+        """silu(gate) * up of a prompt's rows."""
         act = nn.fused_swiglu(x, self.gate_proj, self.up_proj)
-        if act is None:
-            act = ops.silu_mul(self.gate_proj(x), self.up_proj(x))
-        return all_reduce_sum(self.down_proj(act), getattr(self, "tp", None))
+        return ops.silu_mul(self.gate_proj(x), self.up_proj(x)) if act is None else act
 
 
 class TransformerBlock(nn.Module):
@@ -187,24 +196,46 @@ class TransformerBlock(nn.Module):
         y = self._few_rows(x, mask, cache)
         if y is not None:
             return y
+        y = self._prompt_rows(x, mask, cache)
+        if y is not None:
+            return y
         r = self.self_attn(self.input_layernorm(x), mask, cache)
         h = ops.add(x, r)
         r = self.mlp(self.post_attention_layernorm(h))
         return ops.add(h, r)
 
+    def _alone(self, x) -> bool:
+        """The layer is these classes' own and one GPU's."""
+        at = self.self_attn
+        tp = getattr(at, "tp", None)
+        return type(at) is Attention and type(self.mlp) is MLP and not (tp is not None and tp.on) and x.dim() == 3
+
+    def _prompt_rows(self, x, mask, cache):
+        """A prompt on one GPU: q, k and v in one launch, residual sums in the matmuls in front of them.  None where that does not apply."""
+        at, mlp = self.self_attn, self.mlp
+        if x.numel() <= 128 * x.shape[-1] or not self._alone(x):   # (up to 128 rows the feed-forward may go with the few)
+            return None
+        qkv = nn.fused_prompt(self.input_layernorm(x), (at.q_proj, at.k_proj, at.v_proj))
+        if qkv is None:
+            return None
+        out = at.attend_beside(qkv, x, mask, cache)
+        h = nn.fused_prompt(out, (at.o_proj,), residual=x)
+        if h is None:
+            h = ops.add(x, at.o_proj(out))
+        act = mlp.activations(self.post_attention_layernorm(h))
+        y = nn.fused_prompt(act, (mlp.down_proj,), residual=h)
+        return ops.add(h, mlp.down_proj(act)) if y is None else y
+
     def _few_rows(self, x, mask, cache):
         """Few rows on one GPU: norms, residual sums and SwiGLU ride in the four quantized matmuls (nn.fused_rows).  None where
         they do not apply."""
         at, mlp = self.self_attn, self.mlp
-        tp = getattr(at, "tp", None)
-        if type(at) is not Attention or type(mlp) is not MLP or (tp is not None and tp.on) or x.dim() != 3:
+        if not self._alone(x):
             return None
         qkv = nn.fused_rows(x, (at.q_proj, at.k_proj, at.v_proj), norm=self.input_layernorm)
         if qkv is None:
             return None
-        B, L, _ = x.shape
-        nq, nk = at.q_proj.weight.shape[0], at.k_proj.weight.shape[0]
-        out = at.attend(qkv[..., :nq], qkv[..., nq:nq + nk], qkv[..., nq + nk:], B, L, mask, cache)
+        out = at.attend_beside(qkv, x, mask, cache)
         h = nn.fused_rows(out, (at.o_proj,), residual=x)
         if h is None:
             h = ops.add(x, at.o_proj(out))

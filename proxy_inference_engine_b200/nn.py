@@ -134,6 +134,24 @@ def fused_swiglu(x, gate, up):
     return ops.qmm_swiglu(x, gate, up, x.numel() // K, K)
 
 
+def fused_prompt(x, linears, residual=None):
+    """A prompt's rows (64 and more) through several bias-free QuantizedLinears in one launch, [..., sum N] their outputs side by side, and a
+    residual added to them: the bits of the separate calls.  None where that does not apply (the caller then makes those)."""
+    K = x.shape[-1]
+    if x.dtype != torch.bfloat16 or not x.is_contiguous() or K == 0 or K % 128 or x.numel() < 64 * K:
+        return None
+    bits, N = getattr(linears[0], "bits", None), 0
+    if bits not in (4, 8):
+        return None
+    for lin in linears:
+        if not _plain(lin, bits, K):
+            return None
+        N += lin.weight.shape[0]
+    if residual is not None and (residual.shape != x.shape[:-1] + (N,) or residual.dtype != torch.bfloat16 or not residual.is_contiguous()):
+        return None
+    return ops.qmm_rows(x, linears, x.numel() // K, K, N, residual)
+
+
 def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
     """Up to 32 rows, and up to 128 where that is sooner done, through several bias-free QuantizedLinears in ONE pass over their weights, with
     the RMSNorm in front of them, and the residual sum or SwiGLU behind them where asked for:

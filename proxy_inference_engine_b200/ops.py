@@ -244,6 +244,19 @@ def qmm_swiglu(x, gate, up, rows: int, K: int):
     return out
 
 
+def qmm_rows(x, linears, rows: int, K: int, N: int, residual):
+    """pie_qmm_rows on operands nn.fused_prompt has checked; None where the library leaves them to the separate calls."""
+    segs = (QmvSeg * len(linears))()
+    for seg, lin in zip(segs, linears):
+        seg.wq, seg.scales, seg.biases, seg.N = lin.weight.data_ptr(), lin.scales.data_ptr(), lin.biases.data_ptr(), lin.weight.shape[0]
+    out = torch.empty(x.shape[:-1] + (N,), dtype=_BF16, device=x.device)
+    status = _lib.load().pie_qmm_rows(_p(out), N, _p(x), segs, len(linears), _p(residual), rows, K, 64, linears[0].bits, _stream())
+    if status == _lib.EUNSUPPORTED:
+        return None
+    _lib.check(status, "qmm_rows")
+    return out
+
+
 def rms_norm(x, weight, eps: float):
     """mx.fast.rms_norm (MLX/mlx/fast.cpp:56-123): bf16(bf16(x * rsqrt(mean(x^2) + eps)) * weight)."""
     if x.dim() < 1:
