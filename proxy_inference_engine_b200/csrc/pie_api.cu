@@ -167,7 +167,8 @@ static bool qmt_pays(int M, long long n_total, int K, int bits, int dual) {
   const int mode = env_int("PIE_QMT", 1);
   if (mode != 1) return mode == 2;
   const long long tiles = dual ? (n_total + 63) / 64 : (n_total + 127) / 128, work = tiles * ((long long)K * bits / 1024);
-  if (M <= 8) return false;
+  // (3 to 8 rows so long that pie_qmv2.cu has no room for them beside its ring: 4096 x 14336, 5 rows 20.2 / 17.6)
+  if (M <= 8) return bits == 4 && M >= 3 && work >= 1500 && qmv2_smem_bytes(M, K) > (size_t)kQmvMaxSmem;
   if (M <= 32) return bits == 4 && work >= (M <= 16 ? 700 : 400);
   if (M < 64) return work >= 100;
   if (work < 700) return false;

@@ -153,7 +153,8 @@ __global__ void __launch_bounds__(1024) qmt_prep_kernel(uint8_t* img, float* rsc
   const int e = max((int)(top >> 7), 1) - 127;
   const int sh = top == 0 || e == 128 ? 0 : 4 - e;                       // -123 .. 130
   const float f1 = __int_as_float((127 + sh / 2) << 23), f2 = __int_as_float((127 + sh - sh / 2) << 23);
-  if (tid == 0) rscale[m] = ldexpf(1.f, -sh - 7);                        // 2^-137 at the least: a subnormal, and exact
+  // 2^-137 at the least: a subnormal, and exact.  A row with an infinity or a NaN has NaN for results, and nobody looks for a marked row there.
+  if (tid == 0) rscale[m] = e == 128 ? __int_as_float(0x7fffffff) : ldexpf(1.f, -sh - 7);
   const size_t slot_bytes = (size_t)np * 288;
 #pragma unroll
   for (int u = 0; u < U; ++u) {
@@ -595,8 +596,9 @@ __global__ void __launch_bounds__(kQtThreads, 1) qmt_kernel(const __grid_constan
             const uint32_t r4[4] = {rs.x, rs.y, rs.z, rs.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              if (c + 4 * q + e < rows) odd |= y[4 * q + e] != y[4 * q + e];
-              y[4 * q + e] *= __uint_as_float(r4[e]);
+              const float f = __uint_as_float(r4[e]);
+              if (c + 4 * q + e < rows) odd |= y[4 * q + e] != y[4 * q + e] && f == f;
+              y[4 * q + e] *= f;
             }
           }
           for (unsigned left_odd = __ballot_sync(0xffffffffu, odd && live); left_odd; left_odd &= left_odd - 1) {

@@ -463,7 +463,7 @@ class DecodeEngine:
                 n0 = ops.launch_count()
                 self._step_kernels()
                 self.launches_per_step = ops.launch_count() - n0
-        if self.B > 8:
+        if self.B > 2:
             self.watch.post()   # as a prompt's (steps of fewer rows have no such waits)
         for c in self.cache:
             c.offset += n
