@@ -71,7 +71,7 @@ class QuantizedLinear(Module):
             self.bias = torch.zeros((output_dims,), dtype=torch.bfloat16, device=device)
 
     def __call__(self, x):
-        if x.is_cuda:   # few rows: the bits of the call below, without its way through Python
+        if x.is_cuda and x.numel() <= 32 * x.shape[-1]:   # few rows: the bits of the call below, without its way through Python
             y = ops.native_fused_rows()(x, (self,), None, None, False, QuantizedLinear, RMSNorm, ops.qmv_workspace)
             if y is not None:
                 return y
@@ -164,12 +164,17 @@ def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
     sum of squares and the sums over K of several matrices are taken in another order, so that a value near a rounding boundary
     may fall on its other side.
     None where that kernel does not apply (the caller then makes the separate calls, which also report what is wrong)."""
+    K = x.shape[-1]
+    rows = x.numel() // K if K else 0
+    if rows > 32:   # most such calls are the separate ones', and find out before anything else is looked at
+        if rows > 128 or any(type(lin) is not QuantizedLinear for lin in linears):
+            return None
+        if not ops.qmt_scratch_bytes(rows, sum(lin.weight.shape[0] for lin in linears) // (2 if swiglu else 1), K, linears[0].bits, int(swiglu)):
+            return None
     if x.is_cuda:
         y = ops.native_fused_rows()(x, linears, norm, residual, swiglu, QuantizedLinear, RMSNorm, ops.qmv_workspace)
         if y is not None:
             return y
-    K = x.shape[-1]
-    rows = x.numel() // K if K else 0
     if not 0 < rows <= 128 or x.dtype != torch.bfloat16 or not x.is_contiguous() or x.data_ptr() % 16:
         return None
     bits, N = getattr(linears[0], "bits", None), 0
