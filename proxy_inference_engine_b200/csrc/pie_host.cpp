@@ -46,8 +46,12 @@ bool int_of(PyObject* v, long& out) {
   return true;
 }
 
+// The layers' tensors, held until the launch is queued: while the workspace is asked for, and while the launch waits without the lock, another thread
+// may put others in their place, and their memory would be some other tensor's.  (The arguments themselves are the caller's for as long as it calls.)
+using Held = c10::SmallVector<at::Tensor, 10>;
+
 // nn._plain, and the pointers
-bool segment(PyObject* lin, PyObject* type, long& bits, int64_t K, pie_qmv_seg& seg) {
+bool segment(PyObject* lin, PyObject* type, long& bits, int64_t K, pie_qmv_seg& seg, Held& held) {
   if ((PyObject*)Py_TYPE(lin) != type || entry(lin, s_bias)) return false;
   long b = 0, gs = 0;
   if (!int_of(entry(lin, s_bits), b) || !int_of(entry(lin, s_group_size), gs) || gs != 64 || (b != 4 && b != 8) || (bits && b != bits)) return false;
@@ -59,6 +63,7 @@ bool segment(PyObject* lin, PyObject* type, long& bits, int64_t K, pie_qmv_seg& 
       !w->is_contiguous() || !s->is_contiguous() || !z->is_contiguous() || w->size(0) > INT32_MAX)
     return false;
   seg = {(const uint32_t*)w->const_data_ptr(), s->const_data_ptr(), z->const_data_ptr(), (int)w->size(0)};
+  held.append({*w, *s, *z});
   return aligned(seg.wq, 16) && aligned(seg.scales, 8) && aligned(seg.biases, 8);
 }
 
@@ -74,10 +79,11 @@ PyObject* fused_rows(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (M < 1 || M > 128 || K > INT32_MAX || !aligned(x->const_data_ptr(), 16)) Py_RETURN_NONE;
   const bool swiglu = args[4] == Py_True;
   pie_qmv_seg segs[3];
+  Held held;
   long bits = 0;
   int64_t N = 0;
   for (Py_ssize_t i = 0; i < nseg; ++i) {
-    if (!segment(PyTuple_GET_ITEM(args[1], i), args[5], bits, K, segs[i])) Py_RETURN_NONE;
+    if (!segment(PyTuple_GET_ITEM(args[1], i), args[5], bits, K, segs[i], held)) Py_RETURN_NONE;
     N += segs[i].N;
   }
   if (K % (1024 / bits)) Py_RETURN_NONE;
@@ -95,6 +101,7 @@ PyObject* fused_rows(PyObject*, PyObject* const* args, Py_ssize_t n) {
         w->dim() != 1 || w->size(0) != K || !w->is_contiguous() || !aligned(w->const_data_ptr(), 16))
       Py_RETURN_NONE;
     norm_w = w->const_data_ptr();
+    held.push_back(*w);
     eps = PyFloat_AS_DOUBLE(e);
   }
   c10::SmallVector<int64_t, 6> shape(x->sizes().begin(), x->sizes().end());

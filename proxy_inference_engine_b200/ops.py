@@ -193,12 +193,20 @@ def quantized_matmul(x, w, scales, biases, transpose: bool = True, group_size: i
     return y.reshape(x.shape[:-1] + (N,))
 
 
+def _segments(linears):
+    """Segments of a launch, and the tensors they point into: held by the caller until the launch is queued, since another thread may put other
+    tensors in a layer's place meanwhile."""
+    held = [(lin.weight, lin.scales, lin.biases) for lin in linears]
+    segs = (QmvSeg * len(held))()
+    for seg, (w, s, b) in zip(segs, held):
+        seg.wq, seg.scales, seg.biases, seg.N = w.data_ptr(), s.data_ptr(), b.data_ptr(), w.shape[0]
+    return segs, held
+
+
 def qmv_fused(x, linears, rows: int, K: int, N: int, bits: int, norm_weight, eps: float, residual, swiglu: bool):
     """pie_qmt or pie_qmv_fused on operands nn.fused_rows has checked.  N: output columns.  None: more than 32 rows that pie_qmt does not serve."""
     L = _lib.load()
-    segs = (QmvSeg * len(linears))()
-    for seg, lin in zip(segs, linears):
-        seg.wq, seg.scales, seg.biases, seg.N = lin.weight.data_ptr(), lin.scales.data_ptr(), lin.biases.data_ptr(), lin.weight.shape[0]
+    segs, held = _segments(linears)
     out = torch.empty(x.shape[:-1] + (N,), dtype=_BF16, device=x.device)
     epilogue = EPI_SILUMUL if swiglu else EPI_STORE if residual is None else EPI_RESADD
     if _qmt(out, x, segs, len(linears), rows, K, N, bits, norm_weight, float(eps), epilogue, residual, int(swiglu)):
@@ -233,9 +241,7 @@ def qmm_swiglu_pays(rows: int, N: int, K: int, bits: int) -> bool:
 
 def qmm_swiglu(x, gate, up, rows: int, K: int):
     """pie_qmm_swiglu on operands nn.fused_swiglu has checked; None where the library leaves the shape to the separate calls."""
-    segs = (QmvSeg * 2)()
-    for seg, lin in zip(segs, (gate, up)):
-        seg.wq, seg.scales, seg.biases, seg.N = lin.weight.data_ptr(), lin.scales.data_ptr(), lin.biases.data_ptr(), lin.weight.shape[0]
+    segs, held = _segments((gate, up))
     out = torch.empty(x.shape[:-1] + (segs[0].N,), dtype=_BF16, device=x.device)
     status = _lib.load().pie_qmm_swiglu(_p(out), _p(x), segs, rows, K, 64, gate.bits, _stream())
     if status == _lib.EUNSUPPORTED:
@@ -246,9 +252,7 @@ def qmm_swiglu(x, gate, up, rows: int, K: int):
 
 def qmm_rows(x, linears, rows: int, K: int, N: int, residual):
     """pie_qmm_rows on operands nn.fused_prompt has checked; None where the library leaves them to the separate calls."""
-    segs = (QmvSeg * len(linears))()
-    for seg, lin in zip(segs, linears):
-        seg.wq, seg.scales, seg.biases, seg.N = lin.weight.data_ptr(), lin.scales.data_ptr(), lin.biases.data_ptr(), lin.weight.shape[0]
+    segs, held = _segments(linears)
     out = torch.empty(x.shape[:-1] + (N,), dtype=_BF16, device=x.device)
     status = _lib.load().pie_qmm_rows(_p(out), N, _p(x), segs, len(linears), _p(residual), rows, K, 64, linears[0].bits, _stream())
     if status == _lib.EUNSUPPORTED:

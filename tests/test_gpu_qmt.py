@@ -149,3 +149,32 @@ def test_the_native_host_form_is_the_python_one(bits, monkeypatch):
     assert native(x.float()) is None and native(x[:, ::2]) is None and native(x.t()) is None and native(x[:, :1024].contiguous()) is None
     assert native(x, lins[:1], None, x) is None and native(x, lins, lambda v: v) is None and native(x, list(lins)) is None
     assert torch.func.vmap(lambda v: torch.zeros(()) if native(v) is None else torch.ones(()))(x[:, None]).sum() == 0
+
+
+def test_a_call_holds_the_weights_it_was_made_with():
+    """Another thread may put other tensors in a layer's place while a call looks for its workspace: the memory of those the call has read about must
+    not be given to anybody before its launch is queued."""
+    from proxy_inference_engine_b200 import nn, ops
+    g = torch.Generator(device="cuda").manual_seed(5)
+    lin, norm, x = object.__new__(nn.QuantizedLinear), object.__new__(nn.RMSNorm), torch.randn((20, 2048), generator=g, device="cuda").bfloat16()
+    lin.group_size, lin.bits = 64, 4
+    norm.eps = 1e-5
+
+    def call(workspace):
+        torch.cuda.synchronize()
+        lin.weight, lin.scales, lin.biases = _matrix(torch.Generator(device="cuda").manual_seed(6), 512, 2048, 4)
+        norm.weight = torch.ones(2048, dtype=torch.bfloat16, device="cuda")
+        return ops.native_fused_rows()(x, (lin,), norm, None, False, nn.QuantizedLinear, nn.RMSNorm, workspace)
+
+    others, asked = [], []
+
+    def swap(nbytes, device):
+        asked.append(nbytes)
+        for owner, name in ((lin, "weight"), (lin, "scales"), (lin, "biases"), (norm, "weight")):
+            shape, dtype = getattr(owner, name).shape, getattr(owner, name).dtype
+            setattr(owner, name, None)
+            others.append(torch.ones(shape, dtype=dtype, device="cuda"))      # the allocator's next block of this size: the one given back, if any was
+        return ops.qmv_workspace(nbytes, device)
+
+    want, got = call(ops.qmv_workspace), call(swap)
+    assert asked and torch.equal(got, want)
