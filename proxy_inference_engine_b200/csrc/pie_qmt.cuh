@@ -5,8 +5,8 @@
 // The weights are the MMA's A operand (128 rows of the matrix a tile) and the activations its N side.  What bounds such a call is
 // the stream of packed weights and, close behind it, the instructions that turn a code into an operand, so that is kept short:
 //   * s (q - 8) of a 4-bit code has at most 11 significant bits (8 of a bf16 scale, 3 of q - 8): it IS an fp16 number.  A thread lifts
-//     two codes with one mask-or and an exact multiply-add or two: 11 instructions for eight codes, and K can run to its end
-//     in one fp32 accumulator of tensor memory -- no sums per group to be scaled and added afterwards.
+//     two codes with one mask-or and an exact multiply-add or two: 11 instructions for eight codes, and the products of many
+//     groups can run on in one fp32 accumulator of tensor memory -- no sums per group to be scaled and added afterwards.
 //   * an 8-bit code is two of them, q = 16 h + l: h against 16 x and l against x.  One kernel serves both; a matrix of 8-bit codes
 //     is a matrix of twice as many 4-bit ones, in the order the bytes have.
 //   * what is missing, (8 s + b) times the group's sum of x (136 s + b), is 16 more columns of K behind every 128 codes, the sum in three
@@ -48,6 +48,8 @@ struct QtArgs {
   int ntiles, ks;                 // tiles of 128 rows (dual: 64 and 64), stages of a tile
   int nw;                         // stages of packed rows
   int split;                      // > 0: a tile is this many CTAs', and a CTA has no part of a second one
+  int run;                        // turns that one accumulator takes; more are added in fp32
+  int totals_smem;                // where: tensor memory has no room for 32 columns more of turns of 256 codes
   int epi, out_ld;
   uint32_t mask0, mask1, magic0, magic1;   // of qt_word: as arguments, so that a mask-or is one instruction
   QtSeg seg[kMaxSeg];
@@ -226,6 +228,19 @@ __device__ __forceinline__ void qt_tma_2d(uint32_t dst, const CUtensorMap* map, 
 }
 __device__ __forceinline__ void qt_tmem_st4(uint32_t taddr, uint32_t u0, uint32_t u1, uint32_t u2, uint32_t u3) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%4], {%0,%1,%2,%3};" ::"r"(u0), "r"(u1), "r"(u2), "r"(u3), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void qt_tmem_st8(uint32_t taddr, const uint32_t (&u)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::"r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]),
+               "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void qt_tmem_st16(uint32_t taddr, const uint32_t (&u)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"(u[0]), "r"(u[1]),
+               "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]), "r"(u[9]), "r"(u[10]), "r"(u[11]), "r"(u[12]),
+               "r"(u[13]), "r"(u[14]), "r"(u[15]), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void qt_tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]),
+               "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr) : "memory");
 }
 // Issued by the lanes that say `go` (one), without a branch: inside one the operands would leave the uniform registers, and an MMA take
 // longer to issue than to run.
@@ -416,7 +431,8 @@ __global__ void __launch_bounds__(kQtThreads, 1) qmt_kernel(const __grid_constan
     const uint32_t idesc = (1u << 4) | ((uint32_t)(a.np >> 3) << 17) | ((128u >> 4) << 24);   // fp32 sums of fp16 products
     const uint32_t step_k = (uint32_t)(2 * a.np);   // 16 k of x, in 16-byte units
     const bool lead = elect_one();
-    int left = tile_turns - kk_lo * (2 / PER), sg = 0;   // turns to the end of the tile
+    int rest = tile_turns - kk_lo * (2 / PER), left = min(rest, a.run), sg = 0;   // turns to the end of the tile behind this accumulator's
+    rest -= left;
     uint32_t aph = 0, started = 0;
     bool alive = true;
     for (int t0 = 0; t0 < turns; t0 += 3, aph ^= 1) {
@@ -439,7 +455,9 @@ __global__ void __launch_bounds__(kQtThreads, 1) qmt_kernel(const __grid_constan
         if (--left == 0 || t0 + as + 1 == turns) {
           qt_commit_if(go, smem_u32(&acc_full[sg & 1]));
           started = 0;
-          left = tile_turns;
+          rest = rest ? rest : tile_turns;
+          left = min(rest, a.run);
+          rest -= left;
           ++sg;
         }
       }
@@ -514,11 +532,63 @@ __global__ void __launch_bounds__(kQtThreads, 1) qmt_kernel(const __grid_constan
     // come from L2, line by line, when the whole launch waits for these warps.
     bool dry = true;
     while (left > 0) {
-      const int take = min(left, a.ks - kk), b = sg & 1, rows = dry ? 0 : a.M;
+      const int take = min(left, a.ks - kk), rows = dry ? 0 : a.M;
       const bool whole = take == a.ks && !dry;
-      const bool ok = dry || gemm_wait_warp(smem_u32(&acc_full[b]), (sg >> 1) & 1, abortp);
+      // accumulators before the last: all are added up, in tensor memory behind the operands or in shared memory, and the sum takes the last one's
+      // place.  (Not in registers: with 32 more of them live some are spilled, and every call took 1 to 2 us longer.)
+      const int before = dry ? 0 : (take * (2 / PER) - 1) / a.run;
+      bool ok = true;
+      for (int j = 0;; ++j, ++sg) {
+        const uint32_t acc = tmem + (uint32_t)((sg & 1) * a.np) + lanes;
+        ok = dry || gemm_wait_warp(smem_u32(&acc_full[sg & 1]), (sg >> 1) & 1, abortp);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (before == 0) break;
+        const uint32_t kept = tmem + (uint32_t)(2 * a.np + 3 * TURN_COLS) + lanes, kept_s = smR + kQtMaxRows * 4 + (uint32_t)row * 4;
+        if constexpr (PER == 2) {
+#pragma unroll 1
+          for (int c = 0; c < a.np; c += 8) {
+            uint32_t v[8], t[8];   // (t, j = 0: not yet written, and not added)
+            qt_tmem_ld8(acc + c, v);
+            if (a.totals_smem) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q) t[q] = lds32(kept_s + (uint32_t)(c + q) * 512);
+            } else {
+              qt_tmem_ld8(kept + c, t);
+            }
+            tmem_ld_wait();
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              if (j > 0) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(t[q]));
+            if (a.totals_smem && j < before) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q) sts32(kept_s + (uint32_t)(c + q) * 512, v[q]);
+            } else {
+              qt_tmem_st8((j == before ? acc : kept) + c, v);
+            }
+          }
+        } else {
+#pragma unroll 1
+          for (int c = 0; c < a.np; c += 16) {
+            uint32_t v[16], t[16];
+            tmem_ld16(acc + c, v);
+            tmem_ld16(kept + c, t);
+            tmem_ld_wait();
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+              if (j > 0) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(t[q]));
+            qt_tmem_st16((j == before ? acc : kept) + c, v);
+          }
+        }
+        tmem_st_wait();
+        if (j == before) break;
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[sg & 1]);
+      }
       if (!qt_results_and(ok)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int b = sg & 1;
       const QtAt at = qt_tile(a, tile);
       const QtSeg& seg = a.seg[a.dual ? quad >> 1 : at.si];
       const int n = at.n0 + (a.dual ? row & 63 : row);
@@ -575,16 +645,16 @@ __global__ void __launch_bounds__(kQtThreads, 1) qmt_kernel(const __grid_constan
             const float4* part = reinterpret_cast<const float4*>(a.part) + (size_t)(2 * c0 + second) * a.np * 32 + (size_t)(c / 4) * 128 + row;
             const float4* const rest = part + (size_t)(2 - second) * a.np * 32;
 #pragma unroll 1
-            for (int p = 0; p < nparts; p += 3) {   // three parts' loads in flight
-              float4 v[3][4];
+            for (int p = 0; p < nparts; p += 2) {   // two parts' loads in flight
+              float4 v[2][4];
 #pragma unroll
-              for (int u = 0; u < 3; ++u) {
+              for (int u = 0; u < 2; ++u) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) v[u][q] = p + u < nparts ? __ldcg(part + q * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
                 part = p + u == 0 ? rest : part + (size_t)a.np * 64;
               }
 #pragma unroll
-              for (int u = 0; u < 3; ++u)
+              for (int u = 0; u < 2; ++u)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) { y[4 * q] += v[u][q].x; y[4 * q + 1] += v[u][q].y; y[4 * q + 2] += v[u][q].z; y[4 * q + 3] += v[u][q].w; }
             }
@@ -719,7 +789,14 @@ cudaError_t launch_qmt(void* out, int out_ld, const void* x, int x_ld, int M, in
   a.epi = epi; a.out_ld = out_ld; a.out = (uint16_t*)out; a.residual = (const uint16_t*)residual;
   a.mask0 = 0x000f000fu; a.mask1 = 0x00f000f0u; a.magic0 = 0x64006400u; a.magic1 = 0x54005400u;
   const int per = 2 * a.np + 6 * kQtCols <= 512 ? 2 : 1;   // tensor memory has the room for turns of 256 codes
-  const int fixed = 1024 + 3 * per * a.np * 288 + 4096 + 512, room = (kQtSmem - fixed) / kQtStage;
+  // The tensor core cuts the sums it returns, towards zero.  What that makes before the rounding to bf16, measured on products that are next to zero (rms,
+  // of a usual product's size): one accumulator for all of K 1.8e-6 at K 4096 and 8.0e-6 at 14336, a new one every 2048 codes 8.8e-7 and 1.0e-6, every 1024
+  // 3.8e-7 and 5.0e-7; the mma.sync GEMV, which has chains of four, 1.4e-6 and 1.1e-6.  So 1024 codes, and the sums added in fp32 (us, one accumulator / this:
+  // 2 x 14336 x 4096 with SwiGLU 16 rows 26.4 / 27.0, 32 31.2 / 32.4; 128256 x 4096, 16 rows 72.6 / 74.4).  65 rows and more, which the tile kernel would
+  // serve with one accumulator and rounded weights, keep one: at 112 tensor memory has no room for totals.
+  a.run = a.np <= 64 ? 8 / per : 1 << 30;
+  a.totals_smem = a.np <= 64 && 3 * a.np + 3 * per * kQtCols > 512;
+  const int fixed = 1024 + 3 * per * a.np * 288 + 4096 + kQtMaxRows * 4 + (a.totals_smem ? a.np * 512 : 0), room = (kQtSmem - fixed) / kQtStage;
   a.nw = room < kQtMaxStages ? room : kQtMaxStages;
   const size_t smem = (size_t)fixed + (size_t)a.nw * kQtStage;
   uint8_t* p = (uint8_t*)ws;

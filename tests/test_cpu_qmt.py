@@ -14,7 +14,7 @@ COLS, STAGE, SMEM = 72, 128 * 160, 226 * 1024      # kQtCols, kQtStage, kQtSmem
 def geometry(np_):
     """(turn size, stages) as launch_qmt takes them."""
     per = 2 if 2 * np_ + 6 * COLS <= 512 else 1
-    fixed = 1024 + 3 * per * np_ * 288 + 4096 + 512
+    fixed = 1024 + 3 * per * np_ * 288 + 4096 + 512 + (np_ * 512 if np_ == 32 else 0)
     stages = min(12, (SMEM - fixed) // STAGE)
     assert 2 * np_ + 3 * per * COLS <= 512 and fixed + stages * STAGE <= SMEM
     return per, stages
@@ -24,7 +24,7 @@ def test_the_constants_are_the_kernels():
     with open(HEADER) as f:
         text = f.read()
     assert "constexpr int kQtCols = 72;" in text and re.search(r"kQtPacked = 128 \* 128;", text) and "kQtPacked + 2 * 128 * 16;" in text
-    assert "constexpr int kQtSmem = 226 * 1024;" in text and "1024 + 3 * per * a.np * 288 + 4096 + 512" in text
+    assert "constexpr int kQtSmem = 226 * 1024;" in text and "1024 + 3 * per * a.np * 288 + 4096 + kQtMaxRows * 4 + (a.totals_smem ? a.np * 512 : 0)" in text
 
 
 def test_operands_are_exact():
@@ -179,3 +179,40 @@ def test_shares_cover_the_work_and_parts_are_found_again():
         assert len(slots) == len(set(slots)) and all(0 <= s < 2 * 148 for s in slots)
         for t, v in stored.items():
             assert parts[t] == v
+
+
+def test_accumulators_change_hands_at_the_same_turns():
+    """The MMA warp's count of turns and the result warps' count of accumulators of a tile: the same runs, in the same order, whatever a CTA's share."""
+    rng = random.Random(2)
+    with open(HEADER) as f:
+        text = f.read()
+    assert "a.run = a.np <= 64 ? 8 / per : 1 << 30;" in text and "const int before = dry ? 0 : (take * (2 / PER) - 1) / a.run;" in text
+    for np_ in range(16, 129, 16):
+        per, _ = geometry(np_)
+        run = 8 // per if np_ <= 64 else 1 << 30
+        assert (3 * np_ + 3 * per * COLS > 512) == (np_ == 32 or np_ > 96) and per == (2 if np_ <= 32 else 1)    # totals of 32 rows: in shared memory
+        for _ in range(60):
+            ks = 2 * rng.randint(1, 64)
+            lo = rng.randint(0, 5 * ks - 1)
+            hi = rng.randint(lo + 1, 5 * ks)
+            turns, tile_turns = (hi - lo) * 2 // per, ks * 2 // per
+            mma, rest, n = [], tile_turns - lo % ks * 2 // per, 0
+            left = min(rest, run)
+            rest -= left
+            for t in range(turns):
+                left, n = left - 1, n + 1
+                if left == 0 or t + 1 == turns:
+                    mma.append((t + 1, n))
+                    n, rest = 0, rest or tile_turns
+                    left = min(rest, run)
+                    rest -= left
+            results, done, kk, todo = [], 0, lo % ks, hi - lo
+            while todo:
+                take = min(todo, ks - kk)
+                before = (take * 2 // per - 1) // run
+                sizes = [run] * before + [take * 2 // per - before * run]
+                for size in sizes:
+                    done += size
+                    results.append((done, size))
+                todo, kk = todo - take, 0
+            assert mma == results and all(0 < n <= run for _, n in mma)

@@ -151,6 +151,46 @@ def test_the_native_host_form_is_the_python_one(bits, monkeypatch):
     assert torch.func.vmap(lambda v: torch.zeros(()) if native(v) is None else torch.ones(()))(x[:, None]).sum() == 0
 
 
+def _near_zero_targets(g, M, K, w):
+    """x [M, K] whose product with row m of w is far below the sums it is made of: what comes out is the sums' own error, which no rounding of
+    the result hides.  Projected off w's row first, then corrected in one small element after the other."""
+    x, rows = torch.randn((M, K), generator=g, device="cuda"), w[:M]
+    x = (x.double() - (x.double() * rows).sum(1, keepdim=True) / (rows * rows).sum(1, keepdim=True) * rows).bfloat16()
+    at = torch.arange(M, device="cuda")
+    for _ in range(6):
+        r = (x.double() * rows).sum(1)
+        k = torch.where(rows.abs() >= rows.abs().median(), x.double().abs(), torch.inf).argmin(1)
+        x[at, k] = (x[at, k].double() - r / rows[at, k]).bfloat16()
+    return x
+
+
+@pytest.mark.parametrize("bits,M,K", [(4, 9, 512), (4, 16, 4096), (4, 32, 1536), (4, 32, 14336), (4, 48, 14336), (4, 63, 4608), (8, 48, 8192)])
+def test_sums_are_no_further_off_than_the_gemvs(bits, M, K, monkeypatch):
+    """Before their rounding to bf16, over a tile's whole K in one CTA (as many tiles as SMs).  The tensor core cuts the sums it returns, towards zero: with
+    one accumulator for all of K they were off by 1.8e-6 of a product's size at K 4096 and 8.0e-6 at 14336, the GEMV by 1.1e-6 to 1.4e-6 at every K."""
+    from proxy_inference_engine_b200 import _lib
+    L, N = _lib.load(), 128 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(M + K + bits)
+    m = _matrix(g, N, K, bits)
+    w = _dense([t[:128] for t in m], bits)
+    size = float((torch.randn((64, K), generator=g, device="cuda").double() @ w.t()).norm() / (64 * 128) ** 0.5)      # of a product of N(0, 1) rows
+    mine, theirs = [], []
+    for _ in range(3):
+        x = _near_zero_targets(g, M, K, w)
+        ref = (x.double() * w[:M]).sum(1)
+        assert ref.abs().max() < 2e-5 * size                              # its rounding to bf16: at most 4e-8 of a product's size
+        monkeypatch.setenv("PIE_QMT", "2")
+        mine.append(_call(x, [m], bits).diagonal().double() - ref)
+        monkeypatch.setenv("PIE_QMT", "0")
+        y, nb = torch.empty((M, N), dtype=torch.bfloat16, device="cuda"), L.pie_qmv_workspace_bytes(M, N, K, bits, 0, 0)
+        ws = torch.zeros(max(nb, 256), dtype=torch.uint8, device="cuda")
+        _lib.check(L.pie_qmv(y.data_ptr(), x.data_ptr(), *(t.data_ptr() for t in m), M, N, K, 64, bits, ws.data_ptr(), ws.numel(),
+                             torch.cuda.current_stream().cuda_stream), "qmv")
+        theirs.append(y.diagonal().double() - ref)
+    off = [float(torch.cat(v).square().mean().sqrt()) / size for v in (mine, theirs)]
+    assert off[0] <= off[1] and off[0] < 1e-6, off
+
+
 def test_a_call_holds_the_weights_it_was_made_with():
     """Another thread may put other tensors in a layer's place while a call looks for its workspace: the memory of those the call has read about must
     not be given to anybody before its launch is queued."""
