@@ -15,7 +15,8 @@
 //     through shared memory it would cost 2 bytes written and 2 read for each half byte that arrives, and that was the limit of
 //     the earlier kernels.
 // x as fp16: the preparing kernel (RMS norm of the rows where asked for) scales each row by the power of two that brings its
-// largest value into [16, 32), which is exact down to 2^-21 of it (2^-29 of it is the largest error below), and writes the rows in the order
+// largest value into [256, 512) (8 bits: [16, 32)), the most that a group's sum leaves room for, which is exact down to 2^-25 (2^-21) of it, and
+// 2^-33 (2^-29) of it is the largest error below; the GEMV, whose operands are 128 + q, loses 2^-17 of a group's largest value.  It writes the rows in the order
 // the codes are lifted in.  Scales from 6e-8 to 7 (or 0) and |b| < 512 fit; a row of the matrix with others is marked (its operand
 // becomes NaN) and summed in fp32 by the warp that finds the NaN: slow, and right.
 // Roles of a CTA (one an SM): warp 0 packed rows, scales and biases by TMA; warp 1 the prepared x by bulk copies; warp 2 MMAs; warps 4-7
@@ -151,11 +152,11 @@ __global__ void __launch_bounds__(1024) qmt_prep_kernel(uint8_t* img, float* rsc
   if (lane == 0) reinterpret_cast<uint32_t*>(red)[32 + warp] = top;
   __syncthreads();
   top = __reduce_max_sync(0xffffffffu, reinterpret_cast<uint32_t*>(red)[32 + lane]);
-  // x 2^sh has its largest value in [16, 32); infinities and NaN stay what they are
+  // x 2^sh has its largest value in [256, 512), or in [16, 32) where 16 x is to be a number as well; infinities and NaN stay what they are
   const int e = max((int)(top >> 7), 1) - 127;
-  const int sh = top == 0 || e == 128 ? 0 : 4 - e;                       // -123 .. 130
+  const int sh = top == 0 || e == 128 ? 0 : (BITS == 4 ? 8 : 4) - e;     // -123 .. 134
   const float f1 = __int_as_float((127 + sh / 2) << 23), f2 = __int_as_float((127 + sh - sh / 2) << 23);
-  // 2^-137 at the least: a subnormal, and exact.  A row with an infinity or a NaN has NaN for results, and nobody looks for a marked row there.
+  // 2^-141 at the least: a subnormal, and exact.  A row with an infinity or a NaN has NaN for results, and nobody looks for a marked row there.
   if (tid == 0) rscale[m] = e == 128 ? __int_as_float(0x7fffffff) : ldexpf(1.f, -sh - 7);
   const size_t slot_bytes = (size_t)np * 288;
 #pragma unroll

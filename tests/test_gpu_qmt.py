@@ -218,3 +218,15 @@ def test_a_call_holds_the_weights_it_was_made_with():
 
     want, got = call(ops.qmv_workspace), call(swap)
     assert asked and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("bits,M,K,top", [(4, 4, 14336, 23), (4, 16, 4096, 23), (4, 63, 1536, 23), (8, 40, 4096, 19)])
+def test_small_values_beside_a_large_one(bits, M, K, top, monkeypatch):
+    """2^top in a group of zero weights, in rows of N(0, 1): the others are what fp16 leaves them under the row's power of two, off by at most 2^-33 (8 bits:
+    2^-29) of the largest value, which makes 2^-10 / sqrt(3) = 5.6e-4 of a product, below the 1.95e-3 of its rounding: 2.03e-3 together."""
+    monkeypatch.setenv("PIE_QMT", "2")
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    m, x = _matrix(g, 256, K, bits), torch.randn((M, K), generator=g, device="cuda").bfloat16()
+    m[1][:, 0], m[2][:, 0] = 0, 0
+    x[:, 15] = 2.0 ** top
+    assert _rel(_call(x, [m], bits), x.double() @ _dense(m, bits).t()) < 2.1e-3
