@@ -18,7 +18,8 @@
 // largest value into [256, 512) (8 bits: [16, 32)), the most that a group's sum leaves room for, which is exact down to 2^-25 (2^-21) of it, and
 // 2^-33 (2^-29) of it is the largest error below; the GEMV, whose operands are 128 + q, loses 2^-17 of a group's largest value.  It writes the rows in the order
 // the codes are lifted in.  Scales from 6e-8 to 7 (or 0) and |b| < 512 fit; a row of the matrix with others is marked (its operand
-// becomes NaN) and summed in fp32 by the warp that finds the NaN: slow, and right.
+// becomes NaN) and summed in fp32 by the warp that finds the NaN: slow, and right.  A row of x with infinities is found the same way, and its results are
+// what they make of the weights' signs.
 // Roles of a CTA (one an SM): warp 0 packed rows, scales and biases by TMA; warp 1 the prepared x by bulk copies; warp 2 MMAs; warps 4-7
 // the results; warps 8-19 in three sets dequantise, 128 codes of 128 rows in turn.  The work, tiles x 256 codes, is dealt out evenly: a
 // CTA's share may begin and end inside a tile, and the CTA that comes last adds a tile's parts, in the order of K.
@@ -98,11 +99,17 @@ __device__ __forceinline__ void qt_pieces(float v, uint32_t& p0, uint32_t& p1, u
   p2 = qt_pack_f16(r - qt_f16lo(p1), 0.f) & 0xffffu;
 }
 
+// Where entry i of a row's list of infinities lies in its image: k, and bit 15 for a negative one.
+__device__ __forceinline__ size_t qt_list_at(unsigned int i, int np, int m) {
+  return (size_t)(i >> 7) * np * 288 + (size_t)((i >> 3 & 15) * np + m) * 16 + (i & 7) * 2;
+}
+
 // One CTA per row.  U: 8 * 1024 * U >= K.
 template <int BITS, int U>
 __global__ void __launch_bounds__(1024) qmt_prep_kernel(uint8_t* img, float* rscale, unsigned int* cnt, int ntiles, const uint16_t* x,
                                                         int x_ld, const uint16_t* norm_w, float eps, int np, int K) {
   __shared__ float red[64];
+  __shared__ unsigned int infinities;
   const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, chunks = K / 8;
   // the matmul may set itself up and ask for weights, which nothing queued before it writes any more, but reads nothing of this kernel
   pdl_wait();
@@ -156,8 +163,9 @@ __global__ void __launch_bounds__(1024) qmt_prep_kernel(uint8_t* img, float* rsc
   const int e = max((int)(top >> 7), 1) - 127;
   const int sh = top == 0 || e == 128 ? 0 : (BITS == 4 ? 8 : 4) - e;     // -123 .. 134
   const float f1 = __int_as_float((127 + sh / 2) << 23), f2 = __int_as_float((127 + sh - sh / 2) << 23);
-  // 2^-141 at the least: a subnormal, and exact.  A row with an infinity or a NaN has NaN for results, and nobody looks for a marked row there.
-  if (tid == 0) rscale[m] = e == 128 ? __int_as_float(0x7fffffff) : ldexpf(1.f, -sh - 7);
+  // 2^-141 at the least: a subnormal, and exact.  A row with a NaN has NaN for results, and nobody looks for a marked row there; one
+  // with infinities and none has their number here, negative, and a list of them for an image.
+  if (tid == 0 && top != 0x7f80u) rscale[m] = e == 128 ? __int_as_float(0x7fffffff) : ldexpf(1.f, -sh - 7);
   const size_t slot_bytes = (size_t)np * 288;
 #pragma unroll
   for (int u = 0; u < U; ++u) {
@@ -212,6 +220,26 @@ __global__ void __launch_bounds__(1024) qmt_prep_kernel(uint8_t* img, float* rsc
         *reinterpret_cast<uint4*>(at) = make_uint4(p0 | p1 << 16, p2 | q0 << 16, q1 | q2 << 16, r0 | r1 << 16);
         *reinterpret_cast<uint4*>(at + (size_t)np * 16) = make_uint4(r2, 0, 0, 0);
       }
+    }
+  }
+  if (top == 0x7f80u) {   // (what the MMAs make of a list stays in the row's own column)
+    __syncthreads();
+    if (tid == 0) infinities = 0;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t x4[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t b = j & 1 ? x4[j / 2] >> 16 : x4[j / 2] & 0xffffu;
+        if ((b & 0x7fffu) == 0x7f80u)
+          *reinterpret_cast<uint16_t*>(img + qt_list_at(atomicAdd(&infinities, 1u), np, m)) = (uint16_t)(((u * 1024 + tid) * 8 + j) | (b & 0x8000u));
+      }
+    }
+    __syncthreads();
+    if (tid == 0) {
+      *reinterpret_cast<uint16_t*>(img + (size_t)(16 * np + m) * 16) = 0x7fff;   // a group's sum: NaN for all results, which sends for the list
+      rscale[m] = -(float)infinities;
     }
   }
 }
@@ -314,14 +342,24 @@ __device__ __noinline__ bool qt_row_marked(const QtSeg& g, int K, int n) {
   }
   return __any_sync(0xffffffffu, hit);
 }
-// ... whose product with row m a warp sums here, a word of codes a lane at a time, from the prepared x
+// ... whose product with row m (scale f) a warp sums here, a word of codes a lane at a time, from the prepared x.  f < 0: the row has -f infinities,
+// and the product is theirs.
 template <int BITS>
-__device__ __noinline__ float qt_row_dot(const QtSeg& g, const uint8_t* img, int np, int K, int n, int m) {
+__device__ __noinline__ float qt_row_dot(const QtSeg& g, const uint8_t* img, int np, int K, int n, int m, float f) {
   constexpr int PER = 32 / BITS;
   float y = 0.f;
+  auto scale = [&](const uint16_t* p, int k) { return __uint_as_float((uint32_t)__ldg(p + (size_t)n * (K / kGroup) + k / kGroup) << 16); };
+  if (f < 0.f) {
+    for (int i = threadIdx.x & 31; i < (int)-f; i += 32) {
+      const uint32_t entry = __ldcg(reinterpret_cast<const uint16_t*>(img + qt_list_at(i, np, m)));
+      const int k = entry & 0x7fff;
+      const uint32_t q = __ldg(g.wq + (size_t)n * (K / PER) + k / PER) >> (BITS * (k % PER)) & ((1u << BITS) - 1);
+      y += fmaf(scale(g.s, k), (float)q, scale(g.b, k)) * (entry & 0x8000u ? -INFINITY : INFINITY);
+    }
+    return warp_sum(y);
+  }
   for (int i = threadIdx.x & 31; i < K / PER; i += 32) {
-    const size_t at = (size_t)n * (K / kGroup) + i * PER / kGroup;
-    const float s = __uint_as_float((uint32_t)__ldg(g.s + at) << 16), b = __uint_as_float((uint32_t)__ldg(g.b + at) << 16);
+    const float s = scale(g.s, i * PER), b = scale(g.b, i * PER);
     const uint32_t w = __ldg(g.wq + (size_t)n * (K / PER) + i);
     float d = 0.f, sx = 0.f;
     for (int j = 0; j < PER; ++j) {
@@ -333,7 +371,7 @@ __device__ __noinline__ float qt_row_dot(const QtSeg& g, const uint8_t* img, int
     }
     y += s * d + b * sx;
   }
-  return warp_sum(y);
+  return warp_sum(y) * (f * 128.f);
 }
 
 // PER: 128 codes a turn of the dequantisers, or twice as many
@@ -674,11 +712,13 @@ __global__ void __launch_bounds__(kQtThreads, 1) qmt_kernel(const __grid_constan
           }
           for (unsigned left_odd = __ballot_sync(0xffffffffu, odd && live); left_odd; left_odd &= left_odd - 1) {
             const int who = __ffs(left_odd) - 1, row_n = __shfl_sync(0xffffffffu, n, who);
-            if (!qt_row_marked(seg, a.K, row_n)) continue;   // the NaN is the caller's
+            const bool marked = qt_row_marked(seg, a.K, row_n);   // (if not, and no list: the NaN is the caller's)
 #pragma unroll
             for (int q = 0; q < 16; ++q)
               if (c + q < rows) {
-                const float d = qt_row_dot<BITS>(seg, a.img, a.np, a.K, row_n, c + q) * (__uint_as_float(lds32(smR + (uint32_t)(c + q) * 4)) * 128.f);
+                const float f = __uint_as_float(lds32(smR + (uint32_t)(c + q) * 4));
+                if (!marked && !(f < 0.f)) continue;
+                const float d = qt_row_dot<BITS>(seg, a.img, a.np, a.K, row_n, c + q, f);
                 if (lane == who) y[q] = d;
               }
           }

@@ -230,3 +230,25 @@ def test_small_values_beside_a_large_one(bits, M, K, top, monkeypatch):
     m[1][:, 0], m[2][:, 0] = 0, 0
     x[:, 15] = 2.0 ** top
     assert _rel(_call(x, [m], bits), x.double() @ _dense(m, bits).t()) < 2.1e-3
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("M,K", [(16, 512), (40, 4096), (64, 4096), (77, 14336), (128, 28672)])
+def test_rows_with_infinities(bits, M, K, monkeypatch):
+    """Infinities of one sign or of both, first and last of a row, against float64: an infinity times the weights' signs, NaN where they disagree or a weight
+    is zero; marked rows of the matrix among them, and the rows beside as they are without."""
+    monkeypatch.setenv("PIE_QMT", "2")
+    g = torch.Generator(device="cuda").manual_seed(M + K + bits)
+    m, x = _matrix(g, 200, K, bits), torch.randn((M, K), generator=g, device="cuda").bfloat16()
+    m[1][5, 0], m[2][9, 0] = 50.0, 1e5                                  # marked
+    m[1][:, 3], m[2][:, 3] = 0, 0                                       # weights of zero at k 192 .. 255
+    inf = float("inf")
+    y = _call(x, [m], bits)
+    x[0, 0], x[1, K - 1], x[2, 7], x[2, K // 2], x[3, 200], x[M - 1, :] = inf, -inf, inf, -inf, inf, inf
+    x[4, 11], x[4, 12] = inf, float("nan")
+    z, ref = _call(x, [m], bits).double(), x.double() @ _dense(m, bits).t()
+    hit = [0, 1, 2, 3, 4, M - 1]
+    assert torch.equal(z[hit].nan_to_num(0.0), ref[hit].nan_to_num(0.0)) and torch.equal(z[hit].isnan(), ref[hit].isnan())
+    assert z[0].isinf().all() and z[2].isnan().any() and z[2].isinf().any() and z[3].isnan().all()
+    rest = [r for r in range(M) if r not in hit]
+    assert torch.equal(z[rest], y[rest].double())
