@@ -177,7 +177,6 @@ class DecodeEngine:
         # per-layer segment tables (host structs must outlive the captured graph: keep references)
         self.seg_qkv, self.seg_o, self.seg_gu, self.seg_down = [], [], [], []
         nb = 0
-        mb = min(B, 32)
         for ly in model.layers:
             at, mlp = ly.self_attn, ly.mlp
             self.seg_qkv.append(_segs(at.q_proj, at.k_proj, at.v_proj))
@@ -192,7 +191,7 @@ class DecodeEngine:
         qd = self.Hq * self.D
         for (n, k, dual) in (((self.Hq + 2 * self.Hkv) * self.D, h, 0), (h, qd, 0), (a.intermediate_size, h, 1),
                              (h, a.intermediate_size, 0), (hw.shape[0], h, 0)):
-            nb = max(nb, L.pie_qmv_workspace_bytes(mb, n, k, self.bits, dual, 0))
+            nb = max(nb, L.pie_qmv_workspace_bytes(B, n, k, self.bits, dual, 0))
         self.qmv_ws = torch.zeros(max(nb, 256), dtype=torch.uint8, device=dev)
         self.graph = None
         self._next_pos = None

@@ -252,3 +252,17 @@ def test_rows_with_infinities(bits, M, K, monkeypatch):
     assert z[0].isinf().all() and z[2].isnan().any() and z[2].isinf().any() and z[3].isnan().all()
     rest = [r for r in range(M) if r not in hit]
     assert torch.equal(z[rest], y[rest].double())
+
+
+def test_a_decode_engine_has_room_for_it_at_more_than_32_rows():
+    """The workspace of a step of 40 rows holds what the tensor-memory matmul asks for with 40 rows, or the step would fall back to passes of 32."""
+    from parity_util import tiny_args
+    from proxy_inference_engine_b200 import _lib
+    from proxy_inference_engine_b200.decode import DecodeEngine
+    from proxy_inference_engine_b200.llama import Model
+    B, L = 40, _lib.load()
+    args = tiny_args(hidden_size=2048, intermediate_size=2048, num_hidden_layers=1, num_attention_heads=32, num_key_value_heads=8)
+    eng = DecodeEngine(Model(args), B, 64)
+    for n, k, dual in ((3072, 2048, 0), (2048, 2048, 0), (2048, 2048, 1)):
+        need = L.pie_qmt_scratch_bytes(B, n, k, 64, 4, dual)
+        assert need and eng.qmv_ws.numel() >= (128 << 10) + need
