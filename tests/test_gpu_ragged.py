@@ -112,3 +112,21 @@ def test_ragged_step_over_the_quantised_cache():
     for i, sid in enumerate((3, 4)):
         lo = o(np.asarray([seq[sid]], np.int32), o.make_cache(kv_bits=8), last_only=True)[0, -1]
         assert rel_l2(lg[i], lo) < TOL, sid
+
+
+@pytest.mark.parametrize("n", [1, 900, 40000])
+def test_a_steps_tables_reach_the_device_without_a_wait(n):
+    """... behind work that is still queued, from memory that may change at once, and with no page-locked block to be had for it."""
+    from proxy_inference_engine_b200.ragged import to_device
+    a, t = torch.randn((8192, 8192), device="cuda").bfloat16(), torch.arange(n, dtype=torch.int32)
+    to_device(t, "cuda"), torch.mm(a, a)
+    torch.cuda.synchronize()
+    torch._C._host_emptyCache()
+    blocks, queued = torch.cuda.host_memory_stats().get("num_host_alloc"), torch.cuda.Event()
+    for _ in range(20):
+        torch.mm(a, a)                                                  # about 15 ms
+    queued.record()
+    got = to_device(t, "cuda")
+    assert not queued.query()
+    t.fill_(-1)
+    assert got.tolist() == list(range(n)) and torch.cuda.host_memory_stats().get("num_host_alloc") == blocks
