@@ -211,14 +211,17 @@ class TransformerBlock(nn.Module):
         return type(at) is Attention and type(self.mlp) is MLP and not (tp is not None and tp.on) and x.dim() == 3
 
     def _prompt_rows(self, x, mask, cache):
-        """A prompt on one GPU: q, k and v in one launch, residual sums in the matmuls in front of them.  None where that does not apply."""
+        """A prompt on one GPU: q, k and v in one launch, residual sums in the matmuls in front of them, each where that applies.  None where
+        the layer is not that."""
         at, mlp = self.self_attn, self.mlp
         if x.numel() <= 128 * x.shape[-1] or not self._alone(x):   # (up to 128 rows the feed-forward may go with the few)
             return None
-        qkv = nn.fused_prompt(self.input_layernorm(x), (at.q_proj, at.k_proj, at.v_proj))
-        if qkv is None:
-            return None
-        out = at.attend_beside(qkv, x, mask, cache)
+        y = self.input_layernorm(x)
+        qkv = nn.fused_prompt(y, (at.q_proj, at.k_proj, at.v_proj))
+        if qkv is not None:
+            out = at.attend_beside(qkv, x, mask, cache)
+        else:
+            out = at.attend(at.q_proj(y), at.k_proj(y), at.v_proj(y), x.shape[0], x.shape[1], mask, cache)
         h = nn.fused_prompt(out, (at.o_proj,), residual=x)
         if h is None:
             h = ops.add(x, at.o_proj(out))

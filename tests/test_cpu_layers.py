@@ -196,3 +196,30 @@ def test_a_tensor_parallel_block_takes_the_separate_calls(monkeypatch):
     block.self_attn.tp = None
     block.mlp = lambda x: x
     assert block._few_rows(_bf16(1, 1, 512), None, None) is None
+
+
+@pytest.mark.parametrize("odd", [None, "bits", "wrapped"])
+def test_a_prompt_layer_norms_its_input_once(monkeypatch, odd):
+    """... whether or not its q, k and v go in one launch, and with the sums of the separate calls where they do not."""
+    from proxy_inference_engine_b200 import llama, nn
+    calls = []
+    monkeypatch.setattr(nn.RMSNorm, "__call__", lambda self, x: calls.append("norm") or x)
+    monkeypatch.setattr(nn.QuantizedLinear, "__call__", lambda self, x: calls.append("linear") or _bf16(*x.shape[:-1], self.weight.shape[0]))
+    monkeypatch.setattr(ops, "qmm_rows", lambda x, lins, rows, K, N, residual: calls.append(len(lins)) or _bf16(*x.shape[:-1], N))
+    monkeypatch.setattr(ops, "qmm_swiglu_pays", lambda *a: False)
+    monkeypatch.setattr(ops, "silu_mul", lambda g, u: g)
+    monkeypatch.setattr(ops, "add", lambda a, b: a + b)
+    monkeypatch.setattr(llama.Attention, "attend", lambda self, q, k, v, B, L, mask, cache: _bf16(B, L, q.shape[-1]))
+    at, mlp = object.__new__(llama.Attention), object.__new__(llama.MLP)
+    at.q_proj, at.k_proj, at.v_proj, at.o_proj = _plain(512), _plain(256), _plain(256), _plain(512)
+    mlp.gate_proj, mlp.up_proj, mlp.down_proj = _plain(512), _plain(512), _plain(512)
+    if odd == "bits":
+        at.v_proj = _plain(256, bits=8)
+    if odd == "wrapped":
+        at.k_proj = lambda x, inner=at.k_proj: inner(x)
+    layer = object.__new__(llama.TransformerBlock)
+    layer.self_attn, layer.mlp = at, mlp
+    layer.input_layernorm, layer.post_attention_layernorm = object.__new__(nn.RMSNorm), object.__new__(nn.RMSNorm)
+    x = _bf16(1, 200, 512)
+    assert layer(x).shape == x.shape and calls.count("norm") == 2
+    assert calls == ["norm"] + ([3] if odd is None else ["linear"] * 3) + [1, "norm", "linear", "linear", 1]
