@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import subprocess
+import sys
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("PIE_LIB") or os.path.join(_HERE, "libpie_b200.so")  # PIE_LIB: experiment builds
@@ -302,7 +303,7 @@ def build(verbose: bool = False, target: str = "all") -> str:
     out = None if verbose else subprocess.DEVNULL
     with open(os.path.join(CSRC, ".build.lock"), "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
-        subprocess.check_call(["make", "-s", "-j8", "-C", CSRC, target], stdout=out)
+        subprocess.check_call(["make", "-s", "-j8", "-C", CSRC, target, "PYTHON=" + sys.executable], stdout=out)
     return LIB_PATH
 
 

@@ -11,6 +11,7 @@ import ctypes as C
 import functools
 import importlib.util
 import os
+import warnings
 
 import torch
 
@@ -221,14 +222,18 @@ def qmv_fused(x, linears, rows: int, K: int, N: int, bits: int, norm_weight, eps
 
 @functools.cache
 def native_fused_rows():
-    """csrc/pie_host.cpp's form of nn.fused_rows, which takes the common calls and answers None to the others; where it was not built: None to
-    every call."""
+    """csrc/pie_host.cpp's form of nn.fused_rows, which takes the common calls and answers None to the others; where it was not built, or for another torch or
+    interpreter, so that it does not load: None to every call."""
     path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_pie_host.so")
     if not os.path.exists(path):
         return lambda *args: None
-    spec = importlib.util.spec_from_file_location("_pie_host", path)
-    host = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(host)
+    try:
+        spec = importlib.util.spec_from_file_location("_pie_host", path)
+        host = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(host)
+    except (ImportError, OSError) as e:
+        warnings.warn(f"{path} does not load ({e}): build it again with make -C {_lib.CSRC}.  Calls of few rows take the Python form meanwhile.")
+        return lambda *args: None
     L = _lib.load()
     host.bind(*(C.cast(fn, C.c_void_p).value for fn in (L.pie_qmv_fused, L.pie_qmv_workspace_bytes, L.pie_qmt, L.pie_qmt_scratch_bytes)))
     return host.fused_rows

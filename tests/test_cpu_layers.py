@@ -223,3 +223,19 @@ def test_a_prompt_layer_norms_its_input_once(monkeypatch, odd):
     x = _bf16(1, 200, 512)
     assert layer(x).shape == x.shape and calls.count("norm") == 2
     assert calls == ["norm"] + ([3] if odd is None else ["linear"] * 3) + [1, "norm", "linear", "linear", 1]
+
+
+def test_a_host_module_that_does_not_load_leaves_the_calls_to_python(monkeypatch):
+    """... as one that was built for another torch or interpreter does: a warning, once, and no answer to any call."""
+    def refuse(*args):
+        raise ImportError("undefined symbol")
+    ops.native_fused_rows.cache_clear()
+    try:
+        with monkeypatch.context() as m:
+            m.setattr(ops.os.path, "exists", lambda path: True)
+            m.setattr(ops.importlib.util, "module_from_spec", refuse)
+            with pytest.warns(UserWarning, match="does not load"):
+                assert ops.native_fused_rows()(1, 2, 3) is None
+            assert ops.native_fused_rows()(1, 2, 3) is None
+    finally:
+        ops.native_fused_rows.cache_clear()
