@@ -188,8 +188,6 @@ def fused_rows(x, linears, norm=None, residual=None, swiglu: bool = False):
         if linears[0].weight.shape[0] != linears[1].weight.shape[0]:
             return None
         N //= 2
-    if rows > 32 and not ops.qmt_scratch_bytes(rows, N, K, bits, int(swiglu)):
-        return None
     if norm is not None:
         if type(norm) is not RMSNorm:
             return None

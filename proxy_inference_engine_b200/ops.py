@@ -35,9 +35,8 @@ def _qmv_workspace_bytes(M: int, N: int, K: int, bits: int, dual: int) -> int:
     return _lib.load().pie_qmv_workspace_bytes(M, N, K, bits, dual, 0)
 
 
-@functools.lru_cache(maxsize=4096)
 def qmt_scratch_bytes(M: int, N: int, K: int, bits: int, dual: int) -> int:
-    """0: the call is not for pie_qmt.  (A pure function of the sizes.)"""
+    """0: the call is not for pie_qmt.  (Asked each time: it is the current device's answer.)"""
     return _lib.load().pie_qmt_scratch_bytes(M, N, K, 64, bits, dual) if 0 < M <= 128 else 0
 
 

@@ -239,3 +239,12 @@ def test_a_host_module_that_does_not_load_leaves_the_calls_to_python(monkeypatch
             assert ops.native_fused_rows()(1, 2, 3) is None
     finally:
         ops.native_fused_rows.cache_clear()
+
+
+def test_the_matmuls_route_is_asked_for_at_every_call(monkeypatch):
+    """PIE_QMT and the current device may change between two calls: the Python form answers as the library, and so as the native form, does."""
+    answers = []
+    for mode in ("2", "0", "2"):
+        monkeypatch.setenv("PIE_QMT", mode)
+        answers.append(ops.qmt_scratch_bytes(40, 2048, 2048, 4, 0))
+    assert answers[0] == answers[2] > 0 == answers[1]

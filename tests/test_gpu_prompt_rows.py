@@ -24,7 +24,6 @@ def test_one_launch_has_the_bits_of_its_products(monkeypatch, bits, M, K, widths
     from proxy_inference_engine_b200 import nn, ops
     from proxy_inference_engine_b200._lib import load
     monkeypatch.setenv("PIE_QMT", "0")                 # the separate calls on the same kernel at 64 to 128 rows, too
-    ops.qmt_scratch_bytes.cache_clear()
     g = torch.Generator(device="cuda").manual_seed(M + K + bits)
     x, lins = torch.randn((M, K), generator=g, device="cuda").bfloat16(), tuple(_layer(g, n, K, bits) for n in widths)
     want = torch.cat([ops.quantized_matmul(x, l.weight, l.scales, l.biases, bits=bits) for l in lins], 1)
@@ -38,4 +37,3 @@ def test_one_launch_has_the_bits_of_its_products(monkeypatch, bits, M, K, widths
     assert torch.equal(alone, want[:, :widths[0]])     # the choice of a matrix alone: the same bits
     res = torch.randn((M, widths[0]), generator=g, device="cuda").bfloat16()
     assert torch.equal(nn.fused_prompt(x, lins[:1], residual=res), ops.add(res, alone))
-    ops.qmt_scratch_bytes.cache_clear()
