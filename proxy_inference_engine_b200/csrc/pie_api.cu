@@ -277,9 +277,11 @@ int pie_qmv_fused_tp(void* out, int out_ld, const void* x, int x_ld, int M, int 
       long long n_total = 0;
       for (int i = 0; i < nseg; ++i) n_total += segs[i].N;
       if (a.dual) n_total = segs[0].N;
-      if (workspace && qmt_pays(M, n_total, K, bits, a.dual) && kWsCntBytes + qmt_scratch(M, n_total, K, group_size, bits, a.dual) <= workspace_bytes)
-        return cuda_status(launch_qmt(out, out_ld, x, x_ld, M, K, segs, nseg, bits, norm_weight, eps, epilogue, residual,
-                                      (uint8_t*)workspace + kWsCntBytes, (cudaStream_t)stream));
+      if (workspace && qmt_pays(M, n_total, K, bits, a.dual) && kWsCntBytes + qmt_scratch(M, n_total, K, group_size, bits, a.dual) <= workspace_bytes) {
+        const cudaError_t e = launch_qmt(out, out_ld, x, x_ld, M, K, segs, nseg, bits, norm_weight, eps, epilogue, residual,
+                                         (uint8_t*)workspace + kWsCntBytes, (cudaStream_t)stream);
+        if (e != cudaErrorNotSupported) return cuda_status(e);   // (a tensor map that cannot be made: nothing was launched, and the others below need none)
+      }
     }
     // TMA-fed GEMV (pie_qmv2.cu): 4-bit weights, up to 8 rows, K a multiple of 512 -- every matrix of a Llama decode
     // step.  PIE_QMV2=0 keeps the cp.async kernel below (B200, 8B shapes, one row, us cp.async / TMA: q/k/v 7.8 / 7.7,

@@ -28,9 +28,11 @@ int pie_qmm(void* y, const void* x, const uint32_t* wq, const void* scales, cons
                   !(reinterpret_cast<uintptr_t>(biases) & 3) && env_int("PIE_QMM_TC", 1) != 0;
   if (tc && workspace && M <= kQmtRows && qmt_pays(M, N, K, bits, 0)) {
     pie_qmv_seg seg = {wq, scales, biases, N};
-    if (qmt_takes(M, K, K, &seg, 1, group_size, bits) && kWsCntBytes + qmt_scratch(M, N, K, group_size, bits, 0) <= workspace_bytes)
-      return cuda_status(launch_qmt(y, N, x, K, M, K, &seg, 1, bits, nullptr, 0.f, PIE_EPI_STORE, nullptr, (uint8_t*)workspace + kWsCntBytes,
-                                    (cudaStream_t)stream));
+    if (qmt_takes(M, K, K, &seg, 1, group_size, bits) && kWsCntBytes + qmt_scratch(M, N, K, group_size, bits, 0) <= workspace_bytes) {
+      const cudaError_t e = launch_qmt(y, N, x, K, M, K, &seg, 1, bits, nullptr, 0.f, PIE_EPI_STORE, nullptr, (uint8_t*)workspace + kWsCntBytes,
+                                       (cudaStream_t)stream);
+      if (e != cudaErrorNotSupported) return cuda_status(e);
+    }
   }
   if (tc)
     return cuda_status(launch_qmm_tc((uint16_t*)y, (const uint16_t*)x, wq, (const uint16_t*)scales,

@@ -40,7 +40,7 @@ constexpr int kQtMaxRows = kQmtRows, kQtMaxK = 32768;
 constexpr int kQtPacked = 128 * 128;            // packed bytes of a stage: 128 rows, 256 codes
 constexpr int kQtStage = kQtPacked + 2 * 128 * 16;   // ... and scales and biases of 128 rows, the 8 groups its own are among
 constexpr int kQtCols = 72;                     // tensor-memory columns of 128 codes (64) and the 16 columns behind them (8)
-constexpr int kQtMaxStages = 12;
+constexpr int kQtMaxStages = 9;               // what 16 rows leave room for
 constexpr int kQtThreads = 640;
 constexpr int kQtSmem = 226 * 1024;             // dynamic; the barriers are static
 

@@ -6,6 +6,7 @@ import re
 
 import numpy as np
 import pytest
+import torch
 
 HEADER = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "proxy_inference_engine_b200", "csrc", "pie_qmt.cuh")
 COLS, STAGE, SMEM = 72, 128 * 160, 226 * 1024      # kQtCols, kQtStage, kQtSmem
@@ -216,3 +217,18 @@ def test_accumulators_change_hands_at_the_same_turns():
                     results.append((done, size))
                 todo, kk = todo - take, 0
             assert mma == results and all(0 < n <= run for _, n in mma)
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the pointers are none")
+@pytest.mark.parametrize("M", [40, 77])
+def test_calls_go_on_where_no_tensor_map_can_be_made(M, monkeypatch):
+    """Without a driver none can: the call goes on to the kernels that need none, and fails at their launch for want of a device."""
+    from proxy_inference_engine_b200 import _lib
+    L, at = _lib.load(), 1 << 20
+    monkeypatch.setenv("PIE_QMT", "2")
+    monkeypatch.setenv("PIE_QMM_TC", "0" if M < 64 else "1")
+    n0 = L.pie_launch_count()
+    assert L.pie_qmt(at, 4096, at, 4096, M, 4096, (_lib.QmvSeg * 1)(_lib.QmvSeg(at, at, at, 4096)), 1, 64, 4, None, 0.0, 0, None, at, 1 << 30, None) == _lib.EUNSUPPORTED
+    assert L.pie_launch_count() == n0
+    L.pie_qmm(at, at, at, at, at, M, 4096, 4096, 64, 4, at, 1 << 30, None)
+    assert L.pie_launch_count() > n0 or b"NotSupported" not in L.pie_last_cuda_error()
