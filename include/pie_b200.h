@@ -119,7 +119,8 @@ int pie_qmm_swiglu_pays(int M, int N, int K, int group_size, int bits);
 int pie_qmm_swiglu(void* y, const void* x, const pie_qmv_seg* gate_up, int M, int K, int group_size, int bits, void* stream);
 
 /* 64 rows and more: the products of up to three matrices of one K side by side in rows of y (y_ld elements apart), and residual (as y lies; may be
- * y; NULL: none) added to them: the bits of pie_qmm on each and pie_add.  PIE_EUNSUPPORTED (nothing launched): operands it cannot take. */
+ * y; NULL: none) added to them.  One matrix: the bits of the tile kernel of pie_qmm (which takes every call of more than 128 rows) and pie_add.  Several: the tile
+ * is chosen for all of them, so that K may be cut in other places than for each and its fp32 sums added in another order.  PIE_EUNSUPPORTED (nothing launched): operands it cannot take. */
 int pie_qmm_rows(void* y, int y_ld, const void* x, const pie_qmv_seg* segs_host, int nseg, const void* residual, int M, int K, int group_size,
                  int bits, void* stream);
 

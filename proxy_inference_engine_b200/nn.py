@@ -140,7 +140,8 @@ def fused_swiglu(x, gate, up):
 
 def fused_prompt(x, linears, residual=None):
     """A prompt's rows (64 and more) through several bias-free QuantizedLinears in one launch, [..., sum N] their outputs side by side, and a
-    residual added to them: the bits of the separate calls.  None where that does not apply (the caller then makes those)."""
+    residual added to them.  One matrix of more than 128 rows: the bits of the separate calls; several: theirs up to the order of fp32 sums over K, which
+    may be cut in other places.  None where that does not apply (the caller then makes those)."""
     K = x.shape[-1]
     if x.dtype != torch.bfloat16 or not x.is_contiguous() or K == 0 or K % 128 or x.numel() < 64 * K:
         return None

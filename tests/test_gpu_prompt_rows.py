@@ -1,5 +1,6 @@
-"""pie_qmm_rows, several matrices and a residual in one launch of the prompt's matmul, against pie_qmm on each and pie_add: the same bits at every
-tile the choice can take (pairs and single CTAs, K over a cluster's ranks), at ragged widths and in place."""
+"""pie_qmm_rows, several matrices and a residual in one launch of the prompt's matmul, against pie_qmm's tile kernel on each and pie_add, at every tile the choice
+can take (pairs and single CTAs, K over a cluster's ranks) and at ragged widths.  One matrix, with or without a residual, which may be the output itself: the
+same bits.  Several: the choice is the whole's, so that K may be cut in other places and fp32 sums added in another order."""
 import pytest
 import torch
 
@@ -20,10 +21,10 @@ def _layer(g, n, k, bits):
 @pytest.mark.parametrize("M,K,widths", [(64, 4096, (256, 128, 128)), (70, 256, (200, 36, 7)), (129, 2048, (2048, 512, 512)), (300, 640, (264, 8)),
                                         (1000, 4096, (4096, 1024, 1024)), (1531, 2048, (2048, 512, 512)), (2100, 1024, (4000,)),
                                         (513, 512, (129, 129, 129))])
-def test_one_launch_has_the_bits_of_its_products(monkeypatch, bits, M, K, widths):
+def test_one_launch_and_its_products_apart(monkeypatch, bits, M, K, widths):
     from proxy_inference_engine_b200 import nn, ops
-    from proxy_inference_engine_b200._lib import load
-    monkeypatch.setenv("PIE_QMT", "0")                 # the separate calls on the same kernel at 64 to 128 rows, too
+    from proxy_inference_engine_b200._lib import QmvSeg, check, load
+    monkeypatch.setenv("PIE_QMT", "0")                 # the separate calls on the tile kernel at 64 to 128 rows, too
     g = torch.Generator(device="cuda").manual_seed(M + K + bits)
     x, lins = torch.randn((M, K), generator=g, device="cuda").bfloat16(), tuple(_layer(g, n, K, bits) for n in widths)
     want = torch.cat([ops.quantized_matmul(x, l.weight, l.scales, l.biases, bits=bits) for l in lins], 1)
@@ -36,4 +37,8 @@ def test_one_launch_has_the_bits_of_its_products(monkeypatch, bits, M, K, widths
     alone = nn.fused_prompt(x, lins[:1])
     assert torch.equal(alone, want[:, :widths[0]])     # the choice of a matrix alone: the same bits
     res = torch.randn((M, widths[0]), generator=g, device="cuda").bfloat16()
-    assert torch.equal(nn.fused_prompt(x, lins[:1], residual=res), ops.add(res, alone))
+    want = ops.add(res, alone)
+    assert torch.equal(nn.fused_prompt(x, lins[:1], residual=res), want)
+    seg = (QmvSeg * 1)(QmvSeg(lins[0].weight.data_ptr(), lins[0].scales.data_ptr(), lins[0].biases.data_ptr(), widths[0]))
+    check(load().pie_qmm_rows(res.data_ptr(), widths[0], x.data_ptr(), seg, 1, res.data_ptr(), M, K, 64, bits, torch.cuda.current_stream().cuda_stream), "in place")
+    assert torch.equal(res, want)

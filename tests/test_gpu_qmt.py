@@ -1,6 +1,7 @@
 """pie_qmt (csrc/pie_qmt.cuh), some dozens of rows with the weights through tensor memory, against float64 at the edges of its rows, tiles and
-shares.  Operands are exact and sums are fp32, so what is left is the rounding of the result to bf16: 2^-9 of a value at the most, in the
-2-norm 2^-9 / sqrt(3) = 1.13e-3 to 1.95e-3 as the values lie in their binade."""
+shares.  Weights are exact, activations are down to 2^-25 (8 bits: 2^-21) of a row's largest, and sums are off by less than 1e-6, so what is left is the
+rounding of the result to bf16: 2^-9 of a value at the most, in the 2-norm 2^-9 / sqrt(3) = 1.13e-3 to 1.95e-3 as the values lie in their binade.  Two tests
+below look under that: products next to zero show the sums, a large value that meets no weight the activations."""
 import ctypes as C
 
 import pytest
@@ -266,3 +267,58 @@ def test_a_decode_engine_has_room_for_it_at_more_than_32_rows():
     for n, k, dual in ((3072, 2048, 0), (2048, 2048, 0), (2048, 2048, 1)):
         need = L.pie_qmt_scratch_bytes(B, n, k, 64, 4, dual)
         assert need and eng.qmv_ws.numel() >= (128 << 10) + need
+
+
+def _many_rows(g, K=2048, n=6144, rows=48):
+    from proxy_inference_engine_b200 import nn
+    lin = object.__new__(nn.QuantizedLinear)
+    lin.group_size, lin.bits = 64, 4
+    lin.weight, lin.scales, lin.biases = _matrix(g, n, K, 4)
+    return lin, torch.randn((rows, K), generator=g, device="cuda").bfloat16()
+
+
+def _native(x, lin):
+    from proxy_inference_engine_b200 import nn, ops
+    y = ops.native_fused_rows()(x, (lin,), None, None, False, nn.QuantizedLinear, nn.RMSNorm, ops.qmv_workspace)
+    assert y is not None
+    return y
+
+
+def test_the_native_form_on_a_stream_of_its_own_and_in_a_capture():
+    lin, x = _many_rows(torch.Generator(device="cuda").manual_seed(8))
+    want, twice = _native(x, lin), _native(2 * x, lin)
+    side, a = torch.cuda.Stream(), torch.randn((8192, 8192), device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        late = x * 0
+        for _ in range(3):
+            torch.mm(a, a)                                               # the copy below comes behind it, and the call behind that
+        late.copy_(x)
+        got = _native(late, lin)
+    side.synchronize()
+    assert torch.equal(got, want)
+    graph, fed = torch.cuda.CUDAGraph(), x.clone()
+    with torch.cuda.graph(graph):
+        out = _native(fed, lin)
+    for v, y in ((x, want), (2 * x, twice), (x, want)):
+        fed.copy_(v)
+        graph.replay()
+        assert torch.equal(out, y)
+
+
+def test_two_threads_call_the_native_form_on_streams_of_their_own():
+    from concurrent.futures import ThreadPoolExecutor
+    g = torch.Generator(device="cuda").manual_seed(9)
+    work = [_many_rows(g), _many_rows(g, n=4000, rows=63)]
+    want = [_native(x, lin) for lin, x in work]
+    torch.cuda.synchronize()
+
+    def loop(i):
+        (lin, x), bad = work[i], 0
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(200):
+                bad += int(not torch.equal(_native(x, lin), want[i]))
+        return bad
+
+    with ThreadPoolExecutor(2) as pool:
+        assert list(pool.map(loop, range(2))) == [0, 0]
