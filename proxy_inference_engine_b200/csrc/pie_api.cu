@@ -157,17 +157,17 @@ static size_t qmt_scratch(int M, long long n_total, int K, int group_size, int b
   return qmt_ws_bytes(M, dual ? (n_total + 63) / 64 : (n_total + 127) / 128 + kMaxSeg, K, bits);
 }
 // Whether a call is sooner done by it.  Measured, 4 bits, B200, us before / with it (graphs of calls, the preparing kernel included): 16 rows
-// 4096 x 4096 10.9 / 11.5, 6144 x 4096 16.4 / 13.1, 2 x 14336 x 4096 with SwiGLU 42.5 / 26.6, 4096 x 14336 27.6 / 17.8, 128256 x 4096 147 / 72;
-// 32 rows 2048 x 2048 11.2 / 13.1, 3072 x 2048 11.8 / 13.2, 4096 x 4096 18.3 / 14.0, 128256 x 4096 198 / 79; 40 rows (two passes of the
-// GEMV before) 2048 x 2048 16.9 / 14.7, 4096 x 14336 54.6 / 24.2.  So up to 32 rows the line is drawn by the work, in stages of 128 rows of
-// 256 codes, that covers the 8 to 10 us a call takes at the least; 33 to 63 rows are sooner done here but for the smallest matrices (8 bits: 4096 x 4096 23.9 / 18.1,
-// 4096 x 14336 44.0 / 34.6), and from 64 on the estimates of both kernels decide (rows: 64 4096 x 4096 13.9 / 17.6, 2 x 14336 x 4096 54.2 / 41.5).
+// 4096 x 4096 10.9 / 11.2, 6144 x 4096 16.4 / 13.2, 2 x 14336 x 4096 with SwiGLU 42.5 / 27.0, 4096 x 14336 27.6 / 17.5, 128256 x 4096 147 / 74.5;
+// 32 rows 2048 x 2048 11.2 / 12.3, 3072 x 2048 11.8 / 12.5, 4096 x 4096 18.3 / 13.1, 128256 x 4096 198 / 82; 40 rows (two passes of the
+// GEMV before) 2048 x 2048 16.9 / 15.4, 4096 x 14336 54.6 / 23.7.  So up to 32 rows the line is drawn by the work, in stages of 128 rows of
+// 256 codes, that covers the 8 to 10 us a call takes at the least; 33 to 63 rows are sooner done here but for the smallest matrices (8 bits, 40 rows: 4096 x 4096
+// 23.9 / 18.2, 4096 x 14336 44.0 / 36.8), and from 64 on the estimates of both kernels decide (rows: 64 4096 x 4096 13.9 / 17.4, 2 x 14336 x 4096 54.2 / 43.8).
 // 8-bit calls of up to 32 rows stay with pie_qmi.cu (4096 x 14336, 32 rows 25.3 / 31.2).  PIE_QMT: 0 never, 2 always
 static bool qmt_pays(int M, long long n_total, int K, int bits, int dual) {
   const int mode = env_int("PIE_QMT", 1);
   if (mode != 1) return mode == 2;
   const long long tiles = dual ? (n_total + 63) / 64 : (n_total + 127) / 128, work = tiles * ((long long)K * bits / 1024);
-  // (3 to 8 rows so long that pie_qmv2.cu has no room for them beside its ring: 4096 x 14336, 5 rows 20.2 / 17.6)
+  // (3 to 8 rows so long that pie_qmv2.cu has no room for them beside its ring: 4096 x 14336, 5 rows 20.2 / 17.4)
   if (M <= 8) return bits == 4 && M >= 3 && work >= 1500 && qmv2_smem_bytes(M, K) > (size_t)kQmvMaxSmem;
   if (M <= 32) return bits == 4 && work >= (M <= 16 ? 700 : 400);
   if (M < 64) return work >= 100;

@@ -24,10 +24,11 @@
 // the results; warps 8-19 in three sets dequantise, 128 codes of 128 rows in turn.  The work, tiles x 256 codes, is dealt out evenly: a
 // CTA's share may begin and end inside a tile, and the CTA that comes last adds a tile's parts, in the order of K.
 // Measured, 4 bits, us a call with the preparing kernel (the kernels before it: mma.sync GEMV in passes of 32 rows, or the tile kernel from 64
-// rows on -> this one): 4096 x 14336 16 rows 27.6 -> 17.8, 32 37.1 -> 20.6, 48 62.0 -> 24.2; 2 x 14336 x 4096 with SwiGLU 16 rows 42.5 -> 26.6,
-// 32 60.5 -> 31.3, 77 54.6 -> 46.0; 128256 x 4096 16 rows 147 -> 72 (4.1 TB/s of packed weights), 32 198 -> 79.  A call of next to no work takes
+// rows on -> this one): 4096 x 14336 16 rows 27.6 -> 17.5, 32 37.1 -> 20.9, 48 62.0 -> 25.2; 2 x 14336 x 4096 with SwiGLU 16 rows 42.5 -> 27.0,
+// 32 60.5 -> 32.5, 77 54.6 -> 47.5; 128256 x 4096 16 rows 147 -> 74.5 (4.0 TB/s of packed weights), 32 198 -> 82.  A call of next to no work takes
 // 10: 3 of preparation, 2 until the first words are there, 1.3 for the first turn, 3.5 from the last sum to the stored result.  What
-// bounds the rest is issue: about 3500 warp instructions for 256 codes of 128 rows, 0.6 us a turn where the words alone would take 0.37.
+// bounds the rest is issue and the chain of a turn: 3800 warp instructions for 256 codes of 128 rows, set-up and hand-over among them (4096 x 14336, 16
+// rows: issue slots 45 % busy, half of that launch being set-up and hand-over), 0.6 us a turn where the words alone would take 0.37.
 // Tried and left: operands of a whole turn unrolled, or the next quarter's words and scales ahead (no faster: 73 -> 76 for the head), more
 // accumulators (no change), scales in a ring of their own (73 -> 79), MMAs handed over by 128 codes (84: the issuing warp's turn-round).
 #pragma once
