@@ -165,7 +165,7 @@ def _near_zero_targets(g, M, K, w):
     return x
 
 
-@pytest.mark.parametrize("bits,M,K", [(4, 9, 512), (4, 16, 4096), (4, 32, 1536), (4, 32, 14336), (4, 48, 14336), (4, 63, 4608), (8, 48, 8192)])
+@pytest.mark.parametrize("bits,M,K", [(4, 9, 512), (4, 16, 4096), (4, 32, 1536), (4, 32, 14336), (4, 48, 14336), (4, 63, 4608), (8, 20, 4096), (8, 48, 8192)])
 def test_sums_are_no_further_off_than_the_gemvs(bits, M, K, monkeypatch):
     """Before their rounding to bf16, over a tile's whole K in one CTA (as many tiles as SMs).  The tensor core cuts the sums it returns, towards zero: with
     one accumulator for all of K they were off by 1.8e-6 of a product's size at K 4096 and 8.0e-6 at 14336, the GEMV by 1.1e-6 to 1.4e-6 at every K."""
@@ -255,18 +255,29 @@ def test_rows_with_infinities(bits, M, K, monkeypatch):
     assert torch.equal(z[rest], y[rest].double())
 
 
-def test_a_decode_engine_has_room_for_it_at_more_than_32_rows():
-    """The workspace of a step of 40 rows holds what the tensor-memory matmul asks for with 40 rows, or the step would fall back to passes of 32."""
+def test_a_decode_engine_has_room_for_it_at_more_than_32_rows(monkeypatch):
+    """The workspace of a step of 40 rows holds what the tensor-memory matmul asks for with 40 rows, or the step would fall back to passes of 32; and the
+    captured step's logits are those of the kernels without it."""
     from parity_util import tiny_args
     from proxy_inference_engine_b200 import _lib
     from proxy_inference_engine_b200.decode import DecodeEngine
     from proxy_inference_engine_b200.llama import Model
     B, L = 40, _lib.load()
-    args = tiny_args(hidden_size=2048, intermediate_size=2048, num_hidden_layers=1, num_attention_heads=32, num_key_value_heads=8)
-    eng = DecodeEngine(Model(args), B, 64)
+    model = Model(tiny_args(hidden_size=2048, intermediate_size=2048, num_hidden_layers=1, num_attention_heads=32, num_key_value_heads=8))
+    eng, ids = DecodeEngine(model, B, 64), torch.randint(0, 640, (B, 6), device="cuda")
     for n, k, dual in ((3072, 2048, 0), (2048, 2048, 0), (2048, 2048, 1)):
         need = L.pie_qmt_scratch_bytes(B, n, k, 64, 4, dual)
         assert need and eng.qmv_ws.numel() >= (128 << 10) + need
+    eng.prefill(ids)
+    first = eng.tokens.clone()
+    eng.step(1)
+    logits = eng.logits.double().clone()
+    monkeypatch.setenv("PIE_QMT", "0")
+    other = DecodeEngine(model, B, 64)
+    other.prefill(ids)
+    other.tokens.copy_(first)
+    other.step(1)
+    assert _rel(logits, other.logits.double()) < 2e-2
 
 
 def _many_rows(g, K=2048, n=6144, rows=48):
