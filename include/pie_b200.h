@@ -161,6 +161,14 @@ int pie_kv_write_strided(void* kcache, void* vcache, const pie_kv_layout* kv_hos
 int pie_rope_heads(void* out, const void* x, int B, int H, int L, int D, long long stride_b, long long stride_h,
                    long long stride_l, int offset, const float* freqs, void* stream);
 
+/* rotation of q and k and the cache write of k and v in one launch, from wherever the projections' rows lie: rows of head h of sequence b at
+ * p + b stride_b + h stride_h + l stride_l (elements, contiguous features).  q_out [B, Hq, L, D] contiguous; cache rows offset .. offset + L - 1;
+ * positions_out (or NULL): int32 [B], offset + L - 1.  Bit for bit pie_rope_heads and pie_kv_write_strided.                                     */
+typedef struct pie_head_rows { const void* p; long long stride_b, stride_h, stride_l; } pie_head_rows;
+int pie_rope_kv_rows(void* q_out, void* kcache, void* vcache, const pie_kv_layout* kv_host, const pie_head_rows* q, const pie_head_rows* k,
+                     const pie_head_rows* v, int32_t* positions_out, const float* freqs, int B, int Hq, int Hkv, int L, int D, int offset,
+                     void* stream);
+
 /* ---- a9  mx.fast.scaled_dot_product_attention, L == 1, mask None (PIE/models/base.py:92-113) ----------
  * split-K flash-decode (the scheme of Metal sdpa_vector_2pass, kernels/sdpa_vector.h:168-392).
  * q bf16 [B, Hq, D]; context length of row b = positions[b] + 1; out bf16 [B, Hq * D].
@@ -234,6 +242,9 @@ int pie_kvq_append(void* q_out, const void* qkv, const pie_kvq_cache* cache_host
                    const float* freqs, int B, int Hq, int Hkv, int D, void* stream);
 int pie_kvq_write(const pie_kvq_cache* cache_host, const void* k, const void* v, int B, int Hkv, int L, int D,
                   int offset, void* stream);
+/* pie_rope_kv_rows with a quantised cache, up to 1024 rows (PIE_EUNSUPPORTED: more) */
+int pie_rope_kvq_rows(void* q_out, const pie_kvq_cache* cache_host, const pie_head_rows* q, const pie_head_rows* k, const pie_head_rows* v,
+                      int32_t* positions_out, const float* freqs, int B, int Hq, int Hkv, int L, int D, int offset, void* stream);
 int pie_decode_attn_q8_pick_splits(int B, int Hq, int Hkv, int max_context);
 int pie_decode_attn_q8(void* out, const void* q, const pie_kvq_cache* cache_host, const int32_t* positions, int B,
                        int Hq, int Hkv, int D, float scale, int nsplit, void* workspace, size_t workspace_bytes,

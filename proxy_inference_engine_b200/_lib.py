@@ -39,6 +39,11 @@ class KvqCache(C.Structure):
                 ("group_size", C.c_int), ("bits", C.c_int)]
 
 
+class HeadRows(C.Structure):
+    """pie_head_rows"""
+    _fields_ = [("p", C.c_void_p), ("stride_b", C.c_longlong), ("stride_h", C.c_longlong), ("stride_l", C.c_longlong)]
+
+
 class TpPeers(C.Structure):
     """pie_tp_peers"""
     _fields_ = [("base", C.c_void_p * 8), ("rank", C.c_int), ("world", C.c_int), ("max_elems", C.c_int),
@@ -101,6 +106,10 @@ SIGNATURES = {
     "pie_rope_kv_append": (_i, [_vp, _vp, _vp, _vp, C.POINTER(KvLayout), _vp, _vp, _i, _i, _i, _i, _vp]),
     "pie_kv_write_strided": (_i, [_vp, _vp, C.POINTER(KvLayout), _vp, _ll, _ll, _ll, _vp, _ll, _ll, _ll, _i, _i, _i, _i, _i, _vp]),
     "pie_rope_heads": (_i, [_vp, _vp, _i, _i, _i, _i, _ll, _ll, _ll, _i, _vp, _vp]),
+    "pie_rope_kv_rows": (_i, [_vp, _vp, _vp, C.POINTER(KvLayout), C.POINTER(HeadRows), C.POINTER(HeadRows), C.POINTER(HeadRows), _vp, _vp, _i, _i, _i,
+                              _i, _i, _i, _vp]),
+    "pie_rope_kvq_rows": (_i, [_vp, C.POINTER(KvqCache), C.POINTER(HeadRows), C.POINTER(HeadRows), C.POINTER(HeadRows), _vp, _vp, _i, _i, _i, _i, _i,
+                               _i, _vp]),
     "pie_kv_write": (_i, [_vp, _vp, C.POINTER(KvLayout), _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "pie_decode_attn_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "pie_decode_attn_pick_splits": (_i, [_i, _i, _i, _i]),

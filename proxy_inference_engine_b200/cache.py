@@ -43,7 +43,21 @@ class KVCache:
             self._grow(B, H, D, L, keys.device)
         ops.kv_write(self.keys, self.values, ops.kv_layout(self.keys), keys, values, self.offset)
         self.offset += L
-        return self.keys[:, :, : self.offset], self.values[:, :, : self.offset]
+        return self.state
+
+    def rotate_and_fetch(self, queries, keys, values, freqs):
+        """update_and_fetch of rotated keys, with the rotation of queries and keys in the same launch: (queries, keys, values), or None where that does not
+        apply (nothing was done)."""
+        B, H, L, D = keys.shape
+        if self.keys is None or self.offset + L > self.keys.shape[2]:
+            self._grow(B, H, D, L, keys.device)
+        q = None
+        if self.keys.shape[:2] == (B, H) and self.keys.shape[3] == D and self.keys.stride() == self.values.stride():
+            q = ops.rope_kv_rows(queries, keys, values, freqs, self.offset, (self.keys, self.values, ops.kv_layout(self.keys)))
+        if q is None:
+            return None
+        self.offset += L
+        return q, *self.state
 
     @property
     def state(self):
@@ -79,6 +93,17 @@ class PagedKVCache:
         ops.kv_write(self.k_pool, self.v_pool, self.layout(), keys, values, self.offset)
         self.offset += L
         return self, self
+
+    def rotate_and_fetch(self, queries, keys, values, freqs):
+        """As KVCache.rotate_and_fetch."""
+        L = keys.shape[2]
+        if self.offset + L > self.page_table.shape[1] * self.page_size:
+            raise ValueError("PagedKVCache: page table too small for this many tokens")
+        q = ops.rope_kv_rows(queries, keys, values, freqs, self.offset, (self.k_pool, self.v_pool, self.layout()))
+        if q is None:
+            return None
+        self.offset += L
+        return q, self, self
 
     def gather(self):
         """Logical [B, n_kv, offset, D] copies (tests only: the kernels read the pages in place)."""
@@ -139,6 +164,17 @@ class QuantizedKVCache:
         self.offset += L
         return self.state
 
+    def rotate_and_fetch(self, queries, keys, values, freqs):
+        """As KVCache.rotate_and_fetch."""
+        B, H, L, D = keys.shape
+        if self.keys is None or self.offset + L > self.keys[0].shape[2]:
+            self._grow(B, H, D, L, keys.device)
+        q = ops.rope_kv_rows(queries, keys, values, freqs, self.offset, self.desc())
+        if q is None:
+            return None
+        self.offset += L
+        return q, *self.state
+
     @property
     def state(self):
         if self.keys is None:
@@ -180,6 +216,17 @@ class PagedQuantizedKVCache:
         ops.kvq_write(self.desc(), keys, values, self.offset)
         self.offset += L
         return self, self
+
+    def rotate_and_fetch(self, queries, keys, values, freqs):
+        """As KVCache.rotate_and_fetch."""
+        L = keys.shape[2]
+        if self.offset + L > self.page_table.shape[1] * self.page_size:
+            raise ValueError("PagedQuantizedKVCache: page table too small for this many tokens")
+        q = ops.rope_kv_rows(queries, keys, values, freqs, self.offset, self.desc())
+        if q is None:
+            return None
+        self.offset += L
+        return q, self, self
 
     def gather(self):
         """Logical (quants, scales, biases) [B, n_kv, offset, .] copies of K and V (tests and the L > 1 attention)."""

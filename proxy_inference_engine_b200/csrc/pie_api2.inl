@@ -123,6 +123,19 @@ int pie_rope_heads(void* out, const void* x, int B, int H, int L, int D, long lo
                                        (cudaStream_t)stream));
 }
 
+int pie_rope_kv_rows(void* q_out, void* kcache, void* vcache, const pie_kv_layout* kv, const pie_head_rows* q, const pie_head_rows* k,
+                     const pie_head_rows* v, int32_t* positions_out, const float* freqs, int B, int Hq, int Hkv, int L, int D, int offset,
+                     void* stream) {
+  if (B == 0 || L == 0) return PIE_OK;
+  if (!q_out || !kcache || !vcache || !q || !k || !v || !q->p || !k->p || !v->p || !freqs) return PIE_ENULL;
+  if (B < 0 || Hq <= 0 || Hkv <= 0 || L < 0 || offset < 0 || (D != 64 && D != 128) || B > 65535 || Hq > 65535 - 2LL * Hkv) return PIE_EINVAL_SHAPE;
+  if (int s = check_kv(kv, D)) return s;
+  const RopeRows r = {(const uint16_t*)q->p, (const uint16_t*)k->p, (const uint16_t*)v->p, {q->stride_b, q->stride_h, q->stride_l},
+                      {k->stride_b, k->stride_h, k->stride_l}, {v->stride_b, v->stride_h, v->stride_l}};
+  return cuda_status(launch_rope_kv_rows((uint16_t*)q_out, positions_out, r, (uint16_t*)kcache, (uint16_t*)vcache, to_kv(kv), freqs, B, Hq, Hkv,
+                                         L, D, offset, (cudaStream_t)stream));
+}
+
 int pie_kv_write_strided(void* kcache, void* vcache, const pie_kv_layout* kv, const void* k, long long k_stride_b,
                          long long k_stride_h, long long k_stride_l, const void* v, long long v_stride_b, long long v_stride_h,
                          long long v_stride_l, int B, int Hkv, int L, int D, int offset, void* stream) {

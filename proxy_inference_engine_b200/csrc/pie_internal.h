@@ -105,6 +105,10 @@ cudaError_t launch_kv_write(uint16_t* kc, uint16_t* vc, const KvLayout& kv, cons
                             const KvSrc& vs, int B, int Hkv, int L, int D, int offset, cudaStream_t st);
 cudaError_t launch_rope_heads(uint16_t* out, const uint16_t* x, int B, int H, int L, int D, long long sb, long long sh,
                               long long sl, int offset, const float* freqs, cudaStream_t st);
+// rotation and cache write of q, k, v in one launch; pos_out: nullptr or [B]
+struct RopeRows { const uint16_t *q, *k, *v; KvSrc qs, ks, vs; };
+cudaError_t launch_rope_kv_rows(uint16_t* q_out, int32_t* pos_out, const RopeRows& r, uint16_t* kc, uint16_t* vc, const KvLayout& kv,
+                                const float* freqs, int B, int Hq, int Hkv, int L, int D, int offset, cudaStream_t st);
 cudaError_t launch_decode_attn(uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc,
                                const KvLayout& kv, const int32_t* pos, int B, int Hq, int Hkv, int D,
                                float scale, int nsplit, float* ws, cudaStream_t st);

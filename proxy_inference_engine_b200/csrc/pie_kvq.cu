@@ -119,6 +119,44 @@ __global__ void kvq_write_kernel(const KvqArgs c, const uint16_t* k, const uint1
                   c.vb + slot * G + warp);
 }
 
+// rope_kv_pairs_kernel (pie_rope_kv.cu) with a quantised cache: rows wherever they lie, the codes of kvq_append_kernel
+__global__ void kvq_rows_kernel(uint16_t* q_out, int32_t* pos_out, const RopeRows r, const KvqArgs c, const float* freqs, int Hq, int D, int offset) {
+  __shared__ float row[128];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int l = blockIdx.x, L = gridDim.x, h = blockIdx.y, b = blockIdx.z, i = threadIdx.x, half = D / 2;
+  const int lane = i & 31, warp = i >> 5, G = D / 64;
+  if (pos_out && h == 0 && i == 0 && l == L - 1) pos_out[b] = offset + l;
+  const bool is_v = h >= Hq + c.Hkv;
+  const int kvh = is_v ? h - Hq - c.Hkv : h - Hq;
+  if (is_v) {
+    const uint16_t* src = r.v + b * r.vs.sb + kvh * r.vs.sh + l * r.vs.sl;
+    row[i] = bf16lo((uint32_t)src[i]);
+    row[i + half] = bf16lo((uint32_t)src[i + half]);
+  } else {
+    const uint16_t* src = h < Hq ? r.q + b * r.qs.sb + h * r.qs.sh + l * r.qs.sl : r.k + b * r.ks.sb + kvh * r.ks.sh + l * r.ks.sl;
+    float s, co;
+    rope_sincos(((float)l + (float)offset) * (1.0f / freqs[i]), &s, &co);
+    const float x1 = bf16lo((uint32_t)src[i]), x2 = bf16lo((uint32_t)src[i + half]);
+    const uint16_t o1 = f2bf(__fsub_rn(__fmul_rn(x1, co), __fmul_rn(x2, s)));
+    const uint16_t o2 = f2bf(__fadd_rn(__fmul_rn(x1, s), __fmul_rn(x2, co)));
+    if (h < Hq) {
+      uint16_t* dst = q_out + (((size_t)b * Hq + h) * L + l) * D;
+      dst[i] = o1;
+      dst[i + half] = o2;
+      return;
+    }
+    row[i] = bf16lo((uint32_t)o1);
+    row[i + half] = bf16lo((uint32_t)o2);
+  }
+  __syncthreads();
+  const size_t slot = kvq_slot(c, b, kvh, offset + l);
+  uint32_t* dq = (is_v ? c.vq : c.kq) + slot * (D / 4) + warp * 16;
+  uint16_t* ds = (is_v ? c.vs : c.ks) + slot * G + warp;
+  uint16_t* db = (is_v ? c.vb : c.kb) + slot * G + warp;
+  kvq_store_group(row[warp * 64 + 2 * lane], row[warp * 64 + 2 * lane + 1], lane, dq, ds, db);
+}
+
 struct DecAttnQArgs {
   uint16_t* out;
   const uint16_t* q;
@@ -761,6 +799,23 @@ int pie_kvq_write(const pie_kvq_cache* cache, const void* k, const void* v, int 
   kvq_write_kernel<<<dim3(L, Hkv, B), D / 2, 0, (cudaStream_t)stream>>>(c, (const uint16_t*)k, (const uint16_t*)v, L, D,
                                                                        offset);
   return status_of(cudaGetLastError());
+}
+
+int pie_rope_kvq_rows(void* q_out, const pie_kvq_cache* cache, const pie_head_rows* q, const pie_head_rows* k, const pie_head_rows* v,
+                      int32_t* positions_out, const float* freqs, int B, int Hq, int Hkv, int L, int D, int offset, void* stream) {
+  if (B == 0 || L == 0) return PIE_OK;
+  if (!q_out || !q || !k || !v || !q->p || !k->p || !v->p || !freqs) return PIE_ENULL;
+  if (B < 0 || Hq <= 0 || Hkv <= 0 || L < 0 || offset < 0 || B > 65535 || Hq > 65535 - 2LL * Hkv) return PIE_EINVAL_SHAPE;
+  KvqArgs c;
+  if (int s = kvq_check(cache, Hkv, D, &c)) return s;
+  if (!c.page_table && offset + L > c.cap) return PIE_EINVAL_SHAPE;
+  // a block per row and head: 4000 rows of 48 heads take as long as the separate launches, which read 16 bytes an access
+  if ((long long)B * L > 1024) return PIE_EUNSUPPORTED;
+  const RopeRows r = {(const uint16_t*)q->p, (const uint16_t*)k->p, (const uint16_t*)v->p, {q->stride_b, q->stride_h, q->stride_l},
+                      {k->stride_b, k->stride_h, k->stride_l}, {v->stride_b, v->stride_h, v->stride_l}};
+  count_launch();
+  return status_of(launch_pdl(kvq_rows_kernel, dim3((unsigned)L, (unsigned)(Hq + 2 * Hkv), (unsigned)B), dim3((unsigned)(D / 2)), 0,
+                              (cudaStream_t)stream, (uint16_t*)q_out, positions_out, r, c, freqs, Hq, D, offset));
 }
 
 int pie_decode_attn_q8_pick_splits(int B, int Hq, int Hkv, int max_context) {

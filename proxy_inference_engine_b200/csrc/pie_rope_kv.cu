@@ -131,6 +131,103 @@ cudaError_t launch_rope_kv_append(uint16_t* q_out, const uint16_t* qkv, uint16_t
                     Hkv, D);
 }
 
+// A layer's whole way from projected rows to attention in one launch: q [B, Hq, L, D] rotated into q_out (contiguous), k rotated and v copied
+// into cache rows offset .. offset + L - 1, from wherever the rows lie; pos_out[b] = offset + L - 1 where a decode step asks for it.  Bit for
+// bit what rope of q, rope of k and kv_write give, of which this replaces the three launches (and the fill of the positions): the rotated k is
+// not written and read once more, and a layer of few rows is bound by its launches.  From the projection's end to this one's, three launches / one:
+// 8192 tokens of 32 + 8 heads of 128 53 -> 40 us, 1531 of 64 16 -> 12.
+// Few rows: a block per (token, head), a thread per pair -- one sine each, nothing but latency.
+__global__ void rope_kv_pairs_kernel(uint16_t* q_out, int32_t* pos_out, const RopeRows r, uint16_t* kc, uint16_t* vc, const KvLayout kv,
+                                     const float* freqs, int Hq, int Hkv, int D, int offset) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int l = blockIdx.x, L = gridDim.x, h = blockIdx.y, b = blockIdx.z, i = threadIdx.x, half = D / 2;
+  if (pos_out && h == 0 && i == 0 && l == L - 1) pos_out[b] = offset + l;
+  if (h >= Hq + Hkv) {
+    const uint16_t* src = r.v + b * r.vs.sb + (h - Hq - Hkv) * r.vs.sh + l * r.vs.sl;
+    uint16_t* dst = vc + kv_addr(kv, b, h - Hq - Hkv, offset + l);
+    dst[i] = src[i];
+    dst[i + half] = src[i + half];
+    return;
+  }
+  const uint16_t* src = h < Hq ? r.q + b * r.qs.sb + h * r.qs.sh + l * r.qs.sl : r.k + b * r.ks.sb + (h - Hq) * r.ks.sh + l * r.ks.sl;
+  float s, c;
+  rope_sincos(((float)l + (float)offset) * (1.0f / freqs[i]), &s, &c);
+  const float x1 = bf16lo((uint32_t)src[i]), x2 = bf16lo((uint32_t)src[i + half]);
+  uint16_t* dst = h < Hq ? q_out + (((size_t)b * Hq + h) * L + l) * D : kc + kv_addr(kv, b, h - Hq, offset + l);
+  dst[i] = f2bf(__fsub_rn(__fmul_rn(x1, c), __fmul_rn(x2, s)));
+  dst[i + half] = f2bf(__fadd_rn(__fmul_rn(x1, s), __fmul_rn(x2, c)));
+}
+// More: rope_heads_kernel's way over all Hq + 2 Hkv heads, 16 bytes an access, a token's sines for all heads of a lane.
+__global__ void __launch_bounds__(128) rope_kv_heads_kernel(uint16_t* q_out, int32_t* pos_out, const RopeRows r, uint16_t* kc, uint16_t* vc,
+                                                            const KvLayout kv, const float* freqs, int Hq, int Hkv, int L, int D,
+                                                            int offset, int HL) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int half = D / 2, PB = half / 8, pb = threadIdx.x % PB, rest = threadIdx.x / PB, hl = rest % HL;
+  const int l = blockIdx.x * (128 / PB / HL) + rest / HL, b = blockIdx.y;
+  if (l >= L) return;
+  if (pos_out && l == L - 1 && hl == 0 && pb == 0) pos_out[b] = offset + l;
+  float sn[8], cs[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) rope_sincos(((float)l + (float)offset) * (1.0f / freqs[pb * 8 + e]), &sn[e], &cs[e]);
+  const size_t slot = kv_addr(kv, b, 0, offset + l) + pb * 8;
+  // heads hl, hl + HL ...: the loads of four of them in flight before the first store
+  auto heads = [&](const uint16_t* src, long long sh, uint16_t* dst, long long dh, int H, bool turn) {
+    for (int h0 = hl; h0 < H; h0 += 4 * HL) {
+      uint4 v1[4], v2[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (h0 + i * HL < H) {
+          const uint16_t* xr = src + (h0 + i * HL) * sh;
+          v1[i] = *reinterpret_cast<const uint4*>(xr);
+          v2[i] = *reinterpret_cast<const uint4*>(xr + half);
+        }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (h0 + i * HL >= H) break;
+        if (turn) {
+          const uint32_t a[4] = {v1[i].x, v1[i].y, v1[i].z, v1[i].w}, c[4] = {v2[i].x, v2[i].y, v2[i].z, v2[i].w};
+          uint32_t r1[4], r2[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float x1 = bf16lo(a[e]), y1 = bf16hi(a[e]), x2 = bf16lo(c[e]), y2 = bf16hi(c[e]);
+            r1[e] = pack_bf16(__fsub_rn(__fmul_rn(x1, cs[2 * e]), __fmul_rn(x2, sn[2 * e])),
+                              __fsub_rn(__fmul_rn(y1, cs[2 * e + 1]), __fmul_rn(y2, sn[2 * e + 1])));
+            r2[e] = pack_bf16(__fadd_rn(__fmul_rn(x1, sn[2 * e]), __fmul_rn(x2, cs[2 * e])),
+                              __fadd_rn(__fmul_rn(y1, sn[2 * e + 1]), __fmul_rn(y2, cs[2 * e + 1])));
+          }
+          v1[i] = make_uint4(r1[0], r1[1], r1[2], r1[3]);
+          v2[i] = make_uint4(r2[0], r2[1], r2[2], r2[3]);
+        }
+        uint16_t* o = dst + (h0 + i * HL) * dh;
+        *reinterpret_cast<uint4*>(o) = v1[i];
+        *reinterpret_cast<uint4*>(o + half) = v2[i];
+      }
+    }
+  };
+  heads(r.q + b * r.qs.sb + l * r.qs.sl + pb * 8, r.qs.sh, q_out + ((size_t)b * Hq * L + l) * D + pb * 8, (long long)L * D, Hq, true);
+  heads(r.k + b * r.ks.sb + l * r.ks.sl + pb * 8, r.ks.sh, kc + slot, kv.head_stride, Hkv, true);
+  heads(r.v + b * r.vs.sb + l * r.vs.sl + pb * 8, r.vs.sh, vc + slot, kv.head_stride, Hkv, false);
+}
+
+cudaError_t launch_rope_kv_rows(uint16_t* q_out, int32_t* pos_out, const RopeRows& r, uint16_t* kc, uint16_t* vc, const KvLayout& kv,
+                                const float* freqs, int B, int Hq, int Hkv, int L, int D, int offset, cudaStream_t st) {
+  if (B == 0 || L == 0) return cudaSuccess;
+  count_launch();
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc) |
+                         reinterpret_cast<uintptr_t>(r.q) | reinterpret_cast<uintptr_t>(r.k) | reinterpret_cast<uintptr_t>(r.v);
+  const long long strides = r.qs.sb | r.qs.sh | r.qs.sl | r.ks.sb | r.ks.sh | r.ks.sl | r.vs.sb | r.vs.sh | r.vs.sl | kv.batch_stride |
+                            kv.head_stride | kv.tok_stride;
+  if ((long long)B * L > 64 && (ptrs & 15) == 0 && strides % 8 == 0) {
+    const int lanes = 128 / (D / 16), HL = (long long)B * L >= 1024 ? 4 : lanes, per = lanes / HL;
+    return launch_pdl(rope_kv_heads_kernel, dim3((unsigned)((L + per - 1) / per), (unsigned)B), dim3(128), 0, st, q_out, pos_out, r, kc, vc, kv,
+                      freqs, Hq, Hkv, L, D, offset, HL);
+  }
+  return launch_pdl(rope_kv_pairs_kernel, dim3((unsigned)L, (unsigned)(Hq + 2 * Hkv), (unsigned)B), dim3((unsigned)(D / 2)), 0, st, q_out,
+                    pos_out, r, kc, vc, kv, freqs, Hq, Hkv, D, offset);
+}
+
 // prefill: k, v [B, Hkv, L, D], any strides with contiguous features -> cache rows offset .. offset + L - 1.  A copy: a thread per
 // 16 bytes where everything is 16-byte aligned, else a block per row, element by element.  8192 tokens of
 // 8 heads of 128: copy of v 42 + 36 -> 10 us.  Few rows are all latency, and a block that knows its row has no divisions in front of its

@@ -116,6 +116,9 @@ def scaled_dot_product_attention(queries, keys, values, cache, scale, mask):
     return ops.scaled_dot_product_attention(queries, keys, values, scale=scale, mask=mask)
 
 
+_ROTATING_CACHES = (KVCache, PagedKVCache, QuantizedKVCache, PagedQuantizedKVCache)   # (not classes made from them, whose update_and_fetch may be another)
+
+
 class Attention(nn.Module):
     def __init__(self, args: ModelArgs, device="cuda"):
         dim = args.hidden_size
@@ -144,6 +147,10 @@ class Attention(nn.Module):
     def attend_beside(self, qkv, x, mask, cache):
         """attend() of projections that lie side by side in rows."""
         B, L, _ = x.shape
+        if L == 1 and mask is None and qkv.is_cuda and type(cache) in (KVCache, QuantizedKVCache):   # a step of decoding, in one native call
+            out = ops.native_host().attend_rows(self, qkv, cache, KVCache, QuantizedKVCache, Llama3RoPE, ops.attention_workspace)
+            if out is not None:
+                return out
         nq, nk = self.q_proj.weight.shape[0], self.k_proj.weight.shape[0]
         return self.attend(qkv[..., :nq], qkv[..., nq:nq + nk], qkv[..., nq + nk:], B, L, mask, cache)
 
@@ -152,10 +159,15 @@ class Attention(nn.Module):
         queries = queries.reshape(B, L, self.num_heads, -1).transpose(1, 2)
         keys = keys.reshape(B, L, self.n_kv_heads, -1).transpose(1, 2)
         values = values.reshape(B, L, self.n_kv_heads, -1).transpose(1, 2)
+        fetched = None
         if cache is not None:
-            queries = self.rope(queries, offset=cache.offset)
-            keys = self.rope(keys, offset=cache.offset)
-            keys, values = cache.update_and_fetch(keys, values)
+            if type(cache) in _ROTATING_CACHES and type(self.rope) is Llama3RoPE and not self.rope.traditional and self.rope.dimensions == queries.shape[-1]:
+                fetched = cache.rotate_and_fetch(queries, keys, values, self.rope._freqs)
+            if fetched is None:
+                queries = self.rope(queries, offset=cache.offset)
+                keys = self.rope(keys, offset=cache.offset)
+                fetched = queries, *cache.update_and_fetch(keys, values)
+            queries, keys, values = fetched
         else:
             queries, keys = self.rope(queries), self.rope(keys)
             values = values.contiguous()   # in the layout of the rotated keys; a cache would have copied both
@@ -172,11 +184,18 @@ class MLP(nn.Module):
         self.up_proj = mk(args.hidden_size, args.intermediate_size)
 
     def __call__(self, x):
-        act, y = nn.fused_rows(x, (self.gate_proj, self.up_proj), swiglu=True), None
-        if act is not None:
-            y = nn.fused_rows(act, (self.down_proj,))
-        else:
-            act = self.activations(x)
+        act = y = None
+        if x.is_cuda and x.numel() <= 128 * x.shape[-1]:   # few rows: both launches in one native call
+            y = ops.native_host().mlp_rows(x, self.gate_proj, self.up_proj, self.down_proj, nn.QuantizedLinear, nn.RMSNorm, ops.qmv_workspace)
+            if type(y) is tuple:                           # as far as it came
+                (act,), y = y, None
+        if y is None:
+            if act is None:
+                act = nn.fused_rows(x, (self.gate_proj, self.up_proj), swiglu=True)
+            if act is not None:
+                y = nn.fused_rows(act, (self.down_proj,))
+            else:
+                act = self.activations(x)
         return all_reduce_sum(self.down_proj(act) if y is None else y, getattr(self, "tp", None))
 
     def activations(self, x):

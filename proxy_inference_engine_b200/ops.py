@@ -16,7 +16,7 @@ import warnings
 import torch
 
 from . import _lib
-from ._lib import EPI_RESADD, EPI_SILUMUL, EPI_STORE, KvLayout, KvqCache, QmvSeg
+from ._lib import EPI_RESADD, EPI_SILUMUL, EPI_STORE, HeadRows, KvLayout, KvqCache, QmvSeg
 
 _BF16 = torch.bfloat16
 
@@ -219,6 +219,17 @@ def qmv_fused(x, linears, rows: int, K: int, N: int, bits: int, norm_weight, eps
     return out
 
 
+def attention_workspace(units: int, nbytes: int, device) -> torch.Tensor:
+    """Counters and partial sums of a decode step's attention over ``units`` (rows x query heads).  Keyed by the size of the counter region: the counters must
+    be zero at a launch, and a buffer that served another (rows, heads) geometry holds that call's partial sums where this call's counters lie."""
+    return workspaces.get(("attn", (units * 4 + 255) // 256), nbytes, device)
+
+
+class _NoHost:
+    """Where csrc/pie_host.cpp's module was not built, or for another torch or interpreter: None to every call."""
+    mlp_rows = attend_rows = staticmethod(lambda *args: None)
+
+
 @functools.cache
 def native_fused_rows():
     """csrc/pie_host.cpp's form of nn.fused_rows, which takes the common calls and answers None to the others; where it was not built, or for another torch or
@@ -234,8 +245,13 @@ def native_fused_rows():
         warnings.warn(f"{path} does not load ({e}): build it again with make -C {_lib.CSRC}.  Calls of few rows take the Python form meanwhile.")
         return lambda *args: None
     L = _lib.load()
-    host.bind(*(C.cast(fn, C.c_void_p).value for fn in (L.pie_qmv_fused, L.pie_qmv_workspace_bytes, L.pie_qmt, L.pie_qmt_scratch_bytes)))
+    host.bind({name: C.cast(getattr(L, name), C.c_void_p).value for name in host.functions})
     return host.fused_rows
+
+
+def native_host():
+    """The module native_fused_rows() is of: several launches of few rows (mlp_rows, attend_rows), with the same None."""
+    return getattr(native_fused_rows(), "__self__", _NoHost)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -341,6 +357,31 @@ def kv_write(kbuf, vbuf, lay: "KvLayout", keys, values, offset: int):
                                                 B, H, Lq, D, offset, _stream()), "update_and_fetch")
 
 
+def rope_kv_rows(queries, keys, values, freqs, offset: int, write):
+    """Rotation of queries and keys [B, heads, L, D] at positions offset .. and the cache write of keys and values in one launch: the bits of rope of the
+    two and kv_write / kvq_write.  ``write``: (kbuf, vbuf, KvLayout), or a KvqCache.  Returns the rotated queries, contiguous; None where the separate calls
+    are to be made (which also report what is wrong)."""
+    B, Hq, Lq, D = queries.shape
+    Hkv = keys.shape[1]
+    if D not in (64, 128) or keys.shape != (B, Hkv, Lq, D) or values.shape != keys.shape or freqs.dtype != torch.float32 or freqs.shape != (D // 2,) \
+            or not freqs.is_contiguous() or not 0 < B <= 65535 or Hq + 2 * Hkv > 65535 or Lq == 0 \
+            or any(t.dtype != _BF16 or not t.is_cuda or t.stride(3) != 1 for t in (queries, keys, values)):
+        return None
+    out = torch.empty((B, Hq, Lq, D), dtype=_BF16, device=queries.device)
+    rows = [HeadRows(t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)) for t in (queries, keys, values)]
+    L = _lib.load()
+    if isinstance(write, KvqCache):
+        status = L.pie_rope_kvq_rows(_p(out), C.byref(write), *map(C.byref, rows), None, _p(freqs), B, Hq, Hkv, Lq, D, int(offset), _stream())
+        if status == _lib.EUNSUPPORTED:
+            return None
+    else:
+        kbuf, vbuf, lay = write
+        status = L.pie_rope_kv_rows(_p(out), _p(kbuf), _p(vbuf), C.byref(lay), *map(C.byref, rows), None, _p(freqs), B, Hq, Hkv, Lq, D, int(offset),
+                                    _stream())
+    _lib.check(status, "update_and_fetch")
+    return out
+
+
 class CausalMask:
     """What create_attention_mask returns for L > 1 (PIE/models/base.py:37-53): the additive -1e9 causal mask
     [L, offset + L], kept symbolic because the attention kernel builds it from (offset, L)."""
@@ -372,9 +413,7 @@ def decode_attention(q, kbuf, vbuf, lay: KvLayout, positions, scale: float, nspl
     if nsplit <= 0:
         nsplit = L.pie_decode_attn_pick_splits(B, Hq, Hkv, max_context if max_context > 0 else 1)
     nb = L.pie_decode_attn_workspace_bytes(B, Hq, D, nsplit)
-    # keyed by the size of the counter region: the counters must be zero at a launch, and a buffer that served another
-    # (rows, heads) geometry holds that call's partial sums where this call's counters lie
-    ws = workspaces.get(("attn", (B * Hq * 4 + 255) // 256), nb, q.device)
+    ws = attention_workspace(B * Hq, nb, q.device)
     out = torch.empty((B, Hq * D), dtype=_BF16, device=q.device)
     _lib.check(L.pie_decode_attn(_p(out), _p(q), _p(kbuf), _p(vbuf), C.byref(lay), _p(positions), B, Hq, Hkv, D,
                                  float(scale), nsplit, _p(ws), ws.numel(), _stream()), "scaled_dot_product_attention")
@@ -476,9 +515,7 @@ def decode_attention_q8(q, desc: KvqCache, positions, scale: float, Hkv: int, ns
     if nsplit <= 0:
         nsplit = L.pie_decode_attn_q8_pick_splits(B, Hq, Hkv, max_context if max_context > 0 else 1)
     nb = L.pie_decode_attn_workspace_bytes(B, Hq, D, nsplit)
-    # keyed by the size of the counter region: the counters must be zero at a launch, and a buffer that served another
-    # (rows, heads) geometry holds that call's partial sums where this call's counters lie
-    ws = workspaces.get(("attn", (B * Hq * 4 + 255) // 256), nb, q.device)
+    ws = attention_workspace(B * Hq, nb, q.device)
     if out is None:
         out = torch.empty((B, Hq * D), dtype=_BF16, device=q.device)
     qc = q.contiguous()
