@@ -87,8 +87,9 @@ int pie_qmv(void* y, const void* x, const uint32_t* wq, const void* scales, cons
  * the way in (a6: norm_weight != NULL -> x <- rms_norm(x, norm_weight, eps)) and residual-add / SwiGLU on
  * the way out (a11).  For PIE_EPI_SILUMUL pass exactly two segments (gate, up) of equal N; the output row
  * is then N wide.  residual (ld = out_ld) may alias out.  x_ld = elements between rows of x.
- * pdl != 0 launches with programmatic stream serialization: the kernel prefetches its weights while the
- * previous kernel on the stream drains, and reads x only after that kernel has completed.               */
+ * pdl 1 launches with programmatic stream serialization: the kernel reads its first weights while the
+ * previous kernel on the stream drains, and x only after that kernel has completed.  pdl 2: the same where that
+ * kernel may have written the weights: they are only asked of L2 meanwhile.                               */
 typedef struct pie_qmv_seg {
   const uint32_t* wq;
   const void* scales;

@@ -126,7 +126,7 @@ int build_qmv_args(QmvArgs& a, QmvPlan& p, void* out, int out_ld, const void* x,
   a.M = mb; a.ntiles = p.ntiles; a.ksplit = p.ksplit; a.kslice = p.kslice; a.ks_w = p.ks_w;
   a.ks_w_log2 = 0; while ((1 << a.ks_w_log2) < p.ks_w) ++a.ks_w_log2;
   a.nch = p.kslice / (stage_k(bits) * p.ks_w);
-  a.lift_mask = 0x000f000fu; a.lift_magic = 0x43004300u;
+  a.lift_mask = 0x000f000fu; a.lift_magic = 0x43004300u; a.late = 0;
   a.x = (const uint16_t*)x + (size_t)m0 * x_ld;
   a.out = (uint16_t*)out + (size_t)m0 * out_ld;
   a.residual = residual ? (const uint16_t*)residual + (size_t)m0 * out_ld : nullptr;
@@ -291,7 +291,7 @@ int pie_qmv_fused_tp(void* out, int out_ld, const void* x, int x_ld, int M, int 
       Qmv2Args a2;
       const int st1 = build_qmv2_args(a2, out, out_ld, x, x_ld, mb, K, segs, nseg, norm_weight, eps, epilogue, residual, tp);
       if (st1 == PIE_OK) {
-        const int st2 = cuda_status(launch_qmv2(a2, pdl != 0, (cudaStream_t)stream));
+        const int st2 = cuda_status(launch_qmv2(a2, pdl, (cudaStream_t)stream));
         if (st2 != PIE_OK) return st2;
         continue;
       }
@@ -344,6 +344,7 @@ int pie_qmv_fused_tp(void* out, int out_ld, const void* x, int x_ld, int M, int 
         continue;
       }
     }
+    a.late = pdl == 2;
     const int st = cuda_status(launch_qmv(a, bits, p.warps, p.grid, pdl != 0, (cudaStream_t)stream));
     if (st != PIE_OK) return st;
   }
@@ -387,7 +388,7 @@ int pie_qmv(void* y, const void* x, const uint32_t* wq, const void* scales, cons
   if (fast) {
     pie_qmv_seg seg = {wq, scales, biases, N};
     return pie_qmv_fused(y, N, x, K, M, K, &seg, 1, group_size, bits, nullptr, 0.f, PIE_EPI_STORE, nullptr, 0,
-                         workspace, workspace_bytes, 0, stream);
+                         workspace, workspace_bytes, 2, stream);
   }
   if (group_size != 32 && group_size != 64 && group_size != 128) return PIE_EUNSUPPORTED;
   if (bits != 2 && bits != 4 && bits != 8) return PIE_EUNSUPPORTED;

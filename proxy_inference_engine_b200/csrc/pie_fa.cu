@@ -61,6 +61,8 @@ __global__ void __launch_bounds__(kFaThreads) fa_prefill_kernel(const __grid_con
   constexpr int CPR = D / 8;   // 16-byte chunks per tile row
   constexpr int TILE = kFaBKV * D * 2;
   extern __shared__ __align__(128) uint8_t smem[];
+  pdl_launch_dependents();
+  pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   // causal: query tile i needs i + 1 key tiles.  Blocks are dispatched in index order, so the LONGEST tiles go first
   // (the last CTAs to start are then the one-tile ones and the grid's tail is short)
@@ -478,9 +480,8 @@ cudaError_t launch_prefill_attn_tc(uint16_t* out, const uint16_t* q, const uint1
   }
   const dim3 grid((L + kFaBQ - 1) / kFaBQ, Hq, B);
   count_launch();
-  if (D == 128) fa_prefill_kernel<128><<<grid, kFaThreads, smem, st>>>(a);
-  else fa_prefill_kernel<64><<<grid, kFaThreads, smem, st>>>(a);
-  return cudaGetLastError();
+  return D == 128 ? launch_pdl(fa_prefill_kernel<128>, grid, dim3(kFaThreads), smem, st, a)
+                  : launch_pdl(fa_prefill_kernel<64>, grid, dim3(kFaThreads), smem, st, a);
 }
 
 }  // namespace pie

@@ -154,8 +154,6 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   __shared__ __align__(8) uint64_t q_full[2], q_empty[2], k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], o_full[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
-  pdl_launch_dependents();
-  pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -182,6 +180,8 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
   volatile int* const abortp = &abort_flag;
+  pdl_launch_dependents();
+  pdl_wait();   // (the set-up above ran under the end of the launch before this one)
 
   // All barriers are counted over the CTA's items: a role keeps the number of key tiles (of its query tile, of K and V) before its item.
   // Registers: 384 threads x 168 at launch = 64512; the eight softmax warps hold a row of scores each and take 216, the other
@@ -458,8 +458,7 @@ static cudaError_t launch_fap(const CUtensorMap& mq, const CUtensorMap& mk, cons
   if (set != cudaSuccess) return set;
   count_launch();
   const long long items = (long long)a.B * a.Hq * a.qt;
-  fa_prefill_umma_kernel<D><<<(unsigned)(items < num_sms() ? items : num_sms()), T::THREADS, T::SMEM, st>>>(mq, mk, mv, a);
-  return cudaGetLastError();
+  return launch_pdl(fa_prefill_umma_kernel<D>, dim3((unsigned)(items < num_sms() ? items : num_sms())), dim3(T::THREADS), T::SMEM, st, mq, mk, mv, a);
 }
 
 cudaError_t launch_fa_prefill_umma(uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc, const KvLayout& kv, int B,

@@ -1,10 +1,10 @@
 // The host side of calls of few rows, natively: nn.fused_rows (a norm, matrices of one input, and what follows them), the two launches of a
 // feed-forward, and a decode step's attention (rotation and cache write, attention).  Each looks the layers and the activations over and makes the
 // launches.  From Python a launch spends 13 of its 19 us on attributes, checks, argument tables and conversions, and a decode layer makes
-// eight.  The second launch of a native call also overlaps the end of the first (programmatic dependent launch): what it reads ahead
-// of its wait, weights, the first does not write, and that one waits for all before it.  One row of a 1B feed-forward, whose kernels take 9 us: 39 us
-// from Python, 18.5 as two native calls, 17.8 as one; a 1B layer's step of 4 to 8 sequences, attention from Python / natively: 137 -> 57 to 62 (8-bit
-// cache 165 -> 68), of an 8B model with five over 7000 tokens of 8-bit cache 166 -> 135.  What they do not take in full they leave to the Python
+// eight.  Launches are programmatic dependents of whatever is before them on the stream and only ask L2 for weights ahead of their wait; the
+// second of a native call reads them ahead of it: the first does not write them, and starts its dependents behind its own wait for all before it.  One row of a 1B feed-forward, whose kernels take 9 us: 39 us
+// from Python, 18.5 as two native calls, 14.9 as one; a 1B layer's step of 4 to 8 sequences, attention from Python / natively: 137 -> 57 to 62 (8-bit
+// cache 165 -> 68), of an 8B model with five over 7000 tokens of 8-bit cache 166 -> 128.  What they do not take in full they leave to the Python
 // form, which also reports what is wrong: None.
 //
 // Nothing is kept between calls but the addresses of the library's functions.
@@ -156,7 +156,7 @@ Answer rows_call(const at::Tensor& x, PyObject* device, PyObject* const* linears
   } else {
     status = lib.pie_qmv_fused(out.mutable_data_ptr(), (int)N, x.const_data_ptr(), (int)K, (int)M, (int)K, segs, nseg, 64, (int)bits, norm_w,
                                (float)eps, epi, res, 0, ws.defined() ? ws.mutable_data_ptr() : nullptr, ws.defined() ? (size_t)ws.numel() : 0,
-                               chained, stream);
+                               chained ? 1 : 2, stream);
   }
   Py_END_ALLOW_THREADS
   return status == PIE_OK ? DONE : NOT_MINE;

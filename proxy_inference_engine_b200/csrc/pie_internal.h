@@ -52,6 +52,7 @@ struct QmvArgs {
   int out_ld;
   const uint16_t* residual;  // EPI_RESADD (ld = out_ld)
   int epi;
+  int late;              // 1: weights are asked of L2 ahead of the dependency wait, and read behind it
   float* ws_part;        // [ntiles][ksplit][128 * mt] fp32, only if ksplit > 1
   unsigned int* ws_cnt;  // [ntiles], zero before the first launch, self-cleaning
 };

@@ -107,6 +107,8 @@ __device__ __forceinline__ float rms_row_scale(float ss, int dims, float eps) {
 }
 template <int NV>
 __global__ void __launch_bounds__(256) rms_norm_rows_kernel(uint16_t* out, const uint16_t* x, const uint16_t* w, int nvec, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   const uint4* xr = reinterpret_cast<const uint4*>(x) + (size_t)blockIdx.x * nvec;
   uint4* o = reinterpret_cast<uint4*>(out) + (size_t)blockIdx.x * nvec;
   uint4 v[NV], wv[NV];
@@ -140,6 +142,8 @@ __global__ void __launch_bounds__(256) rms_norm_rows_kernel(uint16_t* out, const
 }
 __global__ void __launch_bounds__(256) rms_norm_kernel(uint16_t* out, const uint16_t* x, const uint16_t* w,
                                                        int dims, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   const uint16_t* xr = x + (size_t)blockIdx.x * dims;
   uint16_t* o = out + (size_t)blockIdx.x * dims;
   float ss = 0.f;
@@ -162,13 +166,10 @@ cudaError_t launch_rms_norm(uint16_t* out, const uint16_t* x, const uint16_t* w,
   count_launch();
   const unsigned n = (unsigned)rows;
   if (dims % 8 == 0 && dims <= 8192 && all_aligned16(out, x, w)) {
-    if (dims <= 2048) rms_norm_rows_kernel<1><<<n, 256, 0, st>>>(out, x, w, dims / 8, eps);
-    else if (dims <= 4096) rms_norm_rows_kernel<2><<<n, 256, 0, st>>>(out, x, w, dims / 8, eps);
-    else rms_norm_rows_kernel<4><<<n, 256, 0, st>>>(out, x, w, dims / 8, eps);
-  } else {
-    rms_norm_kernel<<<n, 256, 0, st>>>(out, x, w, dims, eps);
+    auto rows_kernel = dims <= 2048 ? rms_norm_rows_kernel<1> : dims <= 4096 ? rms_norm_rows_kernel<2> : rms_norm_rows_kernel<4>;
+    return launch_pdl(rows_kernel, dim3(n), dim3(256), 0, st, out, x, w, dims / 8, eps);
   }
-  return cudaGetLastError();
+  return launch_pdl(rms_norm_kernel, dim3(n), dim3(256), 0, st, out, x, w, dims, eps);
 }
 
 // ---- a11 glue (PIE/models/llama/language.py:126-127,150-154; nn.silu activations.py:125-132) ----------------
@@ -185,6 +186,8 @@ struct Add {
 };
 template <class Op>
 __global__ void __launch_bounds__(256) pairwise_kernel(uint16_t* out, const uint16_t* a, const uint16_t* b, long long nvec, long long n) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long step = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
 #pragma unroll 4
   for (long long i = first; i < nvec; i += step) {
@@ -198,8 +201,7 @@ static cudaError_t launch_pairwise(uint16_t* out, const uint16_t* a, const uint1
   if (n == 0) return cudaSuccess;
   count_launch();
   const long long nvec = all_aligned16(out, a, b) ? n / 8 : 0, items = nvec ? nvec : n, grid = (items + 255) / 256;
-  pairwise_kernel<Op><<<(unsigned)(grid < num_sms() * 8 ? grid : num_sms() * 8), 256, 0, st>>>(out, a, b, nvec, n);
-  return cudaGetLastError();
+  return launch_pdl(pairwise_kernel<Op>, dim3((unsigned)(grid < num_sms() * 8 ? grid : num_sms() * 8)), dim3(256), 0, st, out, a, b, nvec, n);
 }
 cudaError_t launch_silu_mul(uint16_t* out, const uint16_t* g, const uint16_t* u, long long n, cudaStream_t st) {
   return launch_pairwise<SiluMul>(out, g, u, n, st);

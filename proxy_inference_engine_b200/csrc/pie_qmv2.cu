@@ -48,7 +48,7 @@ size_t qmv2_smem_bytes(int M, int K) {
 }
 
 // ------------------------------------------------------------------------------------------- the kernel
-template <bool ONECOL, bool F16, bool DUAL>
+template <bool ONECOL, bool F16, bool DUAL, bool LATE>
 __global__ void __launch_bounds__(kQ2Warps * 32, 1) qmv2_kernel(const __grid_constant__ Qmv2Args a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -129,7 +129,12 @@ __global__ void __launch_bounds__(kQ2Warps * 32, 1) qmv2_kernel(const __grid_con
   // in every warp's staging path).  PIE_QMV2_DBG: 8 = both before the wait, 16 = both behind x, 4 = both after the staging.
   Q2_STAMP(8)
   const int pf_mode = a.dbg & (4 | 8 | 16);
-  if (pf_mode == 0 || pf_mode == 8) {
+  if (LATE) {
+    if (p_u < ue && elect_one()) {
+      q2_prefetch_unit(a, p_tile, p_kc);
+      if (p_u + 1 < ue) q2_prefetch_unit(a, p_kc + 1 == upt ? p_tile + 1 : p_tile, p_kc + 1 == upt ? 0 : p_kc + 1);
+    }
+  } else if (pf_mode == 0 || pf_mode == 8) {
     if (p_u < ue) { if (elect_one()) issue(p_tile, p_kc, 0); advance(); }
     if (pf_mode == 8 && p_u < ue) { if (elect_one()) issue(p_tile, p_kc, 1); advance(); }
   }
@@ -138,8 +143,10 @@ __global__ void __launch_bounds__(kQ2Warps * 32, 1) qmv2_kernel(const __grid_con
     if ((pf_mode == 0 || pf_mode == 16) && p_u < ue) { if (elect_one()) issue(p_tile, p_kc, 1); advance(); }
   };
   Q2_STAMP(1)
+  if (LATE) pdl_wait();   // (only then may the next launch start: it may read weights ahead of its own wait)
   pdl_launch_dependents();
   pdl_wait();
+  if (LATE && p_u < ue) { if (elect_one()) issue(p_tile, p_kc, 0); advance(); }
   Q2_STAMP(2)
   unsigned int tp_e = 0, tp_set = 0;
   if (ONECOL && a.tp_mode == 1) { tp_e = *reinterpret_cast<volatile unsigned int*>(a.tp_epoch); tp_set = tp_e & 1u; }
@@ -578,9 +585,9 @@ unsigned long long* next_stamp_slot() {
   return g_stamp_buf + (g_stamp_next++) * (kStampSlotBytes / 8);
 }
 
-template <bool ONECOL, bool F16, bool DUAL>
+template <bool ONECOL, bool F16, bool DUAL, bool LATE>
 static cudaError_t launch_qmv2_t(const Qmv2Args& a, bool pdl, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(qmv2_kernel<ONECOL, F16, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQmvMaxSmem);
+  cudaError_t e = cudaFuncSetAttribute(qmv2_kernel<ONECOL, F16, DUAL, LATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQmvMaxSmem);
   if (e != cudaSuccess) return e;
   const int grid = a.tiles_q > 0 ? num_sms() : a.ntiles;   // (launch_qmv2 set the partition for this grid)
   cudaLaunchConfig_t cfg = {};
@@ -594,14 +601,15 @@ static cudaError_t launch_qmv2_t(const Qmv2Args& a, bool pdl, cudaStream_t st) {
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
   count_launch();
-  return cudaLaunchKernelEx(&cfg, qmv2_kernel<ONECOL, F16, DUAL>, a);
+  return cudaLaunchKernelEx(&cfg, qmv2_kernel<ONECOL, F16, DUAL, LATE>, a);
 }
 template <bool ONECOL, bool F16>
-static cudaError_t launch_qmv2_d(const Qmv2Args& a, bool pdl, cudaStream_t st) {
-  return a.dual ? launch_qmv2_t<ONECOL, F16, true>(a, pdl, st) : launch_qmv2_t<ONECOL, F16, false>(a, pdl, st);
+static cudaError_t launch_qmv2_d(const Qmv2Args& a, int pdl, cudaStream_t st) {   // (2: a kernel of its own, the decode step's has every instruction counted)
+  if (pdl == 2) return a.dual ? launch_qmv2_t<ONECOL, F16, true, true>(a, true, st) : launch_qmv2_t<ONECOL, F16, false, true>(a, true, st);
+  return a.dual ? launch_qmv2_t<ONECOL, F16, true, false>(a, pdl != 0, st) : launch_qmv2_t<ONECOL, F16, false, false>(a, pdl != 0, st);
 }
 
-cudaError_t launch_qmv2(const Qmv2Args& a0, bool pdl, cudaStream_t st) {
+cudaError_t launch_qmv2(const Qmv2Args& a0, int pdl, cudaStream_t st) {
   Qmv2Args a = a0;
   a.stamps = next_stamp_slot();
   {

@@ -55,7 +55,7 @@ bool qmv2_supported(int M, int K, int bits, int group_size, const pie_qmv_seg* s
 int build_qmv2_args(Qmv2Args& a, void* out, int out_ld, const void* x, int x_ld, int M, int K, const pie_qmv_seg* segs,
                     int nseg, const void* norm_weight, float eps, int epilogue, const void* residual,
                     const pie_tp_fused* tp = nullptr);
-cudaError_t launch_qmv2(const Qmv2Args& a, bool pdl, cudaStream_t st);
+cudaError_t launch_qmv2(const Qmv2Args& a, int pdl, cudaStream_t st);   // pdl: 0, 1, 2 as pie_qmv_fused's
 // profiling aid (pie_debug_stamps): slots of 256 CTAs x 16 stamps handed to consecutive launches
 constexpr size_t kStampSlotBytes = 256 * 16 * 8;
 void debug_stamps(void* buf, size_t bytes);

@@ -146,6 +146,23 @@ __device__ __forceinline__ void q2_issue_unit(const Qmv2Args& d, const Qmv2Args&
   }
 }
 
+// The same arrays of a unit on their way to L2.
+__device__ __forceinline__ void q2_prefetch_4d(const CUtensorMap* map, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(0) : "memory");
+}
+__device__ __forceinline__ void q2_prefetch_unit(const Qmv2Args& a, int tile, int kc) {
+  int si = 0;
+  if (!a.dual && a.nseg > 1 && tile >= a.tile0[1]) si = 1;
+  if (!a.dual && a.nseg > 2 && tile >= a.tile0[2]) si = 2;
+  const int r0 = a.dual ? tile * 8 : (tile - a.tile0[si]) * 16;
+#pragma unroll 1
+  for (int m = si; m < (a.dual && !a.gu_stacked ? 2 : si + 1); ++m) {
+    q2_prefetch_4d(&a.wmap[m], 0, r0, 2 * kc);
+    q2_prefetch_4d(&a.smap[m], 8 * kc, r0, 0);
+    if (!a.sb_stacked) q2_prefetch_4d(&a.bmap[m], 8 * kc, r0, 0);
+  }
+}
+
 // ------------------------------------------------------------------------------------------- x staging
 // x (optionally RMS-normalised: mx.fast.rms_norm, MLX/mlx/fast.cpp:93-111) -> shared memory in B-fragment order:
 // within every block of 16 k, position 4 m + 2 h + l holds k = m + 8 h + 4 l (what lane t of the MMA needs for step m).

@@ -329,7 +329,13 @@ __device__ __forceinline__ void qmv_body(const QmvArgs& a_in, uint8_t* smem, boo
     prod_save();
   };
 
-  // ---- prologue: weights first (they never depend on the previous kernel), then x --------------------
+  // ---- prologue: weights first (they never depend on the previous kernel, unless it is not known: `late`), then x --------------------
+  if (MODE == QMV_FULL && !COHERENT && a.late) {
+    if (total > 0 && (lane & 7) == 0)   // a lane per row
+#pragma unroll
+      for (int i = 0; i < 4; ++i) l2_prefetch(i & 1 ? wsrc[i - 1] + wdelta[i >> 1] : wsrc[i], min(S - 1, nch) * kRowBytes);
+    pdl_wait();   // (only then may the next launch start: it may read weights ahead of its own wait)
+  }
 #pragma unroll
   for (int s = 0; s < S - 1; ++s) produce(MODE != QMV_MAIN);
   if (MODE == QMV_PREFETCH) return;

@@ -63,7 +63,7 @@ static cudaError_t launch_qmv_smemargs(const QmvArgs& a, int warps, int grid, bo
 cudaError_t launch_qmv(const QmvArgs& a, int bits, int warps, int grid, bool pdl, cudaStream_t st) {
   const int mt = qmv_mt(a.M);
   static const bool smemargs = getenv("PIE_QMV_SMEMARGS") && atoi(getenv("PIE_QMV_SMEMARGS")) != 0;
-  if (smemargs && bits == 4 && a.M == 1 && warps == 16) return launch_qmv_smemargs(a, warps, grid, pdl, st);
+  if (smemargs && !a.late && bits == 4 && a.M == 1 && warps == 16) return launch_qmv_smemargs(a, warps, grid, pdl, st);
   if (bits == 4) {
     if (a.M == 1) return launch_qmv_t<4, 1, true>(a, warps, grid, pdl, st);
     if (mt == 1) return launch_qmv_t<4, 1, false>(a, warps, grid, pdl, st);

@@ -215,7 +215,7 @@ def qmv_fused(x, linears, rows: int, K: int, N: int, bits: int, norm_weight, eps
         return None
     ws = qmv_workspace(_qmv_workspace_bytes(rows, N, K, bits, int(swiglu)), x.device)
     _lib.check(L.pie_qmv_fused(_p(out), N, _p(x), K, rows, K, segs, len(linears), 64, bits, _p(norm_weight), float(eps), epilogue,
-                               _p(residual), 0, _p(ws), ws.numel(), 0, _stream()), "qmv_fused")
+                               _p(residual), 0, _p(ws), ws.numel(), 2, _stream()), "qmv_fused")
     return out
 
 
