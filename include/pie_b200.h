@@ -243,7 +243,7 @@ int pie_kvq_append(void* q_out, const void* qkv, const pie_kvq_cache* cache_host
                    const float* freqs, int B, int Hq, int Hkv, int D, void* stream);
 int pie_kvq_write(const pie_kvq_cache* cache_host, const void* k, const void* v, int B, int Hkv, int L, int D,
                   int offset, void* stream);
-/* pie_rope_kv_rows with a quantised cache, up to 1024 rows (PIE_EUNSUPPORTED: more) */
+/* pie_rope_kv_rows with a quantised cache, up to 9216 rows of heads, B L (Hq + 2 Hkv) (PIE_EUNSUPPORTED: more) */
 int pie_rope_kvq_rows(void* q_out, const pie_kvq_cache* cache_host, const pie_head_rows* q, const pie_head_rows* k, const pie_head_rows* v,
                       int32_t* positions_out, const float* freqs, int B, int Hq, int Hkv, int L, int D, int offset, void* stream);
 int pie_decode_attn_q8_pick_splits(int B, int Hq, int Hkv, int max_context);

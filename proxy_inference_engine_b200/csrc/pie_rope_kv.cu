@@ -219,7 +219,8 @@ cudaError_t launch_rope_kv_rows(uint16_t* q_out, int32_t* pos_out, const RopeRow
                          reinterpret_cast<uintptr_t>(r.q) | reinterpret_cast<uintptr_t>(r.k) | reinterpret_cast<uintptr_t>(r.v);
   const long long strides = r.qs.sb | r.qs.sh | r.qs.sl | r.ks.sb | r.ks.sh | r.ks.sl | r.vs.sb | r.vs.sh | r.vs.sl | kv.batch_stride |
                             kv.head_stride | kv.tok_stride;
-  if ((long long)B * L > 64 && (ptrs & 15) == 0 && strides % 8 == 0) {
+  // 32 + 8 heads, rows: pairs / heads, us, 32 2.1 / 2.9, 48 2.9 / 2.9, 64 3.6 / 2.9, 256 13.2 / 3.6 (D 64; 128 the same)
+  if ((long long)B * L > 48 && (ptrs & 15) == 0 && strides % 8 == 0) {
     const int lanes = 128 / (D / 16), HL = (long long)B * L >= 1024 ? 4 : lanes, per = lanes / HL;
     return launch_pdl(rope_kv_heads_kernel, dim3((unsigned)((L + per - 1) / per), (unsigned)B), dim3(128), 0, st, q_out, pos_out, r, kc, vc, kv,
                       freqs, Hq, Hkv, L, D, offset, HL);
