@@ -7,6 +7,7 @@
 // that every load instruction covers whole 128-byte lines).  Partials (m, l, acc[D]) of the splits are
 // merged in split order by the last CTA to arrive (deterministic).
 #include "pie_internal.h"
+#include "pie_attn_merge.cuh"
 #include "pie_ptx.cuh"
 
 namespace pie {
@@ -153,28 +154,8 @@ __global__ void __launch_bounds__(128) decode_attn_kernel(const DecAttnArgs a) {
     }
   }
   if (a.nsplit == 1) return;
-  __threadfence();
-  __syncthreads();
-  const int cidx = (b * a.Hkv + kvh) * a.rg + rgi;
-  if (threadIdx.x == 0) s_last = (atomicAdd(&a.ws_cnt[cidx], 1u) == (unsigned)a.nsplit - 1);
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  for (int i = threadIdx.x; i < R * D; i += 128) {
-    const int r = i / D, d = i % D;
-    const float* rec = a.ws_part + (rec0 + (size_t)r * a.nsplit) * PW;
-    float mn = -INFINITY;
-    for (int s = 0; s < a.nsplit; ++s) mn = fmaxf(mn, ldcg_f32(rec + (size_t)s * PW + D));
-    float lt = 0.f, at = 0.f;
-    for (int s = 0; s < a.nsplit; ++s) {
-      const float ms = ldcg_f32(rec + (size_t)s * PW + D);
-      const float cw = ms == -INFINITY ? 0.f : exp2f(ms - mn);
-      lt += ldcg_f32(rec + (size_t)s * PW + D + 1) * cw;
-      at += ldcg_f32(rec + (size_t)s * PW + d) * cw;
-    }
-    a.out[((size_t)b * a.Hq + qh0 + r) * D + d] = f2bf(at / lt);
-  }
-  if (threadIdx.x == 0) a.ws_cnt[cidx] = 0;
+  if (last_to_arrive(&a.ws_cnt[(b * a.Hkv + kvh) * a.rg + rgi], a.nsplit, &s_last))
+    merge_splits<D>(a.out + ((size_t)b * a.Hq + qh0) * D, a.ws_part + rec0 * PW, R, a.nsplit);
 }
 
 }  // namespace pie

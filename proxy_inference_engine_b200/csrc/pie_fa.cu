@@ -14,6 +14,7 @@
 // rounded to bf16 for the second product.  GQA: the n_rep query heads of a kv head are separate CTAs; their K/V tiles
 // come from L2.
 #include "pie_internal.h"
+#include "pie_attn_merge.cuh"
 #include "pie_ptx.cuh"
 
 namespace pie {
@@ -242,7 +243,6 @@ __global__ void __launch_bounds__(kFaThreads) fa_decode_kernel(const __grid_cons
   constexpr int KC = D / 16, DT = D / 8, CPR = D / 8, TILE = kFaBKV * D * 2, PW = D + 2, NS = kFaDecStages;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ int s_last;
-  __shared__ float s_m[16][kFaMaxSplits], s_l[16][kFaMaxSplits], s_w[16][kFaMaxSplits];
   pdl_launch_dependents();
   pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
@@ -408,41 +408,8 @@ __global__ void __launch_bounds__(kFaThreads) fa_decode_kernel(const __grid_cons
     }
   }
   if (a.nsplit == 1) return;
-  __threadfence();
-  __syncthreads();
-  const int cidx = b * a.Hkv + kvh;
-  if (tid == 0) s_last = (atomicAdd(&a.ws_cnt[cidx], 1u) == (unsigned)a.nsplit - 1);
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  // merge of the splits: (max, sum) of every record first (one parallel round trip), then the weighted rows with the
-  // loads of 8 splits in flight per thread
-  for (int i = tid; i < n_rep * a.nsplit; i += kFaThreads) {
-    const int r = i / a.nsplit, sp = i % a.nsplit;
-    const float* pr = a.ws_part + (rec0 + (size_t)r * a.nsplit + sp) * PW;
-    s_m[r][sp] = ldcg_f32(pr + D);
-    s_l[r][sp] = ldcg_f32(pr + D + 1);
-  }
-  __syncthreads();
-  for (int i = tid; i < n_rep * a.nsplit; i += kFaThreads) {
-    const int r = i / a.nsplit, sp = i % a.nsplit;
-    float mn = -INFINITY;
-    for (int k = 0; k < a.nsplit; ++k) mn = fmaxf(mn, s_m[r][k]);
-    s_w[r][sp] = s_m[r][sp] == -INFINITY ? 0.f : exp2f(s_m[r][sp] - mn);
-  }
-  __syncthreads();
-  for (int i = tid; i < n_rep * D; i += kFaThreads) {
-    const int r = i / D, d = i % D;
-    const float* pr = a.ws_part + (rec0 + (size_t)r * a.nsplit) * PW + d;
-    float lt = 0.f, at = 0.f;
-#pragma unroll 8
-    for (int sp = 0; sp < a.nsplit; ++sp) {  // split order: deterministic
-      lt += s_l[r][sp] * s_w[r][sp];
-      at += ldcg_f32(pr + (size_t)sp * PW) * s_w[r][sp];
-    }
-    a.out[((size_t)b * a.Hq + qh0 + r) * D + d] = f2bf(at / lt);
-  }
-  if (tid == 0) a.ws_cnt[cidx] = 0;
+  if (last_to_arrive(&a.ws_cnt[b * a.Hkv + kvh], a.nsplit, &s_last))
+    merge_splits<D>(a.out + ((size_t)b * a.Hq + qh0) * D, a.ws_part + rec0 * PW, n_rep, a.nsplit);
 }
 
 cudaError_t launch_decode_attn_tc(uint16_t* out, const uint16_t* q, const uint16_t* kc, const uint16_t* vc,

@@ -17,6 +17,7 @@
 #include <stdlib.h>
 
 #include "pie_internal.h"
+#include "pie_attn_merge.cuh"
 #include "pie_ptx.cuh"
 
 namespace pie {
@@ -404,28 +405,8 @@ __global__ void __launch_bounds__(128, 2) decode_attn_q8_kernel(const DecAttnQAr
     }
   }
   if (a.nsplit == 1) return;
-  __threadfence();
-  __syncthreads();
-  const int cidx = (b * a.c.Hkv + kvh) * a.rg + rgi;
-  if (threadIdx.x == 0) s_last = (atomicAdd(&a.ws_cnt[cidx], 1u) == (unsigned)a.nsplit - 1);
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  for (int i = threadIdx.x; i < R * D; i += 128) {
-    const int r = i / D, d = i % D;
-    const float* rec = a.ws_part + (rec0 + (size_t)r * a.nsplit) * PW;
-    float mn = -INFINITY;
-    for (int s = 0; s < a.nsplit; ++s) mn = fmaxf(mn, ldcg_f32(rec + (size_t)s * PW + D));
-    float lt = 0.f, at = 0.f;
-    for (int s = 0; s < a.nsplit; ++s) {
-      const float ms = ldcg_f32(rec + (size_t)s * PW + D);
-      const float cw = ms == -INFINITY ? 0.f : exp2f(ms - mn);
-      lt += ldcg_f32(rec + (size_t)s * PW + D + 1) * cw;
-      at += ldcg_f32(rec + (size_t)s * PW + d) * cw;
-    }
-    a.out[((size_t)b * a.Hq + qh0 + r) * D + d] = f2bf(at / lt);
-  }
-  if (threadIdx.x == 0) a.ws_cnt[cidx] = 0;
+  if (last_to_arrive(&a.ws_cnt[(b * a.c.Hkv + kvh) * a.rg + rgi], a.nsplit, &s_last))
+    merge_splits<D>(a.out + ((size_t)b * a.Hq + qh0) * D, a.ws_part + rec0 * PW, R, a.nsplit);
 }
 
 // ---- the same attention on tensor cores (D = 128, up to 8 query heads per kv head) ---------------------------------
@@ -689,28 +670,8 @@ __global__ void __launch_bounds__(kQtThreads) decode_attn_q8_tc_kernel(const __g
     }
   }
   if (a.nsplit == 1) return;
-  __threadfence();
-  __syncthreads();
-  const int cidx = b * a.c.Hkv + kvh;
-  if (tid == 0) s_last = (atomicAdd(&a.ws_cnt[cidx], 1u) == (unsigned)a.nsplit - 1);
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  for (int i = tid; i < n_rep * D; i += kQtThreads) {
-    const int r = i / D, d = i % D;
-    const float* pr = a.ws_part + (rec0 + (size_t)r * a.nsplit) * PW;
-    float mn = -INFINITY;
-    for (int s = 0; s < a.nsplit; ++s) mn = fmaxf(mn, ldcg_f32(pr + (size_t)s * PW + D));
-    float lt = 0.f, at = 0.f;
-    for (int s = 0; s < a.nsplit; ++s) {
-      const float ms = ldcg_f32(pr + (size_t)s * PW + D);
-      const float cw = ms == -INFINITY ? 0.f : exp2f(ms - mn);
-      lt += ldcg_f32(pr + (size_t)s * PW + D + 1) * cw;
-      at += ldcg_f32(pr + (size_t)s * PW + d) * cw;
-    }
-    a.out[((size_t)b * a.Hq + qh0 + r) * D + d] = f2bf(at / lt);
-  }
-  if (tid == 0) a.ws_cnt[cidx] = 0;
+  if (last_to_arrive(&a.ws_cnt[b * a.c.Hkv + kvh], a.nsplit, &s_last))
+    merge_splits<D>(a.out + ((size_t)b * a.Hq + qh0) * D, a.ws_part + rec0 * PW, n_rep, a.nsplit);
 }
 
 static cudaError_t launch_decode_attn_q8_tc(const DecAttnQArgs& a, int B, cudaStream_t st) {
