@@ -160,10 +160,11 @@ class DecodeEngine:
             B, self.Hq, self.Hkv, max_context)
         # Two forms of decode attention.  Latency form: rope + KV append + SIMT flash-decode in ONE launch
         # (pie_decode_attn_fused).  Throughput form: pie_rope_kv_append + the tensor-core kernel of pie_fa.cu, which
-        # reads K/V once per kv head.  Measured per layer on B200 (8B shapes, us):
-        #   bs1 ctx500 10.8 / 12.9, bs1 ctx2048 16.9 / 17.4, bs1 ctx8000 40.5 / 22.2, bs4 ctx2048 32.6 / 23.1,
-        #   bs32 ctx2048 203 / 77  ->  the latency form while batch x context stays within 4096 keys.
-        self.attn_fused = (batch * max_context <= 4096) if attn_fused is None else attn_fused
+        # reads K/V once per kv head.  Measured a step of four 8B layers and the head on B200, us, one launch / two:
+        #   bs1 ctx512 247 / 248, ctx1000 254 / 253, ctx4000 303 / 275; bs4 ctx128 324 / 325, ctx300 330 / 329, ctx512 337 / 331,
+        #   ctx1000 369 / 348; bs8 ctx128 368 / 371, ctx300 383 / 375, ctx512 411 / 391
+        #   ->  the latency form while batch x context stays within 1024 keys.
+        self.attn_fused = (batch * max_context <= 1024) if attn_fused is None else attn_fused
         # the splits of a unit form one thread-block cluster and merge through distributed shared memory; measured on
         # B200 (8B, bs1): 3..6 splits cost the same, clusters of 8 are markedly slower to schedule -> cap at 6
         self.nsplit_fused = min(6, L.pie_decode_step_pick_splits(B, self.Hq, self.Hkv, max_context))
