@@ -186,3 +186,21 @@ def test_a_layer_on_a_stream_of_its_own_and_in_a_capture():
         fed.copy_(v)
         graph.replay()
         assert torch.equal(out, y)
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("rows", [1, 4, 9, 40, 200])
+def test_weights_written_by_the_launch_before(bits, rows):
+    """Launches set themselves up, and ask L2 for weights, under the end of the launch before them: what that one writes into the weights is what they multiply by."""
+    g, mlp, other = torch.Generator(device="cuda").manual_seed(rows), _block(bits, 64).mlp, _block(bits, 64, seed=1).mlp
+    x = torch.randn((rows, 512), generator=g, device="cuda").bfloat16()
+    names = [(l, n) for l in ("gate_proj", "up_proj", "down_proj") for n in ("weight", "scales", "biases")]
+    both = [[getattr(getattr(m, l), n).clone() for l, n in names] for m in (mlp, other)]
+    want = [mlp(x), other(x)]
+    assert not torch.equal(*want)
+    got = []
+    for i in range(60):
+        for (l, n), t in zip(names, both[i % 2]):
+            getattr(getattr(mlp, l), n).copy_(t)
+        got.append(mlp(x))
+    assert all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))
