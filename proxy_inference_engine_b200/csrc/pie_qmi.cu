@@ -10,9 +10,9 @@
 //     planes, x ~= rscale[m] * (128 * hi + lo) with |128 hi + lo| <= 16383 (15-bit fixed point against the row maximum: finer
 //     than the bf16 rounding of x for every element above 2^-6 of the maximum, 3e-5 of the maximum below), and the exact
 //     per-group sums of x for the bias term.  The planes are the MMA's int8 B operand: 64 "columns" = 32 rows x {hi, lo}.
-//   * qmi_kernel, persistent, 6 warps: warp 0 feeds a 6-stage ring (128 weight rows x 128 k = 16 KB + the planes' 64 x 128
+//   * qmi_kernel, persistent, 10 warps: warp 0 feeds a 6-stage ring (128 weight rows x 128 k = 16 KB + the planes' 64 x 128
 //     = 8 KB per stage) by TMA; warp 1 issues, per 64-element quantization group, two tcgen05.mma M128 N64 K32 into one of
-//     four TMEM accumulators (int32, exact); warps 2..5 (one TMEM lane quadrant each, a lane = a weight row) read a group's
+//     four TMEM accumulators (int32, exact); warps 2..9 (two to a TMEM lane quadrant, a lane = a weight row) read a group's
 //     accumulator back, form 128 hi + lo exactly in int32, and apply that group's scale and bias in fp32.
 //   * few-tile matrices are split along K over CTAs; partials meet in the workspace and the last slice to arrive sums them
 //     in slice order (deterministic), as in pie_qmd.cu.  Epilogues as the GEMV: store / residual add / SwiGLU (a unit then
@@ -36,13 +36,13 @@ constexpr int kQiMb = 32;        // activation rows (MMA N = 2 planes x 32)
 constexpr int kQiStages = 6;     // (8 measured no faster: the stream is not depth-limited)
 constexpr int kQiABytes = kQiRows * kQiBK, kQiBBytes = 2 * kQiMb * kQiBK, kQiStageBytes = kQiABytes + kQiBBytes;
 constexpr int kQiAcc = 4;        // TMEM accumulator sets (one per stage in flight: 2 groups x 64 columns each)
-constexpr int kQiThreads = 320;   // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue (two per TMEM lane quadrant: 16 rows of the batch each)
-constexpr int kQiMh = kQiMb / 2;
+constexpr int kQiThreads = 320;   // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue (two per TMEM lane quadrant)
+constexpr int kQiMh = kQiMb / 2;  // rows of the batch of an epilogue warp
 // epilogue operands travel by TMA too, one batch per 4 stages (8 groups): scales and biases of the tile's 128 rows
 // (16 B per row each) and the activations' group sums (8 x 32 floats)
 constexpr int kQiBatchStages = 4, kQiBatches = 3;
 constexpr int kQiSbBytes = kQiRows * 16, kQiGsBytes = 8 * kQiMb * 4, kQiBatchBytes = 2 * kQiSbBytes + kQiGsBytes;
-constexpr int kQiSmem = kQiStages * kQiStageBytes + kQiBatches * kQiBatchBytes + 1024;
+constexpr int kQiSmem = kQiStages * kQiStageBytes + kQiBatches * kQiBatchBytes + 4 * kQiMh * 32 * 4 + 1024;   // (up to 16 rows: four warps' sums on their way to the others)
 constexpr int kQiMaxK = 16384;   // the prep kernel keeps a row in registers
 // D = s32, A = u8, B = s8, both K-major, N = 64, M = 128   (cute::UMMA::InstrDescriptor)
 constexpr uint32_t kQiIdesc = (2u << 4) | (0u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
@@ -154,7 +154,17 @@ __device__ __forceinline__ void qi_tile_seg(const QmiArgs& a, int tile, int pass
   nb = (tile - a.seg[si].tile0) * kQiRows;
 }
 
+__device__ __forceinline__ void qi_prefetch_2d(const CUtensorMap* map, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(c0), "r"(c1) : "memory");
+}
+
 // ---- the matmul --------------------------------------------------------------------------------------------------------
+// SETS: with up to 16 rows the two epilogue warps of a quadrant take every other stage (2), with more a half of the batch each (1).  The epilogue is what
+// bounds the kernel: reading sums back, and 4 instructions for each, a conversion among them.  By halves of the batch the second warp worked for rows that
+// are not there.  16 rows, preparation included, us, halves -> stages in turn: 4096 x 4096 14.7 -> 13.2, 4096 x 14336 25.0 -> 22.2, 28672 x 4096 57.3 -> 49.2,
+// 128256 x 4096 126 -> 103 (5.3 TB/s of weights).  Tried and left, 32 rows, 128256 x 4096 126 us: 16 warps in two sets 127; conversions by additions to
+// accumulators that start at 3 2^22 138, with 16 warps 122 but the smaller ones slower (4096 x 4096 14.7 -> 15.0).
+template <int SETS>
 __global__ void __launch_bounds__(kQiThreads, 1) qmi_kernel(const __grid_constant__ QmiArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -173,7 +183,7 @@ __global__ void __launch_bounds__(kQiThreads, 1) qmi_kernel(const __grid_constan
   }
   if (tid == 0) {
     for (int i = 0; i < kQiStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-    for (int i = 0; i < kQiAcc; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
+    for (int i = 0; i < kQiAcc; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], SETS == 2 ? 4 : 8); }
     for (int i = 0; i < kQiBatches; ++i) { mbar_init(&sb_full[i], 1); mbar_init(&sb_empty[i], 8); }
     fence_mbar_init();
     fence_proxy_async();
@@ -187,14 +197,24 @@ __global__ void __launch_bounds__(kQiThreads, 1) qmi_kernel(const __grid_constan
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
-  pdl_wait();   // the planes, row scales and group sums of qmi_prep_kernel are complete and visible
-  pdl_launch_dependents();   // the next kernel may be scheduled as SMs free up; it waits for this grid before it reads
   // slice `sl` of a tile covers stages [kb, ke)
   auto k_range = [&](int sl, int& kb, int& ke) {
     const int nb4 = a.nstages / kQiBatchStages;   // whole batches: K is a multiple of 512
     kb = (int)((long long)sl * nb4 / a.ksplit) * kQiBatchStages;
     ke = (int)((long long)(sl + 1) * nb4 / a.ksplit) * kQiBatchStages;
   };
+
+  if (warp == 0 && lane == 0) {   // the first words on their way to L2 under the kernels before this one (nothing is read: they may have written them)
+    int si, nb, kb, ke;
+    k_range(blockIdx.x % a.ksplit, kb, ke);
+    qi_tile_seg(a, blockIdx.x / a.ksplit, 0, si, nb);
+    for (int ks = kb; ks < min(ke, kb + kQiStages); ++ks) {
+      qi_prefetch_2d(&a.wmap[si], ks * kQiBK, nb);
+      if (ks % kQiBatchStages == 0) { qi_prefetch_2d(&a.smap[si], 2 * ks, nb); qi_prefetch_2d(&a.bmap[si], 2 * ks, nb); }
+    }
+  }
+  pdl_wait();   // the planes, row scales and group sums of qmi_prep_kernel are complete and visible
+  pdl_launch_dependents();   // the next kernel may be scheduled as SMs free up; it waits for this grid before it reads
 
   if (warp == 0) {
     // ================= TMA producer ==================================================================================
@@ -267,9 +287,10 @@ __global__ void __launch_bounds__(kQiThreads, 1) qmi_kernel(const __grid_constan
       }
     }
   } else {
-    // ================= epilogue: TMEM lane quadrant warp % 4, lane = weight row, half = which 16 rows of the batch ======
-    const int quad = warp & 3, half = (warp - 2) >> 2, row = quad * 32 + lane, m0 = half * kQiMh;
-    unsigned gc = 0;
+    // ================= epilogue: TMEM lane quadrant warp % 4, lane = weight row, half = which 16 rows of the batch, set = which stages ======
+    const int quad = warp & 3, half = SETS == 1 ? (warp - 2) >> 2 : 0, set = SETS == 1 ? 0 : (warp - 2) >> 2, row = quad * 32 + lane, m0 = half * kQiMh;
+    float* const merge = reinterpret_cast<float*>(smem + kQiStages * kQiStageBytes + kQiBatches * kQiBatchBytes) + quad * (kQiMh * 32) + lane;
+    unsigned gc = 0;   // stages of all sets so far
     int bs = 0, buse = 0;
     for (int u = blockIdx.x; u < units; u += gridDim.x) {
       const int tile = u / a.ksplit, sl = u % a.ksplit;
@@ -290,12 +311,15 @@ __global__ void __launch_bounds__(kQiThreads, 1) qmi_kernel(const __grid_constan
           const uint8_t* bb = batch_base + bs * kQiBatchBytes;
           const uint4 sq = *reinterpret_cast<const uint4*>(bb + row * 16);
           const uint4 bq = *reinterpret_cast<const uint4*>(bb + kQiSbBytes + row * 16);
-          const uint32_t sw[4] = {sq.x, sq.y, sq.z, sq.w}, bw[4] = {bq.x, bq.y, bq.z, bq.w};
+          const uint32_t sws[4] = {sq.x, sq.y, sq.z, sq.w}, bws[4] = {bq.x, bq.y, bq.z, bq.w};
           const float4* gs_b = reinterpret_cast<const float4*>(bb + 2 * kQiSbBytes);
 #pragma unroll
-          for (int sg = 0; sg < kQiBatchStages; ++sg) {
-            const unsigned buf = gc & (kQiAcc - 1), n_use = gc / kQiAcc;   // gc counts stages
-            ++gc;
+          for (int i = 0; i < kQiBatchStages / SETS; ++i) {
+            const int sg = i * SETS + set;
+            const unsigned buf = (gc + set) & (kQiAcc - 1), n_use = gc / kQiAcc;
+            gc += SETS;
+            const uint32_t sw = SETS == 1 ? sws[i] : set ? sws[(2 * i + 1) & 3] : sws[(2 * i) & 3];   // two groups'
+            const uint32_t bw = SETS == 1 ? bws[i] : set ? bws[(2 * i + 1) & 3] : bws[(2 * i) & 3];
             if (a.dbg & 32) continue;
             mbar_wait(&acc_full[buf], n_use & 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -312,8 +336,7 @@ __global__ void __launch_bounds__(kQiThreads, 1) qmi_kernel(const __grid_constan
 #pragma unroll
             for (int g2 = 0; g2 < 2; ++g2) {
               const int g = 2 * sg + g2;
-              const float s = (g & 1) ? bf16hi(sw[g >> 1]) : bf16lo(sw[g >> 1]);
-              const float b = (g & 1) ? bf16hi(bw[g >> 1]) : bf16lo(bw[g >> 1]);
+              const float s = g2 ? bf16hi(sw) : bf16lo(sw), b = g2 ? bf16hi(bw) : bf16lo(bw);
 #pragma unroll
               for (int m4 = 0; m4 < kQiMh / 4; ++m4) {
                 const float4 q = gs_b[g * (kQiMb / 4) + half * (kQiMh / 4) + m4];
@@ -334,7 +357,18 @@ __global__ void __launch_bounds__(kQiThreads, 1) qmi_kernel(const __grid_constan
         }
 #pragma unroll
         for (int m = 0; m < kQiMh; ++m) acc1[m] = fmaf(__ldg(a.rscale + m0 + m), acc1[m], acc2[m]);
+        if (SETS == 2) {   // the two sets' sums of a row meet in set 0
+          if (set)
+#pragma unroll
+            for (int m = 0; m < kQiMh; ++m) merge[m * 32] = y[m];
+          asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");
+          if (!set)
+#pragma unroll
+            for (int m = 0; m < kQiMh; ++m) y[m] += merge[m * 32];
+          asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");
+        }
       }
+      if (set) continue;
       int si, nb;
       qi_tile_seg(a, tile, 0, si, nb);
       const int n = nb + row;
@@ -518,8 +552,9 @@ cudaError_t launch_qmi(void* out, int out_ld, const void* x, int x_ld, int M, in
   a.ws_part = (float*)((uint8_t*)gsum + ((((size_t)(K / kGroup) * kQiMb * 4) + 255) & ~(size_t)255));
   a.ws_cnt = ws_cnt;
   if (!qi_map(&a.xmap, xq, 2 * kQiMb, K, 2 * kQiMb)) return cudaErrorInvalidValue;
+  const auto kernel = M <= kQiMh ? qmi_kernel<2> : qmi_kernel<1>;
   {  // (per launch, not once per process: the attribute is per device)
-    cudaError_t e = cudaFuncSetAttribute(qmi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kQiSmem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kQiSmem);
     if (e != cudaSuccess) return e;
   }
   count_launch();
@@ -541,7 +576,7 @@ cudaError_t launch_qmi(void* out, int out_ld, const void* x, int x_ld, int M, in
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, qmi_kernel, a);
+  return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
 }  // namespace pie

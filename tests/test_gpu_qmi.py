@@ -74,3 +74,33 @@ def test_int8_form_zero_and_tiny_rows(env, monkeypatch):
     assert np.isfinite(y).all() and (y[2] == 0).all()
     assert rel_l2(np.delete(y, 5, 0), np.delete(ref, 5, 0)) < 2e-3
     assert np.abs(y[5]).max() <= 1e-25
+
+
+@pytest.mark.parametrize("K,N", [(512, 128), (512, 150 * 128), (4096, 384), (14336, 128)])      # a batch of stages; more tiles than SMs; K in slices
+@pytest.mark.parametrize("M", [9, 16, 17])
+def test_up_to_16_rows_stages_go_to_two_sets_of_warps(env, K, N, M, monkeypatch):
+    """Against float64.  x is held to half a 16383th of its row's largest value where it meets s q (against b its sums are exact), the sums are fp32 and the
+    result is rounded to bf16: |error| <= amax / 32766 sum s q + 2^-20 sum (s q + |b|) |x| + 2^-8 |y|.  SwiGLU's second tile, and the sums of one tile
+    where the next one's are kept, too."""
+    orc, ops = env
+    monkeypatch.setenv("PIE_QMI", "1")
+    g = torch.Generator(device="cuda").manual_seed(K + M)
+    x = torch.randn((M, K), generator=g, device="cuda").bfloat16()
+
+    def matrix():
+        q = torch.randint(0, 256, (N, K), generator=g, device="cuda", dtype=torch.uint8)
+        s = (torch.rand((N, K // 64), generator=g, device="cuda") / K ** 0.5 / 100).bfloat16()
+        b = (-128 * s.float()).bfloat16()
+        w = s.double().repeat_interleave(64, 1) * q.double() + b.double().repeat_interleave(64, 1)
+        return (q.view(torch.int32), s, b), w, s.double().repeat_interleave(64, 1) * q.double()
+
+    (up, wu, sq), (gate, wg, _) = matrix(), matrix()
+    y = ops.quantized_matmul(x, *up, True, 64, 8).double()
+    exact = x.double() @ wu.T
+    amax = x.double().abs().amax(1, keepdim=True)
+    bound = amax / 32766 * sq.sum(1) + 2 ** -20 * (x.double().abs() @ (sq + (wu - sq).abs()).T) + 2 ** -8 * exact.abs()
+    assert ((y - exact).abs() <= bound).all()
+    act = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    _fused(ops, act, x, [gate, up], M, K, 8, None, 2, None)
+    want = torch.nn.functional.silu(x.double() @ wg.T) * exact
+    assert float((act.double() - want).norm() / want.norm()) < 2 ** -6      # four bf16 roundings in a row, each 2^-8 at most
