@@ -191,12 +191,17 @@ __device__ __forceinline__ void umma_store(const LinArgs& a, int z, int row0, in
     return;
   }
   float y[32];
-  if (a.bias && n0 + 32 <= a.N) {
 #pragma unroll
-    for (int q = 0; q < 32; ++q) y[q] = __uint_as_float(v[q]) + __ldg(a.bias + n0 + q);
-  } else {
+  for (int q = 0; q < 32; ++q) y[q] = __uint_as_float(v[q]);
+  if (a.bias) {
+    if (n0 + 32 <= a.N) {
 #pragma unroll
-    for (int q = 0; q < 32; ++q) y[q] = __uint_as_float(v[q]) + (a.bias && n0 + q < a.N ? a.bias[n0 + q] : 0.f);
+      for (int q = 0; q < 32; ++q) y[q] += __ldg(a.bias + n0 + q);
+    } else {
+      const float mine = n0 + lane < a.N ? a.bias[n0 + lane] : 0.f;
+#pragma unroll
+      for (int q = 0; q < 32; ++q) y[q] += __shfl_sync(0xffffffffu, mine, q);
+    }
   }
   if (act_in_loop(a.epi)) {
     tile_act_out<OT>(a, reinterpret_cast<OT*>(a.out) + (size_t)z * a.out_bs, a.out_ld, row0, m_end, n0, a.N, y, buf, lane);
