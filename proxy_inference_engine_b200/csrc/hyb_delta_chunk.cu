@@ -4,15 +4,15 @@
 //   u_t = beta_t v_t - beta_t G_t S^T k_t - sum_{i < t} A[t, i] u_i,   A[t, i] = beta_t D[t, i] (k_t . k_i),
 // so U = U0 - W S, where U0 and W solve the same triangle for beta v and beta G k and know nothing of S; and with M[t, i] = D[t, i] (q_t . k_i), i <= t,
 //   o = M U0 + (G q - M W) S,       S <- G S + sum_i D[end, i] k_i u_i^T.
-// delta_chunk_kernel   a CTA per chunk and head, all at once: A, M, the triangle solved for the dk + dv columns of [W | U0], a thread a column of each with
-//                      their 32 values in registers, and the products of M with them.
+// delta_chunk_kernel   a CTA per chunk and head, all at once: A, M, the triangle solved for the dk + dv columns of [W | U0], a thread a column, and the products of M
+//                      with them.  (Half the threads with two columns each: 75 us for 56.)
 // delta_walk_kernel    a CTA per head and 16 columns of S walks the chunks: [W; G q - M W] S, and the update of S.
 // Ratios of decays are products of decays, never quotients: every one is at most 1 and none is 0 / 0 where a decay is tiny.  They and the products k . k and
 // q . k, which most of the error comes from, are computed in double (on its matrix instructions) and rounded once.  Off from float64 by, o / state, a token
 // at a time and so (1200 rows, 16 heads of 128 x 128, relative): keys as the model makes them 9.2e-8 / 8.0e-8 and 7.2e-8 / 7.5e-8, random 1.1e-7 / 8.0e-8 and
 // 7.8e-8 / 7.6e-8, keys that all but coincide 5.9e-8 / 7.4e-8 and 8.8e-8 / 9.7e-8.
 // The walk is a chain not of a token's few operations but of a chunk's two products through shared memory, which bound it: a token at a
-// time is 200 ns.  1200 rows, 16 heads of 128 x 128, one sequence: 245 us -> 185 (chunks 75, walk 109).
+// time is 200 ns.  1200 rows, 16 heads of 128 x 128, one sequence: 245 us -> 167 (chunks 56, walk 109).
 // A sum of the chunk form holds terms that come later than the token (with a zero in front), and is in parts that may be infinite where the whole is
 // not: where some u of a chunk, or some o, is no number, or infinite, the CTA takes that chunk a token at a time, so that it spoils what comes after it and
 // nothing else.
@@ -21,7 +21,7 @@
 namespace pieh {
 
 constexpr int kC = 32;                       // tokens of a chunk
-constexpr int kChunkThreads = 128, kWalkCols = 16, kWalkThreads = 256;
+constexpr int kChunkThreads = 256, kWalkCols = 16, kWalkThreads = 256;
 
 // scratch: W and G q - M W [T, H, dk], U0 [T, H, dv], (G_t, D[end, t]) [T, H, 2]
 struct ChunkScratch { float *w, *q, *u, *a; };
@@ -33,7 +33,7 @@ __device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
 }
 
-constexpr int kChunkCols = 2 * kChunkThreads;   // columns of [W | U0] in hand at once, two a thread
+constexpr int kChunkCols = kChunkThreads;   // columns of [W | U0] in hand at once, one a thread
 template <int DK>
 struct ChunkSmem {
   static constexpr int LD = DK + 4;
@@ -84,97 +84,79 @@ __global__ void __launch_bounds__(kChunkThreads, 3) delta_chunk_kernel(float* o,
     Gs[tid] = (float)g;
     if (tid < n) *reinterpret_cast<float2*>(s.a + ((size_t)(row0 + tid) * d.H + h) * 2) = make_float2((float)g, tid == n - 1 ? 1.f : (float)Ds[n - 1][tid]);
   }
-  // k . k and q . k in tiles of 8 x 8 on and below the diagonal, every fourth run of four k a warp; a tile's parts meet in one warp
-  double acc[20][2];             // [k . k, q . k][row of tiles r, column c <= r: r (r + 1) / 2 + c]
+  // k . k (warps 0 to 3) and q . k (4 to 7) in tiles of 8 x 8 on and below the diagonal, every fourth run of four k a warp; a tile's parts meet in one warp
+  const int part = warp & 3;
+  const bool with_q = warp >= 4;
+  double acc[10][2];             // [row of tiles r, column e <= r: r (r + 1) / 2 + e]
 #pragma unroll
-  for (int j = 0; j < 20; ++j) acc[j][0] = acc[j][1] = 0.;
+  for (int j = 0; j < 10; ++j) acc[j][0] = acc[j][1] = 0.;
 #pragma unroll 1
-  for (int c = 4 * warp; c < DK; c += 16) {
-    double kf[4], qf[4];
+  for (int c = 4 * part; c < DK; c += 16) {
+    double kf[4], xf[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      kf[r] = ks[(8 * r + (lane >> 2)) * LD + c + (lane & 3)];
-      qf[r] = qs[(8 * r + (lane >> 2)) * LD + c + (lane & 3)];
+      const int at = (8 * r + (lane >> 2)) * LD + c + (lane & 3);
+      kf[r] = ks[at];
+      xf[r] = with_q ? qs[at] : ks[at];
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int e = 0; e <= r; ++e) {
-        mma_f64(acc[r * (r + 1) / 2 + e], kf[r], kf[e]);
-        mma_f64(acc[10 + r * (r + 1) / 2 + e], qf[r], kf[e]);
-      }
+      for (int e = 0; e <= r; ++e) mma_f64(acc[r * (r + 1) / 2 + e], xf[r], kf[e]);
   }
-  double2* const parts = reinterpret_cast<double2*>(xs);
+  double2* const parts = reinterpret_cast<double2*>(xs) + (with_q ? 10 * 3 * 32 : 0);
 #pragma unroll
-  for (int j = 0; j < 20; ++j) {
-    const int from = ((warp - j) & 3) - 1;   // -1: the tile's own warp
+  for (int j = 0; j < 10; ++j) {
+    const int from = ((part - j) & 3) - 1;   // -1: the tile's own warp
     if (from >= 0) parts[(j * 3 + from) * 32 + lane] = make_double2(acc[j][0], acc[j][1]);
   }
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int e = 0; e <= r; ++e)
+    for (int e = 0; e <= r; ++e) {
+      const int j = r * (r + 1) / 2 + e;
+      if ((j & 3) == part) {
+        double y[2] = {acc[j][0], acc[j][1]};
 #pragma unroll
-      for (int w = 0; w < 2; ++w) {
-        const int j = 10 * w + r * (r + 1) / 2 + e;
-        if ((j & 3) == warp) {
-          double y[2] = {acc[j][0], acc[j][1]};
-#pragma unroll
-          for (int f = 0; f < 3; ++f) {
-            const double2 part = parts[(j * 3 + f) * 32 + lane];
-            y[0] += part.x; y[1] += part.y;
-          }
-          const int t = 8 * r + (lane >> 2);
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int m = 8 * e + 2 * (lane & 3) + u;
-            if (w) { if (m <= t) Ms[t * kC + m] = (float)(m < t ? Ds[t][m] * y[u] : y[u]); }
-            else if (m < t) As[t * kC + m] = (float)((double)bs[t] * Ds[t][m] * y[u]);
-          }
+        for (int f = 0; f < 3; ++f) {
+          const double2 p = parts[(j * 3 + f) * 32 + lane];
+          y[0] += p.x; y[1] += p.y;
         }
-      }
-  __syncthreads();
-  // Columns c and c + 128 of [W | U0]: eight rows at a time, what the rows before them take from them in a loop (unrolled, the triangle is more
-  // instructions than the caches hold), and the products of M with them on the way
-  for (int c0 = tid; c0 < dk + dv; c0 += kChunkCols) {
-    const int col[2] = {c0, c0 + kChunkThreads};
-    bool has[2], is_v[2];
-    size_t at[2], step[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      has[u] = col[u] < dk + dv;
-      is_v[u] = col[u] >= dk;
-      step[u] = (size_t)d.H * (is_v[u] ? dv : dk);
-      at[u] = is_v[u] ? ((size_t)row0 * d.H + h) * dv + (col[u] - dk) : ((size_t)row0 * d.H + h) * dk + col[u];
-#pragma unroll 8
-      for (int t = 0; t < kC; ++t)
-        xs[t * kChunkCols + u * kChunkThreads + tid] =
-            !has[u] ? 0.f : bs[t] * (is_v[u] ? (t < n ? v[at[u] + t * step[u]] : 0.f) : Gs[t] * ks[t * LD + col[u]]);
-    }
-#pragma unroll 1
-    for (int t0 = 0; t0 < kC; t0 += 8) {
-      float y[2][8], m[2][8];
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int r = 0; r < 8; ++r) y[u][r] = m[u][r] = 0.f;
-#pragma unroll 1
-      for (int j = 0; j < t0; j += 4) {
-        float4 x[2];
+        const int t = 8 * r + (lane >> 2);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          const float* p = xs + j * kChunkCols + u * kChunkThreads + tid;
-          x[u] = make_float4(p[0], p[kChunkCols], p[2 * kChunkCols], p[3 * kChunkCols]);
-        }
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          const float4 a = *reinterpret_cast<const float4*>(As + (t0 + r) * kC + j), mm = *reinterpret_cast<const float4*>(Ms + (t0 + r) * kC + j);
-#pragma unroll
-          for (int u = 0; u < 2; ++u) { y[u][r] += dot4(a, x[u]); m[u][r] += dot4(mm, x[u]); }
+          const int m = 8 * e + 2 * (lane & 3) + u;
+          if (with_q) { if (m <= t) Ms[t * kC + m] = (float)(m < t ? Ds[t][m] * y[u] : y[u]); }
+          else if (m < t) As[t * kC + m] = (float)((double)bs[t] * Ds[t][m] * y[u]);
         }
       }
-      float x[2][8];
+    }
+  __syncthreads();
+  // A column of [W | U0] a thread: eight rows at a time, what the rows before them take from them in a loop (unrolled, the triangle is more
+  // instructions than the caches hold), and the products of M with them on the way
+  for (int c0 = tid; c0 < dk + dv; c0 += kChunkCols) {
+    const bool is_v = c0 >= dk;
+    const size_t step = (size_t)d.H * (is_v ? dv : dk), at = is_v ? ((size_t)row0 * d.H + h) * dv + (c0 - dk) : ((size_t)row0 * d.H + h) * dk + c0;
+    float* const column = xs + tid;
+#pragma unroll 8
+    for (int t = 0; t < kC; ++t) column[t * kChunkCols] = bs[t] * (is_v ? (t < n ? v[at + t * step] : 0.f) : Gs[t] * ks[t * LD + c0]);
+#pragma unroll 1
+    for (int t0 = 0; t0 < kC; t0 += 8) {
+      float y[8], m[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) y[r] = m[r] = 0.f;
+#pragma unroll 1
+      for (int j = 0; j < t0; j += 4) {
+        const float* const p = column + j * kChunkCols;
+        const float4 x = make_float4(p[0], p[kChunkCols], p[2 * kChunkCols], p[3 * kChunkCols]);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          y[r] += dot4(*reinterpret_cast<const float4*>(As + (t0 + r) * kC + j), x);
+          m[r] += dot4(*reinterpret_cast<const float4*>(Ms + (t0 + r) * kC + j), x);
+        }
+      }
+      float x[8];
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
         const float* const ar = As + (t0 + r) * kC + t0;
@@ -182,25 +164,19 @@ __global__ void __launch_bounds__(kChunkThreads, 3) delta_chunk_kernel(float* o,
         const float4 a0 = *reinterpret_cast<const float4*>(ar), a1 = *reinterpret_cast<const float4*>(ar + 4);
         const float4 m0 = *reinterpret_cast<const float4*>(mr), m1 = *reinterpret_cast<const float4*>(mr + 4);
         const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, mm[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+        float p = 0.f, f = 0.f;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          float p = 0.f, f = 0.f;
-#pragma unroll
-          for (int e = 0; e < r; ++e) { p = fmaf(a[e], x[u][e], p); f = fmaf(mm[e], x[u][e], f); }
-          float* const place = xs + (t0 + r) * kChunkCols + u * kChunkThreads + tid;
-          x[u][r] = *place - (y[u][r] + p);
-          *place = x[u][r];
-          m[u][r] += fmaf(mm[r], x[u][r], f);
-        }
+        for (int e = 0; e < r; ++e) { p = fmaf(a[e], x[e], p); f = fmaf(mm[e], x[e], f); }
+        float* const place = column + (t0 + r) * kChunkCols;
+        x[r] = *place - (y[r] + p);
+        *place = x[r];
+        m[r] += fmaf(mm[r], x[r], f);
         const int t = t0 + r;
-        if (t < n)
-#pragma unroll
-          for (int u = 0; u < 2; ++u)
-            if (has[u]) {
-              (is_v[u] ? s.u : s.w)[at[u] + t * step[u]] = x[u][r];
-              if (is_v[u]) o[at[u] + t * step[u]] = m[u][r];
-              else s.q[at[u] + t * step[u]] = fmaf(Gs[t], qs[t * LD + col[u]], -m[u][r]);
-            }
+        if (t < n) {
+          (is_v ? s.u : s.w)[at + t * step] = x[r];
+          if (is_v) o[at + t * step] = m[r];
+          else s.q[at + t * step] = fmaf(Gs[t], qs[t * LD + c0], -m[r]);
+        }
       }
     }
   }
@@ -450,8 +426,8 @@ static cudaError_t launch_chunks(float* o, const float* q, const float* k, const
 
 // Where chunks are sooner done than a token at a time: as long as every column of S has an SM of its own (beyond that the other kernel, of which six CTAs
 // share an SM, loses nothing), from sequences of some 200 tokens on.  us, a token at a time / chunks, 16 heads of
-// 128 x 128: 128 tokens 30 / 42, 256 56 / 52, 400 85 / 70, 4096 825 / 613; four sequences of 300 166 / 199; 32 heads, 1200 tokens 325 / 385; 16 heads of 64 x 64: 128 tokens
-// 27 / 33, 256 50 / 43, 1200 214 / 134.  (Scratch is 1.5 KB a row and head: up to half a GB, some 20000 rows.)
+// 128 x 128: 128 tokens 30 / 36, 256 56 / 46, 400 85 / 63, 4096 825 / 560; four sequences of 300 166 / 179; 32 heads, 1200 tokens 325 / 349; 16 heads of 64 x 64: 128 tokens
+// 27 / 29, 256 50 / 39, 1200 214 / 124.  (Scratch is 1.5 KB a row and head: up to half a GB, some 20000 rows.)
 static bool chunks_pay(const pieh_delta& d, const pieh_batch& b) {
   return d.dk % 4 == 0 && d.dk > 32 && d.dk <= 128 && d.dv % 4 == 0 && b.n_tiles > 0 && b.T >= 192LL * b.n_seq &&
          (size_t)b.T * d.H * chunk_floats(d.dk, d.dv) * 4 <= (size_t)512 << 20 &&
