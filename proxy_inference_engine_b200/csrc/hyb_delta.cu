@@ -74,7 +74,8 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(float* q, float* k, 
 }
 
 // The same with a WARP per token and unit, four channels a lane (16-byte loads; units of n = dk or dv channels, multiples of 4):
-// no barrier, a quarter of the loads and of the index arithmetic.  1200 rows of 48 units of 128: 84.9 -> 39.0 us.  TAPS: the convolution's length, its weights in registers.
+// no barrier, a quarter of the loads and of the index arithmetic.  1200 rows of 48 units of 128: 84.9 -> 39.0 us, and 30.5 with a channel's
+// weights in one load (a load a weight is 16 lines of 128 bytes each time, more than the rows').  TAPS: the convolution's length, its weights in registers.
 template <int TAPS>
 __global__ void __launch_bounds__(256) delta_prepare_warp_kernel(float* q, float* k, float* v, float* beta, float* decay,
                                                                  const float* proj, long long ld, const pieh_delta d,
@@ -89,11 +90,13 @@ __global__ void __launch_bounds__(256) delta_prepare_warp_kernel(float* q, float
   for (int c0 = 4 * lane; c0 < ((n + 127) & ~127); c0 += 128) {   // n <= 128 here unless the unit is a value (see below)
     const bool in = c0 < n;
     const int c = base + (in ? c0 : 0);
+    static_assert(TAPS == 4, "a channel's weights are one load");
     float w[4][TAPS];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-#pragma unroll
-      for (int r = 0; r < TAPS; ++r) w[e][r] = __ldg(d.conv_w + (size_t)(c + e) * TAPS + r);
+    for (int e = 0; e < 4; ++e) {
+      const float4 f = __ldg(reinterpret_cast<const float4*>(d.conv_w) + c + e);
+      w[e][0] = f.x; w[e][1] = f.y; w[e][2] = f.z; w[e][3] = f.w;
+    }
 #pragma unroll
     for (int x = 0; x < TOKENS; ++x) {
       const int t = blockIdx.x * TOKENS + x;
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(256) delta_prepare_warp_kernel(float* q, float
 static bool delta_prepare_by_warps(const float* q, const float* k, const float* v, const float* proj, long long ld,
                                    const pieh_delta& d, int T) {
   const uintptr_t p = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
-                      reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(d.conv_state);
+                      reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(d.conv_state) | reinterpret_cast<uintptr_t>(d.conv_w);
   return (long long)T * (2 * d.G + d.H) >= 6144 && d.taps == 4 && d.dk <= 128 && d.dk % 4 == 0 && d.dv % 4 == 0 && ld % 4 == 0 && (p & 15) == 0;
 }
 
