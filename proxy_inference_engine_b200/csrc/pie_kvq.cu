@@ -787,11 +787,12 @@ int pie_decode_attn_q8_pick_splits(int B, int Hq, int Hkv, int max_context) {
   const int n_rep = Hq / Hkv, R = n_rep % 4 == 0 ? 4 : (n_rep % 2 == 0 ? 2 : 1);
   const long long units = (long long)B * Hkv * (n_rep <= 8 ? 1 : n_rep / R);   // <= 8: the tensor-core kernel, one CTA per kv head
   // two CTAs of four warps fit an SM, and a split of 128 tokens still pays for its part of the merge; a second CTA on an SM slows the first down, so it has to
-  // save 256.  Measured (D 128, 8 kv heads, us at 1 / 2 / 4 / 8 / 15 / 32 splits): bs1 ctx1000 13.3 / 9.8 / 7.2 / 6.0 / 6.6, bs1 ctx4000 45.4 / 26.2 / 15.4 /
-  // 10.2 / 8.8 / 9.3, bs2 ctx2000 24.4 / 15.3 / 9.9 / 7.5 / 9.0 / 12.5, bs4 ctx500 8.1 / 7.3 / 5.9 / 6.4, bs8 ctx1066 14.8 / 11.1 / 9.8 / 11.4, bs16 ctx1000
-  // 14.8 / 13.7 / 17.3, bs32 ctx2048 33 / 38 / 38
-  const long long one = num_sms() / units, two = 2LL * num_sms() / units, by_ctx = max_context / 128;
-  long long n = one >= by_ctx ? by_ctx : std::max(one, std::min(two, by_ctx / 2));
+  // save 256, and more than 16 splits pay from 512 tokens each.  Measured (D 128, 8 kv heads, us at 1 / 2 / 4 / 8 / 15 / 32 splits): bs1 ctx1000 13.3 / 9.8 /
+  // 7.2 / 6.0 / 6.6, bs1 ctx4000 45.4 / 26.2 / 15.4 / 10.2 / 8.8 / 9.3, bs2 ctx2000 24.4 / 15.3 / 9.9 / 7.5 / 9.0 / 12.5, bs4 ctx500 8.1 / 7.3 / 5.9 / 6.4, bs8
+  // ctx1066 14.8 / 11.1 / 9.8 / 11.4, bs16 ctx1000 14.8 / 13.7 / 17.3, bs32 ctx2048 33 / 38 / 38
+  const long long one = num_sms() / units, two = 2LL * num_sms() / units;
+  const long long by_ctx = std::max<long long>({max_context / 512, std::min(16, max_context / 256), std::min<long long>({16, one, max_context / 128})});
+  long long n = std::min(two, by_ctx);
   if (n > 64) n = 64;
   return n < 1 ? 1 : (int)n;
 }
