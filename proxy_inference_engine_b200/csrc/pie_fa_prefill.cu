@@ -26,8 +26,8 @@
 // Measured, 32 query / 8 kv heads, us (TFLOP/s): the mma.sync kernel of pie_fa.cu -> this one with a lane of its own issuing the MMAs
 // and all exponentials on the approximation unit -> as it is.  D 128: 8192 tokens 2190 (251) -> 547 (1005) -> 460 (1196); 2 x 3000
 // tokens 640 (231) -> 190 (774) -> 164 (901).  D 64: 1531 behind 517 92 -> 51 -> 42; 8192 tokens 485 -> 386 (712).
-// (Behind the last arrow: warm, before the walk.)  What is left is one tile's chain, which the other tile covers only in part: of about 3000 cycles per pair of tiles, 1700 are a
-// softmax and 1300 the two products and their hand-overs.
+// (The last figures are those of a CTA an item.)  What is left is one tile's chain, which the other tile covers only in part: of about 3000
+// cycles per pair of tiles, 1700 are a softmax and 1300 the two products and their hand-overs.
 #include "pie_gemm.cuh"
 #include "pie_internal.h"
 
