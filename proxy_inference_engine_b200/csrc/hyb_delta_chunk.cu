@@ -425,11 +425,11 @@ static cudaError_t launch_chunks(float* o, const float* q, const float* k, const
 }
 
 // Where chunks are sooner done than a token at a time: as long as every column of S has an SM of its own (beyond that the other kernel, of which six CTAs
-// share an SM, loses nothing), from sequences of some 200 tokens on.  us, a token at a time / chunks, 16 heads of
-// 128 x 128: 128 tokens 30 / 36, 256 56 / 46, 400 85 / 63, 4096 825 / 560; four sequences of 300 166 / 179; 32 heads, 1200 tokens 325 / 349; 16 heads of 64 x 64: 128 tokens
-// 27 / 29, 256 50 / 39, 1200 214 / 124.  (Scratch is 1.5 KB a row and head: up to half a GB, some 20000 rows.)
+// share an SM, loses nothing), from sequences of 224 tokens on (from some 150 the two are within 5 us, and this is one launch more).  us, a token at a time /
+// chunks, 16 heads of 128 x 128: 128 tokens 30 / 36, 256 56 / 46, 400 85 / 63, 4096 825 / 560; four sequences of 300 166 / 179; 32 heads, 1200 tokens 325 / 349; 16
+// heads of 64 x 64: 128 tokens 27 / 29, 256 50 / 39, 1200 214 / 124.  (Scratch is 1.5 KB a row and head: up to half a GB, some 20000 rows.)
 static bool chunks_pay(const pieh_delta& d, const pieh_batch& b) {
-  return d.dk % 4 == 0 && d.dk > 32 && d.dk <= 128 && d.dv % 4 == 0 && b.n_tiles > 0 && b.T >= 192LL * b.n_seq &&
+  return d.dk % 4 == 0 && d.dk > 32 && d.dk <= 128 && d.dv % 4 == 0 && b.n_tiles > 0 && b.T >= 224LL * b.n_seq &&
          (size_t)b.T * d.H * chunk_floats(d.dk, d.dv) * 4 <= (size_t)512 << 20 &&
          (long long)b.n_seq * d.H * ((d.dv + kWalkCols - 1) / kWalkCols) <= num_sms();
 }
