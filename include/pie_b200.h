@@ -178,6 +178,8 @@ int pie_rope_kv_rows(void* q_out, void* kcache, void* vcache, const pie_kv_layou
  * captured in a CUDA graph; splits beyond the current context are empty and cost nothing.              */
 size_t pie_decode_attn_workspace_bytes(int B, int Hq, int D, int nsplit);
 int pie_decode_attn_pick_splits(int B, int Hq, int Hkv, int max_context);
+/* ... for heads of D, which may pay for more */
+int pie_decode_attn_pick_splits_for(int B, int Hq, int Hkv, int D, int max_context);
 int pie_decode_attn(void* out, const void* q, const void* kcache, const void* vcache,
                     const pie_kv_layout* kv_host, const int32_t* positions, int B, int Hq, int Hkv, int D,
                     float scale, int nsplit, void* workspace, size_t workspace_bytes, void* stream);

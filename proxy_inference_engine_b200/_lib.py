@@ -113,6 +113,7 @@ SIGNATURES = {
     "pie_kv_write": (_i, [_vp, _vp, C.POINTER(KvLayout), _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "pie_decode_attn_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "pie_decode_attn_pick_splits": (_i, [_i, _i, _i, _i]),
+    "pie_decode_attn_pick_splits_for": (_i, [_i, _i, _i, _i, _i]),
     "pie_decode_attn": (_i, [_vp, _vp, _vp, _vp, C.POINTER(KvLayout), _vp, _i, _i, _i, _i, _f, _i, _vp, _sz, _vp]),
     "pie_rope_table": (_i, [_vp, _vp, _vp, _i, _i, _vp]),
     "pie_kvq_append": (_i, [_vp, _vp, C.POINTER(KvqCache), _vp, _vp, _i, _i, _i, _i, _vp]),

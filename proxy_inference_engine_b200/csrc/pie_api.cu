@@ -6,6 +6,7 @@
 
 #include <atomic>
 #include <cstdio>
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 

@@ -23,7 +23,7 @@ namespace {
 
 #define PIE_FUNCTIONS(X)                                                                                                                \
   X(pie_qmv_fused) X(pie_qmv_workspace_bytes) X(pie_qmt) X(pie_qmt_scratch_bytes) X(pie_rope_kv_rows) X(pie_rope_kvq_rows)                \
-  X(pie_decode_attn) X(pie_decode_attn_pick_splits) X(pie_decode_attn_q8) X(pie_decode_attn_q8_pick_splits) X(pie_decode_attn_workspace_bytes)
+  X(pie_decode_attn) X(pie_decode_attn_pick_splits_for) X(pie_decode_attn_q8) X(pie_decode_attn_q8_pick_splits) X(pie_decode_attn_workspace_bytes)
 struct Library {
 #define X(name) decltype(&::name) name = nullptr;
   PIE_FUNCTIONS(X)
@@ -264,7 +264,7 @@ Answer attend_call(const at::Tensor& qkv, PyObject* device, PyObject* at_, PyObj
   }
   held.push_back(*freqs);
   const int splits = quantized ? lib.pie_decode_attn_q8_pick_splits(B, (int)Hq, (int)Hkv, (int)offset + 1)
-                               : lib.pie_decode_attn_pick_splits(B, (int)Hq, (int)Hkv, (int)offset + 1);
+                               : lib.pie_decode_attn_pick_splits_for(B, (int)Hq, (int)Hkv, (int)D, (int)offset + 1);
   at::Tensor ws;
   if (const Answer a = buffer(Py_BuildValue("(lnO)", (long)B * Hq, (Py_ssize_t)lib.pie_decode_attn_workspace_bytes(B, (int)Hq, (int)D, splits), device),
                               attention_workspace, ws))

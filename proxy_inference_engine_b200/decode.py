@@ -156,8 +156,8 @@ class DecodeEngine:
         L = _lib.load()
         self.L = L
         self.watch = ops.PipelineWatch(L, "pie")
-        self.nsplit = (L.pie_decode_attn_q8_pick_splits if kv_bits is not None else L.pie_decode_attn_pick_splits)(
-            B, self.Hq, self.Hkv, max_context)
+        self.nsplit = (L.pie_decode_attn_q8_pick_splits(B, self.Hq, self.Hkv, max_context) if kv_bits is not None
+                       else L.pie_decode_attn_pick_splits_for(B, self.Hq, self.Hkv, self.D, max_context))
         # Two forms of decode attention.  Latency form: rope + KV append + SIMT flash-decode in ONE launch
         # (pie_decode_attn_fused).  Throughput form: pie_rope_kv_append + the tensor-core kernel of pie_fa.cu, which
         # reads K/V once per kv head.  Measured a step of four 8B layers and the head on B200, us, one launch / two:

@@ -411,7 +411,7 @@ def decode_attention(q, kbuf, vbuf, lay: KvLayout, positions, scale: float, nspl
     Hkv = kbuf.shape[1] if lay.page_table is None else kbuf.shape[2]
     L = _lib.load()
     if nsplit <= 0:
-        nsplit = L.pie_decode_attn_pick_splits(B, Hq, Hkv, max_context if max_context > 0 else 1)
+        nsplit = L.pie_decode_attn_pick_splits_for(B, Hq, Hkv, D, max_context if max_context > 0 else 1)
     nb = L.pie_decode_attn_workspace_bytes(B, Hq, D, nsplit)
     ws = attention_workspace(B * Hq, nb, q.device)
     out = torch.empty((B, Hq * D), dtype=_BF16, device=q.device)
