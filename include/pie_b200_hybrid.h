@@ -117,12 +117,6 @@ int pieh_delta_prepare(float* q, float* k, float* v, float* beta, float* decay, 
  * starts from zero whatever the slot holds); o fp32 [T, H, dv]. */
 int pieh_delta_scan(float* o, const float* q, const float* k, const float* v, const float* beta, const float* decay,
                     const pieh_delta* d, const pieh_batch* b, void* stream);
-/* pieh_delta_scan for prompts, 32 tokens at a time: the same recurrence, fp32, with its sums in another order.  dk a multiple of 4 up to 128, dv one of
- * 4, with a tile list; o, q, k and scratch 16-byte aligned.  pieh_delta_scan_scratch: the bytes it needs where it is sooner done than pieh_delta_scan,
- * 0 elsewhere. */
-size_t pieh_delta_scan_scratch(const pieh_delta* d, const pieh_batch* b);
-int pieh_delta_scan_chunks(float* o, const float* q, const float* k, const float* v, const float* beta, const float* decay, const pieh_delta* d,
-                           const pieh_batch* b, void* scratch, size_t scratch_bytes, void* stream);
 /* out[t, h, :] = o[t, h, :] / rms(o[t, h, :]) * out_norm * silu(gate[t, h, :]); gate = proj + gate_off, row stride ld */
 int pieh_delta_gate(void* out, int out_dtype, const float* o, const float* proj, long long ld, long long gate_off,
                     const pieh_delta* d, int T, void* stream);

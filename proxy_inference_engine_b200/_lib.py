@@ -265,8 +265,6 @@ HYBRID_SIGNATURES = {
     "pieh_stream_update": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "pieh_delta_prepare": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _ll, _PD, _PB, _vp]),
     "pieh_delta_scan": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _PD, _PB, _vp]),
-    "pieh_delta_scan_scratch": (_sz, [_PD, _PB]),
-    "pieh_delta_scan_chunks": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _PD, _PB, _vp, _sz, _vp]),
     "pieh_delta_gate": (_i, [_vp, _i, _vp, _vp, _ll, _ll, _PD, _i, _vp]),
     "pieh_attn_prepare": (_i, [_vp, _vp, _ll, _PA, _PB, _vp]),
     "pieh_attn_run": (_i, [_vp, _i, _vp, _PA, _PB, _vp]),

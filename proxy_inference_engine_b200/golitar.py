@@ -235,14 +235,8 @@ class GolitarModel:
                 o = torch.empty_like(v)
                 _lib.check_hybrid(L.pieh_delta_prepare(_p(q), _p(k), _p(v), _p(beta), _p(decay), _p(proj), ld, C.byref(d),
                                                        bref, _stream()), "delta_prepare")
-                nb = L.pieh_delta_scan_scratch(C.byref(d), bref)
-                if nb:     # a prompt: 32 tokens at a time
-                    scratch = torch.empty(nb, dtype=torch.uint8, device=dev)
-                    _lib.check_hybrid(L.pieh_delta_scan_chunks(_p(o), _p(q), _p(k), _p(v), _p(beta), _p(decay), C.byref(d), bref, _p(scratch), nb,
-                                                               _stream()), "delta_scan_chunks")
-                else:
-                    _lib.check_hybrid(L.pieh_delta_scan(_p(o), _p(q), _p(k), _p(v), _p(beta), _p(decay), C.byref(d), bref,
-                                                        _stream()), "delta_scan")
+                _lib.check_hybrid(L.pieh_delta_scan(_p(o), _p(q), _p(k), _p(v), _p(beta), _p(decay), C.byref(d), bref,
+                                                    _stream()), "delta_scan")
                 mixed = torch.empty((T, H * dv), dtype=self.act_torch, device=dev)
                 _lib.check_hybrid(L.pieh_delta_gate(_p(mixed), self.act, _p(o), _p(proj), ld, 2 * G * dk + H * dv,
                                                     C.byref(d), T, _stream()), "delta_gate")
