@@ -53,6 +53,8 @@ const char* pie_status_string(int status);
 const char* pie_last_cuda_error(void);
 /* number of kernels this library has launched since load (the bench's gpu_launches claim) */
 unsigned long long pie_launch_count(void);
+/* which capture into a graph `stream` is in (the same number for all streams of one capture); 0: none */
+unsigned long long pie_capture_id(void* stream);
 /* 1: a bounded wait inside the prefill GEMM (pie_qmm) or the prefill attention (pie_prefill_attn) expired since the library was
  * loaded or pie_pipeline_error_clear() was called, and that call's results are void; 0: none did.  Reads a device word: synchronises. */
 unsigned int pie_pipeline_error(void);

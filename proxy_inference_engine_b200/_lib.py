@@ -95,6 +95,7 @@ SIGNATURES = {
     "pie_qmv": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _sz, _vp]),
     "pie_qmv_fused": (_i, [_vp, _i, _vp, _i, _i, _i, C.POINTER(QmvSeg), _i, _i, _i, _vp, _f, _i, _vp, _i, _vp,
                            _sz, _i, _vp]),
+    "pie_capture_id": (C.c_ulonglong, [_vp]),
     "pie_qmt_scratch_bytes": (_sz, [_i, _ll, _i, _i, _i, _i]),
     "pie_qmt": (_i, [_vp, _i, _vp, _i, _i, _i, C.POINTER(QmvSeg), _i, _i, _i, _vp, _f, _i, _vp, _vp, _sz, _vp]),
     "pie_qmm_swiglu_pays": (_i, [_i, _i, _i, _i, _i]),

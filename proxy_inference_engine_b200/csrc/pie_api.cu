@@ -207,6 +207,12 @@ const char* pie_status_string(int s) {
 }
 const char* pie_last_cuda_error(void) { return g_cuda_err; }
 unsigned long long pie_launch_count(void) { return g_launches.load(); }
+unsigned long long pie_capture_id(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  const cudaError_t e = cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &id);
+  return e == cudaSuccess && status == cudaStreamCaptureStatusActive ? id : 0;
+}
 
 int pie_quantize(const void* w, int dtype, uint32_t* wq, void* scales, void* biases, long long rows, int K,
                  int group_size, int bits, void* stream) {

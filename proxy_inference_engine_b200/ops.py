@@ -11,6 +11,7 @@ import ctypes as C
 import functools
 import importlib.util
 import os
+import threading
 import warnings
 
 import torch
@@ -75,17 +76,35 @@ def _check_gs_bits(what, group_size, bits, full=False):
                          "(supported: group_size 64, bits 4 or 8)")
 
 
+def _capture_id() -> int:
+    """Which capture into a graph the current stream is in; 0: none."""
+    return _lib.load().pie_capture_id(_stream()) if torch.cuda.is_current_stream_capturing() else 0
+
+
 class _Workspaces:
-    """Zero-initialised scratch owned by the host side (the library never allocates)."""
+    """Zero-initialised scratch owned by the host side (the library never allocates).
+
+    A launch leaves its counters at zero for the next one in its buffer, so a buffer is for launches that come one after the other: one thread's, on one stream.  In a
+    capture the buffers are the graph's, zeroed as part of it and kept for as long as the capture goes on: an eager call never sees one, and no graph holds the address of an
+    eager call's, which is given back when a larger one is asked for.  A thread keeps the last KEEP of them, and gives them back when it ends."""
+
+    KEEP = 96   # (a decode step's attention has one per 64 rows x query heads)
 
     def __init__(self):
-        self.bufs = {}
+        self.mine = threading.local()
 
     def get(self, key, nbytes, device):
-        buf = self.bufs.get((key, device))
+        mine, capture = self.mine.__dict__, _capture_id()
+        if mine.get("capture") != capture:
+            mine["capture"], mine["captured"] = capture, {}
+        bufs = mine["captured"] if capture else mine.setdefault("eager", {})
+        key = (key, device, _stream())
+        buf = bufs.get(key)
         if buf is None or buf.numel() < nbytes:
-            buf = torch.zeros(max(int(nbytes), 256), dtype=torch.uint8, device=device)
-            self.bufs[(key, device)] = buf
+            bufs.pop(key, None)
+            buf = bufs[key] = torch.zeros(max(int(nbytes), 256), dtype=torch.uint8, device=device)
+            if len(bufs) > self.KEEP:
+                del bufs[next(iter(bufs))]   # the oldest; its memory is used again in its stream's order
         return buf
 
 
