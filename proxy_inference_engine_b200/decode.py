@@ -160,11 +160,11 @@ class DecodeEngine:
                        else L.pie_decode_attn_pick_splits_for(B, self.Hq, self.Hkv, self.D, max_context))
         # Two forms of decode attention.  Latency form: rope + KV append + SIMT flash-decode in ONE launch
         # (pie_decode_attn_fused).  Throughput form: pie_rope_kv_append + the tensor-core kernel of pie_fa.cu, which
-        # reads K/V once per kv head.  Measured a step of four 8B layers and the head on B200, us, one launch / two:
-        #   bs1 ctx512 247 / 248, ctx1000 254 / 253, ctx4000 303 / 275; bs4 ctx128 324 / 325, ctx300 330 / 329, ctx512 337 / 331,
-        #   ctx1000 369 / 348; bs8 ctx128 368 / 371, ctx300 383 / 375, ctx512 411 / 391
-        #   ->  the latency form while batch x context stays within 1024 keys.
-        self.attn_fused = (batch * max_context <= 1024) if attn_fused is None else attn_fused
+        # reads K/V once per kv head.  The form stands for every position of the engine's room.  A step of four 8B layers and the head on B200, us, one launch /
+        # two, at position 100 and at the end of the room: bs1 room 2048 243 / 261, 266 / 264; bs1 room 4096 244 / 261, 304 / 272; bs2 room 2048 304 / 319, 345 / 330;
+        # bs4 room 1024 324 / 330, 369 / 348; bs8 room 512 369 / 375, 411 / 391; bs8 ctx 2000 622 / 515
+        #   ->  the latency form while batch x room stays within 4096 keys: what a nearly empty room loses to two launches it loses at most of its positions.
+        self.attn_fused = (batch * max_context <= 4096) if attn_fused is None else attn_fused
         # the splits of a unit form one thread-block cluster and merge through distributed shared memory; measured on
         # B200 (8B, bs1): 3..6 splits cost the same, clusters of 8 are markedly slower to schedule -> cap at 6
         self.nsplit_fused = min(6, L.pie_decode_step_pick_splits(B, self.Hq, self.Hkv, max_context))
