@@ -156,8 +156,16 @@ class DecodeEngine:
         L = _lib.load()
         self.L = L
         self.watch = ops.PipelineWatch(L, "pie")
-        self.nsplit = (L.pie_decode_attn_q8_pick_splits(B, self.Hq, self.Hkv, max_context) if kv_bits is not None
-                       else L.pie_decode_attn_pick_splits_for(B, self.Hq, self.Hkv, self.D, max_context))
+        # The number of splits stands for every position of the room, and more than one is a sum of partial results at each of them: more than one only where
+        # that pays soon.  A step of four layers and the head on B200, us, one split / more: 8-bit cache bs8 room 512 (8B) 365 / 372 at position 40 and 376 / 378 at 300,
+        # bs16 room 1000 (1B) 251 / 259 at 40, 281 / 281 at 660; heads of 64, bs32 room 2048 327 / 338 at 40, 374 / 373 at 660, 464 / 444 at the end.  From two on, more of
+        # them cost nothing (8-bit cache bs1 room 1500, 2 / 11 splits: 265 / 255 at 40, 285 / 257 at 1000).
+        if kv_bits is not None:
+            self.nsplit = L.pie_decode_attn_q8_pick_splits(B, self.Hq, self.Hkv, max_context) if max_context >= 1024 else 1
+        elif L.pie_decode_attn_pick_splits(B, self.Hq, self.Hkv, max_context) > 1:
+            self.nsplit = L.pie_decode_attn_pick_splits_for(B, self.Hq, self.Hkv, self.D, max_context)
+        else:
+            self.nsplit = 1
         # Two forms of decode attention.  Latency form: rope + KV append + SIMT flash-decode in ONE launch
         # (pie_decode_attn_fused).  Throughput form: pie_rope_kv_append + the tensor-core kernel of pie_fa.cu, which
         # reads K/V once per kv head.  The form stands for every position of the engine's room.  A step of four 8B layers and the head on B200, us, one launch /

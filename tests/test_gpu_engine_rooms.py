@@ -24,3 +24,9 @@ def engine():
 @pytest.mark.parametrize("batch,room,one", [(1, 64, True), (1, 4096, True), (1, 4097, False), (4, 1024, True), (4, 1025, False), (32, 128, True), (32, 129, False)])
 def test_one_launch_up_to_4096_keys(engine, batch, room, one):
     assert engine(128, batch, room).attn_fused == one
+
+
+@pytest.mark.parametrize("D,kv_bits,batch,room,splits", [(128, 8, 1, 1023, 1), (128, 8, 1, 1024, 8), (64, 8, 8, 600, 1), (128, 8, 32, 2048, 1), (64, None, 32, 2048, 1),
+                                                         (64, None, 16, 2048, 4), (128, None, 16, 2048, 2), (128, None, 1, 64, 1)])
+def test_splits_only_where_they_pay_soon(engine, D, kv_bits, batch, room, splits):
+    assert engine(D, batch, room, kv_bits=kv_bits).nsplit == splits
