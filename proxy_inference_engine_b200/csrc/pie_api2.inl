@@ -187,9 +187,10 @@ int pie_decode_attn_pick_splits_for(int B, int Hq, int Hkv, int D, int max_conte
   if (D != 64 || B <= 0 || Hq <= 0 || Hkv <= 0 || Hq / Hkv > 16) return ns;
   // Heads of 64: a CTA's stages are half the bytes and four fit an SM, which a wave of two leaves waiting for memory.  Up to four while a split has 128 tokens;
   // us, two / four: bs32 ctx2048 38.1 / 26.8, ctx6000 103.5 / 67.9, ctx500 13.1 / 11.8, bs16 ctx1000 14.7 / 11.8, bs8 ctx4000 22.9 / 17.5, ctx1066 9.9 / 8.4, bs5
-  // ctx7002 23.0 / 18.2.
+  // ctx7002 23.0 / 18.2.  Not for a few more (bs4 ctx1300 9 / 10 splits 9.2 / 9.7), nor a first sum of splits below 384 (bs32 ctx256 8.3 / 8.9, ctx384 10.7 / 10.7, ctx450
+  // 13.2 / 11.9).
   const int more = std::min({148 * 4 / (B * Hkv), max_context / 128, 32});   // (kFaMaxSplits)
-  return std::max(ns, more);
+  return (ns == 1 && max_context < 384) || more < ns + (ns + 3) / 4 ? ns : more;
 }
 
 int pie_decode_attn(void* out, const void* q, const void* kcache, const void* vcache, const pie_kv_layout* kv,

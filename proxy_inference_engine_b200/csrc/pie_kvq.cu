@@ -789,8 +789,12 @@ int pie_decode_attn_q8_pick_splits(int B, int Hq, int Hkv, int max_context) {
   // two CTAs of four warps fit an SM, and a split of 128 tokens still pays for its part of the merge; a second CTA on an SM slows the first down, so it has to
   // save 256, and more than 16 splits pay from 512 tokens each.  Measured (D 128, 8 kv heads, us at 1 / 2 / 4 / 8 / 15 / 32 splits): bs1 ctx1000 13.3 / 9.8 /
   // 7.2 / 6.0 / 6.6, bs1 ctx4000 45.4 / 26.2 / 15.4 / 10.2 / 8.8 / 9.3, bs2 ctx2000 24.4 / 15.3 / 9.9 / 7.5 / 9.0 / 12.5, bs4 ctx500 8.1 / 7.3 / 5.9 / 6.4, bs8
-  // ctx1066 14.8 / 11.1 / 9.8 / 11.4, bs16 ctx1000 14.8 / 13.7 / 17.3, bs32 ctx2048 33 / 38 / 38
+  // ctx1066 14.8 / 11.1 / 9.8 / 11.4, bs16 ctx1000 14.8 / 13.7 / 17.3, bs32 ctx2048 33 / 38 / 38; at 16 / 24 / 32 / 64: bs1 ctx8192 12.1 / 13.1 / 12.2 / 18.3, ctx12000
+  // 14.6 / 14.9 / 13.9 / 20.6, ctx32768 28.5 / 27.2 / 23.3 / 30.2.
+  // A first sum of splits costs what two splits save of some 300 tokens, of 700 where the two share an SM (1 / 2 / 3 splits): bs1 ctx300 5.8 / 6.4, ctx384 6.5 / - / 5.8, bs8
+  // ctx300 6.6 / 7.2, ctx384 7.4 / 7.3, ctx450 8.9 / 8.1; bs16 ctx512 9.2 / 9.8, ctx640 10.6 / 10.8, ctx800 12.7 / 12.7, ctx1000 14.8 / 13.7
   const long long one = num_sms() / units, two = 2LL * num_sms() / units;
+  if (max_context < (one < 2 ? 800 : 384)) return 1;
   const long long by_ctx = std::max<long long>({max_context / 512, std::min(16, max_context / 256), std::min<long long>({16, one, max_context / 128})});
   long long n = std::min(two, by_ctx);
   if (n > 64) n = 64;

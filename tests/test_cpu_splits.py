@@ -15,3 +15,15 @@ def test_heads_of_64_may_have_more_splits(heads, B, ctx):
     assert more >= few
     if more > few:
         assert heads[0] // heads[1] <= 16 and more <= 32 and ctx // more >= 128 and B * heads[1] * more <= 4 * 148
+
+
+@pytest.mark.parametrize("B,ctx,splits", [(1, 383, 1), (1, 384, 3), (8, 383, 1), (8, 450, 2), (10, 799, 1), (16, 799, 1), (16, 800, 2), (16, 1300, 2), (75, 9000, 1), (1, 8192, 16)])
+def test_8_bit_splits_only_where_their_sum_pays(B, ctx, splits):
+    """Two of 128 tokens, or two on one SM below 400 each, measured slower than one."""
+    assert _lib.load().pie_decode_attn_q8_pick_splits(B, 32, 8, ctx) == splits
+
+
+@pytest.mark.parametrize("B,ctx,splits", [(32, 383, 1), (32, 384, 2), (4, 1300, 9), (8, 640, 5), (4, 1536, 12), (16, 384, 3)])
+def test_heads_of_64_have_more_splits_only_where_that_pays(B, ctx, splits):
+    """A first sum of splits, and one split more of nine, measured slower."""
+    assert _lib.load().pie_decode_attn_pick_splits_for(B, 32, 8, 64, ctx) == splits
