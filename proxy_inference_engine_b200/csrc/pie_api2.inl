@@ -163,19 +163,15 @@ size_t pie_decode_attn_workspace_bytes(int B, int Hq, int D, int nsplit) {
 int pie_decode_attn_pick_splits(int B, int Hq, int Hkv, int max_context) {
   if (B <= 0 || Hq <= 0 || Hkv <= 0) return 1;
   const int n_rep = Hq / Hkv;
-  int ctas, want;
-  if (n_rep <= 16) {  // tensor-core kernel: one CTA per (sequence, kv head, split), 2 resident per SM (96 KB of stages)
-    ctas = B * Hkv;
-    want = 148 * 2;
-  } else {
-    const int rg = n_rep % 4 == 0 ? n_rep / 4 : (n_rep % 2 == 0 ? n_rep / 2 : n_rep);
-    ctas = B * Hkv * rg;
-    want = 148 * 4;
+  long long ctas = (long long)B * Hkv, want = 2LL * num_sms();   // tensor-core kernel: one CTA per (sequence, kv head, split), 2 resident per SM (96 KB of stages)
+  if (n_rep > 16) {
+    ctas *= n_rep % 4 == 0 ? n_rep / 4 : (n_rep % 2 == 0 ? n_rep / 2 : n_rep);
+    want *= 2;
   }
   // ONE wave of resident CTAs, never a wave and a fraction: measured on B200 (8B shapes, paged, us per layer at
   // 1 / 2 / 3 / 4 splits): bs32 ctx2048 (256 CTAs per split) 45 / 59 / 62 / 66; bs16 ctx4096 (128) 70 / 50 / 65 / 57;
   // bs8 ctx2048 (64), 2 / 4 / 5 / 8 splits: 27 / 23 / 29 / 24
-  int ns = want / ctas;
+  int ns = (int)(want / ctas);
   const int cap = (max_context + 63) / 64;  // >= 64 tokens (one stage) per split
   if (ns > cap) ns = cap;
   if (ns > 32) ns = 32;  // kFaMaxSplits (pie_fa.cu)
@@ -189,7 +185,7 @@ int pie_decode_attn_pick_splits_for(int B, int Hq, int Hkv, int D, int max_conte
   // us, two / four: bs32 ctx2048 38.1 / 26.8, ctx6000 103.5 / 67.9, ctx500 13.1 / 11.8, bs16 ctx1000 14.7 / 11.8, bs8 ctx4000 22.9 / 17.5, ctx1066 9.9 / 8.4, bs5
   // ctx7002 23.0 / 18.2.  Not for a few more (bs4 ctx1300 9 / 10 splits 9.2 / 9.7), nor a first sum of splits below 384 (bs32 ctx256 8.3 / 8.9, ctx384 10.7 / 10.7, ctx450
   // 13.2 / 11.9).
-  const int more = std::min({148 * 4 / (B * Hkv), max_context / 128, 32});   // (kFaMaxSplits)
+  const int more = (int)std::min<long long>({4LL * num_sms() / ((long long)B * Hkv), max_context / 128, 32});   // (kFaMaxSplits)
   return (ns == 1 && max_context < 384) || more < ns + (ns + 3) / 4 ? ns : more;
 }
 

@@ -27,3 +27,12 @@ def test_8_bit_splits_only_where_their_sum_pays(B, ctx, splits):
 def test_heads_of_64_have_more_splits_only_where_that_pays(B, ctx, splits):
     """A first sum of splits, and one split more of nine, measured slower."""
     assert _lib.load().pie_decode_attn_pick_splits_for(B, 32, 8, 64, ctx) == splits
+
+
+@pytest.mark.parametrize("B,Hkv", [(1 << 16, 1 << 16), (1 << 15, 1 << 16), (1 << 30, 8), ((1 << 31) - 1, 2)])
+def test_more_heads_than_32_bits_count(B, Hkv):
+    """(a product of 2^32 was a division by zero)"""
+    L = _lib.load()
+    for D in (64, 128):
+        assert L.pie_decode_attn_pick_splits_for(B, Hkv, Hkv, D, 4096) == 1
+    assert L.pie_decode_attn_q8_pick_splits(B, Hkv, Hkv, 4096) == 1
