@@ -252,19 +252,20 @@ class _NoHost:
 @functools.cache
 def native_fused_rows():
     """csrc/pie_host.cpp's form of nn.fused_rows, which takes the common calls and answers None to the others; where it was not built, or for another torch or
-    interpreter, so that it does not load: None to every call."""
+    interpreter, or for another of these libraries, so that it does not load or bind: None to every call."""
     path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_pie_host.so")
     if not os.path.exists(path):
         return lambda *args: None
+    L = _lib.load()
     try:
         spec = importlib.util.spec_from_file_location("_pie_host", path)
         host = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(host)
-    except (ImportError, OSError) as e:
+        host.bind({name: C.cast(getattr(L, name), C.c_void_p).value for name in host.functions})
+        host.fused_rows, host.mlp_rows, host.attend_rows
+    except (ImportError, OSError, AttributeError, KeyError, TypeError) as e:   # (one of an earlier build has other functions, or another bind)
         warnings.warn(f"{path} does not load ({e}): build it again with make -C {_lib.CSRC}.  Calls of few rows take the Python form meanwhile.")
         return lambda *args: None
-    L = _lib.load()
-    host.bind({name: C.cast(getattr(L, name), C.c_void_p).value for name in host.functions})
     return host.fused_rows
 
 

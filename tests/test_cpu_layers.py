@@ -241,6 +241,29 @@ def test_a_host_module_that_does_not_load_leaves_the_calls_to_python(monkeypatch
         ops.native_fused_rows.cache_clear()
 
 
+def _four_addresses(a, b, c, d):
+    pass
+
+
+@pytest.mark.parametrize("old", [dict(bind=_four_addresses), dict(bind=_four_addresses, functions=["pie_qmt"]), dict(functions=["pie_no_such_call"]),
+                                 dict(functions=[], bind=lambda table: {}["pie_qmt"]), dict(functions=[], bind=lambda table: None, fused_rows=lambda *a: 1)])
+def test_a_host_module_of_another_build_leaves_the_calls_to_python(old, monkeypatch):
+    """It loads, but wants other functions of the library, is bound in another way, or has fewer calls."""
+    from types import SimpleNamespace
+    spec = SimpleNamespace(loader=SimpleNamespace(exec_module=lambda host: None))
+    ops.native_fused_rows.cache_clear()
+    try:
+        with monkeypatch.context() as m:
+            m.setattr(ops.os.path, "exists", lambda path: True)
+            m.setattr(ops.importlib.util, "spec_from_file_location", lambda *a: spec)
+            m.setattr(ops.importlib.util, "module_from_spec", lambda spec: SimpleNamespace(**old))
+            with pytest.warns(UserWarning, match="does not load"):
+                assert ops.native_fused_rows()(1, 2, 3) is None
+            assert ops.native_host().mlp_rows(1, 2) is None and ops.native_host().attend_rows(1, 2) is None
+    finally:
+        ops.native_fused_rows.cache_clear()
+
+
 def test_the_matmuls_route_is_asked_for_at_every_call(monkeypatch):
     """PIE_QMT and the current device may change between two calls: the Python form answers as the library, and so as the native form, does."""
     answers = []
