@@ -116,7 +116,16 @@ def scaled_dot_product_attention(queries, keys, values, cache, scale, mask):
     return ops.scaled_dot_product_attention(queries, keys, values, scale=scale, mask=mask)
 
 
-_ROTATING_CACHES = (KVCache, PagedKVCache, QuantizedKVCache, PagedQuantizedKVCache)   # (not classes made from them, whose update_and_fetch may be another)
+_FETCH = {c: c.update_and_fetch for c in (KVCache, PagedKVCache, QuantizedKVCache, PagedQuantizedKVCache)}
+
+
+def _is(method, function) -> bool:
+    return getattr(method, "__func__", None) is function
+
+
+def _rotates(cache) -> bool:
+    """The cache is one whose update_and_fetch can have the rotation in its launch: not of a class made from these, and with no other put in that method's place."""
+    return type(cache) in _FETCH and _is(cache.update_and_fetch, _FETCH[type(cache)])
 
 
 class Attention(nn.Module):
@@ -147,7 +156,8 @@ class Attention(nn.Module):
     def attend_beside(self, qkv, x, mask, cache):
         """attend() of projections that lie side by side in rows."""
         B, L, _ = x.shape
-        if L == 1 and mask is None and qkv.is_cuda and type(cache) in (KVCache, QuantizedKVCache):   # a step of decoding, in one native call
+        if L == 1 and mask is None and qkv.is_cuda and type(cache) in (KVCache, QuantizedKVCache) and _is(self.attend, _ATTEND) and _rotates(cache):
+            # a step of decoding, in one native call
             out = ops.native_host().attend_rows(self, qkv, cache, KVCache, QuantizedKVCache, Llama3RoPE, ops.attention_workspace)
             if out is not None:
                 return out
@@ -161,7 +171,7 @@ class Attention(nn.Module):
         values = values.reshape(B, L, self.n_kv_heads, -1).transpose(1, 2)
         fetched = None
         if cache is not None:
-            if type(cache) in _ROTATING_CACHES and type(self.rope) is Llama3RoPE and not self.rope.traditional and self.rope.dimensions == queries.shape[-1]:
+            if _rotates(cache) and type(self.rope) is Llama3RoPE and not self.rope.traditional and self.rope.dimensions == queries.shape[-1]:
                 fetched = cache.rotate_and_fetch(queries, keys, values, self.rope._freqs)
             if fetched is None:
                 queries = self.rope(queries, offset=cache.offset)
@@ -173,6 +183,9 @@ class Attention(nn.Module):
             values = values.contiguous()   # in the layout of the rotated keys; a cache would have copied both
         output = scaled_dot_product_attention(queries, keys, values, cache=cache, scale=self.scale, mask=mask)
         return output.transpose(1, 2).reshape(B, L, -1)
+
+
+_ATTEND = Attention.attend
 
 
 class MLP(nn.Module):

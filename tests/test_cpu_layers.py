@@ -225,6 +225,33 @@ def test_a_prompt_layer_norms_its_input_once(monkeypatch, odd):
     assert calls == ["norm"] + ([3] if odd is None else ["linear"] * 3) + [1, "norm", "linear", "linear", 1]
 
 
+class _Rows:
+    """Projected rows as a GPU has them."""
+    is_cuda = True
+
+    def __getitem__(self, at):
+        return self
+
+
+@pytest.mark.parametrize("where", ["nowhere", "object", "class", "cache", "cache's class"])
+def test_a_decode_step_calls_what_is_put_in_a_methods_place(where, monkeypatch):
+    """... on one attention object or cache, or on its class: the native call is for the methods that it stands for."""
+    from types import SimpleNamespace
+    from proxy_inference_engine_b200 import llama
+    from proxy_inference_engine_b200.cache import KVCache
+    monkeypatch.setattr(ops, "native_host", lambda: SimpleNamespace(attend_rows=lambda *a: "native"))
+    at, cache = object.__new__(llama.Attention), KVCache()
+    at.q_proj, at.k_proj, at.v_proj = _plain(512), _plain(256), _plain(256)
+    theirs = lambda *a: "theirs"
+    if where != "nowhere":
+        monkeypatch.setattr(*{"object": (at, "attend"), "class": (llama.Attention, "attend"), "cache": (cache, "update_and_fetch"),
+                              "cache's class": (KVCache, "update_and_fetch")}[where], theirs, raising=False)
+    if where.startswith("cache"):
+        assert not llama._rotates(cache)
+        monkeypatch.setattr(at, "attend", theirs, raising=False)
+    assert at.attend_beside(_Rows(), torch.zeros((2, 1, 512)), None, cache) == ("native" if where == "nowhere" else "theirs")
+
+
 def test_a_host_module_that_does_not_load_leaves_the_calls_to_python(monkeypatch):
     """... as one that was built for another torch or interpreter does: a warning, once, and no answer to any call."""
     def refuse(*args):
