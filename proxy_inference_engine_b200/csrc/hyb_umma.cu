@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_grouped_kernel(const __gri
   __shared__ __align__(8) uint64_t full_bar[S], empty_bar[S], accum_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
-  pdl_sync();
+  pie::pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smA = base, smB = base + S * A_STAGE;
@@ -294,6 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_grouped_kernel(const __gri
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
+  pie::pdl_launch_dependents();   // behind the allocation of tensor memory: a dependent that holds all of an SM's while it waits would keep this CTA from its own
 
   if (warp < kProducers / 32) {
     const int t = tid;
