@@ -33,8 +33,9 @@ unsigned long long pieh_launch_count(void);
 unsigned int pieh_pipeline_error(void);
 int pieh_pipeline_error_clear(void);
 int pieh_pipeline_words(unsigned int* words, void* stream);
-/* on: every operator is launched as a programmatic dependent of the launch before it on its stream (its blocks may become
- * resident early and wait at their top); captured into CUDA graphs as such.  Off by default. */
+/* on > 0: every operator is launched as a programmatic dependent of the launch before it on its stream (its blocks may become
+ * resident early and wait at their top); captured into CUDA graphs as such.  0: none is.  < 0, and until it is called: the tensor-core
+ * matmuls of dense weights alone are. */
 void pieh_set_pdl(int on);
 
 /* epilogues of pieh_linear */

@@ -11,8 +11,8 @@ namespace pieh {
 
 static std::atomic<unsigned long long> g_launches{0};
 static thread_local char g_err[256] = "";
-static std::atomic<int> g_pdl{0};
-bool pdl_enabled() { return g_pdl.load(std::memory_order_relaxed) != 0; }
+static std::atomic<int> g_pdl{-1};   // -1: not asked for either way
+bool pdl_enabled() { return g_pdl.load(std::memory_order_relaxed) > 0; }
 void count_launch(int n) { g_launches.fetch_add((unsigned long long)n, std::memory_order_relaxed); }
 int status_of(cudaError_t e) {
   if (e == cudaSuccess) return PIE_OK;
@@ -135,13 +135,16 @@ __global__ void stream_update_kernel(float* xs, const float* y, const float* mix
 }
 
 }  // namespace pieh
+namespace pie {
+__attribute__((visibility("hidden"))) bool gemm_programmatic() { return pieh::g_pdl.load(std::memory_order_relaxed) != 0; }
+}  // namespace pie
 
 using namespace pieh;
 
 extern "C" int pieh_abi_version(void) { return 1; }
 extern "C" const char* pieh_last_cuda_error(void) { return g_err; }
 extern "C" unsigned long long pieh_launch_count(void) { return g_launches.load(); }
-extern "C" void pieh_set_pdl(int on) { g_pdl.store(on ? 1 : 0); }
+extern "C" void pieh_set_pdl(int on) { g_pdl.store(on < 0 ? -1 : on ? 1 : 0); }
 
 extern "C" int pieh_embed_streams(float* xs, const void* table, int table_dtype, const int32_t* tokens, int T, int S, int W,
                                   int vocab, void* stream) {

@@ -18,6 +18,7 @@ bool pdl_aux_enabled() {
   static const bool on = [] { const char* e = getenv("PIE_PDL_AUX"); return !(e && e[0] == '0'); }();
   return on;
 }
+__attribute__((visibility("hidden"))) bool gemm_programmatic() { return pdl_aux_enabled(); }
 
 static int cuda_status(cudaError_t e) {
   if (e == cudaSuccess) return PIE_OK;

@@ -30,6 +30,8 @@
 
 namespace pie {
 
+__attribute__((visibility("hidden"))) bool gemm_programmatic();   // each library's own: whether its switch for programmatic launches (PIE_PDL_AUX, pieh_set_pdl) leaves them on
+
 static __device__ unsigned int g_gemm_error = 0;   // 1: a pipeline wait of a kernel of this source file expired
 // the word on the host: now (waits for the device), behind what is queued on a stream, and set back
 static inline unsigned int gemm_error_now() {
@@ -648,8 +650,9 @@ cudaError_t gemm_launch(const CUtensorMap& mx, const CUtensorMap& mw, const Gemm
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = SPLIT ? (unsigned)ranks : (unsigned)CG;
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = CG == 2 || SPLIT ? 2 : 1;
+  const bool pdl = gemm_programmatic(), cluster = CG == 2 || SPLIT;
+  cfg.attrs = pdl ? attr : attr + 1;
+  cfg.numAttrs = (pdl ? 1 : 0) + (cluster ? 1 : 0);
   return cudaLaunchKernelEx(&cfg, kern, mx, mw, a, epi);
 }
 

@@ -575,7 +575,7 @@ cudaError_t launch_qmi(void* out, int out_ld, const void* x, int x_ld, int M, in
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pdl_aux_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 

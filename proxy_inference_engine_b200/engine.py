@@ -85,7 +85,7 @@ class _DecodeGraph:
             finally:
                 gc.enable()
                 if pdl:
-                    pdl(0)
+                    pdl(-1)
             self.graph = g
             self._rewind(seqs)
         self.graph.replay()
