@@ -190,17 +190,29 @@ def test_a_layer_on_a_stream_of_its_own_and_in_a_capture():
 
 @pytest.mark.parametrize("bits", [4, 8])
 @pytest.mark.parametrize("rows", [1, 4, 9, 40, 200])
-def test_weights_written_by_the_launch_before(bits, rows):
-    """Launches set themselves up, and ask L2 for weights, under the end of the launch before them: what that one writes into the weights is what they multiply by."""
-    g, mlp, other = torch.Generator(device="cuda").manual_seed(rows), _block(bits, 64).mlp, _block(bits, 64, seed=1).mlp
+@pytest.mark.parametrize("written", ["gate_proj", "up_proj", "down_proj"])
+def test_weights_written_by_the_launch_before(bits, rows, written):
+    """Launches set themselves up, and ask L2 for weights, under the end of the launch before them: what that one writes into the weights is what they multiply by.
+    It is a norm of one long row, a single block that lets its dependents start at its top and writes a matrix's scales last of all."""
+    from proxy_inference_engine_b200 import _lib
+    L = _lib.load()
+    g, mlp = torch.Generator(device="cuda").manual_seed(rows), _block(bits, 64).mlp
     x = torch.randn((rows, 512), generator=g, device="cuda").bfloat16()
-    names = [(l, n) for l in ("gate_proj", "up_proj", "down_proj") for n in ("weight", "scales", "biases")]
-    both = [[getattr(getattr(m, l), n).clone() for l, n in names] for m in (mlp, other)]
-    want = [mlp(x), other(x)]
+    lin, long = getattr(mlp, written), 1 << 18
+    out, ones, n = torch.ones(long, device="cuda").bfloat16(), torch.ones(long, device="cuda").bfloat16(), lin.scales.numel()
+    sets = []                                                    # a norm of ones is its weight
+    for i in range(2):
+        sets.append(ones.clone())
+        sets[i][long - n:] = lin.scales.flatten() * (1 + 2 * i)
+    lin.scales = out[long - n:].view(lin.scales.shape)
+    want = []
+    for w in sets:
+        out.copy_(w)
+        torch.cuda.synchronize()
+        want.append(mlp(x))
     assert not torch.equal(*want)
     got = []
-    for i in range(60):
-        for (l, n), t in zip(names, both[i % 2]):
-            getattr(getattr(mlp, l), n).copy_(t)
+    for i in range(20):
+        assert L.pie_rms_norm(out.data_ptr(), ones.data_ptr(), sets[i % 2].data_ptr(), 1, long, 0.0, torch.cuda.current_stream().cuda_stream) == 0
         got.append(mlp(x))
-    assert all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))
+    assert torch.equal(out, sets[1]) and all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))
