@@ -10,8 +10,8 @@
 // same ~1000 cycles of an SM, so the kernel is built to keep both going at once:
 //   * warps 0-3 / 4-7: the softmax of query tile 0 / 1, a thread per row.  S comes out of tensor memory (128 columns), is
 //     masked on the diagonal, the running maximum moves only when exceeded by 8 (log2 units; the same sums, and O is rescaled
-//     rarely), p = exp2(scale s - m), seven eighths of them (D = 64: three quarters) by the approximation unit (16 a cycle of an SM: at
-//     D = 64 that alone would take twice the MMAs' time) and the rest by a polynomial on the multiply-add pipe, is rounded to bf16 and put back over
+//     rarely), p = exp2(scale s - m), three quarters of them by the approximation unit (16 a cycle of an SM: at D = 64 that alone
+//     would take twice the MMAs' time) and the rest by a polynomial on the multiply-add pipe, is rounded to bf16 and put back over
 //     S as the A operand of the second product.  Row sums are of the unrounded p, in fp32.
 //   * warp 8: TMA.  Q once; K and V tiles of the contiguous or paged cache into two-deep rings (128-byte swizzle).
 //   * warp 9: MMAs.  S_g = Q_g K^T (both operands in shared memory), O_g += P_g V (P in tensor memory, V as it lies:
@@ -20,8 +20,9 @@
 // Tensor memory: S/P 2 x 128 columns, O 2 x D.
 // A CTA per SM walks its share of the 256-row items, longest first (causal: tile i sees i + 1 key tiles).  An item's first scores are issued behind the
 // last product of the one before it, query tile by query tile, while that one's other tile and its results are still worked on; nothing is set up
-// twice.  (One CTA an item, 5.2 of them an SM at 2 x 3000 tokens: 156.8 us; this 146.4, and 144.7 with an eighth of the exponentials off the
-// approximation unit in place of a quarter, 150 with three eighths, 160 with half; 8192 tokens 468 -> 448.)
+// twice.  (One CTA an item, 5.2 of them an SM at 2 x 3000 tokens: 156.8 us; this 146.4; 8192 tokens 464 -> 447; D 64, 2 x 3000 127.5 -> 123.9, but
+// 1500 tokens 23.3 -> 23.9 and 6001 219.9 -> 222.3.  With three eighths of the exponentials off the approximation unit 150, with half 160.  An eighth at D 128 is
+// 144.7, but the unit is off by 2.4e-7 and the polynomial by 2.0e-7.)
 // Every wait is bounded (pie_gemm.cuh).
 // Measured, 32 query / 8 kv heads, us (TFLOP/s): the mma.sync kernel of pie_fa.cu -> this one with a lane of its own issuing the MMAs
 // and all exponentials on the approximation unit -> as it is.  D 128: 8192 tokens 2190 (251) -> 547 (1005) -> 460 (1196); 2 x 3000
@@ -149,7 +150,6 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   constexpr uint32_t ID_S = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
   constexpr uint32_t ID_O = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(D >> 3) << 17) | ((128u >> 4) << 24);
   constexpr int COL_S = 0, COL_O = 256;   // + g * 128, + g * D
-  constexpr int POLY = D == 128 ? 8 : 4;  // of so many pairs of exponentials one takes the polynomial
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t q_full[2], q_empty[2], k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], o_full[2];
   __shared__ uint32_t tmem_slot;
@@ -249,7 +249,7 @@ fa_prefill_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           for (int i = 0; i < 32; ++i) {
             const f32x2 x = f2_fma(f2_pack(s[64 * hf + 2 * i], s[64 * hf + 2 * i + 1]), sc2, ms2);
             float e0, e1;
-            if (i % POLY == POLY - 1) {        // off the approximation unit, which would otherwise bound the tile
+            if (i % 4 == 3) {        // every fourth pair off the approximation unit, which would otherwise bound the tile
               fap_exp2_poly(x, e0, e1);
             } else {
               float x0, x1;
