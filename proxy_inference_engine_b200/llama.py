@@ -119,13 +119,10 @@ def scaled_dot_product_attention(queries, keys, values, cache, scale, mask):
 _FETCH = {c: c.update_and_fetch for c in (KVCache, PagedKVCache, QuantizedKVCache, PagedQuantizedKVCache)}
 
 
-def _is(method, function) -> bool:
-    return getattr(method, "__func__", None) is function
-
-
 def _rotates(cache) -> bool:
     """The cache is one whose update_and_fetch can have the rotation in its launch: not of a class made from these, and with no other put in that method's place."""
-    return type(cache) in _FETCH and _is(cache.update_and_fetch, _FETCH[type(cache)])
+    kind = type(cache)
+    return kind in _FETCH and kind.update_and_fetch is _FETCH[kind] and "update_and_fetch" not in cache.__dict__
 
 
 class Attention(nn.Module):
@@ -156,7 +153,8 @@ class Attention(nn.Module):
     def attend_beside(self, qkv, x, mask, cache):
         """attend() of projections that lie side by side in rows."""
         B, L, _ = x.shape
-        if L == 1 and mask is None and qkv.is_cuda and type(cache) in (KVCache, QuantizedKVCache) and _is(self.attend, _ATTEND) and _rotates(cache):
+        if L == 1 and mask is None and qkv.is_cuda and type(cache) in (KVCache, QuantizedKVCache) and _rotates(cache) \
+                and type(self).attend is _ATTEND and "attend" not in self.__dict__:
             # a step of decoding, in one native call
             out = ops.native_host().attend_rows(self, qkv, cache, KVCache, QuantizedKVCache, Llama3RoPE, ops.attention_workspace)
             if out is not None:

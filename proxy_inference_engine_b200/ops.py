@@ -76,9 +76,20 @@ def _check_gs_bits(what, group_size, bits, full=False):
                          "(supported: group_size 64, bits 4 or 8)")
 
 
+_raw_stream = torch._C._cuda_getCurrentRawStream
+_capturing = torch.cuda.is_current_stream_capturing
+
+
 def _capture_id() -> int:
-    """Which capture into a graph the current stream is in; 0: none."""
-    return _lib.load().pie_capture_id(_stream()) if torch.cuda.is_current_stream_capturing() else 0
+    """Which capture into a graph the current stream is in."""
+    return _lib.load().pie_capture_id(_stream())
+
+
+class _Mine(threading.local):
+    """A thread's workspaces: {(key, device, stream): buffer}, and those of the capture it is in."""
+
+    def __init__(self):
+        self.eager, self.captured, self.capture = {}, {}, 0
 
 
 class _Workspaces:
@@ -91,14 +102,20 @@ class _Workspaces:
     KEEP = 96   # (a decode step's attention has one per 64 rows x query heads)
 
     def __init__(self):
-        self.mine = threading.local()
+        self.mine = _Mine()
 
     def get(self, key, nbytes, device):
-        mine, capture = self.mine.__dict__, _capture_id()
-        if mine.get("capture") != capture:
-            mine["capture"], mine["captured"] = capture, {}
-        bufs = mine["captured"] if capture else mine.setdefault("eager", {})
-        key = (key, device, _stream())
+        mine, index = self.mine, device.index
+        stream = _raw_stream(index)
+        bufs = mine.eager
+        if stream and _capturing():   # (asking costs what the rest of this does, and the default stream cannot be captured)
+            capture = _capture_id()
+            if capture != mine.capture:
+                mine.capture, mine.captured = capture, {}
+            bufs = mine.captured
+        elif mine.captured:           # that capture has ended, or this is another stream
+            mine.capture, mine.captured = 0, {}
+        key = (key, index, stream)
         buf = bufs.get(key)
         if buf is None or buf.numel() < nbytes:
             bufs.pop(key, None)

@@ -13,8 +13,9 @@ CPU = torch.device("cpu")
 def at(monkeypatch):
     """The stream and the capture that a call finds itself on."""
     now = threading.local()
-    monkeypatch.setattr(ops, "_stream", lambda: getattr(now, "stream", 0))
-    monkeypatch.setattr(ops, "_capture_id", lambda: getattr(now, "capture", 0), raising=False)
+    monkeypatch.setattr(ops, "_raw_stream", lambda index: getattr(now, "stream", 0))
+    monkeypatch.setattr(ops, "_capturing", lambda: getattr(now, "capture", 0) != 0)
+    monkeypatch.setattr(ops, "_capture_id", lambda: getattr(now, "capture", 0))
 
     def move(stream=0, capture=0):
         now.stream, now.capture = stream, capture
@@ -45,13 +46,13 @@ def test_a_capture_has_its_own(at):
     """An eager call never sees a buffer whose zeros are only recorded, and a graph never one that a larger eager call replaces."""
     w = ops._Workspaces()
     eager = w.get("attn", 1000, CPU)
-    at(capture=7)
+    at(stream=3, capture=7)
     captured = w.get("attn", 1000, CPU)
     new = w.get("first in a capture", 1000, CPU)
     assert captured is not eager and w.get("attn", 1000, CPU) is captured
     at()
     assert w.get("attn", 1000, CPU) is eager and w.get("first in a capture", 1000, CPU) is not new
-    at(capture=8)
+    at(stream=3, capture=8)
     assert w.get("attn", 1000, CPU) is not captured
 
 

@@ -54,14 +54,14 @@ def test_a_graph_beside_eager_calls():
     from proxy_inference_engine_b200 import ops
     f, larger = _case(3), _case(4)
     f()                                         # (kernels opt in to their shared memory ahead of the capture)
-    ops.workspaces.mine.__dict__.clear()
+    ops.workspaces.mine.eager.clear()
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         out = f()
         again = f()
     want = f()
     for key in list(ops.workspaces.mine.eager):
-        ops.workspaces.get(key[0], 1 << 24, key[1])
+        ops.workspaces.get(key[0], 1 << 24, torch.device("cuda", key[1]))
     other = larger()
     for _ in range(3):
         out.zero_()
