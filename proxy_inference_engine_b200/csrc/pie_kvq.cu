@@ -421,6 +421,8 @@ __global__ void __launch_bounds__(128, 2) decode_attn_q8_kernel(const DecAttnQAr
 // fragment of K comes from one 32-bit word.  The value product is transposed (V as the A operand, features x keys; p * sv
 // as B, keys x heads -- the score accumulators ARE that B fragment): every accumulator row is live, and rows g, g + 8 of
 // value tile (G, q) are features 64 G + 8 g + 2 q + {0, 1}, so a thread's bytes of a V row are one 64-bit word.
+// SPLIT: the context is cut over blockIdx.x and partial results are added up.  One split has a kernel without that: with the sum's instructions in it the
+// compiler gives the loop over stages 148 registers for 142 and orders it worse (bs32 ctx2048 33.4 us / 32.3, ctx1000 18.9 / 18.25, bs64 ctx700 27.5 / 25.8).
 constexpr int kQtKeys = 64, kQtStages = 4, kQtAhead = 2, kQtThreads = 128, kQtStageBytes = 2 * kQtKeys * 128 + kQtKeys * 16;
 
 __device__ __forceinline__ void mma_f16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -436,6 +438,7 @@ __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
 __device__ __forceinline__ float f16lo(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)(v & 0xffffu))); }
 __device__ __forceinline__ float f16hi(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)(v >> 16))); }
 
+template <bool SPLIT>
 __global__ void __launch_bounds__(kQtThreads) decode_attn_q8_tc_kernel(const __grid_constant__ DecAttnQArgs a) {
   constexpr int D = 128, PW = D + 2, NS = kQtStages;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -443,10 +446,10 @@ __global__ void __launch_bounds__(kQtThreads) decode_attn_q8_tc_kernel(const __g
   pdl_launch_dependents();
   pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, j = lane & 3;
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int split = SPLIT ? blockIdx.x : 0, kvh = blockIdx.y, b = blockIdx.z;
   const int n_rep = a.Hq / a.c.Hkv, qh0 = kvh * n_rep;
   const int p = a.pos[b], ctx = p + 1;
-  const int tiles = (ctx + kQtKeys - 1) / kQtKeys, per = (tiles + a.nsplit - 1) / a.nsplit;
+  const int tiles = (ctx + kQtKeys - 1) / kQtKeys, per = SPLIT ? (tiles + a.nsplit - 1) / a.nsplit : tiles;
   const int j0 = split * per, j1 = min(tiles, j0 + per);
   const uint32_t s0 = smem_u32(smem);
 
@@ -663,7 +666,7 @@ __global__ void __launch_bounds__(kQtThreads) decode_attn_q8_tc_kernel(const __g
       lt += rw[D + 1] * cw;
       at += rw[d] * cw;
     }
-    if (a.nsplit == 1) {
+    if (!SPLIT) {
       a.out[((size_t)b * a.Hq + qh0 + r) * D + d] = f2bf(at / lt);
     } else {
       float* pr = a.ws_part + (rec0 + (size_t)r * a.nsplit + split) * PW;
@@ -671,7 +674,7 @@ __global__ void __launch_bounds__(kQtThreads) decode_attn_q8_tc_kernel(const __g
       if (d == 0) { pr[D] = mn; pr[D + 1] = lt; }
     }
   }
-  if (a.nsplit == 1) return;
+  if (!SPLIT) return;
   if (last_to_arrive(&a.ws_cnt[b * a.c.Hkv + kvh], a.nsplit, &s_last))
     merge_splits<D>(a.out + ((size_t)b * a.Hq + qh0) * D, a.ws_part + rec0 * PW, n_rep, a.nsplit);
 }
@@ -692,12 +695,13 @@ static cudaError_t launch_decode_attn_q8_tc(const DecAttnQArgs& a, int B, cudaSt
       if (want > smem) smem = want & ~(size_t)127;
     }
   }
+  const auto kernel = a.nsplit > 1 ? decode_attn_q8_tc_kernel<true> : decode_attn_q8_tc_kernel<false>;
   {  // per launch, not once per process: the attribute is per device
-    cudaError_t e = cudaFuncSetAttribute(decode_attn_q8_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
   count_launch();
-  return launch_pdl(decode_attn_q8_tc_kernel, dim3(a.nsplit, a.c.Hkv, B), dim3(kQtThreads), smem, st, a);
+  return launch_pdl(kernel, dim3(a.nsplit, a.c.Hkv, B), dim3(kQtThreads), smem, st, a);
 }
 
 template <int D>
