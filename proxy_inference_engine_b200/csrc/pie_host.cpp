@@ -185,18 +185,11 @@ PyObject* fused_rows(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// mlp_rows(x, gate, up, down, QuantizedLinear, RMSNorm, workspace) -> down(silu(gate(x)) * up(x)), or the activations alone in a tuple, or None; False: more
-// than 32 rows that the library does not take as few, as nn.fused_rows would find
+// mlp_rows(x, gate, up, down, QuantizedLinear, RMSNorm, workspace) -> down(silu(gate(x)) * up(x)), or the activations alone in a tuple, or None
 PyObject* mlp_rows(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   const at::Tensor* x = n == 7 && bound ? tensor_of(args[0]) : nullptr;
   if (!x || !x->is_cuda()) Py_RETURN_NONE;
-  if (const int64_t K = x->dim() ? x->size(-1) : 0, M = K > 0 ? x->numel() / K : 0; M > 32 && M <= 128 && K <= INT32_MAX) {
-    long bits = 0;
-    const at::Tensor* w = (PyObject*)Py_TYPE(args[1]) == args[4] ? tensor_of(entry(args[1], s_weight)) : nullptr;
-    if (!w || w->dim() != 2 || !int_of(entry(args[1], s_bits), bits)) Py_RETURN_NONE;
-    if (!lib.pie_qmt_scratch_bytes((int)M, w->size(0), (int)K, 64, (int)bits, 1)) Py_RETURN_FALSE;
-  }
   const Kit kit = {args[4], args[5], args[6]};
   THPObjectPtr device(PyObject_GetAttr(args[0], s_device));
   if (!device) return nullptr;

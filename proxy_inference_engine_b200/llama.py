@@ -196,15 +196,12 @@ class MLP(nn.Module):
 
     def __call__(self, x):
         act = y = None
-        few = x.numel() <= 128 * x.shape[-1]
-        if few and x.is_cuda:                # both launches in one native call
+        if x.is_cuda and x.numel() <= 128 * x.shape[-1]:   # few rows: both launches in one native call
             y = ops.native_host().mlp_rows(x, self.gate_proj, self.up_proj, self.down_proj, nn.QuantizedLinear, nn.RMSNorm, ops.qmv_workspace)
-            if type(y) is tuple:             # as far as it came
+            if type(y) is tuple:                           # as far as it came
                 (act,), y = y, None
-            elif y is False:
-                few, y = False, None
         if y is None:
-            if few and act is None:
+            if act is None:
                 act = nn.fused_rows(x, (self.gate_proj, self.up_proj), swiglu=True)
             if act is not None:
                 y = nn.fused_rows(act, (self.down_proj,))

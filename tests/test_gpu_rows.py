@@ -157,17 +157,6 @@ def test_a_feed_forward_of_few_rows_is_the_python_forms(bits, rows, monkeypatch)
     assert all(torch.equal(y, want) for y in outs)
 
 
-@pytest.mark.parametrize("rows,false", [(1, False), (32, False), (33, True), (128, True)])
-def test_rows_that_do_not_go_with_the_few_are_said_to(rows, false):
-    """512 x 1024 is little work: more than 32 rows are the separate launches', and the feed-forward does not ask for the few's again."""
-    from proxy_inference_engine_b200 import nn, ops
-    mlp, x = _block(4, 64).mlp, torch.ones((rows, 512), device="cuda").bfloat16()
-    got = ops.native_host().mlp_rows(x, mlp.gate_proj, mlp.up_proj, mlp.down_proj, nn.QuantizedLinear, nn.RMSNorm, ops.qmv_workspace)
-    assert (got is False) == false
-    if false:
-        assert nn.fused_rows(x, (mlp.gate_proj, mlp.up_proj), swiglu=True) is None
-
-
 def test_a_layer_on_a_stream_of_its_own_and_in_a_capture():
     from proxy_inference_engine_b200.cache import KVCache
     g, block = torch.Generator(device="cuda").manual_seed(6), _block(4, 128)
